@@ -35,6 +35,7 @@ using namespace dp32;
 }  // namespace sa
 
 #include "sa_fp32_kernel.cuh"
+#include "sa_fp32_columns.cuh"
 
 namespace sa {
 namespace fp32 {
@@ -58,6 +59,7 @@ __global__ void __launch_bounds__(256) fma_probe(float *sink, int iters, float s
 // Slack after the emission and forward stores: the kernels' clamped look-ahead loads past a
 // region's last anti-diagonal stay inside the allocation.
 constexpr size_t kStoreSlack = 1024;
+static_assert(2 * (kStoreFront + kStoreBack) <= kStoreSlack, "the emission store's slack holds both ends");
 
 // device memory bound of a batch's plain-form reads
 constexpr size_t kPlainBatchMaxBytes = (size_t) 64 << 30;
@@ -137,6 +139,7 @@ struct sa_batch {
     int64_t n_segs = 0, n_stitch = 0, stitch_floats = 0;
     int64_t cells = 0, out_total = 0;
     int32_t max_width = 0;
+    int32_t max_span = 0;         // columns that three consecutive anti-diagonals span at most
     float threshold = 0.01f;
     // inputs, staged on the host with the device layout (one copy uploads them all)
     Span<RegionDesc> regions;
@@ -374,13 +377,25 @@ struct ReadPlan {
     std::vector<std::vector<int32_t>> cuts;   // per region: windows that start a forward segment
     int64_t diags = 0, cells = 0, windows = 0, chunks = 0, out = 0;
     int64_t segs = 0, stitches = 0, stitch_floats = 0;
-    int32_t max_width = 0;
+    int32_t max_width = 0, max_span = 0;
     // packing offsets
     int64_t region_base = 0, diag_base = 0, cell_base = 0, win_base = 0, chunk_base = 0, kmer_base = 0,
             event_base = 0, out_base = 0, seg_base = 0, stitch_base = 0, stitch_voff = 0;
 };
 
 int32_t band_width(const Region &rg, int64_t d) { return (rg.xmy_r[d] - rg.xmy_l[d]) / 2 + 1; }
+
+// columns from the first of any three consecutive anti-diagonals to the last of them, at most
+int32_t column_extent(const Region &rg) {
+    const int64_t n = (int64_t) rg.xmy_l.size();
+    int32_t lo[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, hi[3] = {-1, -1, -1}, span = 0;
+    for (int64_t d = 0; d < n; ++d) {
+        lo[d % 3] = (int32_t) ((d + rg.xmy_l[d]) >> 1);
+        hi[d % 3] = (int32_t) ((d + rg.xmy_r[d]) >> 1);
+        span = std::max(span, std::max({hi[0], hi[1], hi[2]}) - std::min({lo[0], lo[1], lo[2]}) + 1);
+    }
+    return span;
+}
 
 // Host planning of a batch (no device work): per read its regions and their windows (in parallel
 // over reads), then the packed inputs, written straight into a host staging block (pinned when
@@ -463,6 +478,7 @@ sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, 
             rp.chunks += (n + kChunkDiags) / kChunkDiags;
             for (const Window &w : rg.windows) rp.out += 4 * (int64_t) (w.from - w.T) + 64;
             rp.max_width = std::max(rp.max_width, rg.max_width);
+            rp.max_span = std::max(rp.max_span, column_extent(rg));
         }
     });
     // forward segments: the cap from the policy and the batch's forward anti-diagonals per worker CTA
@@ -521,6 +537,7 @@ sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, 
             nevent += reads[r].n_events;
         }
         b->max_width = std::max(b->max_width, rp.max_width);
+        b->max_span = std::max(b->max_span, rp.max_span);
     }
     b->plain_of.assign(n_reads, -1);
     for (int64_t r = 0; r < n_reads; ++r)
@@ -709,7 +726,8 @@ Args batch_args(const sa_batch *b) {
     a.kmer = b->d_kmer;
     a.gapx = b->d_gapx;
     a.events = b->d_events;
-    a.E = b->d_E;
+    a.n_cells = b->cells;
+    a.E = reinterpret_cast<float2 *>(b->d_E) + kStoreFront;
     a.F = b->d_F;
     a.base = b->d_base;
     a.fshift = b->d_fshift;
@@ -730,16 +748,16 @@ Args batch_args(const sa_batch *b) {
     a.done_seq = b->run_seq;
     const int cpt = std::max(1, (b->max_width + kThreads - 1) / kThreads);
     a.wmax = (cpt <= 1 ? 1 : (cpt <= 2 ? 2 : 4)) * kThreads;
-    a.warp_windows = 1;
     a.spin_limit = b->wait_limit;
     return a;
 }
 
-// the persistent worker over a.n_segs forward segments and a.n_windows windows
-void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
-    const int cls = a.wmax / kThreads;
-    const size_t smem = sizeof(Shared) + sizeof(float) * (size_t) worker_area_floats(cls);
-    auto launch = [&](auto kern) {
+// The persistent worker over a.n_segs forward segments and a.n_windows windows.  Column-resident warps
+// take every batch whose bands fit their slots (bands up to about 124 or 248 columns), unless the
+// launch configuration asks for a window per CTA; the CTA form takes the rest.
+void launch_worker(const sa_batch *b, Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
+    a.sms = sms;
+    auto launch = [&](auto kern, size_t smem) {
         int per_sm = 0;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
@@ -748,10 +766,13 @@ void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg
                                                                     (int64_t) cfg.grid_per_region * a.n_segs));
         kern<<<(unsigned) grid, kThreads, smem, s>>>(a);
     };
-    if (cls == 1 && cfg.ctas_per_sm >= 3) launch(worker_kernel<1, 3>);
-    else if (cls == 1) launch(worker_kernel<1, 2>);
-    else if (cls == 2) launch(worker_kernel<2, 1>);
-    else launch(worker_kernel<4, 1>);
+    if (cfg.warp_windows && b->max_span <= column_span(4))
+        return launch(column_worker<4, 3>, sizeof(ColumnShared) + kWarps * sizeof(WindowShared<4>));
+    const int cls = a.wmax / kThreads;
+    const size_t smem = sizeof(Shared) + sizeof(float) * (size_t) worker_area_floats(cls);
+    if (cls == 1) launch(worker_kernel<1, 2>, smem);
+    else if (cls == 2) launch(worker_kernel<2, 1>, smem);
+    else launch(worker_kernel<4, 1>, smem);
 }
 
 // Reads whose stitch disagreed run again with every region as one segment (after the batch's
@@ -794,7 +815,6 @@ sa_status redo_disagreed(sa_batch *b, cudaStream_t s) {
     a.use_side = 0;          // T of every window comes from the unsegmented sweep's store
     a.done_host = nullptr;   // every read is gathered below
     const sa_launch_config cfg = b->has_cfg ? b->cfg : launch_for(b->device, a.wmax / kThreads);
-    a.warp_windows = cfg.warp_windows;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     sms = std::max(1, sms);
@@ -919,7 +939,6 @@ sa_status sa_batch_run(sa_batch *b, void *stream) {
         const int cpt_pow2 = cpt <= 1 ? 1 : (cpt <= 2 ? 2 : 4);
         b->width_class = cpt_pow2;
         const sa_launch_config cfg = b->has_cfg ? b->cfg : launch_for(b->device, cpt_pow2);
-        a.warp_windows = cfg.warp_windows;
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
         sms = std::max(1, sms);

@@ -3,7 +3,8 @@
 //   1. emission_kernel: the match and extra-event emissions of every band cell, written to the
 //      emission store.  Fully parallel (a warp per run of 32 anti-diagonals); it takes the
 //      Gaussian / HDP density work off the sequential sweeps.
-//   2. worker_kernel: persistent CTAs of 128 threads pull tasks from one device counter.  The first
+//   2. column_worker (sa_fp32_columns.cuh; bands up to about 124 columns) or worker_kernel (wider
+//      bands): persistent CTAs of 128 threads pull tasks from one device counter.  The first
 //      claims are forward segments (longest first); every later claim is a slot of a ready queue of
 //      traceback windows.  A forward segment sweeps a run of a region's anti-diagonals (the whole
 //      region, or a piece of a long one; see Segment) anti-diagonal by anti-diagonal (cells spread
@@ -39,7 +40,7 @@
 // they describe the stored values exactly.
 //
 // Stores, per anti-diagonal d with first cell c (region relative) and width W:
-//   emission store at 2c: [ match emission | extra-event emission ], W floats each;
+//   emission store at c: (match emission, extra-event emission) of each cell;
 //   forward store at 3c:  [ match | gap-X | gap-Y ], W floats each; the gap states only where a
 //   refresh reads them.
 #pragma once
@@ -54,7 +55,10 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCpt = 4;                     // cells per thread: bands up to 512 cells wide
 constexpr int kChunkDiags = 32;                // anti-diagonals per emission-kernel chunk
 enum { ST_M = 0, ST_X = 1, ST_Y = 2 };         // forward store blocks
-enum { SE_M = 0, SE_Y = 1 };                   // emission store blocks
+
+// Cells before and after the emission store that look-ahead loads may read (never a band cell's own
+// operand): zeroed by the emission kernel, so that what reaches the arithmetic is a number.
+constexpr int kStoreFront = 16, kStoreBack = 480;
 
 // per-anti-diagonal meta: x = xmy of the first cell, y = width | flags
 constexpr int32_t kWidthMask = (1 << 20) - 1;
@@ -168,15 +172,9 @@ struct Control {
     unsigned long long packed;   // pairs in the packed output
 };
 
-// per-warp window area (floats) when windows run one per warp: ring, refresh chain (2 rows) and
-// the staged operands of the next refresh (6 rows)
-constexpr int kWarpWindowCpt = 4;
-constexpr int kWarpWindowWidth = 32 * kWarpWindowCpt;
-constexpr int kWarpWindowFloats = 9 * (kWarpWindowWidth + 2) + 8 * kWarpWindowWidth;
-
-// dynamic shared memory of the worker after the Shared header, in floats
+// dynamic shared memory of the CTA worker after the Shared header, in floats
 __host__ __device__ constexpr int worker_area_floats(int cpt) {
-    return cpt == 1 ? kWarps * kWarpWindowFloats : 9 * (cpt * kThreads + 2) + 2 * cpt * kThreads;
+    return 9 * (cpt * kThreads + 2) + 2 * cpt * kThreads;
 }
 
 struct Args {
@@ -204,7 +202,8 @@ struct Args {
     const int32_t *kmer;
     const float *gapx;              // per k-mer position: skip emission of that k-mer
     const Event32 *events;
-    float *E;                       // emission store, 2 floats per cell
+    int64_t n_cells;
+    float2 *E;                      // emission store, (match, extra event) per cell
     float *F;                       // forward store, 3 floats per cell
     double *base;                   // per anti-diagonal FP64 base of the forward store
     float *fshift;                  // per anti-diagonal base(d) - base(d-1)
@@ -216,7 +215,7 @@ struct Args {
     Control *ctl;
     float threshold;
     int32_t wmax;                   // ring width (cells); rings hold wmax + 2 floats per state
-    int32_t warp_windows;           // bands up to 128 cells: a window per warp (else per CTA)
+    int32_t sms;                    // SMs of the device
     long long spin_limit;           // clock cycles a worker may wait for a window
     // gather
     int64_t n_reads;
@@ -338,53 +337,6 @@ __device__ float ordered_fold(const float4 *tab, const float *vals, int n) {
         for (int k = 0; k < nc; ++k) r = lae(tab, r, __shfl_sync(0xffffffffu, packed, k));
     }
     return r;
-}
-
-// Two independent ordered folds (ordered_fold on a[0..na) and on b[0..nb)) run by one warp with
-// their sequential logAdd chains interleaved.
-__device__ __forceinline__ float2 ordered_fold2(const float4 *tab, const float *a, int na, const float *b, int nb) {
-    const int lane = threadIdx.x & 31;
-    float ma = kNegInf, mb = kNegInf;
-    for (int q = 0; q < max(na, nb); q += 32) {
-        ma = fmaxf(ma, q + lane < na ? a[q + lane] : kNegInf);
-        mb = fmaxf(mb, q + lane < nb ? b[q + lane] : kNegInf);
-    }
-    ma = warp_max(ma);
-    mb = warp_max(mb);
-    // first index within kSeedGap of each maximum
-    int sa = na, sb = nb;
-    for (int q = 0; q < na; q += 32) {
-        const unsigned m = __ballot_sync(0xffffffffu, q + lane < na && a[q + lane] >= ma - kSeedGap);
-        if (m) { sa = q + __ffs(m) - 1; break; }
-    }
-    for (int q = 0; q < nb; q += 32) {
-        const unsigned m = __ballot_sync(0xffffffffu, q + lane < nb && b[q + lane] >= mb - kSeedGap);
-        if (m) { sb = q + __ffs(m) - 1; break; }
-    }
-    float seed_a = 0.0f, seed_b = 0.0f;
-    for (int q = 0; q < max(sa, sb); q += 32) {
-        const float va = q + lane < sa ? a[q + lane] : kNegInf;
-        const float vb = q + lane < sb ? b[q + lane] : kNegInf;
-        seed_a += va > kNegInf ? __expf(va - ma) : 0.0f;
-        seed_b += vb > kNegInf ? __expf(vb - mb) : 0.0f;
-    }
-    seed_a = warp_sum(seed_a);
-    seed_b = warp_sum(seed_b);
-    float ra = ma > kNegInf && seed_a > 0.0f ? ma + __logf(seed_a) : kNegInf;
-    float rb = mb > kNegInf && seed_b > 0.0f ? mb + __logf(seed_b) : kNegInf;
-    const int ea = ma > kNegInf ? na : 0, eb = mb > kNegInf ? nb : 0;
-    // chunk by chunk: candidates compacted, then both sequential chains side by side
-    for (int ca = sa & ~31, cb = sb & ~31; ca < ea || cb < eb; ca += 32, cb += 32) {
-        float pa = kNegInf, pb = kNegInf;
-        const int nca = ca < ea ? fold_candidates(a, ca, sa, ea, ma - kFoldGap, pa) : 0;
-        const int ncb = cb < eb ? fold_candidates(b, cb, sb, eb, mb - kFoldGap, pb) : 0;
-        for (int k = 0; k < max(nca, ncb); ++k) {
-            const float xa = __shfl_sync(0xffffffffu, pa, k), xb = __shfl_sync(0xffffffffu, pb, k);
-            if (k < nca) ra = lae(tab, ra, xa);
-            if (k < ncb) rb = lae(tab, rb, xb);
-        }
-    }
-    return make_float2(ra, rb);
 }
 
 __global__ void prep_events(const double2 *raw, Event32 *out, int64_t n) {
@@ -531,6 +483,10 @@ __device__ __forceinline__ void emit_cell(const Ctx &c, const KmerConst32 &k, in
 __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_constant__ Args A) {
     __shared__ EmitStage stage[kEmitWarps];
     const int lane = threadIdx.x & 31;
+    // what the column sweeps' look-ahead reads before the first and after the last cell
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < kStoreFront + kStoreBack; i += blockDim.x)
+            A.E[i < kStoreFront ? i - kStoreFront : A.n_cells + (i - kStoreFront)] = make_float2(0.0f, 0.0f);
     EmitStage &st = stage[threadIdx.x >> 5];
     const int64_t warps = (int64_t) gridDim.x * (blockDim.x >> 5);
     for (int64_t ch = blockIdx.x * (int64_t) (blockDim.x >> 5) + (threadIdx.x >> 5); ch < A.n_chunks; ch += warps) {
@@ -586,7 +542,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
                 const int32_t d = C.d0 + k;
                 const int32_t L = __shfl_sync(0xffffffffu, mt.x, k);
                 const int32_t W = __shfl_sync(0xffffffffu, w, k);
-                float *Ed = A.E + 2 * (C.cell + __shfl_sync(0xffffffffu, off, k));
+                float2 *Ed = A.E + (C.cell + __shfl_sync(0xffffffffu, off, k));
                 const int32_t xfirst = (d + L) >> 1;   // column of the anti-diagonal's cell 0
 #pragma unroll
                 for (int q = 0; q < kCols; ++q) {
@@ -598,8 +554,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
                         const float4 v = st.ev[y - ylo];
                         emit_gauss(kk[q], Event32{v.x, v.y, v.z, v.w}, c.rs, em, ey);
                     }
-                    Ed[SE_M * W + i] = em;
-                    Ed[SE_Y * W + i] = ey;
+                    Ed[i] = make_float2(em, ey);
                 }
             }
         } else if (staged) {
@@ -627,7 +582,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
             const int32_t d = C.d0 + k;
             const int32_t L = __shfl_sync(0xffffffffu, mt.x, k);
             const int32_t W = __shfl_sync(0xffffffffu, w, k);
-            float *Ed = A.E + 2 * (C.cell + __shfl_sync(0xffffffffu, off, k));
+            float2 *Ed = A.E + (C.cell + __shfl_sync(0xffffffffu, off, k));
             for (int i = lane; i < W; i += 32) {
                 const int32_t xmy = L + 2 * i, x = (d + xmy) >> 1, y = (d - xmy) >> 1;
                 const bool ok = x >= 1 && x <= c.R.lX && y >= 1 && y <= c.R.lY;
@@ -646,8 +601,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
                     const float4 v = __ldg(reinterpret_cast<const float4 *>(A.events + c.R.event_base + yc));
                     emit_cell(c, kk, kid, v, c.hdp ? __ldg(A.events_raw + c.R.event_base + yc).x : 0.0, ok, em, ey);
                 }
-                Ed[SE_M * W + i] = em;
-                Ed[SE_Y * W + i] = ey;
+                Ed[i] = make_float2(em, ey);
             }
         }
         __syncwarp();   // the stage is rewritten by the warp's next chunk
@@ -779,7 +733,7 @@ struct ForwardSweep {
     int32_t n;
     int32_t dbeg, dend;           // owned anti-diagonals (dbeg, dend] (0 is owned by a first segment)
     float *Fd;                    // forward store of the anti-diagonal being computed
-    const float *Ereg;
+    const float2 *Ereg;
     // band facts: metas of d-2, d-1, d (m2, m1, m0); by phase, decoded metas of d+1 .. d+3 and
     // raw metas of d+3 .. d+5 (loaded three steps before they are decoded)
     Meta m2, m1, m0;
@@ -809,8 +763,9 @@ struct ForwardSweep {
             const int i = tid + j * kThreads;
             const int32_t xmy = m.L + 2 * i, x = (dd + xmy) >> 1;
             const int ic = clampi(i, 0, max(m.W - 1, 0));
-            pM[P][j] = __ldg(Ereg + 2 * off + SE_M * m.W + ic);
-            pY[P][j] = __ldg(Ereg + 2 * off + SE_Y * m.W + ic);
+            const float2 e = __ldg(Ereg + off + ic);
+            pM[P][j] = e.x;
+            pY[P][j] = e.y;
             pX[P][j] = raw_gapx(c, x);
             pV[P][j] = x >= 1;
         }
@@ -972,7 +927,7 @@ struct ForwardSweep {
         dend = S.d_end;
         const int32_t s = dbeg - S.warm + (dbeg == 0 ? 1 : 0);
         Fd = A.F + 3 * (R.cell_base + S.cell0);
-        Ereg = A.E + 2 * R.cell_base;
+        Ereg = A.E + R.cell_base;
         ring_init(ring, wmax);
         __syncthreads();
         if (dbeg == 0) {
@@ -1111,7 +1066,7 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
     const int64_t db = R.diag_base;
     const int32_t n = R.n;
     const float *Freg = A.F + 3 * R.cell_base;
-    const float *Ereg = A.E + 2 * R.cell_base;
+    const float2 *Ereg = A.E + R.cell_base;
     const Window W = A.windows[gw];
     const WindowTask wt = A.wtask[gw];
     // a window whose T starts a forward segment reads that segment's own copy of T, kept by the
@@ -1209,16 +1164,16 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
         float tM_n[CPT], tX_n[CPT], tY_n[CPT], tE_n[CPT];
         bool tv_n[CPT];
         {
-            const float *Ed = Ereg + 2 * off0;                  // emissions of d
-            const float *Ep = Ereg + 2 * offp;                  // of d+1 (or d at the window top)
+            const float2 *Ed = Ereg + off0;                     // emissions of d
+            const float2 *Ep = Ereg + offp;                     // of d+1 (or d at the window top)
             const float *Fm = Freg + 3 * offm;                  // forward values of d-1
             const int32_t Wpl = Wp > 0 ? Wp : W0;               // width of the block Ep points at
 #pragma unroll
             for (int j = 0; j < CPT; ++j) {
                 const int i = tid + j * kThreads;
                 const int32_t xmy = mm.L + 2 * i, x = (d - 1 + xmy) >> 1;
-                eMm_n[j] = __ldg(Ep + SE_M * Wpl + clampi((xmy - mp.L) >> 1, 0, max(Wpl - 1, 0)));
-                eYu_n[j] = __ldg(Ed + SE_Y * W0 + clampi((xmy - 1 - m0.L) >> 1, 0, max(W0 - 1, 0)));
+                eMm_n[j] = __ldg(Ep + clampi((xmy - mp.L) >> 1, 0, max(Wpl - 1, 0))).x;
+                eYu_n[j] = __ldg(Ed + clampi((xmy - 1 - m0.L) >> 1, 0, max(W0 - 1, 0))).y;
                 eXl_n[j] = raw_gapx(c, x + 1);
                 fM_n[j] = __ldcg(Fm + ST_M * Wm + clampi(i, 0, max(Wm - 1, 0)));
                 tv_n[j] = false;
@@ -1239,7 +1194,7 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
                     const int32_t r = (xmy0 - mmm.L) >> 1;
                     tv_n[j] = i < W0 && Wmm > 0 && xmy0 >= mmm.L && r < Wmm;
                     const int imm = clampi(r, 0, max(Wmm - 1, 0));
-                    tE_n[j] = __ldg(Ed + SE_M * W0 + clampi(i, 0, max(W0 - 1, 0)));
+                    tE_n[j] = __ldg(Ed + clampi(i, 0, max(W0 - 1, 0))).x;
                     tM_n[j] = __ldcg(Fmm + ST_M * Wml + imm);
                     tX_n[j] = __ldcg(Fmm + ST_X * Wml + imm);
                     tY_n[j] = __ldcg(Fmm + ST_Y * Wml + imm);
@@ -1372,349 +1327,6 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
         if (W.at_end) A.loglik[c.region_index] = ll;
     }
 }
-
-// ------------------------------------------------------------------------------------------------
-// backward sweep of one traceback window by one warp (bands up to 32 * WCPT cells wide)
-// ------------------------------------------------------------------------------------------------
-// The same recursion, posterior and refreshes as window_task, with the anti-diagonal's cells spread
-// over one warp (cell i on lane i mod 32): warp-synchronous exchange through the ring, maxima by one
-// warp reduction, pairs numbered by ballots, no block barrier.  Look-ahead loads go to registers
-// indexed by the parity of the step, so they land without register moves; the operands of a
-// refresh (one anti-diagonal in ten) are loaded when it happens.
-template <int WCPT, bool kSX>
-struct WarpWindow {
-    const Ctx &c;
-    const Args &A;
-    const RegionDesc &R;
-    const float4 *tab;
-    float *ring;                  // 3 slots x 3 states x (wmax + 2)
-    float *chain;                 // 2 x wmax: refresh terms, then 6 x wmax: staged refresh operands
-    int lane, wmax, stride;
-    int64_t db;
-    int32_t n, D, T, from;
-    const float *Freg, *Ereg;
-    const float *Tside;           // the forward segment's own copy of T (see window_task), or null
-    float *s0, *s1, *s2;          // ring slots of d, d+1, d+2
-    Meta mpp, mp, m0, mm;         // band facts of d+2, d+1, d, d-1
-    int2 raw_mmm;                 // raw band facts of d-2
-    int32_t off0, offp;           // first cells of d and d+1
-    // look-ahead operands of a step's cells, by step parity: match emission of the match
-    // successor, extra-event emission of the upper successor, skip emission of the lower
-    // successor, forward match value; and the forward base and shift
-    float qM[2][WCPT], qY[2][WCPT], qX[2][WCPT], qF[2][WCPT];
-    double qB[2];
-    float qS[2];
-    float mxD, mx_last, lm_prev, gamma1;
-    float e0, e1, e2;             // end states on D
-    double bbase, pref, ll;
-    int64_t n_out;
-
-    __device__ __forceinline__ WarpWindow(const Ctx &cc, float *r, float *ch, const float4 *tb)
-        : c(cc), A(*cc.A), R(cc.R), tab(tb), ring(r), chain(ch) {}
-
-    // operands of the cells of anti-diagonal dd (meta m, first cell off) into parity Q; m1 / off1
-    // describe dd+1 (upper successors), m2 / off2 dd+2 (match successors)
-    template <int Q>
-    __device__ __forceinline__ void prefetch(int32_t dd, const Meta &m, int32_t off, const Meta &m1, int32_t off1,
-                                             const Meta &m2, int32_t off2) {
-        const float *E2 = Ereg + 2 * off2, *E1 = Ereg + 2 * off1, *Fm = Freg + 3 * off;
-#pragma unroll
-        for (int j = 0; j < WCPT; ++j) {
-            const int i = lane + 32 * j;
-            const int32_t xmy = m.L + 2 * i, x = (dd + xmy) >> 1;
-            qM[Q][j] = __ldg(E2 + SE_M * m2.W + clampi((xmy - m2.L) >> 1, 0, max(m2.W - 1, 0)));
-            qY[Q][j] = __ldg(E1 + SE_Y * m1.W + clampi((xmy - 1 - m1.L) >> 1, 0, max(m1.W - 1, 0)));
-            qX[Q][j] = raw_gapx(c, x + 1);
-            qF[Q][j] = __ldcg(Fm + ST_M * m.W + clampi(i, 0, max(m.W - 1, 0)));
-        }
-        qB[Q] = __ldcg(A.base + db + max(dd, 0));
-        qS[Q] = __ldcg(A.fshift + db + max(dd, 0));
-    }
-
-    // Operands of a refresh at anti-diagonal dd (meta m, first cell off): its gap states, and for
-    // the cells of dd+1 (m1, off1) the forward values of dd-1 (m_1, off_1) on their match
-    // predecessors and their match emissions.  At the end of the step before the refresh,
-    // load_refresh loads them (forward values through L2: other CTAs wrote them during this
-    // launch) and store_refresh puts them in this warp's staging rows.
-    struct RefreshOps {
-        float x[WCPT], y[WCPT], m[WCPT], tx[WCPT], ty[WCPT], e[WCPT];
-    };
-
-    __device__ __forceinline__ void load_refresh(RefreshOps &o, const Meta &m, int32_t off, const Meta &m1, int32_t off1,
-                                                 const Meta &m_1, int32_t off_1, int32_t d_1) const {
-        const float *Fd = Freg + 3 * off, *E1 = Ereg + 2 * off1;
-        const float *Fm = Tside && d_1 == T ? Tside : Freg + 3 * off_1;
-#pragma unroll
-        for (int j = 0; j < WCPT; ++j) {
-            const int i = lane + 32 * j;
-            const int ic = clampi(i, 0, max(m.W - 1, 0));
-            o.x[j] = __ldcg(Fd + ST_X * m.W + ic);
-            o.y[j] = __ldcg(Fd + ST_Y * m.W + ic);
-            const int32_t r = clampi((m1.L + 2 * i - m_1.L) >> 1, 0, max(m_1.W - 1, 0));
-            o.m[j] = __ldcg(Fm + ST_M * m_1.W + r);
-            o.tx[j] = __ldcg(Fm + ST_X * m_1.W + r);
-            o.ty[j] = __ldcg(Fm + ST_Y * m_1.W + r);
-            o.e[j] = __ldg(E1 + SE_M * m1.W + clampi(i, 0, max(m1.W - 1, 0)));
-        }
-    }
-
-    __device__ __forceinline__ void store_refresh(const RefreshOps &o) const {
-        float *stg = chain + 2 * wmax;
-#pragma unroll
-        for (int j = 0; j < WCPT; ++j) {
-            const int i = lane + 32 * j;
-            stg[i] = o.x[j];
-            stg[wmax + i] = o.y[j];
-            stg[2 * wmax + i] = o.m[j];
-            stg[3 * wmax + i] = o.tx[j];
-            stg[4 * wmax + i] = o.ty[j];
-            stg[5 * wmax + i] = o.e[j];
-        }
-    }
-
-    // anti-diagonal d; K = (D - d) & 1 is the parity of its operands
-    template <int K>
-    __device__ __forceinline__ void step(int32_t d, const WindowTask &wt) {
-        const float *t = c.t;
-        const int32_t W0 = m0.W, Wp = mp.W;
-        // maximum of B on d+1 for the shift of d-1 (d+1 = D holds the end states: known exactly)
-        const float mx_new = warp_max1(lm_prev);
-        float gamma0 = 0.0f;           // base(d) - base(d+1) = max(d+2) - gamma1
-        if (d <= D - 2) {
-            float m = d == D - 2 ? mxD : mx_last;
-            if (!(m > kNegInf)) m = 0.0f;
-            gamma0 = m - gamma1;
-        }
-        bbase += (double) gamma0;
-        // operands of the d-1 cells
-        const Meta mmm = decode_meta(raw_mmm, d - 2 >= 0);
-        raw_mmm = raw_meta(A, db, d - 3, n);
-        const int32_t offm = off0 - mm.W;
-        prefetch<1 - K>(d - 1, mm, offm, m0, off0, mp, offp);
-        const bool refresh_next = d - 1 > T && d - 1 <= from && (mm.flags & kFlagRefresh) != 0;
-        // the recursion on d (D itself holds the end-state values); B of the cells kept in registers
-        float lm = kNegInf;
-        float bM[WCPT], bX[WCPT], bY[WCPT];
-        if (d == D) {
-#pragma unroll
-            for (int j = 0; j < WCPT; ++j) {
-                const bool in = lane + 32 * j < W0;
-                bM[j] = in ? e0 : kNegInf;
-                bX[j] = in ? e1 : kNegInf;
-                bY[j] = in ? e2 : kNegInf;
-            }
-        } else {
-            const float shU = -gamma0, shM = -gamma1 - gamma0;
-            // all ring reads first, then the arithmetic, then the ring writes: the cells' chains are
-            // independent, and no shared-memory store sits between them to order them
-            float bme[WCPT], bue[WCPT], ble[WCPT];
-#pragma unroll
-            for (int j = 0; j < WCPT; ++j) {
-                const int i = lane + 32 * j;
-                const int32_t xmy = m0.L + 2 * i;
-                const int ipp = clampi((xmy - mpp.L) >> 1, -1, wmax);
-                const int iu = clampi((xmy - 1 - mp.L) >> 1, -1, wmax);
-                const int il = clampi((xmy + 1 - mp.L) >> 1, -1, wmax);
-                bme[j] = s2[ipp];
-                bue[j] = s1[2 * stride + iu];
-                ble[j] = s1[stride + il];
-            }
-#pragma unroll
-            for (int j = 0; j < WCPT; ++j) {
-                // each successor's backward value plus its emission, shared by the transitions into it
-                const float me = bme[j] + (qM[K][j] + shM);
-                float vM = me + t[T_MC];
-                float vX = me + t[T_MFGX];
-                float vY = me + t[T_MFGY];
-                const float ue = bue[j] + (qY[K][j] + shU);
-                vM = lae(tab, vM, ue + t[T_OY]);
-                vY = lae(tab, vY, ue + t[T_EY]);
-                const float le = ble[j] + (qX[K][j] + shU);
-                vM = lae(tab, vM, le + t[T_OX]);
-                vX = lae(tab, vX, le + t[T_EX]);
-                if (kSX) vY = lae(tab, vY, le + t[T_SX]);
-                const bool in = lane + 32 * j < W0;
-                bM[j] = in ? vM : kNegInf;
-                bX[j] = in ? vX : kNegInf;
-                bY[j] = in ? vY : kNegInf;
-                lm = fmaxf(lm, fmaxf(bM[j], fmaxf(bX[j], bY[j])));
-            }
-#pragma unroll
-            for (int j = 0; j < WCPT; ++j) {
-                const int i = lane + 32 * j;
-                s0[i] = bM[j];
-                s0[stride + i] = bX[j];
-                s0[2 * stride + i] = bY[j];
-            }
-        }
-        __syncwarp();
-        const double fb = qB[K];
-        const float fsh = qS[K];
-        if (d <= from) {
-            if ((m0.flags & kFlagRefresh) != 0) {
-                // diagonalCalculationTotalProbability (pairwiseAligner.c:1182-1200): F.B on d in
-                // ascending cell order, then the matches from d-1 over d into d+1, dotted with B(d+1)
-                const float *stg = chain + 2 * wmax;
-                const bool have_next = d < D;
-                const int32_t Wm = mm.W;
-                float sx[WCPT], sy[WCPT], tm[WCPT], tx[WCPT], ty[WCPT], te[WCPT], b1[WCPT];
-#pragma unroll
-                for (int j = 0; j < WCPT; ++j) {
-                    const int i = lane + 32 * j;
-                    sx[j] = stg[i];
-                    sy[j] = stg[wmax + i];
-                    tm[j] = stg[2 * wmax + i];
-                    tx[j] = stg[3 * wmax + i];
-                    ty[j] = stg[4 * wmax + i];
-                    te[j] = stg[5 * wmax + i];
-                    b1[j] = s1[i];
-                }
-                float c0[WCPT], c1[WCPT];
-#pragma unroll
-                for (int j = 0; j < WCPT; ++j) {
-                    const int i = lane + 32 * j;
-                    float v = qF[K][j] + bM[j];
-                    v = lae(tab, v, sx[j] + bX[j]);
-                    c0[j] = lae(tab, v, sy[j] + bY[j]);
-                    const int32_t xmy1 = mp.L + 2 * i;
-                    const int32_t r = (xmy1 - mm.L) >> 1;
-                    float mth = kNegInf;
-                    if (Wm > 0 && xmy1 >= mm.L && r < Wm) {
-                        const float e = te[j];
-                        mth = tm[j] + (e + t[T_MC]);
-                        mth = lae(tab, mth, tx[j] + (e + t[T_MFGX]));
-                        mth = lae(tab, mth, ty[j] + (e + t[T_MFGY]));
-                    }
-                    c1[j] = mth + b1[j];
-                }
-#pragma unroll
-                for (int j = 0; j < WCPT; ++j) {
-                    const int i = lane + 32 * j;
-                    if (i < W0) chain[i] = c0[j];
-                    if (have_next && i < Wp) chain[wmax + i] = c1[j];
-                }
-                __syncwarp();
-                const float2 ff = ordered_fold2(tab, chain, W0, chain + wmax, have_next ? Wp : 0);
-                const float f0 = ff.x, f1 = ff.y;
-                // the through-part is relative to base_F(d-1) + base_B(d+1)
-                const float ptil = lae(tab, f0, f1 - fsh - gamma0);
-                pref = (double) ptil + fb + bbase;
-                if (d == n) ll = pref;
-                __syncwarp();
-            }
-            // posteriors of d, emitted in ascending cell order (the reference's order)
-            const float kd = (float) (fb + bbase - pref);
-            int64_t before = n_out;
-#pragma unroll
-            for (int j = 0; j < WCPT; ++j) {
-                const int i = lane + 32 * j;
-                const int32_t xmy = m0.L + 2 * i, x = (d + xmy) >> 1, y = (d - xmy) >> 1;
-                const float p = __expf(qF[K][j] + bM[j] + kd);
-                const bool hit = i < W0 && x > 0 && y > 0 && p >= A.threshold;
-                const unsigned bal = __ballot_sync(0xffffffffu, hit);
-                if (hit) {
-                    const int64_t q = before + __popc(bal & ((1u << lane) - 1u));
-                    if (q < wt.out_cap) {
-                        sa_aligned_pair o;
-                        o.score = (int64_t) floor((double) fminf(p, 1.0f) * 10000000.0);
-                        o.x = R.x1 + x - 1;
-                        o.y = R.y1 + y - 1;
-                        o.kmer = __ldg(A.kmer + R.kmer_base + x - 1);   // 1 <= x <= lX for a pair
-                        A.out[wt.out_base + q] = o;
-                    } else {
-                        atomicMax(A.status + R.read, (int32_t) SA_E_OUTPUT);
-                    }
-                }
-                before += __popc(bal);
-            }
-            n_out = before;
-        }
-        if (refresh_next) {
-            // loaded here rather than a step early: held across the step, the 6 x WCPT operands
-            // pushed the 3-CTAs-per-SM build into spilling (312 B per thread; 16 B this way), and
-            // the latency is paid one step in ten
-            RefreshOps rops;
-            load_refresh(rops, mm, offm, m0, off0, mmm, offm - mmm.W, d - 2);
-            __syncwarp();   // this step's refresh (if any) has read the staging rows
-            store_refresh(rops);
-        }
-        mx_last = mx_new;
-        lm_prev = d == D ? kNegInf : lm;   // D's maximum is known exactly (mxD)
-        gamma1 = gamma0;
-        offp = off0;
-        off0 = offm;
-        float *fr = s2;
-        s2 = s1;
-        s1 = s0;
-        s0 = fr;
-        mpp = mp; mp = m0; m0 = mm; mm = mmm;
-    }
-
-    __device__ void run(int64_t gw) {
-        lane = threadIdx.x & 31;
-        wmax = 32 * WCPT;
-        stride = wmax + 2;
-        db = R.diag_base;
-        n = R.n;
-        Freg = A.F + 3 * R.cell_base;
-        Ereg = A.E + 2 * R.cell_base;
-        const Window Wn = A.windows[gw];
-        const WindowTask wt = A.wtask[gw];
-        D = Wn.D;
-        T = Wn.T;
-        from = Wn.from;
-        Tside = A.use_side && wt.side >= 0 ? A.stitch_vals + A.stitch[wt.side].voff + 3 * A.stitch[wt.side].w0 : nullptr;
-        for (int i = lane; i < 9 * stride; i += 32) ring[i] = kNegInf;
-        s0 = ring + 1;
-        s1 = ring + 3 * stride + 1;
-        s2 = ring + 6 * stride + 1;
-        // end-state values on D (stateMachine.c:1034-1061)
-        const float *t = c.t;
-        const bool ragged_end = Wn.at_end && R.ragged_right;
-        e0 = ragged_end ? (t[T_OX] + t[T_OY]) / 2.0f : t[T_MC];
-        e1 = ragged_end ? t[T_EX] : t[T_MFGX];
-        e2 = ragged_end ? t[T_EY] : t[T_MFGY];
-        mxD = fmaxf(e0, fmaxf(e1, e2));
-        if (!(mxD > kNegInf)) mxD = 0.0f;
-        mpp = mp = Meta{0, 0, 0};
-        m0 = decode_meta(raw_meta(A, db, D, n), true);
-        mm = decode_meta(raw_meta(A, db, D - 1, n), D - 1 >= 0);
-        raw_mmm = raw_meta(A, db, D - 2, n);
-        off0 = offp = wt.first_cell;
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < WCPT; ++j) {
-            const int i = lane + 32 * j;
-            if (i < m0.W) {
-                s0[i] = e0;
-                s0[stride + i] = e1;
-                s0[2 * stride + i] = e2;
-            }
-        }
-        prefetch<0>(D, m0, off0, mp, offp, mpp, offp);
-        if (D <= from && (m0.flags & kFlagRefresh) != 0) {
-            RefreshOps o;
-            load_refresh(o, m0, off0, mp, offp, mm, off0 - mm.W, D - 1);
-            store_refresh(o);
-        }
-        mx_last = kNegInf;
-        lm_prev = kNegInf;
-        gamma1 = 0.0f;
-        bbase = pref = ll = 0.0;
-        n_out = 0;
-        __syncwarp();
-        for (int32_t d = D; d > T; d -= 2) {
-            step<0>(d, wt);
-            if (d - 1 <= T) break;
-            step<1>(d - 1, wt);
-        }
-        if (lane == 0) {
-            A.wcount[gw] = n_out;
-            if (Wn.at_end) A.loglik[c.region_index] = ll;
-        }
-        __syncwarp();
-    }
-};
 
 // ------------------------------------------------------------------------------------------------
 // the persistent worker
@@ -1860,11 +1472,10 @@ __device__ void read_unit_done(const Args &A, int32_t r, int tid, Shared *sh) {
     group_sync<NT>();
 }
 
-// CPT: cells per thread of the forward sweep (128 threads per region).  The first claims are
-// forward sweeps, one per CTA; once none is left, windows are claimed: one per warp for bands up to
-// kWarpWindowWidth cells wide, one per CTA for wider bands.  MINB: CTAs per SM the registers are
-// budgeted for (2: 255 registers per thread; 3: 168, with some spilling, for batches bound by their
-// total work rather than by one forward chain).
+// CPT: cells per thread (128 threads per region).  The first claims are forward sweeps, one per CTA;
+// once none is left, windows are claimed, one per CTA.  MINB: CTAs per SM the registers are budgeted
+// for.  Serves the batches column_worker cannot take, and launch configurations without a window per
+// warp.
 template <int CPT, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) worker_kernel(const __grid_constant__ Args A) {
     extern __shared__ float4 smem_raw[];
@@ -1887,48 +1498,22 @@ __global__ void __launch_bounds__(kThreads, MINB) worker_kernel(const __grid_con
         forward_task<CPT>(c, sg, sh, area);
         __syncthreads();
     }
-    // traceback windows, in publication order: one per warp for bands up to 128 cells (when the
-    // launch configuration asks for it), else one per CTA
-    if (CPT == 1 && A.warp_windows) {
-        const int lane = tid & 31, warp = tid >> 5;
-        float *wring = area + warp * kWarpWindowFloats;
-        float *wchain = wring + 9 * (kWarpWindowWidth + 2);
-        for (;;) {
-            int32_t id = -1;
-            if (lane == 0) {
-                const unsigned claim = atomicAdd(&A.ctl->wclaim, 1u);
-                if ((int64_t) claim < A.n_windows) id = wait_ready(A, claim);
-            }
-            id = __shfl_sync(0xffffffffu, id, 0);
-            if (id < 0) break;
-            Ctx c;
-            ctx_init(c, A, A.wtask[id].region);
-            if (c.t[T_SX] > kNegInf) {
-                WarpWindow<kWarpWindowCpt, true> w(c, wring, wchain, sh->la);
-                w.run(id);
-            } else {
-                WarpWindow<kWarpWindowCpt, false> w(c, wring, wchain, sh->la);
-                w.run(id);
-            }
-            read_unit_done<32>(A, c.R.read, lane, sh);
+    // traceback windows, in publication order, one per CTA
+    float *ring = area, *chain = area + 9 * (A.wmax + 2);
+    for (;;) {
+        if (tid == 0) {
+            const unsigned claim = atomicAdd(&A.ctl->wclaim, 1u);
+            sh->task_id = (int64_t) claim < A.n_windows ? wait_ready(A, claim) : -1;
         }
-    } else {
-        float *ring = area, *chain = area + 9 * (A.wmax + 2);
-        for (;;) {
-            if (tid == 0) {
-                const unsigned claim = atomicAdd(&A.ctl->wclaim, 1u);
-                sh->task_id = (int64_t) claim < A.n_windows ? wait_ready(A, claim) : -1;
-            }
-            __syncthreads();
-            const int32_t id = sh->task_id;
-            if (id < 0) break;
-            Ctx c;
-            ctx_init(c, A, A.wtask[id].region);
-            if (c.t[T_SX] > kNegInf) window_task<CPT, true>(c, sh, ring, chain, id);
-            else window_task<CPT, false>(c, sh, ring, chain, id);
-            __syncthreads();
-            read_unit_done<kThreads>(A, c.R.read, tid, sh);
-        }
+        __syncthreads();
+        const int32_t id = sh->task_id;
+        if (id < 0) break;
+        Ctx c;
+        ctx_init(c, A, A.wtask[id].region);
+        if (c.t[T_SX] > kNegInf) window_task<CPT, true>(c, sh, ring, chain, id);
+        else window_task<CPT, false>(c, sh, ring, chain, id);
+        __syncthreads();
+        read_unit_done<kThreads>(A, c.R.read, tid, sh);
     }
 }
 
