@@ -1046,15 +1046,15 @@ sa_status sa_batch_read_status(const sa_batch *b, int64_t read) {
 int64_t sa_batch_pair_count(const sa_batch *b, int64_t read) {
     if (!b || read < 0 || read >= b->n_reads || !b->downloaded) return -1;
     if (b->read_status[read]) return 0;
-    if (b->plain_of[read] >= 0) return b->plain ? (int64_t) plain_pairs(b->plain, b->plain_of[read]).size() : 0;
+    if (b->plain_of[read] >= 0) return b->plain ? (int64_t) plain_pairs(b->plain, b->plain_of[read]).n : 0;
     return b->read_count[read];
 }
 
 const sa_aligned_pair *sa_batch_pairs(const sa_batch *b, int64_t read) {
     if (!b || read < 0 || read >= b->n_reads || !b->downloaded) return nullptr;
     if (!b->read_status[read] && b->plain_of[read] >= 0 && b->plain) {
-        const auto &v = plain_pairs(b->plain, b->plain_of[read]);
-        if (!v.empty()) return v.data();
+        const PlainPairs v = plain_pairs(b->plain, b->plain_of[read]);
+        if (v.n) return v.p;
     }
     return static_cast<const sa_aligned_pair *>(b->host_pairs.ptr) + (b->read_status[read] ? 0 : b->read_base[read]);
 }

@@ -1,4 +1,5 @@
-// Plain FP64 form: one region (read, or split sub-region) per CTA, sweeping the
+// Plain FP64 form.  Sets whose bands and stores fit run as the launches of sa_fp64_resident.cuh; what
+// follows describes the other route, the rings: one region (read, or split sub-region) per CTA, sweeping the
 // band anti-diagonal by anti-diagonal in log space with the reference's logAdd, windowed traceback
 // and every-10th-anti-diagonal total-probability refresh (getPosteriorProbsWithBanding,
 // pairwiseAligner.c:1282-1420).  It is the parity anchor of the engine: results agree with
@@ -62,6 +63,14 @@ struct Region64 {
     double threshold;
     double *loglik;
     int32_t *status;
+    // resident kernels (sa_fp64_resident.cuh): per anti-diagonal {first path, paths, first slot - first
+    // path, window}; the paths; F.B of the match state per slot; the region's first window among the
+    // set's; the read's accumulators; the region's first column in the read
+    const int4 *info;
+    const struct Path64 *path;
+    double *S;
+    int64_t win_base, x_base;
+    int32_t reader, pad2;
 };
 
 // where two forward segments of a region meet, at anti-diagonal b (the later one's first window's T):
@@ -423,6 +432,11 @@ __device__ void expect_diagonal(const Model64 &M, const Region64 &R, const Expec
 // pairs or (expectations mode) the expectation updates.
 // path slots of anti-diagonal d: the first slot (of its first cell) and their number
 __device__ __forceinline__ void diag_slots(const Region64 &R, int32_t d, int32_t &first, int32_t &count) {
+    if (R.info) {
+        first = R.info[d].x;
+        count = R.info[d].y;
+        return;
+    }
     first = R.pfirst[(d + R.xl[d]) >> 1];
     count = R.pfirst[((d + R.xr[d]) >> 1) + 1] - first;
 }
@@ -643,6 +657,8 @@ __device__ void run_region(const Model64 &M, const Region64 &R, int32_t region, 
     if (R.st_out >= 0) stitch_arrive64(R, O, R.st_out);
 }
 
+#include "sa_fp64_resident.cuh"
+
 // Expectations mode (XS: one ExpectOut per read): CTA b walks read b's regions in order.
 __global__ void __launch_bounds__(128) region_kernel(const Model64 *models, const Region64 *regions, SetOut O,
                                                      const ExpectOut *XS) {
@@ -700,10 +716,22 @@ sa_status compute_kmer_logs(sa_state_machine *sm) {
 // ------------------------------------------------------------------------------------------------
 namespace {
 
+// resident route: its store of every anti-diagonal, at most (the rings of the other route take a few
+// MB a region whatever its length), and the threads its sweeps may use
+constexpr size_t kResidentBytes = (size_t) 24 << 30;
+constexpr int kResidentThreads[] = {128, 256, 512};
+
 // host plan of one region: geometry (band, windows) and its paths
 struct PlainRegion {
     int32_t read = 0, model = 0;
     Region rg;
+    bool active = true;          // runs (expectations: reads with an error do not)
+    int32_t reader = 0;          // expectations: its read among the running ones
+    int64_t slots = 0;           // path slots of all its anti-diagonals
+    int32_t span = 0;            // paths that three consecutive anti-diagonals span, at most
+    std::vector<int4> info;      // resident route: Region64::info
+    std::vector<Path64> path;    // and Region64::path
+    bool regular = true;         // every path's predecessors are evenly spaced
     std::vector<int32_t> xl, xr, pfirst, pid, ppre, psuf, row;
     int32_t ring = 3, stride = 1, max_paths = 1;
     size_t ev_off = 0;   // first event of the region in the set's event array
@@ -750,12 +778,28 @@ struct PlainSet {
     int32_t *d_tag = nullptr;
     double *d_P = nullptr;
     size_t p_bytes = 0;
-    // results
+    // resident route
+    bool resident = false, expect = false, multi = false, finite_sx = false;
+    int nt = 128;
+    int64_t n_windows = 0, n_totals = 0, n_chunks = 0, n_rows = 0, n_run_tasks = 0;
+    int64_t term_stride = 1;
+    Window64 *d_windows = nullptr;
+    Total64 *d_totals = nullptr;
+    int32_t *d_chunk_region = nullptr, *d_chunk_d0 = nullptr, *d_run_tasks = nullptr, *d_task_of = nullptr;
+    int64_t *d_row_base = nullptr, *d_region_total = nullptr, *d_region_count = nullptr;
+    int32_t *d_count_rows = nullptr;
+    double *d_terms = nullptr;
+    size_t res_region_count = 0;
+    std::vector<int64_t> read_chunk;   // expectations: first chunk of each running read, and the end
+    MemBlock host_pairs;
+    // results: a read's pairs lie in host_pairs (resident route) or in its own vector
     std::vector<std::vector<sa_aligned_pair>> pairs;
+    std::vector<PlainPairs> spans;
     std::vector<double> ll;
     std::vector<int32_t> status;
 
     ~PlainSet() {
+        mem_put(host_pairs);
         mem_put(host_in);
         mem_put(host_res);
         mem_put(dev);
@@ -766,9 +810,36 @@ namespace {
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t) 255; }
 
+// the device descriptors of the set's machines (resident tables) and the reads' scaling
+void put_models(const PlainSet *s, unsigned char *to) {
+    for (size_t m = 0; m < s->models.size(); ++m) {
+        const sa_state_machine *sm = s->models[m].sm;
+        if (!sm) continue;
+        Model64 M;
+        std::memset(&M, 0, sizeof(M));
+        M.emission = sm->emission;
+        for (int i = 0; i < 9; ++i) M.t[i] = sm->t[i];
+        M.match = sm->dev.match;
+        M.gapy = sm->dev.gapy;
+        M.gapx = sm->dev.gapx;
+        M.klog = sm->dev.klog;
+        M.scale = s->models[m].scale;
+        M.shift = s->models[m].shift;
+        M.var = s->models[m].var;
+        if (sm->emission == SA_EMIT_HDP) {
+            M.grid_length = sm->hdp.grid_length;
+            M.grid = sm->dev.hdp_grid;
+            M.density = sm->dev.hdp_density;
+            M.slope = sm->dev.hdp_slope;
+            M.kmer_row = sm->dev.hdp_kmer_row;
+        }
+        std::memcpy(to + m * sizeof(Model64), &M, sizeof(M));
+    }
+}
+
 // Places every buffer of the set; with non-null bases writes the staged inputs and the Region64 /
 // Model64 descriptors (device addresses).  Returns the device bytes.
-size_t plain_layout(PlainSet *s, unsigned char *host, unsigned char *dev) {
+size_t ring_layout(PlainSet *s, unsigned char *host, unsigned char *dev) {
     size_t at = 0;
     auto take = [&](size_t bytes) {
         at = align256(at);
@@ -930,31 +1001,213 @@ size_t plain_layout(PlainSet *s, unsigned char *host, unsigned char *dev) {
         }
         if (!T.empty()) std::memcpy(host + o_tasks, T.data(), T.size() * sizeof(Region64));
         if (!ST.empty()) std::memcpy(host + o_stitch, ST.data(), ST.size() * sizeof(Stitch64));
-        for (size_t m = 0; m < s->models.size(); ++m) {
-            const sa_state_machine *sm = s->models[m].sm;
-            Model64 M;
-            std::memset(&M, 0, sizeof(M));
-            M.emission = sm->emission;
-            for (int i = 0; i < 9; ++i) M.t[i] = sm->t[i];
-            M.match = sm->dev.match;
-            M.gapy = sm->dev.gapy;
-            M.gapx = sm->dev.gapx;
-            M.klog = sm->dev.klog;
-            M.scale = s->models[m].scale;
-            M.shift = s->models[m].shift;
-            M.var = s->models[m].var;
-            if (sm->emission == SA_EMIT_HDP) {
-                M.grid_length = sm->hdp.grid_length;
-                M.grid = sm->dev.hdp_grid;
-                M.density = sm->dev.hdp_density;
-                M.slope = sm->dev.hdp_slope;
-                M.kmer_row = sm->dev.hdp_kmer_row;
-            }
-            std::memcpy(host + o_models + m * sizeof(Model64), &M, sizeof(M));
-        }
+        put_models(s, host + o_models);
         if (!s->events.empty()) std::memcpy(host + o_events, s->events.data(), s->events.size() * sizeof(double2));
     }
     return s->dev_bytes;
+}
+
+// The same for the resident route: every anti-diagonal's values of every task (a later forward
+// segment's from two anti-diagonals before its sweep), the emissions and F.B of every slot once.
+size_t resident_layout(PlainSet *s, unsigned char *host, unsigned char *dev) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        at = align256(at);
+        const size_t o = at;
+        at += std::max<size_t>(bytes, 1);
+        return o;
+    };
+    const size_t nreg = s->regs.size();
+    s->n_windows = s->n_totals = s->n_chunks = s->n_rows = s->n_run_tasks = 0;
+    s->term_stride = 1;
+    for (size_t i = 0; i < nreg; ++i) {
+        const PlainRegion &pr = s->regs[i];
+        if (!pr.active) continue;
+        const int64_t n = pr.rg.lX + pr.rg.lY;
+        s->n_windows += (int64_t) pr.rg.windows.size();
+        for (const Window &w : pr.rg.windows) s->n_totals += (w.from - w.T + 9) / 10;
+        s->n_chunks += (n + 32) / 32;
+        s->n_run_tasks += 1 + (int64_t) pr.cuts.size();
+        s->term_stride = std::max<int64_t>(s->term_stride, pr.stride);
+    }
+    for (size_t i = 0; i < nreg; ++i) s->n_rows += s->regs[i].rg.lX + s->regs[i].rg.lY + 1;
+    const size_t o_regions = take(nreg * sizeof(Region64));
+    const size_t o_models = take(s->models.size() * sizeof(Model64));
+    const size_t o_tasks = take((size_t) s->n_run_tasks * sizeof(Region64));
+    const size_t o_stitch = take((size_t) s->n_stitch * sizeof(Stitch64));
+    const size_t o_windows = take((size_t) s->n_windows * sizeof(Window64));
+    const size_t o_totals = take((size_t) s->n_totals * sizeof(Total64));
+    const size_t o_chreg = take((size_t) s->n_chunks * sizeof(int32_t));
+    const size_t o_chd0 = take((size_t) s->n_chunks * sizeof(int32_t));
+    const size_t o_taskof = take((size_t) s->n_windows * sizeof(int32_t));
+    const size_t o_rowbase = take(nreg * sizeof(int64_t));
+    struct Off { size_t info, path, pid, win; };
+    std::vector<Off> off(nreg);
+    for (size_t i = 0; i < nreg; ++i) {
+        const PlainRegion &pr = s->regs[i];
+        off[i].info = take(pr.info.size() * sizeof(int4));
+        off[i].path = take(pr.path.size() * sizeof(Path64));
+        off[i].pid = take(pr.pid.size() * sizeof(int32_t));
+        off[i].win = take(pr.rg.windows.size() * sizeof(Window));
+    }
+    const size_t o_events = take(s->events.size() * sizeof(double2));
+    s->in_bytes = align256(at);
+    at = s->in_bytes;
+    s->res_off = at;
+    const size_t o_loglik = take(nreg * sizeof(double));
+    const size_t o_status = take(nreg * sizeof(int32_t));
+    const size_t o_count = take(sizeof(unsigned long long));
+    const size_t o_stres = take((size_t) s->n_stitch * sizeof(Stitch64Res));
+    const size_t o_fail = take(nreg * sizeof(int32_t));
+    const size_t o_rcount = take(nreg * sizeof(int64_t));
+    const size_t o_rtotal = take(nreg * sizeof(int64_t));
+    s->res_bytes = align256(at) - s->res_off;
+    s->res_status = o_status - s->res_off;
+    s->res_count = o_count - s->res_off;
+    s->res_stres = o_stres - s->res_off;
+    s->res_fail = o_fail - s->res_off;
+    s->res_region_count = o_rcount - s->res_off;
+    at = s->res_off + s->res_bytes;
+    const size_t o_P = take((size_t) s->n_rows * sizeof(double));
+    s->p_bytes = (size_t) s->n_rows * sizeof(double);
+    const size_t o_rows = take((size_t) s->n_rows * sizeof(int32_t));
+    const size_t o_terms = take((size_t) s->n_totals * 2 * (size_t) s->term_stride * sizeof(double));
+    std::vector<size_t> o_E(nreg), o_S(nreg), o_B(nreg), o_F((size_t) s->n_run_tasks), o_sv((size_t) s->n_stitch);
+    size_t t = 0;
+    auto first_row = [](const PlainRegion &pr, size_t q) {   // of task q's store
+        return q == 0 ? 0 : pr.rg.windows[pr.cuts[q - 1]].T - pr.warm - 2;
+    };
+    auto slot_at = [](const PlainRegion &pr, int32_t d) -> int64_t { return (int64_t) pr.info[d].z + pr.info[d].x; };
+    for (size_t i = 0; i < nreg; ++i) {
+        const PlainRegion &pr = s->regs[i];
+        if (!pr.active) continue;
+        o_E[i] = take((size_t) pr.slots * 2 * sizeof(double));
+        o_S[i] = take((size_t) pr.slots * sizeof(double));
+        o_B[i] = take(s->expect ? (size_t) pr.slots * 3 * sizeof(double) : 1);
+        for (size_t q = 0; q <= pr.cuts.size(); ++q) {
+            const int32_t r0 = first_row(pr, q);
+            const int32_t r1 = q == pr.cuts.size() ? (int32_t) (pr.rg.lX + pr.rg.lY) : pr.rg.windows[pr.cuts[q] - 1].D;
+            o_F[t++] = take((size_t) (slot_at(pr, r1) + pr.info[r1].y - slot_at(pr, r0)) * 3 * sizeof(double));
+        }
+        for (size_t q = 0; q < pr.cuts.size(); ++q)
+            o_sv[(size_t) s->stitch_first[i] + q] = take(4 * 3 * sizeof(double) * (size_t) pr.stride);
+    }
+    const size_t o_out = take(s->expect ? 1 : (size_t) s->cap * sizeof(sa_aligned_pair));
+    s->dev_bytes = align256(at);
+    if (dev) {
+        s->d_regions = reinterpret_cast<Region64 *>(dev + o_regions);
+        s->d_models = reinterpret_cast<Model64 *>(dev + o_models);
+        s->d_tasks = reinterpret_cast<Region64 *>(dev + o_tasks);
+        s->d_stitch = reinterpret_cast<Stitch64 *>(dev + o_stitch);
+        s->d_windows = reinterpret_cast<Window64 *>(dev + o_windows);
+        s->d_totals = reinterpret_cast<Total64 *>(dev + o_totals);
+        s->d_chunk_region = reinterpret_cast<int32_t *>(dev + o_chreg);
+        s->d_chunk_d0 = reinterpret_cast<int32_t *>(dev + o_chd0);
+        s->d_task_of = reinterpret_cast<int32_t *>(dev + o_taskof);
+        s->d_row_base = reinterpret_cast<int64_t *>(dev + o_rowbase);
+        s->d_loglik = reinterpret_cast<double *>(dev + o_loglik);
+        s->d_status = reinterpret_cast<int32_t *>(dev + o_status);
+        s->d_count = reinterpret_cast<unsigned long long *>(dev + o_count);
+        s->d_stres = reinterpret_cast<Stitch64Res *>(dev + o_stres);
+        s->d_fail = reinterpret_cast<int32_t *>(dev + o_fail);
+        s->d_region_count = reinterpret_cast<int64_t *>(dev + o_rcount);
+        s->d_region_total = reinterpret_cast<int64_t *>(dev + o_rtotal);
+        s->d_P = reinterpret_cast<double *>(dev + o_P);
+        s->d_count_rows = reinterpret_cast<int32_t *>(dev + o_rows);
+        s->d_terms = reinterpret_cast<double *>(dev + o_terms);
+        s->d_out = reinterpret_cast<sa_aligned_pair *>(dev + o_out);
+    }
+    if (!host || !dev) return s->dev_bytes;
+    auto put = [&](size_t o, const void *src, size_t bytes) {
+        if (bytes) std::memcpy(host + o, src, bytes);
+    };
+    auto *regions = reinterpret_cast<Region64 *>(host + o_regions);
+    auto *tasks = reinterpret_cast<Region64 *>(host + o_tasks);
+    auto *stitches = reinterpret_cast<Stitch64 *>(host + o_stitch);
+    auto *windows = reinterpret_cast<Window64 *>(host + o_windows);
+    auto *totals = reinterpret_cast<Total64 *>(host + o_totals);
+    auto *chunk_region = reinterpret_cast<int32_t *>(host + o_chreg), *chunk_d0 = reinterpret_cast<int32_t *>(host + o_chd0);
+    auto *task_of = reinterpret_cast<int32_t *>(host + o_taskof);
+    auto *row_base = reinterpret_cast<int64_t *>(host + o_rowbase);
+    int64_t rows = 0, nw = 0, nt = 0, nc = 0, ntask = 0;
+    for (size_t i = 0; i < nreg; ++i) {
+        const PlainRegion &pr = s->regs[i];
+        put(off[i].info, pr.info.data(), pr.info.size() * sizeof(int4));
+        put(off[i].path, pr.path.data(), pr.path.size() * sizeof(Path64));
+        put(off[i].pid, pr.pid.data(), pr.pid.size() * sizeof(int32_t));
+        put(off[i].win, pr.rg.windows.data(), pr.rg.windows.size() * sizeof(Window));
+        Region64 r;
+        std::memset(&r, 0, sizeof(r));
+        r.lX = (int32_t) pr.rg.lX;
+        r.lY = (int32_t) pr.rg.lY;
+        r.n = (int32_t) (pr.rg.lX + pr.rg.lY);
+        r.n_windows = (int32_t) pr.rg.windows.size();
+        r.ragged_left = pr.rg.ragged_left;
+        r.ragged_right = pr.rg.ragged_right;
+        r.model = pr.model;
+        r.ev_base = pr.rg.y1;
+        r.x_base = pr.rg.x1;
+        r.threshold = s->threshold;
+        r.stride = pr.stride;
+        r.reader = pr.reader;
+        r.info = reinterpret_cast<const int4 *>(dev + off[i].info);
+        r.path = reinterpret_cast<const Path64 *>(dev + off[i].path);
+        r.pid = reinterpret_cast<const int32_t *>(dev + off[i].pid);
+        r.ev = reinterpret_cast<const double2 *>(dev + o_events) + pr.ev_off;
+        r.win = reinterpret_cast<const Window *>(dev + off[i].win);
+        r.E = reinterpret_cast<double *>(dev + o_E[i]);
+        r.S = reinterpret_cast<double *>(dev + o_S[i]);
+        r.B = reinterpret_cast<double *>(dev + o_B[i]);
+        r.s0 = 1;
+        r.w1 = r.n_windows;
+        r.tag = (int32_t) i;
+        r.st_in = r.st_out = -1;
+        r.win_base = nw;
+        r.P = s->d_P + rows;
+        r.loglik = s->d_loglik + i;
+        r.status = s->d_status + i;
+        row_base[i] = rows;
+        rows += r.n + 1;
+        regions[i] = r;
+        if (!pr.active) continue;
+        for (int32_t d0 = 0; d0 <= r.n; d0 += 32, ++nc) {
+            chunk_region[nc] = (int32_t) i;
+            chunk_d0[nc] = d0;
+        }
+        for (size_t q = 0; q <= pr.cuts.size(); ++q, ++ntask) {
+            Region64 k = r;
+            k.F = reinterpret_cast<double *>(dev + o_F[(size_t) ntask]) - 3 * slot_at(pr, first_row(pr, q));
+            k.w0 = q == 0 ? 0 : pr.cuts[q - 1];
+            k.w1 = q == pr.cuts.size() ? r.n_windows : pr.cuts[q];
+            k.s0 = q == 0 ? 1 : pr.rg.windows[pr.cuts[q - 1]].T - pr.warm;
+            k.st_in = q == 0 ? -1 : (int32_t) (s->stitch_first[i] + (int64_t) q - 1);
+            k.st_out = q == pr.cuts.size() ? -1 : (int32_t) (s->stitch_first[i] + (int64_t) q);
+            tasks[ntask] = k;
+            for (int32_t w = k.w0; w < k.w1; ++w, ++nw) {
+                const Window &W = pr.rg.windows[w];
+                windows[nw] = Window64{(int32_t) ntask, w, (int32_t) nt, 0};
+                task_of[nw] = (int32_t) ntask;
+                for (int32_t d = W.from; d > W.T; d -= 10)
+                    totals[nt++] = Total64{(int32_t) i, d, d < W.D ? 1 : 0, d == r.n ? 1 : 0};
+            }
+        }
+        for (size_t q = 0; q < pr.cuts.size(); ++q) {
+            Stitch64 st;
+            std::memset(&st, 0, sizeof(st));
+            st.vals = reinterpret_cast<double *>(dev + o_sv[(size_t) s->stitch_first[i] + q]);
+            st.b = pr.rg.windows[pr.cuts[q]].T;
+            st.region = (int32_t) i;
+            st.stride = pr.stride;
+            stitches[(size_t) s->stitch_first[i] + q] = st;
+        }
+    }
+    put_models(s, host + o_models);
+    put(o_events, s->events.data(), s->events.size() * sizeof(double2));
+    return s->dev_bytes;
+}
+
+size_t plain_layout(PlainSet *s, unsigned char *host, unsigned char *dev) {
+    return s->resident ? resident_layout(s, host, dev) : ring_layout(s, host, dev);
 }
 
 }  // namespace
@@ -995,6 +1248,15 @@ void plan_region(const PathTable &pt, int32_t asz, int64_t kpow, PlainRegion &pr
     }
     pr.max_paths = 1;
     for (int64_t x = 0; x <= rg.lX; ++x) pr.max_paths = std::max(pr.max_paths, pr.pfirst[x + 1] - pr.pfirst[x]);
+    // paths of any three consecutive anti-diagonals, first to last
+    int32_t lo3[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, hi3[3] = {-1, -1, -1};
+    pr.slots = 0;
+    for (int32_t d = 0; d <= n; ++d) {
+        lo3[d % 3] = pr.pfirst[(d + rg.xmy_l[d]) / 2];
+        hi3[d % 3] = pr.pfirst[(d + rg.xmy_r[d]) / 2 + 1] - 1;
+        pr.slots += hi3[d % 3] - lo3[d % 3] + 1;
+        pr.span = std::max(pr.span, std::max({hi3[0], hi3[1], hi3[2]}) - std::min({lo3[0], lo3[1], lo3[2]}) + 1);
+    }
     int32_t span = 0;
     for (const Window &w : rg.windows) span = std::max(span, w.D - w.T + 1);
     pr.ring = std::max(3, span) + 1;
@@ -1007,10 +1269,124 @@ void plan_region(const PathTable &pt, int32_t asz, int64_t kpow, PlainRegion &pr
 
 }  // namespace
 
+// Resident route of a region: per anti-diagonal its paths, slots and window; per path its neighbours.
+void plan_resident(const sa_state_machine *sm, PlainRegion &pr) {
+    const Region &rg = pr.rg;
+    const int32_t n = (int32_t) (rg.lX + rg.lY);
+    pr.info.resize((size_t) n + 1);
+    int64_t at = 0;
+    size_t w = 0;
+    for (int32_t d = 0; d <= n; ++d) {
+        while (w + 1 < rg.windows.size() && d > rg.windows[w].from) ++w;
+        const int32_t lo = pr.pfirst[(d + rg.xmy_l[d]) / 2], cnt = pr.pfirst[(d + rg.xmy_r[d]) / 2 + 1] - lo;
+        pr.info[d] = make_int4(lo, cnt, (int32_t) (at - lo), (int32_t) w);
+        at += cnt;
+    }
+    pr.path.assign(pr.pid.size(), Path64{});
+    for (int64_t x = 0; x <= rg.lX; ++x) {
+        for (int32_t q = pr.pfirst[x]; q < pr.pfirst[x + 1]; ++q) {
+            Path64 &P = pr.path[q];
+            const int32_t kid = pr.pid[q];
+            P.col = (int32_t) x;
+            P.gapx = sm->emission == SA_EMIT_HDP ? kLogPointOne : kid < 0 ? -INFINITY : sm->gapx[kid];
+            P.pred = P.succ = q;
+            auto legal = [&](int32_t a, int32_t b) { return pr.pid[a] < 0 || pr.pid[b] < 0 || pr.psuf[a] == pr.ppre[b]; };
+            if (x > 0) {
+                int32_t last = -1;
+                for (int32_t a = pr.pfirst[x - 1]; a < pr.pfirst[x]; ++a) {
+                    if (!legal(a, q)) continue;
+                    if (P.pred_n == 0) P.pred = a;
+                    else if (P.pred_n == 1) P.pred_step = a - last;
+                    else if (a - last != P.pred_step) pr.regular = false;
+                    ++P.pred_n;
+                    last = a;
+                }
+            }
+            if (x < rg.lX) {
+                int32_t last = -1;
+                for (int32_t b = pr.pfirst[x + 1]; b < pr.pfirst[x + 2]; ++b) {
+                    if (!legal(q, b)) continue;
+                    if (P.succ_n == 0) P.succ = b;
+                    else if (b != last + 1) pr.regular = false;
+                    ++P.succ_n;
+                    last = b;
+                }
+            }
+        }
+    }
+}
+
+// Forward segments (alignment runs, and expectations on the resident route): long regions cut at
+// window starts like the batched form's, the automatic cap from twice the set's anti-diagonals per
+// CTA slot (four plain CTAs per SM)
+void plan_segments(PlainSet *s, bool segments) {
+    int32_t policy = -1, warm0 = 1024;
+    if (segments) segment_policy(policy, warm0);
+    int64_t target = policy;
+    if (segments && policy == 0) {
+        int64_t diags = 0;
+        for (const PlainRegion &pr : s->regs) diags += pr.rg.lX + pr.rg.lY + 1;
+        int sms = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) != cudaSuccess) {
+            cudaGetLastError();
+            sms = 0;
+        }
+        if (sms <= 0) sms = 148;
+        target = std::max<int64_t>(segment_min(), 2 * diags / ((int64_t) sms * 4));
+    }
+    s->n_tasks = s->n_stitch = 0;
+    s->task_first.assign(s->regs.size(), 0);
+    s->stitch_first.assign(s->regs.size(), 0);
+    for (size_t i = 0; i < s->regs.size(); ++i) {
+        PlainRegion &pr = s->regs[i];
+        pr.cuts.clear();
+        pr.warm = 0;
+        if (segments && policy >= 0) {
+            const int32_t wr = segment_warm(pr.rg, warm0);
+            segment_cuts(pr.rg, target, wr, pr.cuts);
+            pr.warm = wr;
+        }
+        s->task_first[i] = s->n_tasks;
+        s->stitch_first[i] = s->n_stitch;
+        s->n_tasks += 1 + (int64_t) pr.cuts.size();
+        s->n_stitch += (int64_t) pr.cuts.size();
+    }
+}
+
+// The resident route for sets whose bands fit its threads (the paths of three consecutive
+// anti-diagonals, and a path's neighbours beyond them, on threads of their own) and, in plain_create,
+// whose store fits kResidentBytes.  Both sides measured on B200, whole call, rings
+// then resident: one 1 kb read 14.0 and 2.1 ms, one 3 kb read with sites 29.4 and 3.8, ten reads of
+// 1 to 10 kb with sites 48 and 5.6, the expectations of six reads of 1 to 5 kb 222 and 6.0.
+// The rings stay for wider bands, for larger sets, and for regions re-run whole.
+void plan_route(PlainSet *s, const sa_read *reads, size_t max_bytes) {
+    int32_t span = 0, paths = 1;
+    int64_t slots = 0;
+    for (const PlainRegion &pr : s->regs) {
+        span = std::max(span, pr.span + 2 * pr.max_paths);
+        paths = std::max(paths, pr.max_paths);
+        slots += pr.slots;
+        if (pr.slots > INT32_MAX / 4) return;
+    }
+    s->multi = paths > 1;
+    s->nt = 0;
+    for (int nt : kResidentThreads)
+        if (!s->nt && span <= nt) s->nt = nt;
+    if (!s->nt || (s->multi && s->nt > 256)) return;
+    if ((size_t) slots * 48 > std::min(kResidentBytes, max_bytes)) return;   // not worth planning in full
+    s->finite_sx = false;
+    for (PlainRegion &pr : s->regs) {
+        plan_resident(reads[pr.read].sm, pr);
+        if (!pr.regular) return;
+        s->finite_sx = s->finite_sx || reads[pr.read].sm->t[T_SX] > -INFINITY;
+    }
+    s->resident = true;
+}
+
 // Plans a set of reads for the plain form.  Reads that fail planning keep their status and get no
 // regions.  `max_bytes` bounds the device block (SA_E_CAPACITY above it).
 sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p, size_t max_bytes, PlainSet **out,
-                       bool segments) {
+                       bool segments, bool expect, bool rings) {
     *out = nullptr;
     auto *s = new (std::nothrow) PlainSet();
     if (!s) return SA_E_NOMEM;
@@ -1075,39 +1451,17 @@ sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p
     }
     s->device = device < 0 ? 0 : device;
     s->cap = cap;
-    // Forward segments (alignment runs): long regions cut at window starts like the batched form's,
-    // the automatic cap from twice the set's anti-diagonals per CTA slot (four plain CTAs per SM)
-    int32_t policy = -1, warm0 = 1024;
-    if (segments) segment_policy(policy, warm0);
-    int64_t target = policy;
-    if (segments && policy == 0) {
-        int64_t diags = 0;
-        for (const PlainRegion &pr : s->regs) diags += pr.rg.lX + pr.rg.lY + 1;
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) != cudaSuccess) {
-            cudaGetLastError();
-            sms = 0;
-        }
-        if (sms <= 0) sms = 148;
-        target = std::max<int64_t>(segment_min(), 2 * diags / ((int64_t) sms * 4));
-    }
-    s->task_first.assign(s->regs.size(), 0);
-    s->stitch_first.assign(s->regs.size(), 0);
-    for (size_t i = 0; i < s->regs.size(); ++i) {
-        PlainRegion &pr = s->regs[i];
-        pr.cuts.clear();
-        pr.warm = 0;
-        if (segments && policy >= 0) {
-            const int32_t wr = segment_warm(pr.rg, warm0);
-            segment_cuts(pr.rg, target, wr, pr.cuts);
-            pr.warm = wr;
-        }
-        s->task_first[i] = s->n_tasks;
-        s->stitch_first[i] = s->n_stitch;
-        s->n_tasks += 1 + (int64_t) pr.cuts.size();
-        s->n_stitch += (int64_t) pr.cuts.size();
-    }
+    s->expect = expect;
+    if (!rings) plan_route(s, reads, max_bytes);
+    segments = segments || (expect && s->resident);
+    plan_segments(s, segments);
     plain_layout(s, nullptr, nullptr);
+    if (s->resident && s->dev_bytes > std::min(kResidentBytes, max_bytes)) {
+        // more than the store may hold: the rings, and whole regions where there are no pairs
+        s->resident = false;
+        plan_segments(s, segments && !expect);
+        plain_layout(s, nullptr, nullptr);
+    }
     if (s->dev_bytes > max_bytes) {
         delete s;
         return SA_E_CAPACITY;
@@ -1128,11 +1482,71 @@ sa_status plain_upload(PlainSet *s, cudaStream_t stream) {
     return SA_OK;
 }
 
-// One launch: every region one CTA.
+namespace {
+
+template <int NT, bool kMulti, bool kSX>
+bool sweeps64(PlainSet *s, const SetOut &O, cudaStream_t stream) {
+    constexpr size_t fwd = sizeof(Forward64Shared<NT, kMulti>), bwd = sizeof(Backward64Shared<NT, kMulti>);
+    auto f = forward64<NT, kMulti, kSX>;
+    auto b = backward64<NT, kMulti, kSX>;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd) != cudaSuccess ||
+        cudaFuncSetAttribute(b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd) != cudaSuccess)
+        return false;
+    f<<<(unsigned) s->n_run_tasks, NT, fwd, stream>>>(s->d_models, s->d_tasks, O);
+    b<<<(unsigned) s->n_windows, NT, bwd, stream>>>(s->d_models, s->d_tasks, s->d_windows, s->d_terms, s->term_stride,
+                                                   s->expect ? 1 : 0);
+    return cudaGetLastError() == cudaSuccess;
+}
+
+template <int NT, bool kMulti>
+bool sweeps64(PlainSet *s, const SetOut &O, cudaStream_t stream) {
+    return s->finite_sx ? sweeps64<NT, kMulti, true>(s, O, stream) : sweeps64<NT, kMulti, false>(s, O, stream);
+}
+
+// emissions, sweeps and total probabilities of the resident route
+sa_status resident_sweeps(PlainSet *s, const SetOut &O, cudaStream_t stream) {
+    emit64<<<(unsigned) s->n_chunks, 256, 0, stream>>>(s->d_models, s->d_regions, s->d_chunk_region, s->d_chunk_d0);
+    bool ok = false;
+    if (s->multi) ok = s->nt == 128 ? sweeps64<128, true>(s, O, stream) : sweeps64<256, true>(s, O, stream);
+    else if (s->nt == 128) ok = sweeps64<128, false>(s, O, stream);
+    else if (s->nt == 256) ok = sweeps64<256, false>(s, O, stream);
+    else ok = sweeps64<512, false>(s, O, stream);
+    if (!ok) return SA_E_CUDA;
+    totals64<<<(unsigned) ((s->n_totals + 63) / 64), 64, 0, stream>>>(s->d_regions, s->d_totals, s->n_totals, s->d_terms,
+                                                                     s->term_stride, s->multi ? 1 : 0);
+    count_launch(4);
+    return cudaGetLastError() == cudaSuccess ? SA_OK : SA_E_CUDA;
+}
+
+// counted, scanned and written in the reference's order: pairs, or assignments (first: the groups)
+template <bool kAssign>
+sa_status resident_outputs(PlainSet *s, const ExpectOut *reads, const int32_t *first, cudaStream_t stream) {
+    Output64 O;
+    std::memset(&O, 0, sizeof(O));
+    O.out = s->d_out;
+    O.reads = reads;
+    O.count = s->d_count_rows;
+    O.region_total = s->d_region_total;
+    O.cap = s->cap;
+    O.threshold = s->threshold;
+    const unsigned nc = (unsigned) s->n_chunks, nr = (unsigned) s->regs.size();
+    // regions that do not run have no counts
+    if (cudaMemsetAsync(s->d_count_rows, 0, (size_t) s->n_rows * sizeof(int32_t), stream) != cudaSuccess) return SA_E_CUDA;
+    outputs64<kAssign, false><<<nc, 256, 0, stream>>>(s->d_regions, s->d_chunk_region, s->d_chunk_d0, s->d_row_base, O);
+    scan64<<<nr, 1024, 0, stream>>>(s->d_regions, s->d_row_base, O);
+    place64<<<1, 32, 0, stream>>>((int64_t) nr, s->d_region_total, s->d_region_count, s->d_count, first);
+    outputs64<kAssign, true><<<nc, 256, 0, stream>>>(s->d_regions, s->d_chunk_region, s->d_chunk_d0, s->d_row_base, O);
+    count_launch(4);
+    return cudaGetLastError() == cudaSuccess ? SA_OK : SA_E_CUDA;
+}
+
+}  // namespace
+
+// The set's launches: one CTA per task and everything in it, or the resident kernels.
 sa_status plain_run(PlainSet *s, cudaStream_t stream) {
     auto *dev = static_cast<unsigned char *>(s->dev.ptr);
     if (cudaMemsetAsync(dev + s->res_off, 0, s->res_bytes, stream) != cudaSuccess ||
-        cudaMemsetAsync(s->d_P, 0, std::max<size_t>(s->p_bytes, 1), stream) != cudaSuccess)
+        (!s->resident && cudaMemsetAsync(s->d_P, 0, std::max<size_t>(s->p_bytes, 1), stream) != cudaSuccess))
         return SA_E_CUDA;
     if (s->regs.empty()) return SA_OK;
     SetOut O;
@@ -1146,10 +1560,116 @@ sa_status plain_run(PlainSet *s, cudaStream_t stream) {
     O.fail = s->d_fail;
     O.stitch_tol = s->stitch_tol;
     s->n_redone = 0;
+    if (s->resident) {
+        const sa_status st = resident_sweeps(s, O, stream);
+        return st ? st : resident_outputs<false>(s, nullptr, nullptr, stream);
+    }
     region_kernel<<<(unsigned) s->n_tasks, 128, 0, stream>>>(s->d_models, s->d_tasks, O, nullptr);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? SA_OK : SA_E_CUDA;
 }
+
+namespace {
+
+// Results of the resident route: the pairs lie in order, region after region; a region whose stitch
+// disagreed runs again whole, in the rings of a set of its own.
+sa_status resident_download(PlainSet *s, cudaStream_t stream) {
+    const auto *res = static_cast<const unsigned char *>(s->host_res.ptr);
+    const auto *loglik = reinterpret_cast<const double *>(res);
+    const auto *rstatus = reinterpret_cast<const int32_t *>(res + s->res_status);
+    const auto *stres = reinterpret_cast<const Stitch64Res *>(res + s->res_stres);
+    const auto *fail = reinterpret_cast<const int32_t *>(res + s->res_fail);
+    const auto *counts = reinterpret_cast<const int64_t *>(res + s->res_region_count);
+    const auto all = *reinterpret_cast<const unsigned long long *>(res + s->res_count);
+    const size_t npairs = (size_t) std::min<unsigned long long>(all, (unsigned long long) s->cap);
+    const size_t nreg = s->regs.size();
+    const size_t bytes = std::max<size_t>(npairs, 1) * sizeof(sa_aligned_pair);
+    if (s->host_pairs.bytes < bytes) {
+        mem_put(s->host_pairs);
+        const sa_status st = mem_get(MemKind::Pinned, s->device, bytes, s->host_pairs);
+        if (st) return st;
+    }
+    auto *pairs = static_cast<sa_aligned_pair *>(s->host_pairs.ptr);
+    if (npairs && (cudaMemcpyAsync(pairs, s->d_out, npairs * sizeof(sa_aligned_pair), cudaMemcpyDeviceToHost, stream) !=
+                       cudaSuccess ||
+                   cudaStreamSynchronize(stream) != cudaSuccess))
+        return SA_E_CUDA;
+    // the regions that run again
+    PlainSet again;
+    std::vector<int64_t> at(nreg, -1);
+    for (size_t i = 0; i < nreg; ++i) {
+        if (!fail[i]) continue;
+        at[i] = (int64_t) again.regs.size();
+        PlainRegion pr = s->regs[i];
+        pr.read = (int32_t) again.regs.size();
+        pr.cuts.clear();
+        again.cap += 4 * (pr.rg.lX + pr.rg.lY + 1) * std::min<int64_t>(pr.max_paths, 4) + 256;
+        again.regs.push_back(std::move(pr));
+    }
+    if (!again.regs.empty()) {
+        const int64_t k = (int64_t) again.regs.size();
+        again.device = s->device;
+        again.models = s->models;
+        again.threshold = s->threshold;
+        again.events = s->events;
+        again.n_tasks = k;
+        again.read_status.assign(k, SA_OK);
+        again.read_count.assign(k, 1);
+        for (int64_t i = 0; i < k; ++i) {
+            again.read_first.push_back(i);
+            again.task_first.push_back(i);
+            again.stitch_first.push_back(0);
+        }
+        plain_layout(&again, nullptr, nullptr);
+        sa_status st = plain_upload(&again, stream);
+        if (!st) st = plain_run(&again, stream);
+        if (!st) st = plain_download(&again, stream);
+        if (st) return st;
+        s->n_redone = k;
+    }
+    const int64_t n_reads = (int64_t) s->read_status.size();
+    s->pairs.assign(n_reads, {});
+    s->spans.assign(n_reads, PlainPairs{});
+    s->ll.assign(n_reads, 0.0);
+    s->status = s->read_status;
+    size_t from = 0;
+    for (int64_t r = 0; r < n_reads; ++r) {
+        bool mixed = false;
+        const size_t first = from;
+        for (int64_t ri = s->read_first[r]; ri < s->read_first[r] + s->read_count[r]; ++ri) {
+            mixed = mixed || at[ri] >= 0;
+            from = std::min(npairs, from + (size_t) counts[ri]);
+            if (at[ri] >= 0) {
+                if (again.status[at[ri]] && !s->status[r]) s->status[r] = again.status[at[ri]];
+                s->ll[r] += again.ll[at[ri]];
+                continue;
+            }
+            if (rstatus[ri] && !s->status[r]) s->status[r] = rstatus[ri];
+            s->ll[r] += loglik[ri];
+            // the last segment's total is in its own frame: the stitches' constants bring it back
+            for (size_t q = 0; q < s->regs[ri].cuts.size(); ++q) s->ll[r] += stres[s->stitch_first[ri] + q].delta;
+        }
+        if (all > (unsigned long long) s->cap && s->read_count[r] && !s->status[r]) s->status[r] = SA_E_OUTPUT;
+        s->spans[r] = PlainPairs{pairs + first, from - first};
+        if (!mixed) continue;
+        auto &v = s->pairs[r];
+        size_t k = first;
+        for (int64_t ri = s->read_first[r]; ri < s->read_first[r] + s->read_count[r]; ++ri) {
+            const size_t n = std::min((size_t) counts[ri], npairs - k);
+            if (at[ri] >= 0) {
+                const PlainPairs g = plain_pairs(&again, at[ri]);
+                v.insert(v.end(), g.p, g.p + g.n);
+            } else {
+                v.insert(v.end(), pairs + k, pairs + k + n);
+            }
+            k += n;
+        }
+        s->spans[r] = PlainPairs{v.data(), v.size()};
+    }
+    return SA_OK;
+}
+
+}  // namespace
 
 // Results to the host (synchronises `stream`): per read its pairs in the reference's emission
 // order, coordinates shifted back from the regions (alignedPairCoordinateCorrectionFn,
@@ -1159,6 +1679,7 @@ sa_status plain_download(PlainSet *s, cudaStream_t stream) {
                         cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
         cudaStreamSynchronize(stream) != cudaSuccess)
         return SA_E_CUDA;
+    if (s->resident) return resident_download(s, stream);
     const auto *res = static_cast<const unsigned char *>(s->host_res.ptr);
     const auto *loglik = reinterpret_cast<const double *>(res);
     const auto *rstatus = reinterpret_cast<const int32_t *>(res + s->res_status);
@@ -1251,6 +1772,8 @@ sa_status plain_download(PlainSet *s, cudaStream_t stream) {
         s->pairs[r].resize(v.size());
         for (size_t i = 0; i < v.size(); ++i) s->pairs[r][i] = v[i].pair;
     }
+    s->spans.assign(n_reads, PlainPairs{});
+    for (int64_t r = 0; r < n_reads; ++r) s->spans[r] = PlainPairs{s->pairs[r].data(), s->pairs[r].size()};
     return SA_OK;
 }
 
@@ -1258,7 +1781,7 @@ int plain_device(const PlainSet *s) { return s->device; }
 int64_t plain_cells(const PlainSet *s) { return s->cells; }
 size_t plain_in_bytes(const PlainSet *s) { return s->in_bytes; }
 sa_status plain_read_status(const PlainSet *s, int64_t r) { return (sa_status) s->status[r]; }
-const std::vector<sa_aligned_pair> &plain_pairs(const PlainSet *s, int64_t r) { return s->pairs[r]; }
+PlainPairs plain_pairs(const PlainSet *s, int64_t r) { return s->spans[r]; }
 double plain_log_likelihood(const PlainSet *s, int64_t r) { return s->ll[r]; }
 void plain_destroy(PlainSet *s) { delete s; }
 void plain_set_stitch_tolerance(PlainSet *s, double scale) { s->stitch_tol = scale; }
@@ -1332,25 +1855,82 @@ extern "C" sa_status sa_getAlignedPairsUsingAnchors(const sa_state_machine *sm_c
         plain_destroy(s);
         return st;
     }
-    const auto &v = plain_pairs(s, 0);
-    auto *outp = (sa_aligned_pair *) std::malloc(std::max<size_t>(1, v.size()) * sizeof(sa_aligned_pair));
+    const PlainPairs v = plain_pairs(s, 0);
+    auto *outp = (sa_aligned_pair *) std::malloc(std::max<size_t>(1, v.n) * sizeof(sa_aligned_pair));
     if (!outp) {
         plain_destroy(s);
         return SA_E_NOMEM;
     }
-    if (!v.empty()) std::memcpy(outp, v.data(), v.size() * sizeof(sa_aligned_pair));
+    if (v.n) std::memcpy(outp, v.p, v.n * sizeof(sa_aligned_pair));
     *pairs_out = outp;
-    *n_pairs_out = (int64_t) v.size();
+    *n_pairs_out = (int64_t) v.n;
     if (log_likelihood) *log_likelihood = plain_log_likelihood(s, 0);
     plain_destroy(s);
     return SA_OK;
 }
 
-// Expectations of many reads in one launch: CTA i walks read i's regions in order into ex[i]'s
+// What the expectations' kernels of the resident route read beside the set: each running read's
+// k-mers with their columns, in the reference's order of regions and columns, and its ranges.
+struct ExpectPlan {
+    std::vector<Kmer64> kmers;
+    std::vector<Column64> cols;
+    std::vector<int64_t> read_chunk, read_task;   // per running read its first chunk and task, and the ends
+    std::vector<int32_t> first;                   // per region the first region of its read
+    bool hdp = false;
+};
+
+static void plan_expectations(const PlainSet *s, const sa_read *reads, const std::vector<int64_t> &run, ExpectPlan &E) {
+    E.first.resize(s->regs.size());
+    for (size_t r = 0; r < s->regs.size(); ++r) E.first[r] = (int32_t) s->read_first[s->regs[r].read];
+    int64_t chunks = 0, tasks = 0;
+    std::vector<int32_t> at, dlo, dhi;
+    for (size_t j = 0; j < run.size(); ++j) {
+        const int64_t i = run[j];
+        E.read_chunk.push_back(chunks);
+        E.read_task.push_back(tasks);
+        const int64_t r0 = s->read_first[i], r1 = r0 + s->read_count[i];
+        for (int64_t r = r0; r < r1; ++r) {
+            chunks += (s->regs[r].rg.lX + s->regs[r].rg.lY + 32) / 32;
+            tasks += 1 + (int64_t) s->regs[r].cuts.size();
+        }
+        if (reads[i].sm->emission == SA_EMIT_HDP) {
+            E.hdp = true;
+            continue;
+        }
+        // columns by k-mer (counted), each k-mer's in order of region and column
+        at.assign((size_t) reads[i].sm->n_kmers + 1, 0);
+        for (int64_t r = r0; r < r1; ++r)
+            for (int64_t x = 1; x <= s->regs[r].rg.lX; ++x) ++at[s->regs[r].pid[x] + 1];
+        const int32_t base = (int32_t) E.cols.size();
+        for (size_t k = 0; k + 1 < at.size(); ++k) {
+            if (at[k + 1]) E.kmers.push_back(Kmer64{(int32_t) j, (int32_t) k, base + at[k], at[k + 1]});
+            at[k + 1] += at[k];
+        }
+        E.cols.resize((size_t) base + at.back());
+        for (int64_t r = r0; r < r1; ++r) {
+            const PlainRegion &pr = s->regs[r];
+            const int32_t n = (int32_t) (pr.rg.lX + pr.rg.lY), lX = (int32_t) pr.rg.lX;
+            // anti-diagonals that may hold a column's cells (ascending in the column both ways)
+            dlo.assign(lX + 1, n + 1);
+            dhi.assign(lX + 1, -1);
+            for (int32_t d = 0, x = 0; d <= n; ++d)
+                for (; x <= lX && x < pr.info[d].x + pr.info[d].y; ++x) dlo[x] = d;
+            for (int32_t d = n, x = lX; d >= 0; --d)
+                for (; x >= 0 && x >= pr.info[d].x; --x) dhi[x] = d;
+            for (int32_t x = 1; x <= lX; ++x)
+                E.cols[base + at[pr.pid[x]]++] = Column64{(int32_t) r, x, dlo[x], dhi[x]};
+        }
+    }
+    E.read_chunk.push_back(chunks);
+    E.read_task.push_back(tasks);
+}
+
+// Expectations of many reads: on the resident route every read's sweeps side by side and its
+// accumulators filled from their posteriors; else CTA i walks read i's regions in order into ex[i]'s
 // accumulators (the single-read call is this with one read).  Per read on the device: the
 // anti-diagonal scratch and cell masks, the accumulators, and (HDP machines) the assignment lists.
 static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_params &p, sa_expectations *ex,
-                                    int32_t *read_status) {
+                                    int32_t *read_status, bool rings = false) {
     for (int64_t i = 0; i < n; ++i) {
         read_status[i] = SA_OK;
         const sa_state_machine *sm = reads[i].sm;
@@ -1364,7 +1944,7 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
         }
     }
     PlainSet *s = nullptr;
-    sa_status st = plain_create(reads, n, p, kExpectMaxBytes, &s);
+    sa_status st = plain_create(reads, n, p, kExpectMaxBytes, &s, false, true, rings);
     if (st) return st;
     std::vector<int32_t> width(n, 1);
     for (int64_t i = 0; i < n; ++i) {
@@ -1392,7 +1972,18 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
         plain_destroy(s);
         return st;
     }
-    // one device block: per running read its buffers, then the ExpectOut array
+    ExpectPlan E;
+    if (s->resident) {
+        for (PlainRegion &pr : s->regs) pr.active = false;
+        for (size_t j = 0; j < run.size(); ++j)
+            for (int64_t r = s->read_first[run[j]]; r < s->read_first[run[j]] + s->read_count[run[j]]; ++r) {
+                s->regs[r].active = true;
+                s->regs[r].reader = (int32_t) j;
+            }
+        plain_layout(s, nullptr, nullptr);
+        plan_expectations(s, reads, run, E);
+    }
+    // one device block: per running read its buffers, then the ExpectOut array and the plan
     struct Off { size_t scratch, mask, acc, ee, po, ob, ak, ae, na; int64_t nk, cap; bool hdp; };
     auto up = [](size_t v) { return (v + 255) & ~(size_t) 255; };
     std::vector<Off> off(run.size());
@@ -1416,7 +2007,15 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
     }
     const size_t o_xs = total;
     total += up(sizeof(ExpectOut) * run.size());
-    std::vector<unsigned char> host(total, 0);
+    const size_t o_kmers = total; total += up(sizeof(Kmer64) * E.kmers.size());
+    const size_t o_cols = total; total += up(sizeof(Column64) * E.cols.size());
+    const size_t o_rchunk = total; total += up(sizeof(int64_t) * E.read_chunk.size());
+    const size_t o_rtask = total; total += up(sizeof(int64_t) * E.read_task.size());
+    const size_t o_first = total; total += up(sizeof(int32_t) * E.first.size());
+    const size_t staged = total;
+    const size_t o_partial = total; total += s->resident ? up(sizeof(double) * 9 * (size_t) s->n_chunks) : 0;
+    std::vector<unsigned char> host(staged, 0);
+    std::vector<int64_t> again;
     MemBlock blk;
     st = plain_upload(s, nullptr);
     if (!st) st = mem_get(MemKind::Device, s->device, total, blk);
@@ -1449,14 +2048,49 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
             X.n_assign = reinterpret_cast<int64_t *>(d + o.na);
             X.assign_cap = o.cap;
         }
+        auto put = [&](size_t o, const void *src, size_t bytes) {
+            if (bytes) std::memcpy(host.data() + o, src, bytes);
+        };
+        put(o_kmers, E.kmers.data(), sizeof(Kmer64) * E.kmers.size());
+        put(o_cols, E.cols.data(), sizeof(Column64) * E.cols.size());
+        put(o_rchunk, E.read_chunk.data(), sizeof(int64_t) * E.read_chunk.size());
+        put(o_rtask, E.read_task.data(), sizeof(int64_t) * E.read_task.size());
+        put(o_first, E.first.data(), sizeof(int32_t) * E.first.size());
         SetOut O;
         std::memset(&O, 0, sizeof(O));
         auto *dev = static_cast<unsigned char *>(s->dev.ptr);
-        if (cudaMemcpy(d, host.data(), total, cudaMemcpyHostToDevice) != cudaSuccess ||
+        if (cudaMemcpy(d, host.data(), staged, cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemsetAsync(dev + s->res_off, 0, s->res_bytes, nullptr) != cudaSuccess ||
-            cudaMemsetAsync(s->d_P, 0, std::max<size_t>(s->p_bytes, 1), nullptr) != cudaSuccess)
+            (!s->resident && cudaMemsetAsync(s->d_P, 0, std::max<size_t>(s->p_bytes, 1), nullptr) != cudaSuccess))
             st = SA_E_CUDA;
-        if (!st) {
+        const auto *X = reinterpret_cast<const ExpectOut *>(d + o_xs);
+        if (!st && s->resident) {
+            O.stitch = s->d_stitch;
+            O.stres = s->d_stres;
+            O.fail = s->d_fail;
+            O.stitch_tol = s->stitch_tol;
+            auto *partial = reinterpret_cast<double *>(d + o_partial);
+            st = resident_sweeps(s, O, nullptr);
+            if (!st) {
+                transitions64<<<(unsigned) s->n_chunks, 256>>>(s->d_models, s->d_tasks, s->d_task_of, s->d_chunk_region,
+                                                              s->d_chunk_d0, s->d_regions, partial);
+                if (!E.kmers.empty())
+                    kmers64<<<(unsigned) ((E.kmers.size() + 3) / 4), 128>>>(
+                        s->d_models, s->d_regions, reinterpret_cast<const Kmer64 *>(d + o_kmers), (int64_t) E.kmers.size(),
+                        reinterpret_cast<const Column64 *>(d + o_cols), X);
+                finish64<<<(unsigned) run.size(), 256>>>(X, reinterpret_cast<const int64_t *>(d + o_rchunk), partial,
+                                                        s->d_tasks, reinterpret_cast<const int64_t *>(d + o_rtask),
+                                                        s->d_stres);
+                count_launch(E.kmers.empty() ? 2 : 3);
+                if (cudaGetLastError() != cudaSuccess) st = SA_E_CUDA;
+            }
+            if (!st && E.hdp)
+                st = resident_outputs<true>(s, X, reinterpret_cast<const int32_t *>(d + o_first), nullptr);
+            if (!st && (cudaMemcpyAsync(s->host_res.ptr, dev + s->res_off, s->res_bytes, cudaMemcpyDeviceToHost, nullptr) !=
+                            cudaSuccess ||
+                        cudaDeviceSynchronize() != cudaSuccess))
+                st = SA_E_CUDA;
+        } else if (!st) {
             region_kernel<<<(unsigned) run.size(), 128>>>(s->d_models, s->d_regions, O,
                                                         reinterpret_cast<const ExpectOut *>(d + o_xs));
             count_launch();
@@ -1464,16 +2098,28 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
         }
         if (!st && cudaMemcpy(host.data(), d, o_xs, cudaMemcpyDeviceToHost) != cudaSuccess) st = SA_E_CUDA;
         if (!st) {
+            const auto *res = static_cast<const unsigned char *>(s->host_res.ptr);
+            const auto *fail = reinterpret_cast<const int32_t *>(res + s->res_fail);
+            const auto *counts = reinterpret_cast<const int64_t *>(res + s->res_region_count);
             for (size_t j = 0; j < run.size(); ++j) {
                 const int64_t i = run[j];
                 const Off &o = off[j];
+                bool agreed = true;   // a read with a disagreeing stitch: again, whole, from its accumulators
+                for (int64_t r = s->read_first[i]; s->resident && r < s->read_first[i] + s->read_count[i]; ++r)
+                    agreed = agreed && !fail[r];
+                if (!agreed) {
+                    again.push_back(i);
+                    continue;
+                }
                 const auto *acc = reinterpret_cast<const double *>(host.data() + o.acc);
                 ex[i].likelihood = acc[0];
                 for (int k = 0; k < 9; ++k) ex[i].transitions[k] = acc[k + 1];
                 std::memcpy(ex[i].event_expectations, host.data() + o.ee, sizeof(double) * 2 * (size_t) o.nk);
                 std::memcpy(ex[i].posteriors, host.data() + o.po, sizeof(double) * (size_t) o.nk);
                 std::memcpy(ex[i].observed, host.data() + o.ob, (size_t) o.nk);
-                const int64_t na = *reinterpret_cast<const int64_t *>(host.data() + o.na);
+                int64_t na = *reinterpret_cast<const int64_t *>(host.data() + o.na);
+                if (s->resident && o.hdp)
+                    for (int64_t r = s->read_first[i]; r < s->read_first[i] + s->read_count[i]; ++r) na += counts[r];
                 ex[i].n_assignments = na;
                 if (o.hdp) {
                     const int64_t got = std::min(na, o.cap);
@@ -1491,6 +2137,8 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
     mem_put(blk);
     cudaSetDevice(prev_dev);
     plain_destroy(s);
+    for (int64_t i : again)
+        if (!st) st = expectations_batch(reads + i, 1, p, ex + i, read_status + i, true);
     return st;
 }
 

@@ -1,0 +1,1058 @@
+// Resident kernels of the plain FP64 form: the same recursion, operation for operation, as a chain of
+// launches that each have the parallelism their part allows.
+//
+//   emit64      the emissions of every path slot
+//   forward64   a CTA per forward segment, a path per thread: stores every anti-diagonal's values
+//   backward64  a CTA per traceback window, a path per thread: stores F.B of the match state of every
+//               slot, and the terms of the total probabilities
+//   totals64    a thread per total probability (the reference's sequential folds)
+//   posterior pairs: count64, scan64, place64, write64, in the reference's order; or, in
+//   expectations mode, transitions64, kmers64 and finish64 (and the HDP machine's assignments with
+//   the pairs' kernels)
+//
+// Why.  One CTA that walked a region's forward sweep, then window after window backward, then the
+// posteriors, with every value in global memory behind four dependent table loads, took ~2.8 us an
+// anti-diagonal and sweep: latency, not arithmetic (issue 0.1 a cycle on its SM, FP64 pipe 3 %).
+// Here the paths of the reference are numbered along it and path q stays on thread q mod NT, so its own
+// column's previous value is in a register and its neighbours' are one shared-memory read away; the
+// operands come by asynchronous copy kAhead64 anti-diagonals ahead; and only what depends on the
+// previous anti-diagonal's neighbour sits between two barriers (gap-X forward, match and gap-X
+// backward).  Windows run side by side, and logarithms, exponentials, totals and outputs are off the
+// sweeps' chain.  Measured on B200: see the dispatch rule in plain_create.
+//
+// A slot not in the band holds log 0 for that anti-diagonal, so an absent neighbour drops out of
+// log_add.  No two paths of three consecutive anti-diagonals share a thread: the host takes this
+// route only if they span at most NT paths.
+#pragma once
+
+constexpr int kAhead64 = 6;            // anti-diagonals between a copy and its use
+constexpr int kRing64 = 8;             // rows of the copy rings
+constexpr int kInfoRing = 128;         // rows of band facts kept
+
+// neighbours of a path: those of the column before (stride apart) and after (consecutive) that it may
+// follow or precede (path_checkLegal), in ascending order
+struct Path64 {
+    double gapx;                       // its skip emission
+    int32_t pred, pred_n;
+    int32_t pred_step, col;
+    int32_t succ, succ_n;
+};
+
+// one traceback window: its task, its place among the region's windows, its first total's terms
+struct Window64 {
+    int32_t task, win;
+    int32_t first_total;               // index of its first total probability
+    int32_t pad;
+};
+
+struct Total64 {
+    int32_t region, d;                 // anti-diagonal
+    int32_t have_next, last;           // d < D; d ends the region
+};
+
+__device__ __forceinline__ void copy64_8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy64_16(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy64_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy64_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// ------------------------------------------------------------------------------------------------
+// emissions: a warp per anti-diagonal
+// ------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) emit64(const Model64 *models, const Region64 *regions, const int32_t *chunk_region,
+                                              const int32_t *chunk_d0) {
+    const Region64 &R = regions[chunk_region[blockIdx.x]];
+    const Model64 &M = models[R.model];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t d0 = chunk_d0[blockIdx.x];
+    for (int32_t d = d0 + warp; d < d0 + 32 && d <= R.n; d += 8) {
+        const int4 in = R.info[d];
+        for (int32_t k = lane; k < in.y; k += 32) {
+            const int32_t q = in.x + k, kid = R.pid[q], y = d - R.path[q].col;
+            double em = kNegInf, ey = kNegInf;
+            if (y >= 1 && kid >= 0) {
+                const double2 ev = R.ev[y - 1];
+                em = emit_event(M, kid, ev.x, ev.y, true);
+                ey = M.emission == 2 ? em : emit_event(M, kid, ev.x, ev.y, false);
+            }
+            reinterpret_cast<double2 *>(R.E)[in.z + q] = make_double2(em, ey);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// band facts of the sweeps: 32 anti-diagonals at a time, by the CTA's first warp
+// ------------------------------------------------------------------------------------------------
+// DIR: +1 forward, -1 backward.  The block after the current one is loaded at its start and becomes
+// readable half way through it, long before a copy (kAhead64 ahead) asks for it.
+template <int DIR>
+struct InfoStream {
+    int4 *ring;
+    const int4 *src;
+    int32_t n, start;
+    int4 next;
+
+    __device__ __forceinline__ int32_t row(int32_t k) const { return start + DIR * k; }   // k-th anti-diagonal
+    __device__ __forceinline__ int4 fetch(int32_t k) const {
+        const int32_t d = row(k);
+        int4 v = src[min(max(d, 0), n)];
+        if (d < 0 || d > n) v.y = 0;   // no such anti-diagonal: no slots
+        return v;
+    }
+    __device__ __forceinline__ void open(const int4 *s, int32_t nn, int32_t d0) {
+        src = s;
+        n = nn;
+        start = d0;
+        if (threadIdx.x < 32) {
+            ring[threadIdx.x] = fetch(threadIdx.x);
+            ring[32 + threadIdx.x] = fetch(32 + threadIdx.x);
+        }
+    }
+    // at the k-th step
+    __device__ __forceinline__ void advance(int32_t k) {
+        if (threadIdx.x < 32) {
+            if ((k & 31) == 0) next = fetch(k + 64 + threadIdx.x);
+            else if ((k & 31) == 16) ring[((k - 16) + 64 + threadIdx.x) & (kInfoRing - 1)] = next;
+        }
+    }
+    __device__ __forceinline__ int4 at(int32_t k) const { return ring[k & (kInfoRing - 1)]; }
+};
+
+// ------------------------------------------------------------------------------------------------
+// log_add on the sweeps' chains
+// ------------------------------------------------------------------------------------------------
+// dp64::log_add bit for bit, without its select chains: the cubic's piece comes from shared memory,
+// indexed as in the FP32 form: C - d rounded down, with C's last place 1/64, holds -32 ceil(2 d) mod
+// 512 in bits 5..8, the byte offset of the piece.  -inf less -inf is NaN, which compares as beyond the
+// cut-off.  One after another 117 cycles each, four independent ones 223 (measured; with the
+// coefficients selected, 95 and 295; with the piece found by integer compares, 152 and 480).
+struct LogAdd64 {
+    double2 c[16][2];                  // (a3, a2), (a1, a0) of the piece of -ceil(2 d) mod 16
+};
+
+__device__ __forceinline__ void log_add_table64(LogAdd64 &t, int k) {
+    const double d = 0.5 * ((16 - k) & 15);   // the upper end of the entry's range
+    const bool p0 = d <= 1.0, p1 = d <= 2.5, p2 = d <= 4.5;
+    t.c[k][0] = make_double2(p0 ? (double) -0.009350833524763f : p1 ? (double) -0.014532321752540f
+                             : p2 ? (double) -0.004605031767994f : (double) -0.000458661602210f,
+                             p0 ? (double) 0.130659527668286f : p1 ? (double) 0.139942324101744f
+                             : p2 ? (double) 0.063427417320019f : (double) 0.009695946122598f);
+    t.c[k][1] = make_double2(p0 ? (double) 0.498799810682272f : p1 ? (double) 0.495635523139337f
+                             : p2 ? (double) 0.695956496475118f : (double) 0.930734667215156f,
+                             p0 ? (double) 0.693203116424741f : p1 ? (double) 0.692140569840976f
+                             : p2 ? (double) 0.514272634594009f : (double) 0.168037164329057f);
+}
+
+__device__ __forceinline__ double lad(const LogAdd64 &t, double x, double y) {
+    const double d = fabs(x - y);
+    const int k = __double2loint(__dadd_rd(105553116266496.0, -d)) & 0x1e0;
+    const double2 *c = reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(t.c) + k);
+    const double2 ab = c[0], ce = c[1];
+    const double p = ((ab.x * d + ab.y) * d + ce.x) * d + ce.y;
+    double r;
+    // branch-free: the larger and the smaller argument, and the larger alone from the cut-off on
+    asm("{\n\t.reg .pred q, n;\n\t.reg .f64 hi, lo, s;\n\tsetp.lt.f64 q, %1, %2;\n\tselp.f64 hi, %2, %1, q;\n\t"
+        "selp.f64 lo, %1, %2, q;\n\tadd.rn.f64 s, %3, lo;\n\tsetp.lt.f64 n, %4, 0d401E000000000000;\n\t"
+        "selp.f64 %0, s, hi, n;\n\t}"
+        : "=d"(r) : "d"(x), "d"(y), "d"(p), "d"(d));
+    return r;
+}
+
+// four independent ones, stage by stage
+__device__ __forceinline__ void lad4(const LogAdd64 &t, const double (&x)[4], const double (&y)[4], double (&r)[4]) {
+    double d[4], p[4];
+    double2 ab[4], ce[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) d[j] = fabs(x[j] - y[j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int k = __double2loint(__dadd_rd(105553116266496.0, -d[j])) & 0x1e0;
+        const double2 *c = reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(t.c) + k);
+        ab[j] = c[0];
+        ce[j] = c[1];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = ab[j].x * d[j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = p[j] + ab[j].y;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = p[j] + ce[j].x;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = p[j] + ce[j].y;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        asm("{\n\t.reg .pred q, n;\n\t.reg .f64 hi, lo, s;\n\tsetp.lt.f64 q, %1, %2;\n\tselp.f64 hi, %2, %1, q;\n\t"
+            "selp.f64 lo, %1, %2, q;\n\tadd.rn.f64 s, %3, lo;\n\tsetp.lt.f64 n, %4, 0d401E000000000000;\n\t"
+            "selp.f64 %0, s, hi, n;\n\t}"
+            : "=d"(r[j]) : "d"(x[j]), "d"(y[j]), "d"(p[j]), "d"(d[j]));
+}
+
+// ------------------------------------------------------------------------------------------------
+// forward sweep of one segment
+// ------------------------------------------------------------------------------------------------
+// On anti-diagonal d a thread computes, side by side, the four log_adds whose operands are at hand:
+// gap-X of d (its neighbours on d-1), gap-Y of d (own column on d-1), all but the last term of the
+// match state of d+1 (neighbours on d-1), and the last term of d's.  So a step takes one log_add's
+// latency, a barrier and a shared-memory round trip, where the states one after another took four.
+template <int NT, bool kMulti>
+struct Forward64Shared {
+    LogAdd64 la;
+    int4 info[kInfoRing];
+    double2 e[kRing64][NT];
+    double gx[kRing64][NT];
+    int4 pred[kMulti ? kRing64 : 1][kMulti ? NT : 1];   // pred, pred_n, pred_step
+    double v[2][3][NT];                // states by parity of the anti-diagonal
+};
+
+template <int NT, bool kMulti, bool kSX>
+__global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Region64 *tasks, SetOut O) {
+    extern __shared__ double2 smem64[];
+    using Sh = Forward64Shared<NT, kMulti>;
+    Sh &sh = *reinterpret_cast<Sh *>(smem64);
+    const Region64 R = tasks[blockIdx.x];
+    const double *mt = models[R.model].t;
+    const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY], tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX],
+                 tOY = mt[T_OY], tEY = mt[T_EY];
+    const int tid = threadIdx.x;
+    const int32_t s = R.s0 <= 1 ? 1 : R.s0, dend = R.win[R.w1 - 1].D;
+    InfoStream<1> info{sh.info};
+    info.open(R.info, R.n, s);
+    if (tid < 16) log_add_table64(sh.la, tid);
+    // the values of s-2 (parity 0, as s) and s-1
+    double M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf;
+    for (int st = 0; st < 3; ++st) sh.v[0][st][tid] = kNegInf;
+    if (R.s0 <= 1) {
+        if (tid == 0) {   // startStateProb / raggedStartStateProb (stateMachine.c:1022-1032) on anti-diagonal 0
+            M1 = R.ragged_left ? kNegInf : 0.0;
+            X1 = Y1 = R.ragged_left ? 0.0 : kNegInf;
+            double *c = R.F + 3 * (int64_t) R.info[0].z;
+            c[S_M] = M1;
+            c[S_X] = X1;
+            c[S_Y] = Y1;
+        }
+    } else {   // a later segment: every slot of s-2 and s-1 starts at 0
+        const int4 i2 = R.info[s - 2], i1 = R.info[s - 1];
+        const double z = ((tid - i2.x) & (NT - 1)) < i2.y ? 0.0 : kNegInf;
+        for (int st = 0; st < 3; ++st) sh.v[0][st][tid] = z;
+        M1 = X1 = Y1 = ((tid - i1.x) & (NT - 1)) < i1.y ? 0.0 : kNegInf;
+    }
+    sh.v[1][S_M][tid] = M1;
+    sh.v[1][S_X][tid] = X1;
+    sh.v[1][S_Y][tid] = Y1;
+    __syncthreads();
+    auto issue = [&](int32_t k) {
+        const int4 in = info.at(k);
+        const int32_t i = (tid - in.x) & (NT - 1), q = in.x + i;
+        if (i < in.y) {
+            const int b = k & (kRing64 - 1);
+            copy64_16(&sh.e[b][tid], R.E + 2 * ((int64_t) in.z + q));
+            copy64_8(&sh.gx[b][tid], &R.path[q].gapx);
+            if constexpr (kMulti) {
+                copy64_8(&sh.pred[b][tid].x, &R.path[q].pred);
+                copy64_8(&sh.pred[b][tid].z, &R.path[q].pred_step);
+            }
+        }
+        copy64_commit();
+    };
+    // what a thread needs of the k-th anti-diagonal beside the values, in registers a step early
+    struct Own {
+        int32_t i, q;
+        bool in;
+        int64_t at;
+        double2 e;
+        double gx;
+        int4 pr;
+    };
+    auto own = [&](int32_t k) -> Own {
+        const int4 in = info.at(k);
+        const int b = k & (kRing64 - 1);
+        Own o;
+        o.i = (tid - in.x) & (NT - 1);
+        o.q = in.x + o.i;
+        o.in = o.i < in.y;
+        o.at = (int64_t) in.z + o.q;
+        o.e = sh.e[b][tid];
+        o.gx = sh.gx[b][tid];
+        if constexpr (kMulti) o.pr = o.in ? sh.pred[b][tid] : make_int4(0, 0, 0, 0);
+        else o.pr = make_int4(o.q - 1, 1, 0, 0);
+        return o;
+    };
+    for (int k = 0; k < kAhead64; ++k) issue(k);
+    copy64_wait<kAhead64 - 2>();
+    Own o0 = own(0), o1 = own(1);
+    // match state: all terms but the last, and that
+    double most = kNegInf, last = kNegInf;
+    if (!kMulti || o0.pr.y > 0) {
+        for (int32_t a = 0, p = o0.pr.x; a < o0.pr.y; ++a, p += o0.pr.z) {
+            const int w = p & (NT - 1);
+            if (a) most = lad(sh.la, most, last);
+            most = lad(sh.la, most, sh.v[0][S_M][w] + (o0.e.x + tMC));
+            most = lad(sh.la, most, sh.v[0][S_X][w] + (o0.e.x + tMX));
+            last = sh.v[0][S_Y][w] + (o0.e.x + tMY);
+        }
+    }
+    const int32_t b_in = R.st_in >= 0 ? O.stitch[R.st_in].b : -10, b_out = R.st_out >= 0 ? O.stitch[R.st_out].b : -10;
+#pragma unroll 1
+    for (int32_t d = s, k = 0; d <= dend; ++d, ++k) {
+        info.advance(k);
+        issue(k + kAhead64);
+        copy64_wait<kAhead64 - 2>();   // every copy of d+2 and before has landed
+        const double eOX = o0.gx + tOX, eEX = o0.gx + tEX, eSX = o0.gx + tSX;
+        const double eMC = o1.e.x + tMC, eMX = o1.e.x + tMX, eMY = o1.e.x + tMY;
+        double x[4], y[4], r[4];
+        x[1] = M1 + (o0.e.y + tOY);
+        y[1] = Y1 + (o0.e.y + tEY);
+        x[2] = most;
+        y[2] = last;
+        __syncthreads();   // d-1's values
+        const double(&v)[3][NT] = sh.v[(k + 1) & 1];
+        const int p0 = o0.pr.x & (NT - 1), p1 = o1.pr.x & (NT - 1);
+        x[0] = v[S_M][p0] + eOX;
+        y[0] = v[S_X][p0] + eEX;
+        x[3] = v[S_M][p1] + eMC;
+        y[3] = v[S_X][p1] + eMX;
+        double lY = 0.0;
+        if (kSX) lY = v[S_Y][p0] + eSX;
+        last = v[S_Y][p1] + eMY;
+        const Own o2 = own(k + 2);
+        if constexpr (kMulti) {
+            if (o0.pr.y == 0) x[0] = y[0] = lY = kNegInf;
+            if (o1.pr.y == 0) x[3] = y[3] = last = kNegInf;
+        }
+        lad4(sh.la, x, y, r);
+        if (kSX) r[0] = lad(sh.la, r[0], lY);
+        most = r[3];
+        if constexpr (kMulti) {
+            for (int32_t a = 1, p = o0.pr.x + o0.pr.z; a < o0.pr.y; ++a, p += o0.pr.z) {
+                const int w = p & (NT - 1);
+                r[0] = lad(sh.la, r[0], v[S_M][w] + eOX);
+                r[0] = lad(sh.la, r[0], v[S_X][w] + eEX);
+                if (kSX) r[0] = lad(sh.la, r[0], v[S_Y][w] + eSX);
+            }
+            for (int32_t a = 1, p = o1.pr.x + o1.pr.z; a < o1.pr.y; ++a, p += o1.pr.z) {
+                const int w = p & (NT - 1);
+                most = lad(sh.la, most, last);
+                most = lad(sh.la, most, v[S_M][w] + eMC);
+                most = lad(sh.la, most, v[S_X][w] + eMX);
+                last = v[S_Y][w] + eMY;
+            }
+        }
+        X1 = o0.in ? r[0] : kNegInf;
+        Y1 = o0.in ? r[1] : kNegInf;
+        M1 = o0.in ? r[2] : kNegInf;
+        sh.v[k & 1][S_M][tid] = M1;
+        sh.v[k & 1][S_X][tid] = X1;
+        sh.v[k & 1][S_Y][tid] = Y1;
+        if (o0.in) {
+            double *c = R.F + 3 * o0.at;
+            c[S_M] = M1;
+            c[S_X] = X1;
+            c[S_Y] = Y1;
+        }
+        // the values of b-1 and b to their side of a stitch
+        if (d == b_in - 1 || d == b_in || d == b_out - 1 || d == b_out) {
+            const bool side = d == b_in - 1 || d == b_in;
+            const Stitch64 S = O.stitch[side ? R.st_in : R.st_out];
+            const int blk = side ? d - (b_in - 1) : 2 + d - (b_out - 1);
+            if (o0.in) {
+                double *o = S.vals + 3 * ((int64_t) blk * S.stride + o0.i);
+                o[0] = M1;
+                o[1] = X1;
+                o[2] = Y1;
+            }
+        }
+        o0 = o1;
+        o1 = o2;
+    }
+    copy64_wait<0>();
+    if (R.st_in >= 0) stitch_arrive64(R, O, R.st_in);
+    if (R.st_out >= 0) stitch_arrive64(R, O, R.st_out);
+}
+
+// ------------------------------------------------------------------------------------------------
+// backward sweep of one traceback window
+// ------------------------------------------------------------------------------------------------
+// A path's values go to its predecessors already summed with its emission and the transitions (the
+// pushed sums of backward_cell), so a predecessor only folds.  As forward, the log_adds of a step are
+// side by side: gap-X and gap-Y of d, the match state of d but for its last term, and the last term of
+// d+1's (which nothing needs before d-1).  What d+1's match value goes into (F.B, the terms of a total
+// probability's two folds: F.B on that anti-diagonal, and the matches from the one before it over it
+// into the one after, dotted with B there) is therefore written a step late.
+template <int NT, bool kMulti>
+struct Backward64Shared {
+    LogAdd64 la;
+    int4 info[kInfoRing];
+    double2 e[kRing64][NT];
+    double gx[kRing64][NT];
+    int4 nb[kMulti ? kRing64 : 1][kMulti ? NT : 1];        // succ, succ_n; pred, pred_n
+    int32_t step[kMulti ? kRing64 : 1][kMulti ? NT : 1];   // pred_step
+    double f[kRing64][NT];             // forward match value
+    double fx[2][NT];                  // forward gap values of a total's anti-diagonal
+    double fm[3][NT];                  // forward values of the anti-diagonal before it
+    double a[2][3][NT];                // sums for the match predecessors, by parity
+    double b[2][3][NT];                // sums for the gap-X predecessors, by parity
+};
+
+// the path a thread holds on an anti-diagonal
+struct Held64 {
+    int32_t i, n;                      // its slot, and the anti-diagonal's slots
+    int64_t at;                        // its place in the stores
+    int4 pred;                         // its predecessors: first, count, step
+    double e;                          // its match emission
+    double M;                          // its match value
+};
+
+template <int NT, bool kMulti, bool kSX>
+__global__ void __launch_bounds__(NT) backward64(const Model64 *models, const Region64 *tasks, const Window64 *windows,
+                                                 double *terms, int64_t term_stride, int expect) {
+    extern __shared__ double2 smem64[];
+    using Sh = Backward64Shared<NT, kMulti>;
+    Sh &sh = *reinterpret_cast<Sh *>(smem64);
+    const Window64 wt = windows[blockIdx.x];
+    const Region64 R = tasks[wt.task];
+    const double *mt = models[R.model].t;
+    const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY], tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX],
+                 tOY = mt[T_OY], tEY = mt[T_EY];
+    const Window W = R.win[wt.win];
+    const int tid = threadIdx.x;
+    // endStateProb / raggedEndStateProb (stateMachine.c:1034-1061) on the traceback anti-diagonal
+    const bool ragged_end = W.at_end && R.ragged_right;
+    const double e0 = ragged_end ? (tOX + tOY) / 2.0 : tMC, e1 = ragged_end ? tEX : tMX, e2 = ragged_end ? tEY : tMY;
+    InfoStream<-1> info{sh.info};
+    info.open(R.info, R.n, W.D);
+    if (tid < 16) log_add_table64(sh.la, tid);
+    for (int k = 0; k < 2; ++k)
+        for (int st = 0; st < 3; ++st) sh.a[k][st][tid] = sh.b[k][st][tid] = kNegInf;
+    __syncthreads();
+    const int32_t steps = W.D - W.T;
+    auto issue = [&](int32_t k) {
+        if (k < steps) {
+            const int32_t d = W.D - k;
+            const int4 in = info.at(k);
+            const int32_t i = (tid - in.x) & (NT - 1), q = in.x + i;
+            const bool post = d <= W.from, total = post && (W.from - d) % 10 == 0;
+            const int b = k & (kRing64 - 1);
+            if (i < in.y) {
+                const int64_t at = (int64_t) in.z + q;
+                copy64_16(&sh.e[b][tid], R.E + 2 * at);
+                copy64_8(&sh.gx[b][tid], &R.path[q].gapx);
+                if constexpr (kMulti) {
+                    copy64_8(&sh.nb[b][tid].x, &R.path[q].succ);
+                    copy64_8(&sh.nb[b][tid].z, &R.path[q].pred);
+                    sh.step[b][tid] = R.path[q].pred_step;
+                }
+                if (post) copy64_8(&sh.f[b][tid], R.F + 3 * at);
+                if (total) {
+                    copy64_8(&sh.fx[0][tid], R.F + 3 * at + S_X);
+                    copy64_8(&sh.fx[1][tid], R.F + 3 * at + S_Y);
+                }
+            }
+            if (total) {
+                const int4 bl = info.at(k + 1);
+                const int32_t j = (tid - bl.x) & (NT - 1);
+                if (j < bl.y) {
+                    const double *f = R.F + 3 * ((int64_t) bl.z + bl.x + j);
+                    for (int st = 0; st < 3; ++st) copy64_8(&sh.fm[st][tid], f + st);
+                } else {
+                    for (int st = 0; st < 3; ++st) sh.fm[st][tid] = kNegInf;
+                }
+            }
+        }
+        copy64_commit();
+    };
+    struct Own {
+        int32_t i, n, q;
+        int64_t at;
+        double2 e;
+        double gx, f;
+        int4 nb;
+        int32_t step;
+    };
+    auto own = [&](int32_t k) -> Own {
+        const int4 in = info.at(k);
+        const int b = k & (kRing64 - 1);
+        Own o;
+        o.i = (tid - in.x) & (NT - 1);
+        o.n = k < steps ? in.y : 0;
+        o.q = in.x + o.i;
+        o.at = (int64_t) in.z + o.q;
+        o.e = sh.e[b][tid];
+        o.gx = sh.gx[b][tid];
+        o.f = sh.f[b][tid];
+        o.nb = make_int4(o.q + 1, 1, o.q - 1, 1);
+        o.step = 0;
+        if constexpr (kMulti) {
+            o.nb = o.i < o.n ? sh.nb[b][tid] : make_int4(0, 0, 0, 0);
+            o.step = sh.step[b][tid];
+        }
+        return o;
+    };
+    for (int k = 0; k < kAhead64; ++k) issue(k);
+    copy64_wait<kAhead64 - 1>();
+    Own o0 = own(0);
+    double f1 = 0.0;                                 // forward match value of d+1
+    double u0 = kNegInf, u1 = kNegInf;               // own path's gap-Y sums of d+1
+    double most = kNegInf, last = kNegInf;           // its match state on d+1: all terms but one, and that
+    double X1 = kNegInf, Y1 = kNegInf;               // its gap values on d+1
+    Held64 h1{0, 0, 0, make_int4(0, 0, 0, 0), 0.0, kNegInf}, h2 = h1;   // the paths held on d+1, d+2
+    int64_t total_at = wt.first_total;
+#pragma unroll 1
+    for (int32_t k = 0; k <= steps; ++k) {           // k == steps: only what is a step late
+        const int32_t d = W.D - k;
+        info.advance(k);
+        issue(k + kAhead64);
+        copy64_wait<kAhead64 - 1>();                 // every copy of d-1 and above has landed
+        const bool inb = o0.i < o0.n;
+        const int4 nb = o0.nb;
+        double x[4], y[4], r[4];
+        __syncthreads();   // d+1's sums for gap-X predecessors, d+2's for match predecessors
+        const double(&a)[3][NT] = sh.a[k & 1];
+        const double(&c)[3][NT] = sh.b[(k + 1) & 1];
+        const int p0 = nb.x & (NT - 1);
+        x[0] = a[1][p0];
+        y[0] = c[1][p0];
+        x[1] = a[2][p0];
+        y[1] = u1;
+        x[2] = a[0][p0];
+        y[2] = u0;
+        x[3] = most;
+        y[3] = last;
+        double l = c[0][p0], lY = 0.0;
+        if (kSX) lY = c[2][p0];
+        const Own o1 = own(k + 1);
+        if constexpr (kMulti) {
+            if (nb.y == 0) x[0] = y[0] = x[1] = x[2] = l = lY = kNegInf;
+            for (int32_t j = 1; j < nb.y; ++j) {
+                const int w = (nb.x + j) & (NT - 1);
+                x[0] = lad(sh.la, x[0], a[1][w]);
+                x[1] = lad(sh.la, x[1], a[2][w]);
+                x[2] = lad(sh.la, x[2], a[0][w]);
+            }
+        }
+        lad4(sh.la, x, y, r);
+        if (kSX) r[1] = lad(sh.la, r[1], lY);
+        if constexpr (kMulti) {
+            for (int32_t j = 1; j < nb.y; ++j) {
+                const int w = (nb.x + j) & (NT - 1);
+                r[2] = lad(sh.la, r[2], l);
+                l = c[0][w];
+                r[0] = lad(sh.la, r[0], c[1][w]);
+                if (kSX) r[1] = lad(sh.la, r[1], c[2][w]);
+            }
+        }
+        double vX = r[0], vY = r[1], m = r[2];
+        h1.M = h1.i < h1.n ? r[3] : kNegInf;
+        if (k == 0) {
+            m = e0;
+            l = kNegInf;
+            vX = e1;
+            vY = e2;
+        }
+        most = m;
+        last = l;
+        vX = inb ? vX : kNegInf;
+        vY = inb ? vY : kNegInf;
+        const double2 e = o0.e;
+        const double gx = o0.gx;
+        // match sums of d+1 (a buffer's parity is its anti-diagonal's plus one), gap sums of d
+        const bool in1 = h1.i < h1.n;
+        sh.a[(k + 1) & 1][0][tid] = in1 ? h1.M + (h1.e + tMC) : kNegInf;
+        sh.a[(k + 1) & 1][1][tid] = in1 ? h1.M + (h1.e + tMX) : kNegInf;
+        sh.a[(k + 1) & 1][2][tid] = in1 ? h1.M + (h1.e + tMY) : kNegInf;
+        sh.b[k & 1][0][tid] = inb ? vX + (gx + tOX) : kNegInf;
+        sh.b[k & 1][1][tid] = inb ? vX + (gx + tEX) : kNegInf;
+        if (kSX) sh.b[k & 1][2][tid] = inb ? vX + (gx + tSX) : kNegInf;
+        u0 = inb ? vY + (e.y + tOY) : kNegInf;
+        u1 = inb ? vY + (e.y + tEY) : kNegInf;
+        // d+1's outputs
+        if (k > 0 && d + 1 <= W.from) {
+            const double f = f1;
+            if (in1) {
+                R.S[h1.at] = f + h1.M;
+                if (expect) {
+                    R.B[3 * h1.at + S_M] = h1.M;
+                    R.B[3 * h1.at + S_X] = X1;
+                    R.B[3 * h1.at + S_Y] = Y1;
+                }
+            }
+            if ((W.from - d - 1) % 10 == 0) {
+                double *t0 = terms + total_at * 2 * term_stride;
+                if (in1) {
+                    double s = f + h1.M;
+                    s = lad(sh.la, s, sh.fx[0][tid] + X1);
+                    s = lad(sh.la, s, sh.fx[1][tid] + Y1);
+                    t0[h1.i] = s;
+                }
+                if (k > 1 && h2.i < h2.n) {
+                    // the slot of d+2 this thread held: its predecessors' forward values on d
+                    double w = kNegInf;
+                    if constexpr (!kMulti) {
+                        const int p = h2.pred.x & (NT - 1);
+                        w = lad(sh.la, sh.fm[S_M][p] + (h2.e + tMC), sh.fm[S_X][p] + (h2.e + tMX));
+                        w = lad(sh.la, w, sh.fm[S_Y][p] + (h2.e + tMY));
+                    } else {
+                        for (int32_t j = 0, p = h2.pred.x; j < h2.pred.y; ++j, p += h2.pred.z) {
+                            w = lad(sh.la, w, sh.fm[S_M][p & (NT - 1)] + (h2.e + tMC));
+                            w = lad(sh.la, w, sh.fm[S_X][p & (NT - 1)] + (h2.e + tMX));
+                            w = lad(sh.la, w, sh.fm[S_Y][p & (NT - 1)] + (h2.e + tMY));
+                        }
+                    }
+                    t0[term_stride + h2.i] = w + h2.M;
+                }
+                ++total_at;
+            }
+        }
+        X1 = vX;
+        Y1 = vY;
+        h2 = h1;
+        h1 = Held64{o0.i, o0.n, o0.at, make_int4(nb.z, nb.w, o0.step, 0), e.x, kNegInf};
+        f1 = o0.f;
+        o0 = o1;
+    }
+    copy64_wait<0>();
+}
+
+// ------------------------------------------------------------------------------------------------
+// total probabilities: a thread each
+// ------------------------------------------------------------------------------------------------
+// diagonalCalculationTotalProbability (pairwiseAligner.c:1182-1200) over the terms: cells in ascending
+// order, a cell's paths folded first (hdCell_totalProbability); the two sums side by side.
+__global__ void __launch_bounds__(64) totals64(const Region64 *regions, const Total64 *totals, int64_t n, const double *terms,
+                                               int64_t term_stride, int multi) {
+    __shared__ LogAdd64 la;
+    if (threadIdx.x < 16) log_add_table64(la, threadIdx.x);
+    __syncthreads();
+    const int64_t at = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
+    if (at >= n) return;
+    const Total64 T = totals[at];
+    const Region64 &R = regions[T.region];
+    const double *t0 = terms + at * 2 * term_stride, *t1 = t0 + term_stride;
+    const int4 in = R.info[T.d];
+    const int4 in1 = T.have_next ? R.info[T.d + 1] : make_int4(0, 0, 0, 0);
+    double total = kNegInf, through = kNegInf;
+    if (!multi) {
+        const int32_t most = max(in.y, in1.y);
+#pragma unroll 4
+        for (int32_t i = 0; i < most; ++i) {
+            const double a = i < in.y ? t0[i] : kNegInf, b = i < in1.y ? t1[i] : kNegInf;
+            total = lad(la, total, a);        // log_add(x, log 0) is x
+            through = lad(la, through, b);
+        }
+    } else {
+        auto fold = [&](const double *t, const int4 &f) {
+            double v = kNegInf, cell = kNegInf;
+            int32_t col = -1;
+            for (int32_t i = 0; i < f.y; ++i) {
+                const int32_t c = R.path[f.x + i].col;
+                if (c != col) {
+                    v = lad(la, v, cell);
+                    cell = kNegInf;
+                    col = c;
+                }
+                cell = lad(la, cell, t[i]);
+            }
+            return lad(la, v, cell);
+        };
+        total = fold(t0, in);
+        if (T.have_next) through = fold(t1, in1);
+    }
+    if (T.have_next) total = lad(la, total, through);
+    R.P[T.d] = total;
+    if (T.last) *R.loglik = total;
+}
+
+// ------------------------------------------------------------------------------------------------
+// outputs in the reference's order
+// ------------------------------------------------------------------------------------------------
+// A region's windows come in ascending order and a window's anti-diagonals (T, from] descending, so
+// anti-diagonal d of a window comes T + from - d -th among the region's.
+struct Output64 {
+    sa_aligned_pair *out;         // pairs, or
+    const ExpectOut *reads;       // (expectations of HDP machines) each read's assignments
+    int32_t *count;               // per region its anti-diagonals' counts, then their starts
+    int64_t *region_total;        // per region its count, then its start
+    int64_t cap;
+    double threshold;
+};
+
+// the number of outputs of slot q on d, and (write) the outputs
+template <bool kAssign>
+__device__ __forceinline__ int slot_hits(const Region64 &R, const Output64 &O, int64_t at, double total, int32_t x,
+                                         int32_t y, double &p, unsigned &which) {
+    if (kAssign) {   // match transitions at or above the threshold, from match, gap-X, gap-Y
+        which = 0;
+        if (R.B[3 * at] >= 0.0)
+            for (int j = 0; j < 3; ++j)
+                if (R.B[3 * at + j] >= O.threshold) which |= 1u << j;
+        return __popc(which);
+    }
+    if (x <= 0 || y <= 0) return 0;
+    p = exp(R.S[at] - total);
+    return p >= O.threshold ? 1 : 0;
+}
+
+template <bool kAssign, bool kWrite>
+__global__ void __launch_bounds__(256) outputs64(const Region64 *regions, const int32_t *chunk_region,
+                                                 const int32_t *chunk_d0, const int64_t *row_base, Output64 O) {
+    const int32_t region = chunk_region[blockIdx.x];
+    const Region64 &R = regions[region];
+    if (kAssign && !O.reads[R.reader].hdp) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t d0 = chunk_d0[blockIdx.x];
+    int32_t *count = O.count + row_base[region];
+    for (int32_t d = max(d0, 1) + warp; d < d0 + 32 && d <= R.n; d += 8) {
+        const int4 in = R.info[d];
+        const Window W = R.win[in.w];
+        const int32_t place = W.T + W.from - d;
+        const double total = R.P[W.from - 10 * ((W.from - d) / 10)];
+        int64_t base = kWrite ? O.region_total[region] + count[place] : 0;
+        int32_t found = 0;
+        for (int32_t k0 = 0; k0 < in.y; k0 += 32) {
+            const int32_t k = k0 + lane, q = in.x + k;
+            const int64_t at = (int64_t) in.z + q;
+            double p = 0.0;
+            unsigned which = 0;
+            int hits = 0;
+            int32_t x = 0, y = 0;
+            if (k < in.y) {
+                x = R.path[q].col;
+                y = d - x;
+                hits = slot_hits<kAssign>(R, O, at, total, x, y, p, which);
+            }
+            if (!__any_sync(0xffffffffu, hits > 0)) continue;
+            int32_t inc = hits;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            if (kWrite && hits) {
+                int64_t to = base + found + inc - hits;
+                if (kAssign) {
+                    const ExpectOut &X = O.reads[R.reader];
+                    for (int j = 0; j < 3; ++j) {
+                        if (!((which >> j) & 1u)) continue;
+                        if (to < X.assign_cap) {
+                            X.assign_kmer[to] = R.pid[q];
+                            X.assign_event[to] = R.ev_base + y - 1;
+                        }
+                        ++to;
+                    }
+                } else if (to < O.cap) {
+                    sa_aligned_pair o;
+                    o.score = (int64_t) floor((p > 1.0 ? 1.0 : p) * 10000000.0);
+                    o.x = R.x_base + x - 1;
+                    o.y = R.ev_base + y - 1;
+                    o.kmer = R.pid[q];
+                    O.out[to] = o;
+                } else {
+                    atomicExch(R.status, (int32_t) SA_E_OUTPUT);
+                }
+            }
+            found += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (!kWrite && lane == 0) count[place] = found;
+    }
+}
+
+// counts of a region's anti-diagonals to their starts, a CTA each
+__global__ void __launch_bounds__(1024) scan64(const Region64 *regions, const int64_t *row_base, Output64 O) {
+    __shared__ int32_t sums[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int32_t *c = O.count + row_base[blockIdx.x];
+    const int32_t n = regions[blockIdx.x].n;   // places 0 .. n-1
+    int32_t run = 0;
+    for (int32_t k0 = 0; k0 < n; k0 += 4096) {
+        int32_t v[4], mine = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int32_t k = k0 + 4 * tid + j;
+            v[j] = k < n ? c[k] : 0;
+            mine += v[j];
+        }
+        int32_t inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (lane == 31) sums[warp] = inc;
+        __syncthreads();
+        int32_t before = 0, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) before += sums[w];
+            all += sums[w];
+        }
+        int32_t at = run + before + inc - mine;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int32_t k = k0 + 4 * tid + j;
+            if (k < n) c[k] = at;
+            at += v[j];
+        }
+        run += all;
+        __syncthreads();
+    }
+    if (tid == 0) O.region_total[blockIdx.x] = run;
+}
+
+// regions' counts to their starts, in order; `counts` keeps them, `all` their sum.  `first`: the first
+// region of each group that starts again at 0 (a read's assignments), or null for one group
+__global__ void place64(int64_t n, int64_t *region_total, int64_t *counts, unsigned long long *all, const int32_t *first) {
+    if (threadIdx.x || blockIdx.x) return;
+    int64_t at = 0;
+    for (int64_t r = 0; r < n; ++r) {
+        if (first && first[r] == r) at = 0;
+        const int64_t c = region_total[r];
+        counts[r] = c;
+        region_total[r] = at;
+        at += c;
+    }
+    if (all) *all = (unsigned long long) at;
+}
+
+// ------------------------------------------------------------------------------------------------
+// expectations
+// ------------------------------------------------------------------------------------------------
+// The transition posteriors of every slot (cell_signal_updateExpectations, pairwiseAligner.c:763-793;
+// see expect_diagonal): summed per block, and the three into the match state kept in place of the
+// slot's backward values (-1 where there is no middle neighbour), for the per-k-mer folds.
+__global__ void __launch_bounds__(256) transitions64(const Model64 *models, const Region64 *tasks, const int32_t *task_of,
+                                                     const int32_t *chunk_region, const int32_t *chunk_d0,
+                                                     const Region64 *regions, double *partial) {
+    __shared__ double sums[8][9];
+    const int32_t region = chunk_region[blockIdx.x];
+    const Region64 &R = regions[region];
+    const Model64 &M = models[R.model];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t d0 = chunk_d0[blockIdx.x];
+    double acc[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) acc[j] = 0.0;
+    for (int32_t d = max(d0, 1) + warp; d < d0 + 32 && d <= R.n; d += 8) {
+        const int4 in = R.info[d], l1 = R.info[d - 1], l2 = d >= 2 ? R.info[d - 2] : make_int4(0, 0, 0, 0);
+        const Window W = R.win[in.w];
+        const double total = R.P[W.from - 10 * ((W.from - d) / 10)];
+        const double *F = tasks[task_of[R.win_base + in.w]].F;   // the segment that swept this window
+        if (lane == 0) acc[8] += total;
+        for (int32_t k = lane; k < in.y; k += 32) {
+            const int32_t q = in.x + k;
+            const int64_t at = (int64_t) in.z + q;
+            const double bM = R.B[3 * at], bX = R.B[3 * at + 1], bY = R.B[3 * at + 2];
+            const bool lo = q - 1 >= l1.x && q - 1 < l1.x + l1.y && q > 0;
+            const bool mi = d - 2 >= W.T && q - 1 >= l2.x && q - 1 < l2.x + l2.y && q > 0;
+            const bool up = q >= l1.x && q < l1.x + l1.y;
+            if (lo) {
+                const double *l = F + 3 * ((int64_t) l1.z + q - 1);
+                const double e = R.path[q].gapx;
+                acc[0] += exp(l[S_M] + bX + (e + M.t[T_OX]) - total);
+                acc[1] += exp(l[S_X] + bX + (e + M.t[T_EX]) - total);
+                acc[2] += exp(l[S_Y] + bX + (e + M.t[T_SX]) - total);
+            }
+            double p3 = -1.0, p4 = 0.0, p5 = 0.0;
+            if (mi) {
+                const double *m = F + 3 * ((int64_t) l2.z + q - 1);
+                const double e = R.E[2 * at];
+                p3 = exp(m[S_M] + bM + (e + M.t[T_MC]) - total);
+                p4 = exp(m[S_X] + bM + (e + M.t[T_MFGX]) - total);
+                p5 = exp(m[S_Y] + bM + (e + M.t[T_MFGY]) - total);
+                acc[3] += p3;
+                acc[4] += p4;
+                acc[5] += p5;
+            }
+            if (up) {
+                const double *u = F + 3 * ((int64_t) l1.z + q);
+                const double e = R.E[2 * at + 1];
+                acc[6] += exp(u[S_M] + bY + (e + M.t[T_OY]) - total);
+                acc[7] += exp(u[S_Y] + bY + (e + M.t[T_EY]) - total);
+            }
+            R.B[3 * at] = p3;
+            R.B[3 * at + 1] = p4;
+            R.B[3 * at + 2] = p5;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+        for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+        if (lane == 0) sums[warp][j] = acc[j];
+    }
+    __syncthreads();
+    if (threadIdx.x < 9) {
+        double s = 0.0;
+        for (int w = 0; w < 8; ++w) s += sums[w][threadIdx.x];
+        partial[9 * (int64_t) blockIdx.x + threadIdx.x] = s;
+    }
+}
+
+// a k-mer of a read: the columns it stands at, by region, ascending
+struct Kmer64 {
+    int32_t read, kid, first, count;   // columns cols[first .. first + count)
+};
+struct Column64 {
+    int32_t region, col, dlo, dhi;     // anti-diagonals the column's cells may be on
+};
+
+// continuousPairHmm_addToEmissionExpectation (continuousHmm.c:160-169) for one k-mer of one read, by a
+// warp: 32 anti-diagonals at a time in the reference's order.  The running weight and mean sum that
+// each update's spread needs are scans over the lanes, a lane's cells of one anti-diagonal in order.
+__global__ void __launch_bounds__(128) kmers64(const Model64 *models, const Region64 *regions, const Kmer64 *kmers,
+                                               int64_t n_kmers, const Column64 *cols, const ExpectOut *XS) {
+    const int64_t at = blockIdx.x * (int64_t) 4 + (threadIdx.x >> 5);
+    if (at >= n_kmers) return;
+    const int lane = threadIdx.x & 31;
+    const Kmer64 K = kmers[at];
+    const ExpectOut &X = XS[K.read];
+    double e0 = X.event_exp[2 * (int64_t) K.kid], e1 = X.event_exp[2 * (int64_t) K.kid + 1], po = X.posteriors[K.kid];
+    bool seen = false;
+    for (int32_t c0 = K.first; c0 < K.first + K.count;) {
+        // the columns of one region
+        const int32_t region = cols[c0].region;
+        int32_t c1 = c0 + 1;
+        while (c1 < K.first + K.count && cols[c1].region == region) ++c1;
+        const Region64 &R = regions[region];
+        const Model64 &M = models[R.model];
+        const double mu = M.match[(int64_t) K.kid * 5];
+        const int32_t dlo = max(cols[c0].dlo, 1), dhi = min(cols[c1 - 1].dhi, R.n);
+        for (int32_t w = dlo <= dhi ? R.info[dlo].w : 0; dlo <= dhi && w <= R.info[dhi].w; ++w) {
+            const Window W = R.win[w];
+            const int32_t bottom = max(W.T + 1, dlo);
+            for (int32_t dt = min(W.from, dhi); dt >= bottom; dt -= 32) {
+                // down to an anti-diagonal of the last column that begins at or before this one
+                int32_t l = c0, h = c1;
+                while (l < h) {
+                    const int32_t mid = (l + h) >> 1;
+                    if (cols[mid].dlo <= dt) l = mid + 1;
+                    else h = mid;
+                }
+                if (l == c0) break;
+                dt = min(dt, cols[l - 1].dhi);
+                if (dt < bottom) break;
+                const int32_t d = dt - lane;
+                int32_t a = 0, b = 0;         // columns c0 + a .. c0 + b - 1 are on d
+                int4 in = make_int4(0, 0, 0, 0);
+                if (d >= bottom) {
+                    in = R.info[d];
+                    a = 0;
+                    b = c1 - c0;
+                    if (b == 1) {
+                        const int32_t q = cols[c0].col;
+                        if (!(q >= in.x && q < in.x + in.y)) b = 0;
+                    } else {   // single-path columns: column x is path x
+                        int32_t lo = 0, hi = b;
+                        while (lo < hi) {
+                            const int32_t mid = (lo + hi) >> 1;
+                            if (cols[c0 + mid].col < in.x) lo = mid + 1;
+                            else hi = mid;
+                        }
+                        a = lo;
+                        hi = b;
+                        while (lo < hi) {
+                            const int32_t mid = (lo + hi) >> 1;
+                            if (cols[c0 + mid].col < in.x + in.y) lo = mid + 1;
+                            else hi = mid;
+                        }
+                        b = lo;
+                    }
+                }
+                double s0 = 0.0, sp = 0.0;
+                for (int32_t c = a; c < b; ++c) {
+                    const int32_t q = cols[c0 + c].col;
+                    const double *p = R.B + 3 * ((int64_t) in.z + q);
+                    if (p[0] < 0.0) continue;
+                    seen = true;
+                    const double xe = (R.ev[d - q - 1].x + M.var * mu - M.scale * mu - M.shift) / M.var;
+                    for (int j = 0; j < 3; ++j) {
+                        s0 += p[j] * xe;
+                        sp += p[j];
+                    }
+                }
+                double i0 = s0, ip = sp;   // inclusive scans in the reference's order (lane 0 first)
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double v0 = __shfl_up_sync(0xffffffffu, i0, o), vp = __shfl_up_sync(0xffffffffu, ip, o);
+                    if (lane >= o) {
+                        i0 += v0;
+                        ip += vp;
+                    }
+                }
+                double r0 = __shfl_up_sync(0xffffffffu, i0, 1), rp = __shfl_up_sync(0xffffffffu, ip, 1);
+                r0 = e0 + (lane ? r0 : 0.0);
+                rp = po + (lane ? rp : 0.0);
+                double spread = 0.0;
+                for (int32_t c = a; c < b; ++c) {
+                    const int32_t q = cols[c0 + c].col;
+                    const double *p = R.B + 3 * ((int64_t) in.z + q);
+                    if (p[0] < 0.0) continue;
+                    const double xe = (R.ev[d - q - 1].x + M.var * mu - M.scale * mu - M.shift) / M.var;
+                    for (int j = 0; j < 3; ++j) {
+                        r0 += p[j] * xe;
+                        rp += p[j];
+                        const double uk = r0 / rp;
+                        spread += p[j] * (xe - uk) * (xe - uk);
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) spread += __shfl_xor_sync(0xffffffffu, spread, o);
+                e1 += spread;
+                e0 += __shfl_sync(0xffffffffu, i0, 31);
+                po += __shfl_sync(0xffffffffu, ip, 31);
+            }
+        }
+        c0 = c1;
+    }
+    seen = __any_sync(0xffffffffu, seen);
+    if (lane == 0 && seen) {
+        X.event_exp[2 * (int64_t) K.kid] = e0;
+        X.event_exp[2 * (int64_t) K.kid + 1] = e1;
+        X.posteriors[K.kid] = po;
+        X.observed[K.kid] = 1;
+    }
+}
+
+// A read's likelihood and transition expectations from its blocks' sums, a CTA per read.  Anti-diagonals
+// a later segment swept have their totals in its frame: the stitches' constants bring them back.
+__global__ void __launch_bounds__(256) finish64(const ExpectOut *XS, const int64_t *read_chunk, const double *partial,
+                                                const Region64 *tasks, const int64_t *read_task, const Stitch64Res *stres) {
+    __shared__ double sums[8][9];
+    const ExpectOut &X = XS[blockIdx.x];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double acc[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) acc[j] = 0.0;
+    for (int64_t c = read_chunk[blockIdx.x] + tid; c < read_chunk[blockIdx.x + 1]; c += 256)
+#pragma unroll
+        for (int j = 0; j < 9; ++j) acc[j] += partial[9 * c + j];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+        for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+        if (lane == 0) sums[warp][j] = acc[j];
+    }
+    __syncthreads();
+    if (tid) return;
+    for (int j = 0; j < 9; ++j) {
+        acc[j] = 0.0;
+        for (int w = 0; w < 8; ++w) acc[j] += sums[w][j];
+    }
+    double delta = 0.0;
+    for (int64_t t = read_task[blockIdx.x]; t < read_task[blockIdx.x + 1]; ++t) {
+        const Region64 &R = tasks[t];
+        delta = R.st_in >= 0 ? delta + stres[R.st_in].delta : 0.0;
+        if (R.st_in >= 0) acc[8] += delta * (double) (R.win[R.w1 - 1].from - R.win[R.w0].T);
+    }
+    X.acc[0] += acc[8];
+    constexpr int to[8] = {S_M * 3 + S_X, S_X * 3 + S_X, S_Y * 3 + S_X, S_M * 3 + S_M,
+                           S_X * 3 + S_M, S_Y * 3 + S_M, S_M * 3 + S_Y, S_Y * 3 + S_Y};
+    for (int j = 0; j < 8; ++j) X.acc[1 + to[j]] += acc[j];
+}

@@ -202,8 +202,10 @@ bool batch_run_events(const sa_batch *b, cudaEvent_t *start, cudaEvent_t *end);
 // for reads whose references have degenerate ('X') positions.
 struct PlainSet;
 // segments: cut long regions into forward segments (alignment runs; not the expectations mode)
+// expect: for getExpectations (no pairs; forward segments only on the resident route); rings: not the
+// resident route
 sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p, size_t max_bytes, PlainSet **out,
-                       bool segments = false);
+                       bool segments = false, bool expect = false, bool rings = false);
 // scale of the set's stitch tolerance (negative: every stitch disagrees and its region re-runs whole)
 void plain_set_stitch_tolerance(PlainSet *s, double scale);
 // forward segments of the plain form in use: stitches and regions re-run whole at the last download
@@ -215,7 +217,12 @@ int plain_device(const PlainSet *s);
 int64_t plain_cells(const PlainSet *s);
 size_t plain_in_bytes(const PlainSet *s);
 sa_status plain_read_status(const PlainSet *s, int64_t r);
-const std::vector<sa_aligned_pair> &plain_pairs(const PlainSet *s, int64_t r);
+struct PlainPairs {
+    const sa_aligned_pair *p = nullptr;
+    size_t n = 0;
+};
+// a read's pairs, valid until the set's next download or its end
+PlainPairs plain_pairs(const PlainSet *s, int64_t r);
 double plain_log_likelihood(const PlainSet *s, int64_t r);
 void plain_destroy(PlainSet *s);
 
