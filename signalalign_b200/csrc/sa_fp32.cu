@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
@@ -59,7 +60,6 @@ __global__ void __launch_bounds__(256) fma_probe(float *sink, int iters, float s
 // Slack after the emission and forward stores: the kernels' clamped look-ahead loads past a
 // region's last anti-diagonal stay inside the allocation.
 constexpr size_t kStoreSlack = 1024;
-static_assert(2 * (kStoreFront + kStoreBack) <= kStoreSlack, "the emission store's slack holds both ends");
 
 // device memory bound of a batch's plain-form reads
 constexpr size_t kPlainBatchMaxBytes = (size_t) 64 << 30;
@@ -726,8 +726,7 @@ Args batch_args(const sa_batch *b) {
     a.kmer = b->d_kmer;
     a.gapx = b->d_gapx;
     a.events = b->d_events;
-    a.n_cells = b->cells;
-    a.E = reinterpret_cast<float2 *>(b->d_E) + kStoreFront;
+    a.E = reinterpret_cast<float2 *>(b->d_E);
     a.F = b->d_F;
     a.base = b->d_base;
     a.fshift = b->d_fshift;
@@ -752,27 +751,30 @@ Args batch_args(const sa_batch *b) {
     return a;
 }
 
-// The persistent worker over a.n_segs forward segments and a.n_windows windows.  Column-resident warps
-// take every batch whose bands fit their slots (bands up to about 124 or 248 columns), unless the
-// launch configuration asks for a window per CTA; the CTA form takes the rest.
-void launch_worker(const sa_batch *b, Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
-    a.sms = sms;
-    auto launch = [&](auto kern, size_t smem) {
+// The persistent worker over a.n_segs forward segments and a.n_windows windows: column-resident CTAs of
+// 128, 256 or 512 columns where the bands fit them, the CTA form for other bands and for launch
+// configurations that ask for it.
+void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
+    auto launch = [&](auto kern, int threads, size_t smem) {
         int per_sm = 0;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
         per_sm = std::max(1, std::min(per_sm, cfg.ctas_per_sm));
         const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t) sms * per_sm,
                                                                     (int64_t) cfg.grid_per_region * a.n_segs));
-        kern<<<(unsigned) grid, kThreads, smem, s>>>(a);
+        kern<<<(unsigned) grid, (unsigned) threads, smem, s>>>(a);
     };
-    if (cfg.warp_windows && b->max_span <= column_span(4))
-        return launch(column_worker<4, 3>, sizeof(ColumnShared) + kWarps * sizeof(WindowShared<4>));
+    if (cfg.warp_windows && b->max_span <= column_span(512)) {
+        if (b->max_span <= column_span(128)) launch(column_worker<128, 3>, 128 + kHelpers, sizeof(ColumnShared<128>));
+        else if (b->max_span <= column_span(256)) launch(column_worker<256, 2>, 256 + kHelpers, sizeof(ColumnShared<256>));
+        else launch(column_worker<512, 1>, 512 + kHelpers, sizeof(ColumnShared<512>));
+        return;
+    }
     const int cls = a.wmax / kThreads;
     const size_t smem = sizeof(Shared) + sizeof(float) * (size_t) worker_area_floats(cls);
-    if (cls == 1) launch(worker_kernel<1, 2>, smem);
-    else if (cls == 2) launch(worker_kernel<2, 1>, smem);
-    else launch(worker_kernel<4, 1>, smem);
+    if (cls == 1) launch(worker_kernel<1, 2>, kThreads, smem);
+    else if (cls == 2) launch(worker_kernel<2, 1>, kThreads, smem);
+    else launch(worker_kernel<4, 1>, kThreads, smem);
 }
 
 // Reads whose stitch disagreed run again with every region as one segment (after the batch's

@@ -1,319 +1,589 @@
-// Column-resident form of the batched FP32 worker, for bands up to column_span(NC) columns: a CTA per
-// forward segment (a column per thread), a warp per traceback window (NC columns per lane).
+// Column-resident form of the batched FP32 worker: a CTA per forward segment and per traceback window,
+// a matrix column per thread, for bands up to column_span(NT) columns.
 //
 // Why.  The recursion is bound by the latency of its chain of logAdds and by instruction issue, not by
 // memory.  With cells spread by their place in the band and exchanged through a shared-memory ring,
 // most instructions were not arithmetic: ring addresses, clamps, stores and loads, a look-ahead
 // address per operand (24 warp instructions per band cell, issue 19 to 30 % busy).
 //
-// How.  Matrix column x lives in slot x mod 128, whichever way the band moves.  A cell's neighbours are
-// then in the same slot (the same column) or in the one beside it (column x - 1 forward, x + 1
-// backward): two or three shuffles an anti-diagonal, no ring.  Slots outside the band hold -inf, which
-// makes every absent neighbour drop out of logAdd.  Three anti-diagonals' columns never share a slot:
-// the host takes this path for a batch only if any three consecutive anti-diagonals span at most
-// column_span(NC) columns, so the NC - 1 slots before an anti-diagonal's first column are always
-// outside it, and a lane's cells are consecutive elements of each store, addressed from one place.
+// How.  Column x lives on thread x mod NT, whichever way the band moves.  A cell's neighbours are then
+// on the same thread (the same column) or the one beside it (column x - 1 forward, x + 1 backward):
+// shuffles, and one shared float4 per warp's edge.  Threads outside the band hold -inf, which makes
+// every absent neighbour drop out of logAdd.  Three anti-diagonals' columns never share a thread: the
+// host takes this path for a batch only if any three consecutive anti-diagonals span at most
+// column_span(NT) columns.  A sweep is a chain of anti-diagonals and its warps issue in order, so
+// every instruction that is not the recursion lengthens the chain: three more warps take them, each
+// with less to do a step than the sweep, since they issue in order too (one warp for all of it made
+// the step 760 cycles; the sweep alone takes under 300).  One works out the renormalisation shifts,
+// one brings band facts and copies operands into shared memory kAhead anti-diagonals ahead, and one
+// takes the results out: forward, the values, bases and publication of windows; backward, the total
+// probabilities (sequential folds), posteriors and pairs, ten anti-diagonals at a time.
 //
 // The arithmetic is that of ForwardSweep and window_task, operation for operation, so the values are
-// theirs bit for bit.  Measured on B200, the worker of 8 reads of 8 to 12 kb (2.1e7 cells, 71
-// segments): 3.52 -> 2.35 ms; of 30 reads of 8 to 30 kb (1.5e8 cells): 5.36 -> 3.85 ms.  One warp per
-// forward segment (NC columns a lane) was slower than the form before it: 5.0 ms on the 8 reads.
+// theirs bit for bit.
+//
+// Measured on B200, the worker launch with cells by their place in the band / with four columns a lane,
+// a warp per window, and every thread its own copies / in this form: 8 reads of 8 to 12 kb (2.1e7 cells,
+// 71 segments) 3.52 / 2.35 / 1.27 ms, 30 reads of 8 to 30 kb (1.5e8 cells) 5.36 / 3.85 / 3.04 ms, 6 reads
+// of 3 to 8 kb at expansion 200 (512 threads) 6.79 / - / 3.88 ms.
 #pragma once
 
 namespace sa {
 namespace fp32 {
 
-// NC columns per lane: 32 NC slots, bands up to column_span(NC) columns
-__host__ __device__ constexpr int column_slots(int nc) { return 32 * nc; }
-__host__ __device__ constexpr int column_span(int nc) { return 31 * nc; }
+// NT threads hold bands up to column_span(NT) columns (a neighbour's column included)
+__host__ __device__ constexpr int column_span(int nt) { return nt - 2; }
 
+constexpr int kAhead = 6;                // anti-diagonals between a copy and its use
+constexpr int kRows = 8;                 // rows of the copy rings
+constexpr int kInfoRows = 128;           // rows of band facts kept
+constexpr int kBlock = 10;               // anti-diagonals per total probability
+constexpr int kPostRows = 64;            // anti-diagonals the posteriors' warp may lag (about 2 kBlock)
 
 extern __shared__ float4 column_smem[];
 
-// lae() with the table at the start of shared memory.  C - 2 d rounded down, C a multiple of 16 large
-// enough that the last place is 1/16, holds -ceil(2 d) mod 16 in bits 4..7: the byte offset of the
-// piece, without a shift.  The cut-off is a predicated add.
+// lae() with the table at the start of shared memory, in two halves: entries of 8 bytes lie in banks of
+// their own, so lanes with different pieces do not conflict (16 bytes an entry put two on a bank: the
+// forward sweep's step took 1.3 times as long).  C - 2 d rounded down, C a multiple of 16 large enough
+// that the last place is 1/8, holds -ceil(2 d) mod 16 in bits 3..6: the byte offset of the piece,
+// without a shift.  The cut-off is a predicated add.
+struct LogAddHalves {
+    float2 hi[16], lo[16];               // (a3, a2), (a1, a0) of the piece of -ceil(2 d) mod 16
+};
+
+__device__ __forceinline__ float4 lac_piece(float d) {
+    const int k = __float_as_int(__fmaf_rd(d, -2.0f, 1572864.0f)) & 0x78;
+    const char *t = reinterpret_cast<const char *>(column_smem) + k;
+    const float2 h = *reinterpret_cast<const float2 *>(t);
+    const float2 l = *reinterpret_cast<const float2 *>(t + sizeof(LogAddHalves::hi));
+    return make_float4(h.x, h.y, l.x, l.y);
+}
+
 __device__ __forceinline__ float lac(float x, float y) {
     float mx = fmaxf(x, y);
     const float d = fabsf(x - y);
-    const int k = __float_as_int(__fmaf_rd(d, -2.0f, 786432.0f)) & 0xf0;
-    const float4 c = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(column_smem) + k);
+    const float4 c = lac_piece(d);
     const float h = fmaf(fmaf(fmaf(c.x, d, c.y), d, c.z), d, c.w);
     asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, 0f40F00000;\n\t@p add.rn.f32 %0, %0, %2;\n\t}"
         : "+f"(mx) : "f"(d), "f"(h));
     return mx;
 }
 
-// the element of a lane's first slot on an anti-diagonal whose first column is xf: slots r = 0..3
-// hold cells j + r (negative, or at least the width: outside the band)
-template <int NC>
-__device__ __forceinline__ int32_t first_cell_of_lane(int lane, int32_t xf) {
-    return ((NC * lane - (xf & ~(NC - 1))) & (column_slots(NC) - 1)) - (xf & (NC - 1));
+// N independent ones, stage by stage
+template <int N>
+__device__ __forceinline__ void lacs(const float (&x)[N], const float (&y)[N], float (&r)[N]) {
+    float d[N];
+    float4 c[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) d[j] = fabsf(x[j] - y[j]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) c[j] = lac_piece(d[j]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) r[j] = fmaxf(x[j], y[j]);
+    float h[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) h[j] = fmaf(c[j].x, d[j], c[j].y);
+#pragma unroll
+    for (int j = 0; j < N; ++j) h[j] = fmaf(h[j], d[j], c[j].z);
+#pragma unroll
+    for (int j = 0; j < N; ++j) h[j] = fmaf(h[j], d[j], c[j].w);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+        asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, 0f40F00000;\n\t@p add.rn.f32 %0, %0, %2;\n\t}"
+            : "+f"(r[j]) : "f"(d[j]), "f"(h[j]));
 }
 
-__device__ __forceinline__ bool cell_in(int32_t j, int r, int32_t W) { return (uint32_t) (j + r) < (uint32_t) W; }
+__device__ __forceinline__ void copy_async4(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
 
-// skip emissions of a lane's columns: the machine's one value, or per column
-template <int NC, bool kGX>
-struct Skip {
-    float v[kGX ? NC : 1];
-    __device__ __forceinline__ float operator[](int r) const { return v[kGX ? r : 0]; }
-    // columns x0 .. x0 + 3
-    __device__ __forceinline__ void load(const Ctx &c, int32_t x0) {
-        if (!kGX) {
-            v[0] = c.gx;
-            return;
-        }
-#pragma unroll
-        for (int r = 0; r < NC; ++r) v[kGX ? r : 0] = raw_gapx(c, x0 + r);
-    }
-};
+__device__ __forceinline__ void copy_async8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// barrier `id` of the CTA over n threads (the sweep's warps, or they and the warp of the posteriors)
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+enum { kBarRow = 1, kBarFull = 2, kBarEmpty = 4 };   // kBarFull + b, kBarEmpty + b: block buffer b
+constexpr int kHelpers = 96;             // threads of the warps beside a sweep's: shifts, copies, results
 
 // ------------------------------------------------------------------------------------------------
-// forward sweep of one segment by a CTA: a column per thread
+// band facts of a sweep, 32 anti-diagonals at a time, by its service warp
 // ------------------------------------------------------------------------------------------------
-// The sweep is a chain of dependent anti-diagonals, so its latency is what counts.  Thread t holds the
-// column x with x mod 128 == t.  The recursion needs the column to the left on d-1 (for gap-X) and on
-// d-2 (for the match, so a step early), and its own column on d-1 (gap-Y): the left column comes by
-// shuffle, across a warp's edge through one shared float4, and only gap-X sits between one
-// anti-diagonal's barrier and the next.  Emissions and band facts come in groups of kGroup
-// anti-diagonals, a whole group ahead: waits on loads are then for loads of a group ago, not for the
-// newest ones (a warp waits for all of its loads that share a scoreboard).
-constexpr int kGroup = 4;
-
-struct ColumnForwardShared {
-    float4 edge[2][kWarps];             // match, gap-X, gap-Y of a warp's last column, by parity of d
-    float part[2][kWarps];              // the warps' largest values, by parity of d
+// The k-th anti-diagonal of the sweep is start + DIR k.  A block is loaded when the sweep is 64
+// anti-diagonals before it and becomes readable half a block later.
+struct InfoRing {
+    int4 row[kInfoRows];                 // first column, width | flags, first cell, shift
+    double base[kInfoRows];              // forward base (backward sweeps)
 };
 
-template <bool kSX, bool kGX>
-struct ColumnForward {
-    const Ctx &c;
-    const Args &A;
-    const RegionDesc &R;
-    const Segment &S;
-    ColumnForwardShared *fs;
-    int tid, lane, warp;
+template <int DIR>
+struct RowStream {
+    InfoRing *ring;
+    const Args *A;
     int64_t db;
-    int32_t n, dbeg, dend;
-    const float2 *Ereg;
-    float *Freg;
-    float M1, X1, Y1;             // own column on d-1
-    float lM2, lX2, lY2;          // left column on d-2
-    float2 e[kGroup], e_next[kGroup];
-    float g[kGX ? kGroup : 1], g_next[kGX ? kGroup : 1];
-    int2 m[kGroup], m_next[kGroup];   // raw band facts of this group and the next
-    int32_t off, off_next;        // first cell of d, and of the next group's first anti-diagonal
-    int32_t cap;                  // next anti-diagonal whose values a stitch takes
-    float mxw;                    // this warp's largest value on d-1
-    float delta0, delta1;         // delta(d) = base(d) - base(d-1), delta(d-1)
-    double base0;                 // base(d)
-    double qbase;                 // lane q of warp 0: base and shift of the last d with d mod 32 == q
-    float qshift;
-    int32_t wi;
+    int lane;
+    int32_t n, start, acc;               // acc: first cell of the next block (backward: past it)
+    int2 raw;
+    double base;
+    float shift;
 
-    __device__ __forceinline__ ColumnForward(const Ctx &cc, const Segment &sg, ColumnForwardShared *f)
-        : c(cc), A(*cc.A), R(cc.R), S(sg), fs(f) {}
-
-    __device__ __forceinline__ int32_t cell_of(int32_t d, int2 mt) const {
-        return (tid - ((d + mt.x) >> 1)) & (kThreads - 1);
-    }
-
-    // band facts of dd .. dd + kGroup - 1
-    __device__ __forceinline__ void fetch_meta(int32_t dd, int2 (&o)[kGroup]) const {
-#pragma unroll
-        for (int k = 0; k < kGroup; ++k) o[k] = raw_meta(A, db, dd + k, n);
-    }
-
-    // emissions of dd .. dd + kGroup - 1 (band facts mt, first cell o of dd); returns the first cell after
-    __device__ __forceinline__ int32_t fetch(int32_t dd, const int2 (&mt)[kGroup], int32_t o, float2 (&ee)[kGroup],
-                                             float (&gg)[kGX ? kGroup : 1]) const {
-#pragma unroll
-        for (int k = 0; k < kGroup; ++k) {
-            const int32_t i = cell_of(dd + k, mt[k]);
-            ee[k] = __ldg(Ereg + o + i);
-            if (kGX) gg[kGX ? k : 0] = raw_gapx(c, ((dd + k + mt[k].x) >> 1) + i);
-            o += dd + k <= n ? mt[k].y & kWidthMask : 0;
+    __device__ __forceinline__ void load(int32_t k0) {
+        const int32_t d = start + DIR * (k0 + lane), dc = clampi(d, 0, n);
+        raw = __ldg(A->meta + db + dc);
+        if (d < 0 || d > n) raw.y = 0;   // no such anti-diagonal: no cells
+        if (DIR < 0) {
+            base = __ldcg(A->base + db + dc);
+            shift = __ldcg(A->fshift + db + dc);
         }
-        return o;
     }
+    __device__ __forceinline__ void publish(int32_t k0) {
+        const int32_t k = k0 + lane, d = start + DIR * k, W = raw.y & kWidthMask;
+        int32_t sum = W;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        const int32_t first = DIR > 0 ? acc + sum - W : acc - sum;
+        ring->row[k & (kInfoRows - 1)] = make_int4((d + raw.x) >> 1, raw.y, first, __float_as_int(shift));
+        if (DIR < 0) ring->base[k & (kInfoRows - 1)] = base;
+        acc += DIR * __shfl_sync(0xffffffffu, sum, 31);
+        __syncwarp();
+    }
+    // first: first cell of the first anti-diagonal (backward: past it)
+    __device__ __forceinline__ void open(InfoRing *r, const Args &a, int64_t diag_base, int32_t nn, int32_t d0,
+                                         int32_t first) {
+        ring = r;
+        A = &a;
+        db = diag_base;
+        lane = threadIdx.x & 31;
+        n = nn;
+        start = d0;
+        acc = first;
+        shift = 0.0f;
+        base = 0.0;
+        load(0);
+        publish(0);
+        load(32);
+        publish(32);
+    }
+    __device__ __forceinline__ void advance(int32_t k) {
+        if ((k & 31) == 0) load(k + 64);
+        else if ((k & 31) == 16) publish(k + 48);
+    }
+    __device__ __forceinline__ int4 at(int32_t k) const { return ring->row[k & (kInfoRows - 1)]; }
+};
 
-    // the values of d-1 (own column) and the largest values go out, then d is computed; k: d's place
-    // in its group, Q: the parity of d
-    template <int K, int Q>
-    __device__ __forceinline__ void step(int32_t d) {
-        const float *t = c.t;
-        const int32_t W = m[K].y & kWidthMask, flags = m[K].y & ~kWidthMask;
-        const int32_t i = cell_of(d, m[K]);
-        const bool in = i < W;
-        // d-1 to the right-hand neighbours (Q ^ 1: its parity)
-        if (lane == 31) fs->edge[Q ^ 1][warp] = make_float4(M1, X1, Y1, 0.0f);
-        if (lane == 0) fs->part[Q ^ 1][warp] = mxw;
-        // meanwhile what does not depend on them: match and gap-Y of d
-        const float shL = -delta0, shM = -delta1 - delta0;
-        float vM = lac(lM2 + t[T_MC], lX2 + t[T_MFGX]);
-        vM = lac(vM, lY2 + t[T_MFGY]) + (e[K].x + shM);
-        float vY = lac(M1 + t[T_OY], Y1 + t[T_EY]) + (e[K].y + shL);
+// ------------------------------------------------------------------------------------------------
+// shared memory
+// ------------------------------------------------------------------------------------------------
+// what a sweep's thread needs of an anti-diagonal, from the service warp
+struct alignas(16) RowFacts {
+    int32_t xf, w;                       // first column; width | flags
+    float sh1, sh2;                      // the shifts of the values from one and from two anti-diagonals back
+};
+constexpr int32_t kRowPost = 1 << 23;    // posteriors of the anti-diagonal are the window's
+
+template <int NT>
+struct ColumnForwardShared {
+    float2 e[kRows][NT];                 // match and extra-event emissions, by cell
+    InfoRing info;
+    RowFacts row[4];
+    float4 edge[2][NT / 32];             // match, gap-X, gap-Y of a warp's last column, by parity
+    float part[2][NT / 32];              // the warps' largest values, by parity
+    float v[2][3][NT];                   // values by thread, by parity
+};
+
+template <int NT>
+struct ColumnWindowShared {
+    float2 e[kRows][NT];
+    InfoRing info;
+    RowFacts row[4];
+    float f[kRows][NT];                  // forward match values, by cell
+    float ops[5][NT];                    // a total's anti-diagonal d: gap-X, gap-Y of d; match, gap-X, gap-Y of d-1
+    float4 edge[2][NT / 32];             // match and its emission a row back, gap-X, skip emission of a warp's
+                                         // first column, by parity
+    float part[2][NT / 32];
+    // for the posteriors' warp: by anti-diagonal of the sweep, its base and this window's; and two
+    // blocks of kBlock anti-diagonals: F.B of the match state by thread, the two folds' terms, and the
+    // shift and gamma of the total's anti-diagonal
+    double fb[kPostRows], bb[kPostRows];
+    int2 post[kPostRows];                // first column, width
+    float s[2][kBlock][NT];
+    float chain[2][2][NT];
+    float2 through[2];
+    int2 widths[2];                      // of the two folds
+};
+static_assert(offsetof(ColumnForwardShared<128>, e) == offsetof(ColumnWindowShared<128>, e), "one emission ring");
+
+template <int NT>
+struct alignas(16) ColumnShared {
+    LogAddHalves la;
+    union {
+        ColumnForwardShared<NT> f;
+        ColumnWindowShared<NT> w;
+    };
+    int32_t task;
+};
+
+// ------------------------------------------------------------------------------------------------
+// one side of a stitch, and its check, by one warp (see stitch_check)
+// ------------------------------------------------------------------------------------------------
+__device__ __noinline__ void warp_stitch_check(const Args &A, int32_t si) {
+    const int lane = threadIdx.x & 31;
+    const StitchDesc sd = A.stitch[si];
+    StitchRes &res = A.stitch_res[si];
+    const double sb0 = __ldcg(&res.sbase[0]), sb1 = __ldcg(&res.sbase[1]);
+    const double tb0 = __ldcg(&res.tbase[0]), tb1 = __ldcg(&res.tbase[1]);
+    const int32_t nv = 3 * (sd.w0 + sd.w1);
+    const float *spec = A.stitch_vals + sd.voff, *tru = spec + nv;
+    double amax = -INFINITY, dref = 0.0;
+    for (int q = lane; q < nv; q += 32) {
+        const bool j = q >= 3 * sd.w0;
+        const float tv = __ldcg(tru + q), sv = __ldcg(spec + q);
+        if (tv > kNegInf && sv > kNegInf) {
+            const double a = (double) tv + (j ? tb1 : tb0);
+            if (a > amax) {
+                amax = a;
+                dref = a - ((double) sv + (j ? sb1 : sb0));
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double a2 = __shfl_xor_sync(0xffffffffu, amax, o), d2 = __shfl_xor_sync(0xffffffffu, dref, o);
+        if (a2 > amax || (a2 == amax && d2 < dref)) {
+            amax = a2;
+            dref = d2;
+        }
+    }
+    const double scale = (double) A.stitch_tol;
+    bool ok = scale >= 0.0;
+    double spread = 0.0;
+    for (int q = lane; q < nv; q += 32) {
+        const bool j = q >= 3 * sd.w0;
+        const float tv = __ldcg(tru + q), sv = __ldcg(spec + q);
+        const bool ft = tv > kNegInf, fs = sv > kNegInf;
+        if (ft != fs) {
+            ok = false;
+        } else if (ft) {
+            const double a = (double) tv + (j ? tb1 : tb0);
+            const double dev = fabs((a - ((double) sv + (j ? sb1 : sb0))) - dref);
+            spread = fmax(spread, dev);
+            if (!(dev <= scale * (2e-5 + 1e-6 * (amax - a)))) ok = false;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) spread = fmax(spread, __shfl_xor_sync(0xffffffffu, spread, o));
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) {
+        res.delta = dref;
+        res.spread = (float) spread;
+        res.result = ok ? kStitchAgreed : kStitchDisagreed;
+        if (!ok) atomicExch(A.seg_fail + sd.read, 1);
+        __threadfence();
+    }
+    __syncwarp();
+    read_unit_done<32>(A, sd.read, lane, nullptr);
+}
+
+// one side of stitch si has written its values: the second to arrive checks it (one warp)
+__device__ __forceinline__ void warp_stitch_arrive(const Args &A, int32_t si) {
+    int32_t before = 0;
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence();
+        before = atomicAdd(&A.stitch_res[si].arrive, 1);
+        __threadfence();
+    }
+    if (__shfl_sync(0xffffffffu, before, 0) == 1) warp_stitch_check(A, si);
+}
+
+// ------------------------------------------------------------------------------------------------
+// forward sweep of one segment
+// ------------------------------------------------------------------------------------------------
+// On anti-diagonal d a thread folds, side by side: gap-X of d (left column on d-1), gap-Y of d (own
+// column on d-1), the match state of d+1 but for its last term (left column on d-1), and the last
+// term of d's: one logAdd's latency, a barrier and a shared-memory read a step.
+template <int NT, bool kSX, bool kGX>
+__device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs) {
+    constexpr int NW = NT / 32;
+    const Args &A = *c.A;
+    const RegionDesc &R = c.R;
+    const float *t = c.t;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int32_t dbeg = S.d_begin, s = dbeg - S.warm + (dbeg == 0 ? 1 : 0), steps = S.d_end - s + 1;
+    // own column on d-1, and d's match state but for its last term, and that term
+    float M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf, most = kNegInf, last = kNegInf;
+    float mxw;                           // this warp's largest value on d-1
+    if (dbeg == 0) {
+        // anti-diagonal 0: startStateProb / raggedStartStateProb (stateMachine.c:1022-1032), column 0
+        const float s0 = R.ragged_left ? kNegInf : 0.0f, s1 = R.ragged_left ? 0.0f : kNegInf;
+        if (tid == 0) {
+            M1 = s0;
+            X1 = Y1 = s1;
+        }
+        mxw = warp == 0 ? fmaxf(s0, s1) : kNegInf;
+    } else {
+        // a later segment: every band cell of s-2 and s-1 starts at 0
+        const int2 r2 = raw_meta(A, R.diag_base, s - 2, R.n), r1 = raw_meta(A, R.diag_base, s - 1, R.n);
+        if (((tid - ((s - 1 + r1.x) >> 1)) & (NT - 1)) < (r1.y & kWidthMask)) M1 = X1 = Y1 = 0.0f;
+        const bool left = ((tid - 1 - ((s - 2 + r2.x) >> 1)) & (NT - 1)) < (r2.y & kWidthMask);
+        const float z = left ? 0.0f : kNegInf;
+        most = lac(z + t[T_MC], z + t[T_MFGX]);
+        last = z + t[T_MFGY];
+        mxw = 0.0f;
+    }
+    if (lane == 0) fs->part[1][warp] = mxw;
+    if (lane == 31) fs->edge[1][warp] = make_float4(M1, X1, Y1, 0.0f);
+    const float4 *edge = &fs->edge[0][(warp + NW - 1) & (NW - 1)];
+    bar_sync(kBarRow, NT + kHelpers);          // the first rows are ready
+    RowFacts row = fs->row[0];
+    bool inb = ((tid - row.xf) & (NT - 1)) < (row.w & kWidthMask);
+    float2 e = fs->e[0][(tid - row.xf) & (NT - 1)];
+    float gx = 0.0f;
+    if (kGX) gx = raw_gapx(c, row.xf + ((tid - row.xf) & (NT - 1)));
+#pragma unroll 2
+    for (int32_t k = 0; k < steps; ++k) {
         float lM = __shfl_up_sync(0xffffffffu, M1, 1), lX = __shfl_up_sync(0xffffffffu, X1, 1),
               lY = __shfl_up_sync(0xffffffffu, Y1, 1);
-        // shift of d+1 from the maximum of d-2 (its parity is d's; complete since the last barrier)
-        float delta_next = 0.0f;
-        if (d >= 2) {
-            const float4 fp = *reinterpret_cast<const float4 *>(fs->part[Q]);
-            const float mx = fmaxf(fmaxf(fp.x, fp.y), fmaxf(fp.z, fp.w));
-            delta_next = ((mx > kNegInf ? mx : 0.0f) - delta0) - delta1;
-        }
-        __syncthreads();
-        const float4 ed = fs->edge[Q ^ 1][(warp + kWarps - 1) & (kWarps - 1)];
+        float x[4], y[4], r[4];
+        x[1] = M1 + t[T_OY];
+        y[1] = Y1 + t[T_EY];
+        x[2] = most;
+        y[2] = last;
+        bar_sync(kBarRow, NT + kHelpers);      // d-1's edges; d+1's facts and emissions
+        const float4 ed = edge[((k + 1) & 1) * NW];
+        const RowFacts next = fs->row[(k + 1) & 3];
         if (lane == 0) {
             lM = ed.x;
             lX = ed.y;
             lY = ed.z;
         }
-        float vX = lac(lM + t[T_OX], lX + t[T_EX]);
-        if (kSX) vX = lac(vX, lY + t[T_SX]);
-        vX = vX + ((kGX ? g[kGX ? K : 0] : c.gx) + shL);
-        vM = in ? vM : kNegInf;
-        vX = in ? vX : kNegInf;
-        vY = in ? vY : kNegInf;
-        const bool own = d > dbeg;
-        if (in && own) {
-            float *Fd = Freg + 3 * (int64_t) off + i;
-            Fd[0] = vM;
-            if (flags & kFlagStoreGaps) {
-                Fd[W] = vX;
-                Fd[2 * W] = vY;
+        x[0] = lM + t[T_OX];
+        y[0] = lX + t[T_EX];
+        x[3] = lM + t[T_MC];
+        y[3] = lX + t[T_MFGX];
+        const int32_t i = (tid - next.xf) & (NT - 1);
+        const float2 e_next = fs->e[(k + 1) & (kRows - 1)][i];
+        lacs<4>(x, y, r);
+        if (kSX) r[0] = lac(r[0], lY + t[T_SX]);
+        const float vX = r[0] + ((kGX ? gx : c.gx) + row.sh1);
+        const float vY = r[1] + (e.y + row.sh1);
+        const float vM = r[2] + (e.x + row.sh2);
+        most = r[3];
+        last = lY + t[T_MFGY];
+        M1 = inb ? vM : kNegInf;
+        X1 = inb ? vX : kNegInf;
+        Y1 = inb ? vY : kNegInf;
+        if (lane == 31) fs->edge[k & 1][warp] = make_float4(M1, X1, Y1, 0.0f);
+        mxw = warp_max1(fmaxf(M1, fmaxf(X1, Y1)));
+        if (lane == 0) fs->part[k & 1][warp] = mxw;
+        fs->v[k & 1][0][tid] = M1;
+        fs->v[k & 1][1][tid] = X1;
+        fs->v[k & 1][2][tid] = Y1;
+        row = next;
+        inb = i < (next.w & kWidthMask);
+        e = e_next;
+        if (kGX) gx = raw_gapx(c, row.xf + i);
+    }
+    bar_sync(kBarRow, NT + kHelpers);          // the last anti-diagonal's values go out
+}
+
+// The largest of the warps' values (part: one row of them)
+template <int NW>
+__device__ __forceinline__ float part_max(const float *part) {
+    float m[NW];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) m[w] = part[w];
+#pragma unroll
+    for (int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int w = 0; w < NW / 2; ++w)
+            if (w < o) m[w] = fmaxf(m[w], m[w + o]);
+    return m[0];
+}
+
+// The forward sweep's shifts: at step k (anti-diagonal d) those of d+2, from the maximum of d-1.
+// Renormalisation as in ForwardSweep: base(d+1) = base(d-2) + max(d-2); delta(d) = base(d) - base(d-1).
+template <int NT>
+__device__ __forceinline__ void column_forward_shifts(const Segment &S, ColumnForwardShared<NT> *fs) {
+    const int lane = threadIdx.x & 31;
+    const int32_t s = S.d_begin - S.warm + (S.d_begin == 0 ? 1 : 0), steps = S.d_end - s + 1;
+    float d0 = 0.0f, d1 = 0.0f;          // delta of d and of d+1 (max(s-2) counts as 0)
+    if (lane < 2) *reinterpret_cast<float2 *>(&fs->row[lane].sh1) = make_float2(-d0, -d0 - d0);
+    bar_sync(kBarRow, NT + kHelpers);
+#pragma unroll 2
+    for (int32_t k = 0; k < steps; ++k) {
+        bar_sync(kBarRow, NT + kHelpers);
+        const float mx = part_max<NT / 32>(fs->part[(k + 1) & 1]);
+        const float d2 = ((mx > kNegInf ? mx : 0.0f) - d1) - d0;
+        if (lane == 0) *reinterpret_cast<float2 *>(&fs->row[(k + 2) & 3].sh1) = make_float2(-d2, -d1 - d2);
+        d0 = d1;
+        d1 = d2;
+    }
+    bar_sync(kBarRow, NT + kHelpers);
+}
+
+// The forward sweep's copies: at step k the emissions of the kAhead-th anti-diagonal after, and the
+// place of the second.
+template <int NT>
+__device__ __forceinline__ void column_forward_copies(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs) {
+    constexpr int NW = NT / 32;
+    const Args &A = *c.A;
+    const RegionDesc &R = c.R;
+    const int lane = threadIdx.x & 31;
+    const int32_t s = S.d_begin - S.warm + (S.d_begin == 0 ? 1 : 0), steps = S.d_end - s + 1;
+    const float2 *Ereg = A.E + R.cell_base + lane;
+    RowStream<1> info;
+    info.open(&fs->info, A, R.diag_base, R.n, s, (int32_t) S.cell0);
+    auto issue = [&](int32_t k, const int4 &in) {
+        const int32_t W = in.y & kWidthMask;
+        const float2 *src = Ereg + in.z;
+        float2 *dst = &fs->e[k & (kRows - 1)][lane];
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+            if (lane + 32 * w < W) copy_async8(dst + 32 * w, src + 32 * w);
+        copy_commit();
+    };
+    auto place = [&](int32_t k) {
+        const int4 in = info.at(k);
+        if (lane == 0) *reinterpret_cast<int2 *>(&fs->row[k & 3].xf) = make_int2(in.x, in.y);
+    };
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) issue(k, info.at(k));
+    place(0);
+    place(1);
+    copy_wait<kAhead - 2>();
+    int4 in = info.at(kAhead);
+    bar_sync(kBarRow, NT + kHelpers);
+    for (int32_t k = 0; k < steps; ++k) {
+        bar_sync(kBarRow, NT + kHelpers);
+        issue(k + kAhead, in);
+        place(k + 2);
+        info.advance(k);
+        in = info.at(k + kAhead + 1);
+        copy_wait<kAhead - 2>();         // every copy of d+2 and before has landed
+    }
+    bar_sync(kBarRow, NT + kHelpers);
+    copy_wait<0>();
+}
+
+// The forward sweep's results: at step k d-1's values, base and shift go out, a window that closes there
+// is published, and a stitch there gets its side.
+template <int NT>
+__device__ __forceinline__ void column_forward_results(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs) {
+    constexpr int NW = NT / 32;
+    const Args &A = *c.A;
+    const RegionDesc &R = c.R;
+    const int lane = threadIdx.x & 31;
+    const int64_t db = R.diag_base;
+    const int32_t dbeg = S.d_begin, dend = S.d_end;
+    const int32_t s = dbeg - S.warm + (dbeg == 0 ? 1 : 0), steps = dend - s + 1;
+    float *Freg = A.F + 3 * R.cell_base;
+    if (dbeg == 0 && lane == 0) {
+        const float s0 = R.ragged_left ? kNegInf : 0.0f, s1 = R.ragged_left ? 0.0f : kNegInf;
+        Freg[ST_M] = s0;
+        Freg[ST_X] = s1;
+        Freg[ST_Y] = s1;
+        A.base[db] = 0.0;
+        A.fshift[db] = 0.0f;
+    }
+    double base = 0.0;                   // base(d-1)
+    double qbase = 0.0;                  // lane q: base and shift of the last d with d mod 32 == q
+    float qshift = 0.0f;
+    int32_t wi = S.wi0;
+    int32_t cap = S.stitch_in >= 0 ? dbeg - 1 : (S.stitch_out >= 0 ? dend - 1 : INT32_MAX);
+    bar_sync(kBarRow, NT + kHelpers);
+    bar_sync(kBarRow, NT + kHelpers);    // step 0
+    int4 in = fs->info.row[0];
+    for (int32_t k = 1; k <= steps; ++k) {
+        const int32_t r = s + k - 1;     // the anti-diagonal that goes out
+        const int32_t W = in.y & kWidthMask;
+        const bool own = r > dbeg, gaps = (in.y & kFlagStoreGaps) != 0;
+        float *Fd = Freg + 3 * (int64_t) in.z + lane;
+        int at[NW];
+#pragma unroll
+        for (int w = 0; w < NW; ++w) at[w] = (in.x + lane + 32 * w) & (NT - 1);
+        bar_sync(kBarRow, NT + kHelpers);
+        const float(*v)[NT] = fs->v[(k - 1) & 1];
+        if (own) {
+            float o[NW];
+#pragma unroll
+            for (int w = 0; w < NW; ++w) o[w] = v[0][at[w]];
+#pragma unroll
+            for (int w = 0; w < NW; ++w)
+                if (lane + 32 * w < W) Fd[32 * w] = o[w];
+            if (gaps) {
+#pragma unroll
+                for (int w = 0; w < NW; ++w) {
+                    if (lane + 32 * w < W) {
+                        Fd[W + 32 * w] = v[1][at[w]];
+                        Fd[2 * W + 32 * w] = v[2][at[w]];
+                    }
+                }
             }
         }
-        mxw = warp_max1(fmaxf(vM, fmaxf(vX, vY)));
-        // base and shift of d: lane d mod 32 of warp 0 keeps them and the warp writes them out 32 at a
-        // time and before a window is published (its backward sweep reads them)
-        const bool window_end = own && (flags & kFlagWindowEnd) != 0;
-        const int q = d & 31;
+        const float delta = -fs->row[(k - 1) & 3].sh1, delta_next = -fs->row[k & 3].sh1;
+        const int4 in_next = fs->info.row[k & (kInfoRows - 1)];
+        base += (double) delta;
+        const bool window_end = own && (in.y & kFlagWindowEnd) != 0;
+        const int q = r & 31;
         if (lane == q) {
-            qbase = base0;
-            qshift = delta0;
+            qbase = base;
+            qshift = delta;
         }
-        if (q == 31 || window_end || d == dend) {
-            if (warp == 0 && lane <= q && d - q + lane > dbeg) {
-                A.base[db + (d - q) + lane] = qbase;
-                A.fshift[db + (d - q) + lane] = qshift;
+        if (q == 31 || window_end || r == dend) {
+            if (lane <= q && r - q + lane > dbeg) {
+                A.base[db + (r - q) + lane] = qbase;
+                A.fshift[db + (r - q) + lane] = qshift;
             }
             if (window_end) {
-                __threadfence();   // this anti-diagonal and all before it, device-wide
-                __syncthreads();
-                if (tid == 0) {
-                    const unsigned at = atomicAdd(&A.ctl->pub, 1u);
-                    if ((int64_t) at < A.n_windows) atomicExch(A.ready + at, (int32_t) (R.win_base + wi));
+                __threadfence();         // this anti-diagonal and all before it, device-wide
+                __syncwarp();
+                if (lane == 0) {
+                    const unsigned p = atomicAdd(&A.ctl->pub, 1u);
+                    if ((int64_t) p < A.n_windows) atomicExch(A.ready + p, (int32_t) (R.win_base + wi));
                 }
                 ++wi;
             }
         }
-        off += W;
-        lM2 = lM;
-        lX2 = lX;
-        lY2 = lY;
-        M1 = vM;
-        X1 = vX;
-        Y1 = vY;
-        delta1 = delta0;
-        delta0 = delta_next;
-        base0 += (double) delta_next;
-        if (d == cap) cap = capture(d, i, in);
-    }
-
-    // the values of d (now M1, X1, Y1) to their side of a stitch: called on b-1 and on b, where the
-    // segment begins or ends; base0 and delta0 / delta1 already describe d+1.  Returns the next such d.
-    __device__ __forceinline__ int32_t capture(int32_t d, int32_t i, bool in) const {
-        const bool in_side = S.stitch_in >= 0 && d <= dbeg;
-        const int32_t si = in_side ? S.stitch_in : S.stitch_out, b = in_side ? dbeg : dend;
-        const StitchDesc sd = A.stitch[si];
-        float *o = A.stitch_vals + sd.voff + (in_side ? 0 : 3 * (sd.w0 + sd.w1)) + (d == b ? 3 * sd.w0 : 0) + i;
-        const int32_t W = d == b ? sd.w1 : sd.w0;
-        if (in) {
-            o[0] = M1;
-            o[W] = X1;
-            o[2 * W] = Y1;
-        }
-        if (d == b && tid == 0) {
-            const double base_b = base0 - (double) delta0, base_b1 = base_b - (double) delta1;
-            double *bs = in_side ? A.stitch_res[si].sbase : A.stitch_res[si].tbase;
-            bs[0] = base_b1;
-            bs[1] = base_b;
-        }
-        return d < b ? b : (in_side && S.stitch_out >= 0 ? dend - 1 : INT32_MAX);
-    }
-
-    __device__ __forceinline__ void run(Shared *sh) {
-        tid = threadIdx.x;
-        lane = tid & 31;
-        warp = tid >> 5;
-        db = R.diag_base;
-        n = R.n;
-        dbeg = S.d_begin;
-        dend = S.d_end;
-        const int32_t s = dbeg - S.warm + (dbeg == 0 ? 1 : 0);
-        Ereg = A.E + R.cell_base;
-        Freg = A.F + 3 * R.cell_base;
-        off = (int32_t) S.cell0;
-        M1 = X1 = Y1 = lM2 = lX2 = lY2 = kNegInf;
-        // steps run in pairs of parities 0 and 1 (of d - s): s-1 has parity 1, s-2 parity 0
-        if (dbeg == 0) {
-            // anti-diagonal 0: startStateProb / raggedStartStateProb (stateMachine.c:1022-1032), column 0
-            const float s0 = R.ragged_left ? kNegInf : 0.0f, s1 = R.ragged_left ? 0.0f : kNegInf;
-            if (tid == 0) {
-                M1 = s0;
-                X1 = Y1 = s1;
-                Freg[ST_M] = s0;
-                Freg[ST_X] = s1;
-                Freg[ST_Y] = s1;
-                A.base[db] = 0.0;
-                A.fshift[db] = 0.0f;
+        if (r == cap) {
+            const bool in_side = S.stitch_in >= 0 && r <= dbeg;
+            const int32_t si = in_side ? S.stitch_in : S.stitch_out, b = in_side ? dbeg : dend;
+            const StitchDesc sd = A.stitch[si];
+            float *o = A.stitch_vals + sd.voff + (in_side ? 0 : 3 * (sd.w0 + sd.w1)) + (r == b ? 3 * sd.w0 : 0);
+            for (int i = lane; i < W; i += 32)
+                for (int st = 0; st < 3; ++st) o[st * W + i] = v[st][(in.x + i) & (NT - 1)];
+            if (r == b && lane == 0) {
+                // as ForwardSweep: back from the base past b
+                const double past = base + (double) delta_next, base_b = past - (double) delta_next;
+                double *bs = in_side ? A.stitch_res[si].sbase : A.stitch_res[si].tbase;
+                bs[0] = base_b - (double) delta;
+                bs[1] = base_b;
             }
-            mxw = warp == 0 ? fmaxf(s0, s1) : kNegInf;
-        } else {
-            // a later segment: every band cell of s-2 and s-1 starts at 0
-            const int2 r2 = raw_meta(A, db, s - 2, n), r1 = raw_meta(A, db, s - 1, n);
-            if (cell_of(s - 1, r1) < (r1.y & kWidthMask)) M1 = X1 = Y1 = 0.0f;
-            if (((cell_of(s - 2, r2) - 1) & (kThreads - 1)) < (r2.y & kWidthMask)) lM2 = lX2 = lY2 = 0.0f;
-            mxw = 0.0f;
+            cap = r < b ? b : (in_side && S.stitch_out >= 0 ? dend - 1 : INT32_MAX);
         }
-        if (lane == 0) fs->part[0][warp] = 0.0f;   // maximum of s-2, where there is one
-        fetch_meta(s, m);
-        off_next = fetch(s, m, off, e, g);
-        fetch_meta(s + kGroup, m_next);
-        // renormalisation as in ForwardSweep: base(d+1) = base(d-2) + max(d-2)
-        delta0 = delta1 = 0.0f;
-        base0 = 0.0;
-        qbase = 0.0;
-        qshift = 0.0f;
-        wi = S.wi0;
-        cap = S.stitch_in >= 0 ? dbeg - 1 : (S.stitch_out >= 0 ? dend - 1 : INT32_MAX);
-        __syncthreads();
-        for (int32_t d = s; d <= dend; d += kGroup) {
-            off_next = fetch(d + kGroup, m_next, off_next, e_next, g_next);
-            int2 m_after[kGroup];
-            fetch_meta(d + 2 * kGroup, m_after);
-            step<0, 0>(d);
-            if (d + 1 > dend) break;
-            step<1, 1>(d + 1);
-            if (d + 2 > dend) break;
-            step<2, 0>(d + 2);
-            if (d + 3 > dend) break;
-            step<3, 1>(d + 3);
-#pragma unroll
-            for (int k = 0; k < kGroup; ++k) {
-                e[k] = e_next[k];
-                if (kGX) g[kGX ? k : 0] = g_next[kGX ? k : 0];
-                m[k] = m_next[k];
-                m_next[k] = m_after[k];
-            }
-        }
-        if (S.stitch_in >= 0) stitch_arrive(A, sh, S.stitch_in);
-        if (S.stitch_out >= 0) stitch_arrive(A, sh, S.stitch_out);
-        __syncthreads();
+        in = in_next;
     }
-};
+    if (S.stitch_in >= 0 || S.stitch_out >= 0) {
+        __threadfence();                 // the stitch's values, before the counts below
+        __syncwarp();
+        if (S.stitch_in >= 0) warp_stitch_arrive(A, S.stitch_in);
+        if (S.stitch_out >= 0) warp_stitch_arrive(A, S.stitch_out);
+    }
+}
 
 // ------------------------------------------------------------------------------------------------
 // the two ordered folds of a refresh
@@ -331,7 +601,7 @@ __device__ __forceinline__ float2 column_folds(float *chain, int na, int nb) {
     for (int k = 0; k < NC; ++k) {
         const int i = lane + 32 * k;
         va[k] = i < na ? chain[i] : kNegInf;
-        vb[k] = i < nb ? chain[column_slots(NC) + i] : kNegInf;
+        vb[k] = i < nb ? chain[(32 * NC) + i] : kNegInf;
         ma = fmaxf(ma, va[k]);
         mb = fmaxf(mb, vb[k]);
     }
@@ -375,14 +645,14 @@ __device__ __forceinline__ float2 column_folds(float *chain, int na, int nb) {
         const bool ib = i >= sb && vb[k] > mb - kFoldGap && (i <= xb || mb - vb[k] < 7.5f);
         const unsigned a = __ballot_sync(0xffffffffu, ia), b = __ballot_sync(0xffffffffu, ib);
         if (ia) chain[ca + __popc(a & below)] = va[k];
-        if (ib) chain[column_slots(NC) + cb + __popc(b & below)] = vb[k];
+        if (ib) chain[(32 * NC) + cb + __popc(b & below)] = vb[k];
         ca += __popc(a);
         cb += __popc(b);
     }
     __syncwarp();
     const bool second = lane >= 16;
     const int mine = second ? cb : ca, most = max(ca, cb);
-    const float *list = chain + (second ? column_slots(NC) : 0);
+    const float *list = chain + (second ? (32 * NC) : 0);
     float r = second ? rb : ra;
     float next = mine > 0 ? list[0] : kNegInf;
     for (int k = 0; k < most; ++k) {
@@ -395,412 +665,393 @@ __device__ __forceinline__ float2 column_folds(float *chain, int na, int nb) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// backward sweep of one traceback window by one warp, posteriors fused
+// backward sweep of one traceback window
 // ------------------------------------------------------------------------------------------------
-// A successor's value plus its emission is summed in the successor's own slot and then shifted by one
-// column, so an anti-diagonal takes two shuffles.  Emissions and forward values come through shared
-// memory, copied asynchronously kAhead anti-diagonals ahead by the lane that reads them (lane-private
-// slots, one group of copies per anti-diagonal), so the wait is for copies that old, and no register
-// holds an operand that is not in use.  Band facts and bases come 32 anti-diagonals at a time, a lane
-// each.
-constexpr int kAhead = 5;                // anti-diagonals between a copy and its first use
-constexpr int kRows = 8;                 // rows of the copy ring: d + 2 .. d - kAhead
-
-template <int NC>
-struct WindowShared {
-    float2 e[kRows][NC][32];            // emissions, row d mod kRows, by register and lane
-    float f[kRows][NC][32];             // forward match values
-    float ops[5][NC][32];               // the next refresh: gap-X, gap-Y of d, match, gap-X, gap-Y of d-1
-    int4 info[64];                      // row d mod 64: first column, width | flags, first cell, shift
-    double base[64];                    // forward base
-    float chain[2 * 32 * NC];           // terms of the two folds
-};
-
-__device__ __forceinline__ void copy_async4(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-
-__device__ __forceinline__ void copy_async8(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-template <int N>
-__device__ __forceinline__ void copy_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-template <int NC, bool kSX, bool kGX>
-struct ColumnWindow {
-    const Ctx &c;
-    const Args &A;
-    const RegionDesc &R;
-    WindowShared<NC> *ws;
-    int lane;
-    int32_t D, T, from;
-    const float2 *Ereg;
-    const float *Freg, *Tside;
-    float vM1[NC], vX1[NC], vY1[NC], vM2[NC];   // backward values of d+1, and match of d+2
-    int32_t j1, W1;               // the lane's first cell and the width on d+1
-    int32_t xf1;                  // first column of d+1
-    int2 raw;                     // band facts, base and shift of the next block of 32, a lane each
-    double raw_base;
-    float raw_shift;
-    int32_t block_top;            // first cell past the next block
-    float mx1, mx2, gamma1;
-    double bbase, pref;
-    int64_t n_out;
-
-    __device__ __forceinline__ ColumnWindow(const Ctx &cc, WindowShared<NC> *w) : c(cc), A(*cc.A), R(cc.R), ws(w) {}
-
-    // band facts and bases of anti-diagonals 32 b + lane
-    __device__ __forceinline__ void load_block(int32_t b) {
-        const int32_t d = clampi(32 * b + lane, 0, R.n);
-        raw = __ldg(A.meta + R.diag_base + d);
-        raw_base = __ldcg(A.base + R.diag_base + d);
-        raw_shift = __ldcg(A.fshift + R.diag_base + d);
-    }
-
-    // the loaded block b becomes readable (anti-diagonals up to `last` of it) and the one below loads
-    __device__ __forceinline__ void open_block(int32_t b, int32_t last) {
-        const int32_t d = 32 * b + lane, W = d <= last ? raw.y & kWidthMask : 0;
-        int32_t sum = W;   // widths of d and the block's later anti-diagonals
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t v = __shfl_down_sync(0xffffffffu, sum, o);
-            if (lane + o < 32) sum += v;
+template <int NT, bool kSX, bool kGX>
+__device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &Wn, ColumnWindowShared<NT> *ws) {
+    constexpr int NW = NT / 32;
+    const RegionDesc &R = c.R;
+    const float *t = c.t;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int32_t D = Wn.D, steps = Wn.D - Wn.T, rows = Wn.from - Wn.T;
+    // end-state values on D (stateMachine.c:1034-1061)
+    const bool ragged_end = Wn.at_end && R.ragged_right;
+    const float e0 = ragged_end ? (t[T_OX] + t[T_OY]) / 2.0f : t[T_MC];
+    const float e1 = ragged_end ? t[T_EX] : t[T_MFGX];
+    const float e2 = ragged_end ? t[T_EY] : t[T_MFGY];
+    if (lane == 0) ws->edge[1][warp] = make_float4(kNegInf, 0.0f, kNegInf, 0.0f);
+    const float4 *edge = &ws->edge[0][(warp + 1) & (NW - 1)];
+    // own column: values and emissions of d+1, match value and emission of d+2
+    float M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf, M2 = kNegInf;
+    float2 e1r = make_float2(0.0f, 0.0f);
+    float eM2 = 0.0f, gx = 0.0f, gx1 = 0.0f;
+    int32_t i1 = 0, W1 = 0, xf1 = 0;     // its cell, the width and the first column of d+1
+    int32_t left = rows;                 // posterior anti-diagonals to come
+    int32_t block = 0, in_block = 0;
+    bar_sync(kBarRow, NT + 64);          // the first rows are ready
+    int2 row = *reinterpret_cast<const int2 *>(&ws->row[0].xf);   // first column, width | flags
+    int32_t i = (tid - row.x) & (NT - 1);
+    float2 e = ws->e[0][i];
+    if (kGX) gx = raw_gapx(c, row.x + i);
+#pragma unroll 1
+    for (int32_t k = 0; k < steps; ++k) {
+        const int32_t W = row.y & kWidthMask;
+        const bool inb = i < W;
+        float nM = __shfl_down_sync(0xffffffffu, M2, 1), nE = __shfl_down_sync(0xffffffffu, eM2, 1),
+              nX = __shfl_down_sync(0xffffffffu, X1, 1), nG = kGX ? __shfl_down_sync(0xffffffffu, gx1, 1) : c.gx;
+        bar_sync(kBarRow, NT + 64);      // d+1's edges, d's shifts; d-1's facts and operands
+        const float4 ed = edge[((k + 1) & 1) * NW];
+        const float2 sh = *reinterpret_cast<const float2 *>(&ws->row[k & 3].sh1);
+        const int2 next = *reinterpret_cast<const int2 *>(&ws->row[(k + 1) & 3].xf);
+        if (lane == 31) {
+            nM = ed.x;
+            nE = ed.y;
+            nX = ed.z;
+            if (kGX) nG = ed.w;
         }
-        ws->info[d & 63] = make_int4((d + raw.x) >> 1, raw.y, block_top - sum, __float_as_int(raw_shift));
-        ws->base[d & 63] = raw_base;
-        block_top -= __shfl_sync(0xffffffffu, sum, 0);
-        __syncwarp();
-        if (b > 0) load_block(b - 1);
+        const float me = nM + (nE + sh.y);
+        const float ue = Y1 + (e1r.y + sh.x);
+        const float le = nX + (nG + sh.x);
+        float x[3], y[3], r[3];
+        x[0] = me + t[T_MC];
+        y[0] = ue + t[T_OY];
+        x[1] = me + t[T_MFGX];
+        y[1] = le + t[T_EX];
+        x[2] = me + t[T_MFGY];
+        y[2] = ue + t[T_EY];
+        const int32_t i_next = (tid - next.x) & (NT - 1);
+        const float2 e_next = ws->e[(k + 1) & (kRows - 1)][i_next];
+        const float f = ws->f[k & (kRows - 1)][i];
+        lacs<3>(x, y, r);
+        r[0] = lac(r[0], le + t[T_OX]);
+        if (kSX) r[2] = lac(r[2], le + t[T_SX]);
+        if (k == 0) {
+            r[0] = e0;
+            r[1] = e1;
+            r[2] = e2;
+        }
+        const float vM = inb ? r[0] : kNegInf, vX = inb ? r[1] : kNegInf, vY = inb ? r[2] : kNegInf;
+        if (lane == 0) ws->edge[k & 1][warp] = make_float4(M1, e1r.x, vX, gx);
+        const float mx = warp_max1(fmaxf(vM, fmaxf(vX, vY)));
+        if (lane == 0) ws->part[k & 1][warp] = mx;
+        if ((row.y & kRowPost) != 0) {
+            const int b = block & 1;
+            if (in_block == 0 && block >= 2) bar_sync(kBarEmpty + b, NT + 32);   // the block before last is done with
+            const float v = f + vM;
+            ws->s[b][in_block][tid] = v;
+            if (in_block == 0) {
+                // diagonalCalculationTotalProbability (pairwiseAligner.c:1182-1200): F.B on d in ascending
+                // cell order, then the matches from d-1 over d into d+1, dotted with B(d+1)
+                if (inb) {
+                    float w = lac(v, ws->ops[0][i] + vX);
+                    w = lac(w, ws->ops[1][i] + vY);
+                    ws->chain[b][0][i] = w;
+                }
+                if (k > 0 && i1 < W1) {
+                    const int32_t l = xf1 + i1 - 1 - next.x;   // the column before, on d-1
+                    const bool there = l >= 0 && l < (next.y & kWidthMask);
+                    const int32_t lc = there ? l : 0;
+                    float th = (there ? ws->ops[2][lc] : kNegInf) + (e1r.x + t[T_MC]);
+                    th = lac(th, (there ? ws->ops[3][lc] : kNegInf) + (e1r.x + t[T_MFGX]));
+                    th = lac(th, (there ? ws->ops[4][lc] : kNegInf) + (e1r.x + t[T_MFGY]));
+                    ws->chain[b][1][i1] = th + M1;
+                }
+                if (tid == 0) {
+                    ws->through[b] = make_float2(__int_as_float(ws->info.row[k & (kInfoRows - 1)].w), -sh.x);
+                    ws->widths[b] = make_int2(W, k > 0 ? W1 : 0);
+                }
+            }
+            ++in_block;
+            --left;
+            if (in_block == kBlock || left == 0) {
+                __threadfence_block();
+                bar_arrive(kBarFull + b, NT + 32);
+                ++block;
+                in_block = 0;
+            }
+        }
+        M2 = M1;
+        eM2 = e1r.x;
+        M1 = vM;
+        X1 = vX;
+        Y1 = vY;
+        e1r = e;
+        gx1 = gx;
+        i1 = i;
+        W1 = W;
+        xf1 = row.x;
+        row = next;
+        i = i_next;
+        e = e_next;
+        if (kGX) gx = raw_gapx(c, row.x + i);
     }
+}
 
-    // copies of anti-diagonal d: emissions, forward values, and a refresh's other operands
-    __device__ __forceinline__ void issue(int32_t d) {
-        if (d > T) {
-            if ((d & 31) == 0) open_block((d >> 5) - 1, INT32_MAX);
-            const int4 in = ws->info[d & 63];
-            const int32_t j = first_cell_of_lane<NC>(lane, in.x), W = in.y & kWidthMask;
-            const float2 *es = Ereg + (in.z + j);
-            float2(*ed)[32] = ws->e[d & (kRows - 1)];
+// The window sweep's shifts and bases: at step k (anti-diagonal d) those of d-1, from the maximum of d+1:
+// base(d-1) - base(d) = max(d+1) - (base(d) - base(d+1)).
+template <int NT>
+__device__ __forceinline__ void column_window_shifts(const Ctx &c, const Window &Wn, ColumnWindowShared<NT> *ws) {
+    const float *t = c.t;
+    const int lane = threadIdx.x & 31;
+    const int32_t steps = Wn.D - Wn.T;
+    const bool ragged_end = Wn.at_end && c.R.ragged_right;
+    float mxD = fmaxf(ragged_end ? (t[T_OX] + t[T_OY]) / 2.0f : t[T_MC],
+                      fmaxf(ragged_end ? t[T_EX] : t[T_MFGX], ragged_end ? t[T_EY] : t[T_MFGY]));
+    if (!(mxD > kNegInf)) mxD = 0.0f;
+    float gamma = 0.0f;                  // base(d) - base(d+1)
+    double bbase = 0.0;                  // base(d-1) of this window
+    if (lane < 2) {                      // D and D-1
+        *reinterpret_cast<float2 *>(&ws->row[lane].sh1) = make_float2(-gamma, -gamma - gamma);
+        ws->bb[lane] = bbase;
+    }
+    bar_sync(kBarRow, NT + 64);
+    for (int32_t k = 0; k < steps; ++k) {
+        bar_sync(kBarRow, NT + 64);
+        if (k == 0) continue;
+        float m = part_max<NT / 32>(ws->part[(k + 1) & 1]);
+        if (k == 1) m = mxD;
+        const float g = (m > kNegInf ? m : 0.0f) - gamma;
+        if (lane == 0) *reinterpret_cast<float2 *>(&ws->row[(k + 1) & 3].sh1) = make_float2(-g, -gamma - g);
+        bbase += (double) g;
+        if (lane == 0) ws->bb[(k + 1) & (kPostRows - 1)] = bbase;
+        gamma = g;
+    }
+}
+
+// The window sweep's copies: at step k the operands of the kAhead-th anti-diagonal below, and the place
+// of the second (for the sweep and the posteriors).
+template <int NT>
+__device__ __forceinline__ void column_window_copies(const Ctx &c, const Window &Wn, const WindowTask &wt,
+                                                     ColumnWindowShared<NT> *ws) {
+    constexpr int NW = NT / 32;
+    const Args &A = *c.A;
+    const RegionDesc &R = c.R;
+    const int lane = threadIdx.x & 31;
+    const float2 *Ereg = A.E + R.cell_base + lane;
+    const float *Freg = A.F + 3 * R.cell_base + lane;
+    const int32_t D = Wn.D, T = Wn.T, from = Wn.from, steps = D - T;
+    // a window whose T starts a forward segment reads that segment's own copy of T
+    const float *Tside = A.use_side && wt.side >= 0
+                             ? A.stitch_vals + A.stitch[wt.side].voff + 3 * A.stitch[wt.side].w0 + lane
+                             : nullptr;
+    RowStream<-1> info;
+    info.open(&ws->info, A, R.diag_base, R.n, D, wt.first_cell + (raw_meta(A, R.diag_base, D, R.n).y & kWidthMask));
+    auto issue = [&](int32_t k, const int4 &in) {
+        if (k < steps) {
+            const int32_t d = D - k, W = in.y & kWidthMask;
+            const float2 *es = Ereg + in.z;
+            const float *fd = Freg + 3 * (int64_t) in.z;
+            float2 *ed = &ws->e[k & (kRows - 1)][lane];
+            float *ff = &ws->f[k & (kRows - 1)][lane];
+            const int32_t Wf = d <= from ? W : 0;
 #pragma unroll
-            for (int r = 0; r < NC; ++r) copy_async8(&ed[r][lane], es + r);
-            if (d <= from) {
-                // only the band's cells: what lies past an anti-diagonal may not be written yet
-                const float *fs = Freg + (3 * (int64_t) in.z + j);
-                float(*fd)[32] = ws->f[d & (kRows - 1)];
+            for (int w = 0; w < NW; ++w) {
+                if (lane + 32 * w < W) copy_async8(ed + 32 * w, es + 32 * w);
+                if (lane + 32 * w < Wf) copy_async4(ff + 32 * w, fd + 32 * w);
+            }
+            if (Wf > 0 && (in.y & kFlagRefresh) != 0) {
+                const int4 below = info.at(k + 1);
+                const int32_t Wm = below.y & kWidthMask;
+                const float *fm = Tside && d - 1 == T ? Tside : Freg + 3 * (int64_t) below.z;
 #pragma unroll
-                for (int r = 0; r < NC; ++r)
-                    if (cell_in(j, r, W)) copy_async4(&fd[r][lane], fs + r);
-                if ((in.y & kFlagRefresh) != 0) {
-                    const int4 below = ws->info[(d - 1) & 63];
-                    const int32_t jm = first_cell_of_lane<NC>(lane, below.x), Wm = below.y & kWidthMask;
-                    const float *fm = (Tside && d - 1 == T ? Tside : Freg + 3 * (int64_t) below.z) + jm;
-#pragma unroll
-                    for (int r = 0; r < NC; ++r) {
-                        if (cell_in(j, r, W)) {
-                            copy_async4(&ws->ops[0][r][lane], fs + W + r);
-                            copy_async4(&ws->ops[1][r][lane], fs + 2 * W + r);
-                        }
-                        if (cell_in(jm, r, Wm)) {
-                            copy_async4(&ws->ops[2][r][lane], fm + r);
-                            copy_async4(&ws->ops[3][r][lane], fm + Wm + r);
-                            copy_async4(&ws->ops[4][r][lane], fm + 2 * Wm + r);
-                        } else {
-                            ws->ops[2][r][lane] = ws->ops[3][r][lane] = ws->ops[4][r][lane] = kNegInf;
-                        }
+                for (int w = 0; w < NW; ++w) {
+                    const int i = lane + 32 * w;
+                    if (i < W) {
+                        copy_async4(&ws->ops[0][i], fd + W + 32 * w);
+                        copy_async4(&ws->ops[1][i], fd + 2 * W + 32 * w);
+                    }
+                    if (i < Wm) {
+                        copy_async4(&ws->ops[2][i], fm + 32 * w);
+                        copy_async4(&ws->ops[3][i], fm + Wm + 32 * w);
+                        copy_async4(&ws->ops[4][i], fm + 2 * Wm + 32 * w);
                     }
                 }
             }
         }
         copy_commit();
-    }
-
-    // Total probability through anti-diagonal d (diagonalCalculationTotalProbability,
-    // pairwiseAligner.c:1182-1200): F.B on d in ascending cell order, then the matches from d-1 over d
-    // into d+1 dotted with B(d+1), relative to base_F(d) + base_B(d).  f, bM, bX, bY: forward match
-    // and backward values of d (first cell j, width W).
-    __device__ __forceinline__ float refresh(int32_t d, int32_t j, int32_t W, const float (&f)[NC], const float (&bM)[NC],
-                                             const float (&bX)[NC], const float (&bY)[NC], float shift, float gamma0) {
-        const float *t = c.t;
-        const bool have_next = d < D;
-        const float2(*en)[32] = ws->e[(d + 1) & (kRows - 1)];
-        const int left = (lane + 31) & 31;
-        float m = __shfl_sync(0xffffffffu, ws->ops[2][NC - 1][lane], left);
-        float x = __shfl_sync(0xffffffffu, ws->ops[3][NC - 1][lane], left);
-        float y = __shfl_sync(0xffffffffu, ws->ops[4][NC - 1][lane], left);
-#pragma unroll
-        for (int r = 0; r < NC; ++r) {
-            float v = f[r] + bM[r];
-            v = lac(v, ws->ops[0][r][lane] + bX[r]);
-            v = lac(v, ws->ops[1][r][lane] + bY[r]);
-            if (cell_in(j, r, W)) ws->chain[j + r] = v;
-            const float em = en[r][lane].x;
-            float th = m + (em + t[T_MC]);
-            th = lac(th, x + (em + t[T_MFGX]));
-            th = lac(th, y + (em + t[T_MFGY]));
-            if (have_next && cell_in(j1, r, W1)) ws->chain[column_slots(NC) + j1 + r] = th + vM1[r];
-            m = ws->ops[2][r][lane];
-            x = ws->ops[3][r][lane];
-            y = ws->ops[4][r][lane];
-        }
-        __syncwarp();
-        const float2 ff = column_folds<NC>(ws->chain, W, have_next ? W1 : 0);
-        // the through-part is relative to base_F(d-1) + base_B(d+1)
-        return lac(ff.x, ff.y - shift - gamma0);
-    }
-
-    // pairs of anti-diagonal d in ascending cell order (the reference's): the lanes rotated so that
-    // the one with the first column comes first
-    __device__ __forceinline__ void emit(int32_t d, int32_t xf, int32_t j, int32_t W, const float (&s)[NC],
-                                         const WindowTask &wt) {
-        const int first = (xf / NC) & 31;
-        unsigned b[NC], hits = 0;
-        float p[NC];
-#pragma unroll
-        for (int r = 0; r < NC; ++r) {
-            const int32_t x = xf + j + r, y = d - x;
-            p[r] = __expf(s[r]);
-            const bool hit = cell_in(j, r, W) && x > 0 && y > 0 && p[r] >= A.threshold;
-            hits |= hit ? 1u << r : 0u;
-            const unsigned v = __ballot_sync(0xffffffffu, hit);
-            b[r] = __funnelshift_r(v, v, first);
-        }
-        const unsigned below = (1u << ((lane - first) & 31)) - 1u;
-        int64_t q = n_out;
-#pragma unroll
-        for (int r = 0; r < NC; ++r) q += __popc(b[r] & below);
-        if (hits) {
-#pragma unroll
-            for (int r = 0; r < NC; ++r) {
-                if (!((hits >> r) & 1u)) continue;
-                const int32_t x = xf + j + r, y = d - x;
-                if (q < wt.out_cap) {
-                    sa_aligned_pair o;
-                    o.score = (int64_t) floor((double) fminf(p[r], 1.0f) * 10000000.0);
-                    o.x = R.x1 + x - 1;
-                    o.y = R.y1 + y - 1;
-                    o.kmer = __ldg(A.kmer + R.kmer_base + x - 1);   // 1 <= x <= lX for a pair
-                    A.out[wt.out_base + q] = o;
-                } else {
-                    atomicMax(A.status + R.read, (int32_t) SA_E_OUTPUT);
-                }
-                ++q;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < NC; ++r) n_out += __popc(b[r]);
-    }
-
-    __device__ __forceinline__ void run(int64_t gw) {
-        lane = threadIdx.x & 31;
-        Ereg = A.E + R.cell_base;
-        Freg = A.F + 3 * R.cell_base;
-        const Window Wn = A.windows[gw];
-        const WindowTask wt = A.wtask[gw];
-        D = Wn.D;
-        T = Wn.T;
-        from = Wn.from;
-        // a window whose T starts a forward segment reads that segment's own copy of T
-        Tside = A.use_side && wt.side >= 0 ? A.stitch_vals + A.stitch[wt.side].voff + 3 * A.stitch[wt.side].w0 : nullptr;
-        // a cell can only reach the threshold if its logarithm does
-        const float log_threshold = A.threshold > 0.0f ? logf(A.threshold) - 1e-3f : kNegInf;
-        const float *t = c.t;
-        // end-state values on D (stateMachine.c:1034-1061)
-        const bool ragged_end = Wn.at_end && R.ragged_right;
-        const float e0 = ragged_end ? (t[T_OX] + t[T_OY]) / 2.0f : t[T_MC];
-        const float e1 = ragged_end ? t[T_EX] : t[T_MFGX];
-        const float e2 = ragged_end ? t[T_EY] : t[T_MFGY];
-        float mxD = fmaxf(e0, fmaxf(e1, e2));
-        if (!(mxD > kNegInf)) mxD = 0.0f;
-        __syncwarp();   // the warp's previous window has read its shared memory
-#pragma unroll
-        for (int r = 0; r < NC; ++r) {
-            vM1[r] = vX1[r] = vY1[r] = vM2[r] = kNegInf;
-            ws->e[(D + 1) & (kRows - 1)][r][lane] = ws->e[(D + 2) & (kRows - 1)][r][lane] = make_float2(0.0f, 0.0f);
-        }
-        load_block(D >> 5);
-        block_top = wt.first_cell + (__shfl_sync(0xffffffffu, raw.y, D & 31) & kWidthMask);
-        open_block(D >> 5, D);
-#pragma unroll
-        for (int k = 0; k < kAhead; ++k) issue(D - k);
-        j1 = W1 = xf1 = 0;
-        mx1 = mx2 = kNegInf;
-        gamma1 = 0.0f;
-        bbase = pref = 0.0;
-        double ll = 0.0;
-        n_out = 0;
-#pragma unroll 1
-        for (int32_t d = D; d > T; --d) {
-            issue(d - kAhead);
-            copy_wait<kAhead>();   // every copy of d and above has landed
-            const int4 in = ws->info[d & 63];
-            const int32_t xf = in.x, W = in.y & kWidthMask;
-            const int32_t j = first_cell_of_lane<NC>(lane, xf);
-            float gamma0 = 0.0f;           // base(d) - base(d+1) = max(d+2) - gamma1
-            if (d <= D - 2) gamma0 = (mx2 > kNegInf ? mx2 : 0.0f) - gamma1;
-            bbase += (double) gamma0;
-            float bM[NC], bX[NC], bY[NC];
-            float mx0;
-            if (d == D) {
-#pragma unroll
-                for (int r = 0; r < NC; ++r) {
-                    const bool inb = cell_in(j, r, W);
-                    bM[r] = inb ? e0 : kNegInf;
-                    bX[r] = inb ? e1 : kNegInf;
-                    bY[r] = inb ? e2 : kNegInf;
-                }
-                mx0 = mxD;
-            } else {
-                const float shU = -gamma0, shM = -gamma1 - gamma0;
-                const float2(*ep)[32] = ws->e[(d + 2) & (kRows - 1)], (*eu)[32] = ws->e[(d + 1) & (kRows - 1)];
-                Skip<NC, kGX> g;
-                g.load(c, xf1 + j1);
-                float me[NC + 1], le[NC + 1];
-#pragma unroll
-                for (int r = 0; r < NC; ++r) {
-                    me[r] = vM2[r] + (ep[r][lane].x + shM);
-                    le[r] = vX1[r] + (g[r] + shU);
-                }
-                const int right = (lane + 1) & 31;
-                me[NC] = __shfl_sync(0xffffffffu, me[0], right);
-                le[NC] = __shfl_sync(0xffffffffu, le[0], right);
-                float lm = kNegInf;
-#pragma unroll
-                for (int r = 0; r < NC; ++r) {
-                    float m = me[r + 1] + t[T_MC];
-                    float x = me[r + 1] + t[T_MFGX];
-                    float y = me[r + 1] + t[T_MFGY];
-                    const float ue = vY1[r] + (eu[r][lane].y + shU);
-                    m = lac(m, ue + t[T_OY]);
-                    y = lac(y, ue + t[T_EY]);
-                    m = lac(m, le[r + 1] + t[T_OX]);
-                    x = lac(x, le[r + 1] + t[T_EX]);
-                    if (kSX) y = lac(y, le[r + 1] + t[T_SX]);
-                    const bool inb = cell_in(j, r, W);
-                    bM[r] = inb ? m : kNegInf;
-                    bX[r] = inb ? x : kNegInf;
-                    bY[r] = inb ? y : kNegInf;
-                    lm = fmaxf(lm, fmaxf(bM[r], fmaxf(bX[r], bY[r])));
-                }
-                mx0 = warp_max1(lm);
-            }
-            if (d <= from) {
-                float f[NC];
-#pragma unroll
-                for (int r = 0; r < NC; ++r) f[r] = ws->f[d & (kRows - 1)][r][lane];
-                const double fb = ws->base[d & 63];
-                if ((in.y & kFlagRefresh) != 0) {
-                    pref = (double) refresh(d, j, W, f, bM, bX, bY, __int_as_float(in.w), gamma0) + fb + bbase;
-                    if (d == R.n) ll = pref;
-                }
-                const float kd = (float) (fb + bbase - pref);
-                float s[NC], top = kNegInf;
-#pragma unroll
-                for (int r = 0; r < NC; ++r) {
-                    s[r] = f[r] + bM[r] + kd;
-                    top = fmaxf(top, s[r]);
-                }
-                if (__any_sync(0xffffffffu, top > log_threshold || A.threshold <= 0.0f)) emit(d, xf, j, W, s, wt);
-            }
-            mx2 = mx1;
-            mx1 = mx0;
-            gamma1 = gamma0;
-            j1 = j;
-            W1 = W;
-            xf1 = xf;
-#pragma unroll
-            for (int r = 0; r < NC; ++r) {
-                vM2[r] = vM1[r];
-                vM1[r] = bM[r];
-                vX1[r] = bX[r];
-                vY1[r] = bY[r];
-            }
-        }
-        copy_wait<0>();
+    };
+    auto place = [&](int32_t k) {
+        const int4 in = info.at(k);
+        const double fb = ws->info.base[k & (kInfoRows - 1)];
         if (lane == 0) {
-            A.wcount[gw] = n_out;
-            if (Wn.at_end) A.loglik[c.region_index] = ll;
+            *reinterpret_cast<int2 *>(&ws->row[k & 3].xf) = make_int2(in.x, in.y | (D - k <= from ? kRowPost : 0));
+            ws->post[k & (kPostRows - 1)] = make_int2(in.x, in.y & kWidthMask);
+            ws->fb[k & (kPostRows - 1)] = fb;
+        }
+    };
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) issue(k, info.at(k));
+    place(0);
+    place(1);
+    copy_wait<kAhead - 2>();
+    int4 in = info.at(kAhead);
+    bar_sync(kBarRow, NT + 64);
+    for (int32_t k = 0; k < steps; ++k) {
+        bar_sync(kBarRow, NT + 64);
+        issue(k + kAhead, in);
+        place(k + 2);
+        info.advance(k);
+        in = info.at(k + kAhead + 1);
+        copy_wait<kAhead - 2>();         // every copy of d-2 and above has landed
+    }
+    copy_wait<0>();
+}
+
+// The window's total probabilities, posteriors and pairs (one warp): a block's total first, then its
+// anti-diagonals in the reference's order, descending, cells ascending.
+template <int NT>
+__device__ __forceinline__ void column_window_post(const Ctx &c, const Window &Wn, const WindowTask &wt, int64_t gw,
+                                                   ColumnWindowShared<NT> *ws) {
+    const Args &A = *c.A;
+    const RegionDesc &R = c.R;
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31;
+    const int32_t rows = Wn.from - Wn.T, blocks = (rows + kBlock - 1) / kBlock;
+    // a cell can only reach the threshold if its logarithm does
+    const float log_threshold = A.threshold > 0.0f ? logf(A.threshold) - 1e-3f : kNegInf;
+    double pref = 0.0, ll = 0.0;
+    int64_t n_out = 0;
+    for (int32_t q = 0; q < blocks; ++q) {
+        const int b = q & 1;
+        bar_sync(kBarFull + b, NT + 32);
+        const int2 widths = ws->widths[b];
+        const float2 ff = column_folds<NT / 32>(&ws->chain[b][0][0], widths.x, widths.y);
+        const float2 th = ws->through[b];
+        // the through-part is relative to base_F(d-1) + base_B(d+1)
+        const float ptil = lac(ff.x, ff.y - th.x - th.y);
+        const int32_t top = Wn.from - q * kBlock, k0 = Wn.D - top;   // the total's anti-diagonal
+        pref = (double) ptil + ws->fb[k0 & (kPostRows - 1)] + ws->bb[k0 & (kPostRows - 1)];
+        if (top == R.n) ll = pref;
+        const int m = min(kBlock, rows - q * kBlock);
+        // lane j: what the block's j-th anti-diagonal needs
+        const int32_t at_row = (k0 + lane) & (kPostRows - 1);
+        const float kd_lane = lane < m ? (float) (ws->fb[at_row] + ws->bb[at_row] - pref) : 0.0f;
+        const int2 row_lane = lane < m ? ws->post[at_row] : make_int2(0, 0);
+        for (int j = 0; j < m; ++j) {
+            const float kd = __shfl_sync(0xffffffffu, kd_lane, j);
+            const int32_t xf = __shfl_sync(0xffffffffu, row_lane.x, j), W = __shfl_sync(0xffffffffu, row_lane.y, j);
+            const int32_t d = top - j;
+            float v[NW], most = kNegInf;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                const int i = lane + 32 * w;
+                v[w] = ws->s[b][j][(xf + i) & (NT - 1)] + kd;
+                if (i >= W) v[w] = kNegInf;
+                most = fmaxf(most, v[w]);
+            }
+            if (!__any_sync(0xffffffffu, most > log_threshold || A.threshold <= 0.0f)) continue;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                const int i = lane + 32 * w;
+                const int32_t x = xf + i, y = d - x;
+                const float p = __expf(v[w]);
+                const bool hit = i < W && x > 0 && y > 0 && p >= A.threshold;
+                const unsigned bal = __ballot_sync(0xffffffffu, hit);
+                if (hit) {
+                    const int64_t at = n_out + __popc(bal & ((1u << lane) - 1u));
+                    if (at < wt.out_cap) {
+                        sa_aligned_pair o;
+                        o.score = (int64_t) floor((double) fminf(p, 1.0f) * 10000000.0);
+                        o.x = R.x1 + x - 1;
+                        o.y = R.y1 + y - 1;
+                        o.kmer = 0;      // filled in by the gather: a load here would hold the warp up
+                        A.out[wt.out_base + at] = o;
+                    } else {
+                        atomicMax(A.status + R.read, (int32_t) SA_E_OUTPUT);
+                    }
+                }
+                n_out += __popc(bal);
+            }
         }
         __syncwarp();
+        if (q + 2 < blocks) bar_arrive(kBarEmpty + b, NT + 32);
     }
-};
+    if (lane == 0) {
+        A.wcount[gw] = n_out;
+        if (Wn.at_end) A.loglik[c.region_index] = ll;
+    }
+    __syncwarp();
+}
 
 // ------------------------------------------------------------------------------------------------
 // the persistent worker of column-resident batches
 // ------------------------------------------------------------------------------------------------
-struct alignas(16) ColumnShared {
-    float4 la[16];                      // logAdd cubic pieces, indexed by -ceil(2 d) mod 16
-    ColumnForwardShared fs;
-    Shared sh;                          // the segments' claims and stitch checks
-};
-
-// The first claims are forward segments (longest first), one per CTA; once none is left, each warp
-// claims windows.
-template <bool kSX, bool kGX>
-__device__ __forceinline__ void column_forward(const Ctx &c, const Segment &sg, ColumnForwardShared *fs, Shared *sh) {
-    ColumnForward<kSX, kGX> f(c, sg, fs);
-    f.run(sh);
+// NT / 32 warps sweep, beside the three others.  The first claims are forward segments (longest
+// first); once none is left, windows.
+template <int NT, bool kSX, bool kGX>
+__device__ __forceinline__ void column_forward(const Ctx &c, const Segment &sg, ColumnForwardShared<NT> *fs) {
+    if (threadIdx.x < NT) column_forward_sweep<NT, kSX, kGX>(c, sg, fs);
+    else if (threadIdx.x < NT + 32) column_forward_shifts<NT>(sg, fs);
+    else if (threadIdx.x < NT + 64) column_forward_copies<NT>(c, sg, fs);
+    else column_forward_results<NT>(c, sg, fs);
 }
 
-template <int NC, bool kSX, bool kGX>
-__device__ __forceinline__ void column_window(const Ctx &c, WindowShared<NC> *ws, int64_t id) {
-    ColumnWindow<NC, kSX, kGX> w(c, ws);
-    w.run(id);
+template <int NT, bool kSX, bool kGX>
+__device__ __forceinline__ void column_window(const Ctx &c, ColumnWindowShared<NT> *ws, int64_t id) {
+    const Window Wn = c.A->windows[id];
+    const WindowTask wt = c.A->wtask[id];
+    if (threadIdx.x < NT) column_window_sweep<NT, kSX, kGX>(c, Wn, ws);
+    else if (threadIdx.x < NT + 32) column_window_shifts<NT>(c, Wn, ws);
+    else if (threadIdx.x < NT + 64) column_window_copies<NT>(c, Wn, wt, ws);
+    else column_window_post<NT>(c, Wn, wt, id, ws);
 }
 
-template <int NC, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) column_worker(const __grid_constant__ Args A) {
-    ColumnShared *cs = reinterpret_cast<ColumnShared *>(column_smem);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT + kHelpers, MINB) column_worker(const __grid_constant__ Args A) {
+    ColumnShared<NT> *cs = reinterpret_cast<ColumnShared<NT> *>(column_smem);
+    const int tid = threadIdx.x;
     if (tid < 16) {
-        log_add_piece((16 - tid) & 15, cs->la[tid]);
+        float4 c;
+        log_add_piece((16 - tid) & 15, c);
+        cs->la.hi[tid] = make_float2(c.x, c.y);
+        cs->la.lo[tid] = make_float2(c.z, c.w);
     }
+    // a thread outside the band adds whatever emission its slot holds to -inf: a number, not what a
+    // kernel before this one left there (both unions' members have the ring in one place)
+    for (int q = tid; q < kRows * NT; q += NT + kHelpers) (&cs->w.e[0][0])[q] = make_float2(0.0f, 0.0f);
     for (;;) {
         if (tid == 0) {
             const unsigned claim = atomicAdd(&A.ctl->claim, 1u);
-            cs->sh.task_id = claim < (unsigned) A.n_segs ? A.order[claim] : -1;
+            cs->task = claim < (unsigned) A.n_segs ? A.order[claim] : -1;
         }
         __syncthreads();
-        const int32_t id = cs->sh.task_id;
+        const int32_t id = cs->task;
         if (id < 0) break;
         const Segment sg = A.segs[id];
         Ctx c;
         ctx_init(c, A, sg.region);
         const bool sx = c.t[T_SX] > kNegInf;
         if (c.gx_uniform) {
-            if (sx) column_forward<true, false>(c, sg, &cs->fs, &cs->sh);
-            else column_forward<false, false>(c, sg, &cs->fs, &cs->sh);
+            if (sx) column_forward<NT, true, false>(c, sg, &cs->f);
+            else column_forward<NT, false, false>(c, sg, &cs->f);
         } else {
-            if (sx) column_forward<true, true>(c, sg, &cs->fs, &cs->sh);
-            else column_forward<false, true>(c, sg, &cs->fs, &cs->sh);
+            if (sx) column_forward<NT, true, true>(c, sg, &cs->f);
+            else column_forward<NT, false, true>(c, sg, &cs->f);
         }
+        __syncthreads();
     }
-    WindowShared<NC> *ws = reinterpret_cast<WindowShared<NC> *>(cs + 1) + warp;
+    __syncthreads();
     for (;;) {
-        int32_t id = -1;
-        if (lane == 0) {
+        if (tid == 0) {
             const unsigned claim = atomicAdd(&A.ctl->wclaim, 1u);
-            if ((int64_t) claim < A.n_windows) id = wait_ready(A, claim);
+            cs->task = (int64_t) claim < A.n_windows ? wait_ready(A, claim) : -1;
         }
-        id = __shfl_sync(0xffffffffu, id, 0);
+        __syncthreads();
+        const int32_t id = cs->task;
         if (id < 0) break;
         Ctx c;
         ctx_init(c, A, A.wtask[id].region);
         const bool sx = c.t[T_SX] > kNegInf;
         if (c.gx_uniform) {
-            if (sx) column_window<NC, true, false>(c, ws, id);
-            else column_window<NC, false, false>(c, ws, id);
+            if (sx) column_window<NT, true, false>(c, &cs->w, id);
+            else column_window<NT, false, false>(c, &cs->w, id);
         } else {
-            if (sx) column_window<NC, true, true>(c, ws, id);
-            else column_window<NC, false, true>(c, ws, id);
+            if (sx) column_window<NT, true, true>(c, &cs->w, id);
+            else column_window<NT, false, true>(c, &cs->w, id);
         }
-        read_unit_done<32>(A, c.R.read, lane, nullptr);
+        // the posteriors' warp wrote the window's pairs and counts
+        if (tid >= NT + 64) read_unit_done<32>(A, c.R.read, tid & 31, nullptr);
+        __syncthreads();
     }
 }
 

@@ -56,10 +56,6 @@ constexpr int kMaxCpt = 4;                     // cells per thread: bands up to 
 constexpr int kChunkDiags = 32;                // anti-diagonals per emission-kernel chunk
 enum { ST_M = 0, ST_X = 1, ST_Y = 2 };         // forward store blocks
 
-// Cells before and after the emission store that look-ahead loads may read (never a band cell's own
-// operand): zeroed by the emission kernel, so that what reaches the arithmetic is a number.
-constexpr int kStoreFront = 16, kStoreBack = 480;
-
 // per-anti-diagonal meta: x = xmy of the first cell, y = width | flags
 constexpr int32_t kWidthMask = (1 << 20) - 1;
 constexpr int32_t kFlagWindowEnd = 1 << 20;   // a traceback window closes here
@@ -202,7 +198,6 @@ struct Args {
     const int32_t *kmer;
     const float *gapx;              // per k-mer position: skip emission of that k-mer
     const Event32 *events;
-    int64_t n_cells;
     float2 *E;                      // emission store, (match, extra event) per cell
     float *F;                       // forward store, 3 floats per cell
     double *base;                   // per anti-diagonal FP64 base of the forward store
@@ -215,7 +210,6 @@ struct Args {
     Control *ctl;
     float threshold;
     int32_t wmax;                   // ring width (cells); rings hold wmax + 2 floats per state
-    int32_t sms;                    // SMs of the device
     long long spin_limit;           // clock cycles a worker may wait for a window
     // gather
     int64_t n_reads;
@@ -483,10 +477,6 @@ __device__ __forceinline__ void emit_cell(const Ctx &c, const KmerConst32 &k, in
 __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_constant__ Args A) {
     __shared__ EmitStage stage[kEmitWarps];
     const int lane = threadIdx.x & 31;
-    // what the column sweeps' look-ahead reads before the first and after the last cell
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < kStoreFront + kStoreBack; i += blockDim.x)
-            A.E[i < kStoreFront ? i - kStoreFront : A.n_cells + (i - kStoreFront)] = make_float2(0.0f, 0.0f);
     EmitStage &st = stage[threadIdx.x >> 5];
     const int64_t warps = (int64_t) gridDim.x * (blockDim.x >> 5);
     for (int64_t ch = blockIdx.x * (int64_t) (blockDim.x >> 5) + (threadIdx.x >> 5); ch < A.n_chunks; ch += warps) {
@@ -1023,7 +1013,7 @@ __device__ void forward_task(const Ctx &c, const Segment &sg, Shared *sh, float 
 template <int CPT>
 __device__ __forceinline__ void write_pairs(const Ctx &c, Shared *sh, const WindowTask &wt, int32_t pend_d,
                                             unsigned pend, const float *pv, const int32_t *px, const int32_t *py,
-                                            const int32_t *pk, int64_t &n_out) {
+                                            int64_t &n_out) {
     const Args &A = *c.A;
     const RegionDesc &R = c.R;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1045,7 +1035,7 @@ __device__ __forceinline__ void write_pairs(const Ctx &c, Shared *sh, const Wind
                 o.score = (int64_t) floor((double) fminf(pv[j], 1.0f) * 10000000.0);
                 o.x = R.x1 + px[j] - 1;
                 o.y = R.y1 + py[j] - 1;
-                o.kmer = pk[j];
+                o.kmer = 0;   // filled in by the gather
                 A.out[wt.out_base + slot] = o;
             } else {
                 atomicMax(A.status + R.read, (int32_t) SA_E_OUTPUT);
@@ -1132,7 +1122,7 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
     double pref = 0.0;                 // latest refresh total probability (absolute)
     unsigned pend = 0;
     float pv[CPT];
-    int32_t px[CPT], py[CPT], pk[CPT];
+    int32_t px[CPT], py[CPT];
     int32_t pend_d = -1;
     __syncthreads();
     for (int32_t d = D; d > T; --d) {
@@ -1240,7 +1230,7 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
         __syncthreads();
         // pairs of the previous anti-diagonal, in the reference's order (ascending xmy)
         if (pend_d >= 0) {
-            write_pairs<CPT>(c, sh, wt, pend_d, pend, pv, px, py, pk, n_out);
+            write_pairs<CPT>(c, sh, wt, pend_d, pend, pv, px, py, n_out);
             pend = 0;
             pend_d = -1;
         }
@@ -1298,7 +1288,6 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
                 pv[j] = p;
                 px[j] = x;
                 py[j] = y;
-                pk[j] = __ldg(A.kmer + R.kmer_base + clampi(x - 1, 0, max(R.lX - 1, 0)));
                 const unsigned bal = __ballot_sync(0xffffffffu, hit);
                 if (hit) pend |= 1u << j;
                 if (lane == 0) sh->wcnt[d & 1][j][warp] = __popc(bal);
@@ -1321,7 +1310,7 @@ __device__ void window_task(const Ctx &c, Shared *sh, float *ring, float *chain,
     }
     // flush the last anti-diagonal's pairs
     __syncthreads();
-    if (pend_d >= 0) write_pairs<CPT>(c, sh, wt, pend_d, pend, pv, px, py, pk, n_out);
+    if (pend_d >= 0) write_pairs<CPT>(c, sh, wt, pend_d, pend, pv, px, py, n_out);
     if (tid == 0) {
         A.wcount[gw] = n_out;
         if (W.at_end) A.loglik[c.region_index] = ll;
@@ -1373,6 +1362,12 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
 template <int NT>
 __device__ void gather_read(const Args &A, int64_t r, int tid, long long *red, long long &base, long long &tot) {
     const int64_t w0 = A.read_win[8 * r], nw = A.read_win[8 * r + 1];
+    // k-mer ids of the read's columns
+    const int32_t *kmer = A.kmer;
+    if (nw > 0) {
+        const RegionDesc &R = A.regions[A.read_win[8 * r + 2]];
+        kmer += R.kmer_base - R.x1;
+    }
     long long mine = 0;
     for (int64_t k = tid; k < nw; k += NT)
         mine += min(__ldcg(A.wcount + w0 + k), (int64_t) A.wtask[w0 + k].out_cap);
@@ -1410,9 +1405,17 @@ __device__ void gather_read(const Args &A, int64_t r, int tid, long long *red, l
         for (int jj = 0; jj < m; ++jj) {
             const long long c = __shfl_sync(0xffffffffu, cnt, jj);
             const long long at = run + __shfl_sync(0xffffffffu, inc, jj) - c;
+            // a pair in two halves, (score, x) and (y, k-mer): the k-mer of its column is looked up here
             const int4 *src = reinterpret_cast<const int4 *>(A.out + __shfl_sync(0xffffffffu, ob, jj));
             int4 *dst = reinterpret_cast<int4 *>(A.packed + base + at);
-            for (long long q = tid; q < 2 * c; q += NT) dst[q] = __ldcg(src + q);
+            for (long long q = tid; q < 2 * c; q += NT) {
+                int4 h = __ldcg(src + q);
+                if (q & 1) {
+                    h.z = __ldg(kmer + __ldcg(&src[q - 1].z));
+                    h.w = 0;
+                }
+                dst[q] = h;
+            }
         }
         run += __shfl_sync(0xffffffffu, inc, 31);
     }

@@ -130,35 +130,35 @@ struct InfoStream {
 // log_add on the sweeps' chains
 // ------------------------------------------------------------------------------------------------
 // dp64::log_add bit for bit, without its select chains: the cubic's piece comes from shared memory,
-// indexed as in the FP32 form: C - d rounded down, with C's last place 1/64, holds -32 ceil(2 d) mod
-// 512 in bits 5..8, the byte offset of the piece.  -inf less -inf is NaN, which compares as beyond the
-// cut-off.  One after another 117 cycles each, four independent ones 223 (measured; with the
-// coefficients selected, 95 and 295; with the piece found by integer compares, 152 and 480).
+// indexed as in the FP32 form: C - d rounded down, with C's last place 1/16, holds -8 ceil(2 d) mod
+// 128 in bits 3..6, the byte offset of the piece in each coefficient's table (entries of 8 bytes lie in
+// banks of their own, so lanes with different pieces do not conflict).  -inf less -inf is NaN, which
+// compares as beyond the cut-off.
 struct LogAdd64 {
-    double2 c[16][2];                  // (a3, a2), (a1, a0) of the piece of -ceil(2 d) mod 16
+    double a[16], b[16], c[16], e[16];   // a3 .. a0 of the piece of -ceil(2 d) mod 16
 };
 
 __device__ __forceinline__ void log_add_table64(LogAdd64 &t, int k) {
     const double d = 0.5 * ((16 - k) & 15);   // the upper end of the entry's range
     const bool p0 = d <= 1.0, p1 = d <= 2.5, p2 = d <= 4.5;
-    t.c[k][0] = make_double2(p0 ? (double) -0.009350833524763f : p1 ? (double) -0.014532321752540f
-                             : p2 ? (double) -0.004605031767994f : (double) -0.000458661602210f,
-                             p0 ? (double) 0.130659527668286f : p1 ? (double) 0.139942324101744f
-                             : p2 ? (double) 0.063427417320019f : (double) 0.009695946122598f);
-    t.c[k][1] = make_double2(p0 ? (double) 0.498799810682272f : p1 ? (double) 0.495635523139337f
-                             : p2 ? (double) 0.695956496475118f : (double) 0.930734667215156f,
-                             p0 ? (double) 0.693203116424741f : p1 ? (double) 0.692140569840976f
-                             : p2 ? (double) 0.514272634594009f : (double) 0.168037164329057f);
+    t.a[k] = p0 ? (double) -0.009350833524763f : p1 ? (double) -0.014532321752540f
+             : p2 ? (double) -0.004605031767994f : (double) -0.000458661602210f;
+    t.b[k] = p0 ? (double) 0.130659527668286f : p1 ? (double) 0.139942324101744f
+             : p2 ? (double) 0.063427417320019f : (double) 0.009695946122598f;
+    t.c[k] = p0 ? (double) 0.498799810682272f : p1 ? (double) 0.495635523139337f
+             : p2 ? (double) 0.695956496475118f : (double) 0.930734667215156f;
+    t.e[k] = p0 ? (double) 0.693203116424741f : p1 ? (double) 0.692140569840976f
+             : p2 ? (double) 0.514272634594009f : (double) 0.168037164329057f;
 }
 
-__device__ __forceinline__ double lad(const LogAdd64 &t, double x, double y) {
-    const double d = fabs(x - y);
-    const int k = __double2loint(__dadd_rd(105553116266496.0, -d)) & 0x1e0;
-    const double2 *c = reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(t.c) + k);
-    const double2 ab = c[0], ce = c[1];
-    const double p = ((ab.x * d + ab.y) * d + ce.x) * d + ce.y;
+__device__ __forceinline__ const double *piece64(const LogAdd64 &t, double d) {
+    const int k = __double2loint(__dadd_rd(422212465065984.0, -d)) & 0x78;
+    return reinterpret_cast<const double *>(reinterpret_cast<const char *>(t.a) + k);
+}
+
+// the larger argument alone from the cut-off on; else the cubic p (of the difference d) and the smaller
+__device__ __forceinline__ double pick64(double x, double y, double p, double d) {
     double r;
-    // branch-free: the larger and the smaller argument, and the larger alone from the cut-off on
     asm("{\n\t.reg .pred q, n;\n\t.reg .f64 hi, lo, s;\n\tsetp.lt.f64 q, %1, %2;\n\tselp.f64 hi, %2, %1, q;\n\t"
         "selp.f64 lo, %1, %2, q;\n\tadd.rn.f64 s, %3, lo;\n\tsetp.lt.f64 n, %4, 0d401E000000000000;\n\t"
         "selp.f64 %0, s, hi, n;\n\t}"
@@ -166,37 +166,39 @@ __device__ __forceinline__ double lad(const LogAdd64 &t, double x, double y) {
     return r;
 }
 
+__device__ __forceinline__ double lad(const LogAdd64 &t, double x, double y) {
+    const double d = fabs(x - y);
+    const double *c = piece64(t, d);
+    return pick64(x, y, ((c[0] * d + c[16]) * d + c[32]) * d + c[48], d);
+}
+
 // four independent ones, stage by stage
 __device__ __forceinline__ void lad4(const LogAdd64 &t, const double (&x)[4], const double (&y)[4], double (&r)[4]) {
-    double d[4], p[4];
-    double2 ab[4], ce[4];
+    double d[4], p[4], b[4], c[4], e[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) d[j] = fabs(x[j] - y[j]);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const int k = __double2loint(__dadd_rd(105553116266496.0, -d[j])) & 0x1e0;
-        const double2 *c = reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(t.c) + k);
-        ab[j] = c[0];
-        ce[j] = c[1];
+        const double *q = piece64(t, d[j]);
+        p[j] = q[0];
+        b[j] = q[16];
+        c[j] = q[32];
+        e[j] = q[48];
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = ab[j].x * d[j];
+    for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] + ab[j].y;
+    for (int j = 0; j < 4; ++j) p[j] = p[j] + b[j];
 #pragma unroll
     for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] + ce[j].x;
+    for (int j = 0; j < 4; ++j) p[j] = p[j] + c[j];
 #pragma unroll
     for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] + ce[j].y;
+    for (int j = 0; j < 4; ++j) p[j] = p[j] + e[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-        asm("{\n\t.reg .pred q, n;\n\t.reg .f64 hi, lo, s;\n\tsetp.lt.f64 q, %1, %2;\n\tselp.f64 hi, %2, %1, q;\n\t"
-            "selp.f64 lo, %1, %2, q;\n\tadd.rn.f64 s, %3, lo;\n\tsetp.lt.f64 n, %4, 0d401E000000000000;\n\t"
-            "selp.f64 %0, s, hi, n;\n\t}"
-            : "=d"(r[j]) : "d"(x[j]), "d"(y[j]), "d"(p[j]), "d"(d[j]));
+    for (int j = 0; j < 4; ++j) r[j] = pick64(x[j], y[j], p[j], d[j]);
 }
 
 // ------------------------------------------------------------------------------------------------
