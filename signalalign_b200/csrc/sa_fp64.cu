@@ -1282,6 +1282,8 @@ void plan_resident(const sa_state_machine *sm, PlainRegion &pr) {
         pr.info[d] = make_int4(lo, cnt, (int32_t) (at - lo), (int32_t) w);
         at += cnt;
     }
+    // windows whose posteriors end above where they begin (traceback distances below the overlap): the rings
+    for (const Window &win : rg.windows) pr.regular = pr.regular && win.from > win.T;
     pr.path.assign(pr.pid.size(), Path64{});
     for (int64_t x = 0; x <= rg.lX; ++x) {
         for (int32_t q = pr.pfirst[x]; q < pr.pfirst[x + 1]; ++q) {
@@ -1492,8 +1494,8 @@ bool sweeps64(PlainSet *s, const SetOut &O, cudaStream_t stream) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd) != cudaSuccess ||
         cudaFuncSetAttribute(b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd) != cudaSuccess)
         return false;
-    f<<<(unsigned) s->n_run_tasks, NT, fwd, stream>>>(s->d_models, s->d_tasks, O);
-    b<<<(unsigned) s->n_windows, NT, bwd, stream>>>(s->d_models, s->d_tasks, s->d_windows, s->d_terms, s->term_stride,
+    f<<<(unsigned) s->n_run_tasks, NT + kHelpers64, fwd, stream>>>(s->d_models, s->d_tasks, O);
+    b<<<(unsigned) s->n_windows, NT + kHelpers64, bwd, stream>>>(s->d_models, s->d_tasks, s->d_windows, s->d_terms, s->term_stride,
                                                    s->expect ? 1 : 0);
     return cudaGetLastError() == cudaSuccess;
 }

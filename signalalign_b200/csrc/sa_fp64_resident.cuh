@@ -15,9 +15,7 @@
 // anti-diagonal and sweep: latency, not arithmetic (issue 0.1 a cycle on its SM, FP64 pipe 3 %).
 // Here the paths of the reference are numbered along it and path q stays on thread q mod NT, so its own
 // column's previous value is in a register and its neighbours' are one shared-memory read away; the
-// operands come by asynchronous copy kAhead64 anti-diagonals ahead; and only what depends on the
-// previous anti-diagonal's neighbour sits between two barriers (gap-X forward, match and gap-X
-// backward).  Windows run side by side, and logarithms, exponentials, totals and outputs are off the
+// operands come by asynchronous copy kAhead64 anti-diagonals ahead; and a step's log_adds are independent.  Windows run side by side, and logarithms, exponentials, totals and outputs are off the
 // sweeps' chain.  Measured on B200: see the dispatch rule in plain_create.
 //
 // A slot not in the band holds log 0 for that anti-diagonal, so an absent neighbour drops out of
@@ -25,7 +23,9 @@
 // route only if they span at most NT paths.
 #pragma once
 
-constexpr int kAhead64 = 6;            // anti-diagonals between a copy and its use
+constexpr int kAhead64 = 6;            // anti-diagonals between a copy and its use (forward)
+constexpr int kBehind64 = 5;           // and backward, where a row is read once more after its use
+constexpr int kHelpers64 = 64;         // threads of the warps beside a sweep's: copies, results
 constexpr int kRing64 = 8;             // rows of the copy rings
 constexpr int kInfoRing = 128;         // rows of band facts kept
 
@@ -50,6 +50,10 @@ struct Total64 {
     int32_t have_next, last;           // d < D; d ends the region
 };
 
+__device__ __forceinline__ void copy64_4(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
 __device__ __forceinline__ void copy64_8(void *dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -88,11 +92,13 @@ __global__ void __launch_bounds__(256) emit64(const Model64 *models, const Regio
     }
 }
 
+__device__ __forceinline__ void bar64(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
+
 // ------------------------------------------------------------------------------------------------
-// band facts of the sweeps: 32 anti-diagonals at a time, by the CTA's first warp
+// band facts of the sweeps: 32 anti-diagonals at a time, by the warp of the copies
 // ------------------------------------------------------------------------------------------------
 // DIR: +1 forward, -1 backward.  The block after the current one is loaded at its start and becomes
-// readable half way through it, long before a copy (kAhead64 ahead) asks for it.
+// readable half way through it, long before anything asks for it.
 template <int DIR>
 struct InfoStream {
     int4 *ring;
@@ -100,27 +106,29 @@ struct InfoStream {
     int32_t n, start;
     int4 next;
 
-    __device__ __forceinline__ int32_t row(int32_t k) const { return start + DIR * k; }   // k-th anti-diagonal
-    __device__ __forceinline__ int4 fetch(int32_t k) const {
-        const int32_t d = row(k);
+    __device__ __forceinline__ int4 fetch(int32_t k) const {   // of the k-th anti-diagonal
+        const int32_t d = start + DIR * k;
         int4 v = src[min(max(d, 0), n)];
         if (d < 0 || d > n) v.y = 0;   // no such anti-diagonal: no slots
         return v;
     }
-    __device__ __forceinline__ void open(const int4 *s, int32_t nn, int32_t d0) {
+    __device__ __forceinline__ void open(int4 *r, const int4 *s, int32_t nn, int32_t d0) {
+        ring = r;
         src = s;
         n = nn;
         start = d0;
-        if (threadIdx.x < 32) {
-            ring[threadIdx.x] = fetch(threadIdx.x);
-            ring[32 + threadIdx.x] = fetch(32 + threadIdx.x);
-        }
+        const int lane = threadIdx.x & 31;
+        ring[lane] = fetch(lane);
+        ring[32 + lane] = fetch(32 + lane);
+        __syncwarp();
     }
     // at the k-th step
     __device__ __forceinline__ void advance(int32_t k) {
-        if (threadIdx.x < 32) {
-            if ((k & 31) == 0) next = fetch(k + 64 + threadIdx.x);
-            else if ((k & 31) == 16) ring[((k - 16) + 64 + threadIdx.x) & (kInfoRing - 1)] = next;
+        const int lane = threadIdx.x & 31;
+        if ((k & 31) == 0) next = fetch(k + 64 + lane);
+        else if ((k & 31) == 16) {
+            ring[((k - 16) + 64 + lane) & (kInfoRing - 1)] = next;
+            __syncwarp();
         }
     }
     __device__ __forceinline__ int4 at(int32_t k) const { return ring[k & (kInfoRing - 1)]; }
@@ -208,30 +216,47 @@ __device__ __forceinline__ void lad4(const LogAdd64 &t, const double (&x)[4], co
 // gap-X of d (its neighbours on d-1), gap-Y of d (own column on d-1), all but the last term of the
 // match state of d+1 (neighbours on d-1), and the last term of d's.  So a step takes one log_add's
 // latency, a barrier and a shared-memory round trip, where the states one after another took four.
+// The sweep's warps issue in order, so two more warps take what is not the recursion: the copies, and
+// the stores of the values.
 template <int NT, bool kMulti>
 struct Forward64Shared {
     LogAdd64 la;
     int4 info[kInfoRing];
-    double2 e[kRing64][NT];
+    double2 e[kRing64][NT];            // by slot of the anti-diagonal
     double gx[kRing64][NT];
     int4 pred[kMulti ? kRing64 : 1][kMulti ? NT : 1];   // pred, pred_n, pred_step
-    double v[2][3][NT];                // states by parity of the anti-diagonal
+    double v[2][3][NT];                // states by thread, by parity of the anti-diagonal
 };
 
+// what a thread needs of an anti-diagonal beside the values, in registers before its step
+template <bool kMulti>
+struct ForwardOwn64 {
+    bool in;
+    double2 e;
+    double gx;
+    int4 pr;
+};
+
+template <int NT, bool kMulti>
+__device__ __forceinline__ ForwardOwn64<kMulti> forward_own64(const Forward64Shared<NT, kMulti> &sh, int32_t k) {
+    const int4 in = sh.info[k & (kInfoRing - 1)];
+    const int b = k & (kRing64 - 1);
+    const int32_t i = (threadIdx.x - in.x) & (NT - 1);
+    ForwardOwn64<kMulti> o;
+    o.in = i < in.y;
+    o.e = sh.e[b][i];
+    o.gx = sh.gx[b][i];
+    if constexpr (kMulti) o.pr = o.in ? sh.pred[b][i] : make_int4(0, 0, 0, 0);
+    else o.pr = make_int4((threadIdx.x - 1) & (NT - 1), 1, 0, 0);
+    return o;
+}
+
 template <int NT, bool kMulti, bool kSX>
-__global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Region64 *tasks, SetOut O) {
-    extern __shared__ double2 smem64[];
-    using Sh = Forward64Shared<NT, kMulti>;
-    Sh &sh = *reinterpret_cast<Sh *>(smem64);
-    const Region64 R = tasks[blockIdx.x];
-    const double *mt = models[R.model].t;
+__device__ __forceinline__ void forward_sweep64(const double *mt, const Region64 &R, Forward64Shared<NT, kMulti> &sh) {
     const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY], tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX],
                  tOY = mt[T_OY], tEY = mt[T_EY];
     const int tid = threadIdx.x;
-    const int32_t s = R.s0 <= 1 ? 1 : R.s0, dend = R.win[R.w1 - 1].D;
-    InfoStream<1> info{sh.info};
-    info.open(R.info, R.n, s);
-    if (tid < 16) log_add_table64(sh.la, tid);
+    const int32_t s = R.s0 <= 1 ? 1 : R.s0, steps = R.win[R.w1 - 1].D - s + 1;
     // the values of s-2 (parity 0, as s) and s-1
     double M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf;
     for (int st = 0; st < 3; ++st) sh.v[0][st][tid] = kNegInf;
@@ -239,10 +264,6 @@ __global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Reg
         if (tid == 0) {   // startStateProb / raggedStartStateProb (stateMachine.c:1022-1032) on anti-diagonal 0
             M1 = R.ragged_left ? kNegInf : 0.0;
             X1 = Y1 = R.ragged_left ? 0.0 : kNegInf;
-            double *c = R.F + 3 * (int64_t) R.info[0].z;
-            c[S_M] = M1;
-            c[S_X] = X1;
-            c[S_Y] = Y1;
         }
     } else {   // a later segment: every slot of s-2 and s-1 starts at 0
         const int4 i2 = R.info[s - 2], i1 = R.info[s - 1];
@@ -253,64 +274,20 @@ __global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Reg
     sh.v[1][S_M][tid] = M1;
     sh.v[1][S_X][tid] = X1;
     sh.v[1][S_Y][tid] = Y1;
-    __syncthreads();
-    auto issue = [&](int32_t k) {
-        const int4 in = info.at(k);
-        const int32_t i = (tid - in.x) & (NT - 1), q = in.x + i;
-        if (i < in.y) {
-            const int b = k & (kRing64 - 1);
-            copy64_16(&sh.e[b][tid], R.E + 2 * ((int64_t) in.z + q));
-            copy64_8(&sh.gx[b][tid], &R.path[q].gapx);
-            if constexpr (kMulti) {
-                copy64_8(&sh.pred[b][tid].x, &R.path[q].pred);
-                copy64_8(&sh.pred[b][tid].z, &R.path[q].pred_step);
-            }
-        }
-        copy64_commit();
-    };
-    // what a thread needs of the k-th anti-diagonal beside the values, in registers a step early
-    struct Own {
-        int32_t i, q;
-        bool in;
-        int64_t at;
-        double2 e;
-        double gx;
-        int4 pr;
-    };
-    auto own = [&](int32_t k) -> Own {
-        const int4 in = info.at(k);
-        const int b = k & (kRing64 - 1);
-        Own o;
-        o.i = (tid - in.x) & (NT - 1);
-        o.q = in.x + o.i;
-        o.in = o.i < in.y;
-        o.at = (int64_t) in.z + o.q;
-        o.e = sh.e[b][tid];
-        o.gx = sh.gx[b][tid];
-        if constexpr (kMulti) o.pr = o.in ? sh.pred[b][tid] : make_int4(0, 0, 0, 0);
-        else o.pr = make_int4(o.q - 1, 1, 0, 0);
-        return o;
-    };
-    for (int k = 0; k < kAhead64; ++k) issue(k);
-    copy64_wait<kAhead64 - 2>();
-    Own o0 = own(0), o1 = own(1);
+    bar64(NT + kHelpers64);            // the first rows are ready
+    ForwardOwn64<kMulti> o0 = forward_own64<NT, kMulti>(sh, 0), o1 = forward_own64<NT, kMulti>(sh, 1);
     // match state: all terms but the last, and that
     double most = kNegInf, last = kNegInf;
-    if (!kMulti || o0.pr.y > 0) {
-        for (int32_t a = 0, p = o0.pr.x; a < o0.pr.y; ++a, p += o0.pr.z) {
-            const int w = p & (NT - 1);
-            if (a) most = lad(sh.la, most, last);
-            most = lad(sh.la, most, sh.v[0][S_M][w] + (o0.e.x + tMC));
-            most = lad(sh.la, most, sh.v[0][S_X][w] + (o0.e.x + tMX));
-            last = sh.v[0][S_Y][w] + (o0.e.x + tMY);
-        }
+    for (int32_t a = 0, p = o0.pr.x; a < o0.pr.y; ++a, p += o0.pr.z) {
+        const int w = p & (NT - 1);
+        if (a) most = lad(sh.la, most, last);
+        most = lad(sh.la, most, sh.v[0][S_M][w] + (o0.e.x + tMC));
+        most = lad(sh.la, most, sh.v[0][S_X][w] + (o0.e.x + tMX));
+        last = sh.v[0][S_Y][w] + (o0.e.x + tMY);
     }
-    const int32_t b_in = R.st_in >= 0 ? O.stitch[R.st_in].b : -10, b_out = R.st_out >= 0 ? O.stitch[R.st_out].b : -10;
+    bar64(NT + kHelpers64);            // s-2's values are read
 #pragma unroll 1
-    for (int32_t d = s, k = 0; d <= dend; ++d, ++k) {
-        info.advance(k);
-        issue(k + kAhead64);
-        copy64_wait<kAhead64 - 2>();   // every copy of d+2 and before has landed
+    for (int32_t k = 0; k < steps; ++k) {
         const double eOX = o0.gx + tOX, eEX = o0.gx + tEX, eSX = o0.gx + tSX;
         const double eMC = o1.e.x + tMC, eMX = o1.e.x + tMX, eMY = o1.e.x + tMY;
         double x[4], y[4], r[4];
@@ -318,7 +295,7 @@ __global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Reg
         y[1] = Y1 + (o0.e.y + tEY);
         x[2] = most;
         y[2] = last;
-        __syncthreads();   // d-1's values
+        bar64(NT + kHelpers64);        // d-1's values, d+2's operands
         const double(&v)[3][NT] = sh.v[(k + 1) & 1];
         const int p0 = o0.pr.x & (NT - 1), p1 = o1.pr.x & (NT - 1);
         x[0] = v[S_M][p0] + eOX;
@@ -328,7 +305,7 @@ __global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Reg
         double lY = 0.0;
         if (kSX) lY = v[S_Y][p0] + eSX;
         last = v[S_Y][p1] + eMY;
-        const Own o2 = own(k + 2);
+        const ForwardOwn64<kMulti> o2 = forward_own64<NT, kMulti>(sh, k + 2);
         if constexpr (kMulti) {
             if (o0.pr.y == 0) x[0] = y[0] = lY = kNegInf;
             if (o1.pr.y == 0) x[3] = y[3] = last = kNegInf;
@@ -357,28 +334,107 @@ __global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Reg
         sh.v[k & 1][S_M][tid] = M1;
         sh.v[k & 1][S_X][tid] = X1;
         sh.v[k & 1][S_Y][tid] = Y1;
-        if (o0.in) {
-            double *c = R.F + 3 * o0.at;
-            c[S_M] = M1;
-            c[S_X] = X1;
-            c[S_Y] = Y1;
-        }
-        // the values of b-1 and b to their side of a stitch
-        if (d == b_in - 1 || d == b_in || d == b_out - 1 || d == b_out) {
-            const bool side = d == b_in - 1 || d == b_in;
-            const Stitch64 S = O.stitch[side ? R.st_in : R.st_out];
-            const int blk = side ? d - (b_in - 1) : 2 + d - (b_out - 1);
-            if (o0.in) {
-                double *o = S.vals + 3 * ((int64_t) blk * S.stride + o0.i);
-                o[0] = M1;
-                o[1] = X1;
-                o[2] = Y1;
-            }
-        }
         o0 = o1;
         o1 = o2;
     }
+    bar64(NT + kHelpers64);            // the last anti-diagonal's values go out
+}
+
+template <int NT, bool kMulti>
+__device__ __forceinline__ void forward_copies64(const Region64 &R, Forward64Shared<NT, kMulti> &sh) {
+    const int lane = threadIdx.x & 31;
+    const int32_t s = R.s0 <= 1 ? 1 : R.s0, steps = R.win[R.w1 - 1].D - s + 1;
+    InfoStream<1> info;
+    info.open(sh.info, R.info, R.n, s);
+    auto issue = [&](int32_t k, const int4 &in) {
+        const int b = k & (kRing64 - 1);
+        const double *e = R.E + 2 * ((int64_t) in.z + in.x);
+        const Path64 *path = R.path + in.x;
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) {
+            const int i = lane + 32 * w;
+            if (i < in.y) {
+                copy64_16(&sh.e[b][i], e + 2 * i);
+                copy64_8(&sh.gx[b][i], &path[i].gapx);
+                if constexpr (kMulti) {
+                    copy64_8(&sh.pred[b][i].x, &path[i].pred);
+                    copy64_8(&sh.pred[b][i].z, &path[i].pred_step);
+                }
+            }
+        }
+        copy64_commit();
+    };
+#pragma unroll
+    for (int k = 0; k < kAhead64; ++k) issue(k, info.at(k));
+    copy64_wait<kAhead64 - 3>();
+    int4 in = info.at(kAhead64);
+    bar64(NT + kHelpers64);
+    bar64(NT + kHelpers64);
+    for (int32_t k = 0; k < steps; ++k) {
+        bar64(NT + kHelpers64);
+        issue(k + kAhead64, in);
+        info.advance(k);
+        in = info.at(k + kAhead64 + 1);
+        copy64_wait<kAhead64 - 3>();   // every copy of d+3 and before has landed
+    }
+    bar64(NT + kHelpers64);
     copy64_wait<0>();
+}
+
+// at step k d-1's values go to the store and, where a stitch is, to its side
+template <int NT, bool kMulti>
+__device__ __forceinline__ void forward_results64(const Region64 &R, const SetOut &O, Forward64Shared<NT, kMulti> &sh) {
+    const int lane = threadIdx.x & 31;
+    const int32_t s = R.s0 <= 1 ? 1 : R.s0, steps = R.win[R.w1 - 1].D - s + 1;
+    if (R.s0 <= 1 && lane == 0) {
+        double *c = R.F + 3 * (int64_t) R.info[0].z;
+        c[S_M] = R.ragged_left ? kNegInf : 0.0;
+        c[S_X] = c[S_Y] = R.ragged_left ? 0.0 : kNegInf;
+    }
+    const int32_t b_in = R.st_in >= 0 ? O.stitch[R.st_in].b : -10, b_out = R.st_out >= 0 ? O.stitch[R.st_out].b : -10;
+    bar64(NT + kHelpers64);
+    bar64(NT + kHelpers64);
+    bar64(NT + kHelpers64);            // step 0
+    int4 in = sh.info[0];
+    for (int32_t k = 1; k <= steps; ++k) {
+        const int32_t r = s + k - 1;   // the anti-diagonal that goes out
+        double *c = R.F + 3 * ((int64_t) in.z + in.x + lane);
+        int at[NT / 32];
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) at[w] = (in.x + lane + 32 * w) & (NT - 1);
+        bar64(NT + kHelpers64);
+        const double(&v)[3][NT] = sh.v[(k - 1) & 1];
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) {
+            if (lane + 32 * w < in.y) {
+                c[96 * w + S_M] = v[S_M][at[w]];
+                c[96 * w + S_X] = v[S_X][at[w]];
+                c[96 * w + S_Y] = v[S_Y][at[w]];
+            }
+        }
+        if (r == b_in - 1 || r == b_in || r == b_out - 1 || r == b_out) {
+            const bool side = r == b_in - 1 || r == b_in;
+            const Stitch64 S = O.stitch[side ? R.st_in : R.st_out];
+            double *o = S.vals + 3 * (int64_t) (side ? r - (b_in - 1) : 2 + r - (b_out - 1)) * S.stride;
+            for (int i = lane; i < in.y; i += 32)
+                for (int st = 0; st < 3; ++st) o[3 * i + st] = v[st][(in.x + i) & (NT - 1)];
+        }
+        in = sh.info[k & (kInfoRing - 1)];
+    }
+}
+
+template <int NT, bool kMulti, bool kSX>
+__global__ void __launch_bounds__(NT + kHelpers64) forward64(const Model64 *models, const Region64 *tasks, SetOut O) {
+    extern __shared__ double2 smem64[];
+    using Sh = Forward64Shared<NT, kMulti>;
+    Sh &sh = *reinterpret_cast<Sh *>(smem64);
+    const Region64 R = tasks[blockIdx.x];
+    if (threadIdx.x < 16) log_add_table64(sh.la, threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x < NT) forward_sweep64<NT, kMulti, kSX>(models[R.model].t, R, sh);
+    else if (threadIdx.x < NT + 32) forward_copies64<NT, kMulti>(R, sh);
+    else forward_results64<NT, kMulti>(R, O, sh);
+    __syncthreads();
     if (R.st_in >= 0) stitch_arrive64(R, O, R.st_in);
     if (R.st_out >= 0) stitch_arrive64(R, O, R.st_out);
 }
@@ -391,135 +447,88 @@ __global__ void __launch_bounds__(NT) forward64(const Model64 *models, const Reg
 // side by side: gap-X and gap-Y of d, the match state of d but for its last term, and the last term of
 // d+1's (which nothing needs before d-1).  What d+1's match value goes into (F.B, the terms of a total
 // probability's two folds: F.B on that anti-diagonal, and the matches from the one before it over it
-// into the one after, dotted with B there) is therefore written a step late.
+// into the one after, dotted with B there) is therefore written a step late or later.
 template <int NT, bool kMulti>
 struct Backward64Shared {
     LogAdd64 la;
     int4 info[kInfoRing];
-    double2 e[kRing64][NT];
-    double gx[kRing64][NT];
+    double2 e[kRing64][NT];            // by slot of the anti-diagonal
+    double gx[NT > 256 ? 1 : kRing64][NT > 256 ? 1 : NT];   // (512 threads read it where it is: no room)
     int4 nb[kMulti ? kRing64 : 1][kMulti ? NT : 1];        // succ, succ_n; pred, pred_n
     int32_t step[kMulti ? kRing64 : 1][kMulti ? NT : 1];   // pred_step
     double f[kRing64][NT];             // forward match value
     double fx[2][NT];                  // forward gap values of a total's anti-diagonal
     double fm[3][NT];                  // forward values of the anti-diagonal before it
-    double a[2][3][NT];                // sums for the match predecessors, by parity
-    double b[2][3][NT];                // sums for the gap-X predecessors, by parity
+    double a[2][3][NT];                // sums for the match predecessors, by thread, by parity
+    double b[2][3][NT];                // sums for the gap-X predecessors, by thread, by parity
+    double vm[2][NT];                  // match values by thread, by parity of the anti-diagonal
+    double vx[4][NT], vy[4][NT];       // gap values (expectations)
 };
+
+static_assert(sizeof(Backward64Shared<512, false>) <= 227 * 1024 && sizeof(Backward64Shared<256, true>) <= 227 * 1024 &&
+                  sizeof(Forward64Shared<512, false>) <= 227 * 1024,
+              "a CTA's shared memory");
 
 // the path a thread holds on an anti-diagonal
 struct Held64 {
     int32_t i, n;                      // its slot, and the anti-diagonal's slots
-    int64_t at;                        // its place in the stores
     int4 pred;                         // its predecessors: first, count, step
     double e;                          // its match emission
     double M;                          // its match value
 };
 
 template <int NT, bool kMulti, bool kSX>
-__global__ void __launch_bounds__(NT) backward64(const Model64 *models, const Region64 *tasks, const Window64 *windows,
-                                                 double *terms, int64_t term_stride, int expect) {
-    extern __shared__ double2 smem64[];
-    using Sh = Backward64Shared<NT, kMulti>;
-    Sh &sh = *reinterpret_cast<Sh *>(smem64);
-    const Window64 wt = windows[blockIdx.x];
-    const Region64 R = tasks[wt.task];
-    const double *mt = models[R.model].t;
+__device__ __forceinline__ void backward_sweep64(const double *mt, const Region64 &R, const Window64 &wt, const Window &W,
+                                                 Backward64Shared<NT, kMulti> &sh, double *terms, int64_t term_stride,
+                                                 int expect) {
     const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY], tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX],
                  tOY = mt[T_OY], tEY = mt[T_EY];
-    const Window W = R.win[wt.win];
     const int tid = threadIdx.x;
+    const int32_t steps = W.D - W.T;
     // endStateProb / raggedEndStateProb (stateMachine.c:1034-1061) on the traceback anti-diagonal
     const bool ragged_end = W.at_end && R.ragged_right;
     const double e0 = ragged_end ? (tOX + tOY) / 2.0 : tMC, e1 = ragged_end ? tEX : tMX, e2 = ragged_end ? tEY : tMY;
-    InfoStream<-1> info{sh.info};
-    info.open(R.info, R.n, W.D);
-    if (tid < 16) log_add_table64(sh.la, tid);
     for (int k = 0; k < 2; ++k)
         for (int st = 0; st < 3; ++st) sh.a[k][st][tid] = sh.b[k][st][tid] = kNegInf;
-    __syncthreads();
-    const int32_t steps = W.D - W.T;
-    auto issue = [&](int32_t k) {
-        if (k < steps) {
-            const int32_t d = W.D - k;
-            const int4 in = info.at(k);
-            const int32_t i = (tid - in.x) & (NT - 1), q = in.x + i;
-            const bool post = d <= W.from, total = post && (W.from - d) % 10 == 0;
-            const int b = k & (kRing64 - 1);
-            if (i < in.y) {
-                const int64_t at = (int64_t) in.z + q;
-                copy64_16(&sh.e[b][tid], R.E + 2 * at);
-                copy64_8(&sh.gx[b][tid], &R.path[q].gapx);
-                if constexpr (kMulti) {
-                    copy64_8(&sh.nb[b][tid].x, &R.path[q].succ);
-                    copy64_8(&sh.nb[b][tid].z, &R.path[q].pred);
-                    sh.step[b][tid] = R.path[q].pred_step;
-                }
-                if (post) copy64_8(&sh.f[b][tid], R.F + 3 * at);
-                if (total) {
-                    copy64_8(&sh.fx[0][tid], R.F + 3 * at + S_X);
-                    copy64_8(&sh.fx[1][tid], R.F + 3 * at + S_Y);
-                }
-            }
-            if (total) {
-                const int4 bl = info.at(k + 1);
-                const int32_t j = (tid - bl.x) & (NT - 1);
-                if (j < bl.y) {
-                    const double *f = R.F + 3 * ((int64_t) bl.z + bl.x + j);
-                    for (int st = 0; st < 3; ++st) copy64_8(&sh.fm[st][tid], f + st);
-                } else {
-                    for (int st = 0; st < 3; ++st) sh.fm[st][tid] = kNegInf;
-                }
-            }
-        }
-        copy64_commit();
-    };
     struct Own {
-        int32_t i, n, q;
-        int64_t at;
+        int32_t i, n;
         double2 e;
-        double gx, f;
+        double gx;
         int4 nb;
         int32_t step;
     };
     auto own = [&](int32_t k) -> Own {
-        const int4 in = info.at(k);
+        const int4 in = sh.info[k & (kInfoRing - 1)];
         const int b = k & (kRing64 - 1);
         Own o;
         o.i = (tid - in.x) & (NT - 1);
         o.n = k < steps ? in.y : 0;
-        o.q = in.x + o.i;
-        o.at = (int64_t) in.z + o.q;
-        o.e = sh.e[b][tid];
-        o.gx = sh.gx[b][tid];
-        o.f = sh.f[b][tid];
-        o.nb = make_int4(o.q + 1, 1, o.q - 1, 1);
+        o.e = sh.e[b][o.i];
+        if constexpr (NT > 256) o.gx = o.i < o.n ? __ldg(&R.path[in.x + o.i].gapx) : 0.0;
+        else o.gx = sh.gx[b][o.i];
         o.step = 0;
         if constexpr (kMulti) {
-            o.nb = o.i < o.n ? sh.nb[b][tid] : make_int4(0, 0, 0, 0);
-            o.step = sh.step[b][tid];
+            o.nb = o.i < o.n ? sh.nb[b][o.i] : make_int4(0, 0, 0, 0);
+            o.step = sh.step[b][o.i];
+        } else {
+            o.nb = make_int4(in.x + o.i + 1, 1, in.x + o.i - 1, 1);
         }
         return o;
     };
-    for (int k = 0; k < kAhead64; ++k) issue(k);
-    copy64_wait<kAhead64 - 1>();
+    bar64(NT + kHelpers64);                          // the first rows are ready
     Own o0 = own(0);
-    double f1 = 0.0;                                 // forward match value of d+1
     double u0 = kNegInf, u1 = kNegInf;               // own path's gap-Y sums of d+1
     double most = kNegInf, last = kNegInf;           // its match state on d+1: all terms but one, and that
     double X1 = kNegInf, Y1 = kNegInf;               // its gap values on d+1
-    Held64 h1{0, 0, 0, make_int4(0, 0, 0, 0), 0.0, kNegInf}, h2 = h1;   // the paths held on d+1, d+2
+    Held64 h1{0, 0, make_int4(0, 0, 0, 0), 0.0, kNegInf}, h2 = h1;   // the paths held on d+1, d+2
     int64_t total_at = wt.first_total;
+    int32_t until = W.D - W.from;                    // steps until the next total's anti-diagonal
 #pragma unroll 1
     for (int32_t k = 0; k <= steps; ++k) {           // k == steps: only what is a step late
-        const int32_t d = W.D - k;
-        info.advance(k);
-        issue(k + kAhead64);
-        copy64_wait<kAhead64 - 1>();                 // every copy of d-1 and above has landed
         const bool inb = o0.i < o0.n;
         const int4 nb = o0.nb;
         double x[4], y[4], r[4];
-        __syncthreads();   // d+1's sums for gap-X predecessors, d+2's for match predecessors
+        bar64(NT + kHelpers64);                      // d+1's sums for gap-X predecessors, d+2's for match predecessors
         const double(&a)[3][NT] = sh.a[k & 1];
         const double(&c)[3][NT] = sh.b[(k + 1) & 1];
         const int p0 = nb.x & (NT - 1);
@@ -554,76 +563,172 @@ __global__ void __launch_bounds__(NT) backward64(const Model64 *models, const Re
                 if (kSX) r[1] = lad(sh.la, r[1], c[2][w]);
             }
         }
-        double vX = r[0], vY = r[1], m = r[2];
-        h1.M = h1.i < h1.n ? r[3] : kNegInf;
-        if (k == 0) {
-            m = e0;
-            l = kNegInf;
-            vX = e1;
-            vY = e2;
-        }
-        most = m;
-        last = l;
-        vX = inb ? vX : kNegInf;
-        vY = inb ? vY : kNegInf;
-        const double2 e = o0.e;
-        const double gx = o0.gx;
-        // match sums of d+1 (a buffer's parity is its anti-diagonal's plus one), gap sums of d
         const bool in1 = h1.i < h1.n;
+        h1.M = in1 ? r[3] : kNegInf;
+        if (k == 0) {
+            r[2] = e0;
+            l = kNegInf;
+            r[0] = e1;
+            r[1] = e2;
+        }
+        most = r[2];
+        last = l;
+        const double vX = inb ? r[0] : kNegInf, vY = inb ? r[1] : kNegInf;
+        // match sums of d+1 (a buffer's parity is its anti-diagonal's plus one), gap sums of d
         sh.a[(k + 1) & 1][0][tid] = in1 ? h1.M + (h1.e + tMC) : kNegInf;
         sh.a[(k + 1) & 1][1][tid] = in1 ? h1.M + (h1.e + tMX) : kNegInf;
         sh.a[(k + 1) & 1][2][tid] = in1 ? h1.M + (h1.e + tMY) : kNegInf;
-        sh.b[k & 1][0][tid] = inb ? vX + (gx + tOX) : kNegInf;
-        sh.b[k & 1][1][tid] = inb ? vX + (gx + tEX) : kNegInf;
-        if (kSX) sh.b[k & 1][2][tid] = inb ? vX + (gx + tSX) : kNegInf;
-        u0 = inb ? vY + (e.y + tOY) : kNegInf;
-        u1 = inb ? vY + (e.y + tEY) : kNegInf;
-        // d+1's outputs
-        if (k > 0 && d + 1 <= W.from) {
-            const double f = f1;
+        sh.b[k & 1][0][tid] = inb ? vX + (o0.gx + tOX) : kNegInf;
+        sh.b[k & 1][1][tid] = inb ? vX + (o0.gx + tEX) : kNegInf;
+        if (kSX) sh.b[k & 1][2][tid] = inb ? vX + (o0.gx + tSX) : kNegInf;
+        u0 = inb ? vY + (o0.e.y + tOY) : kNegInf;
+        u1 = inb ? vY + (o0.e.y + tEY) : kNegInf;
+        sh.vm[(k + 1) & 1][tid] = h1.M;              // of the anti-diagonal before, for the warp of the results
+        if (expect) {
+            sh.vx[k & 3][tid] = vX;
+            sh.vy[k & 3][tid] = vY;
+        }
+        if (k == until + 1) {
+            // d+1 is a total's: its terms
+            until += 10;
+            double *t0 = terms + total_at * 2 * term_stride;
             if (in1) {
-                R.S[h1.at] = f + h1.M;
-                if (expect) {
-                    R.B[3 * h1.at + S_M] = h1.M;
-                    R.B[3 * h1.at + S_X] = X1;
-                    R.B[3 * h1.at + S_Y] = Y1;
-                }
+                double s = sh.f[(k - 1) & (kRing64 - 1)][h1.i] + h1.M;
+                s = lad(sh.la, s, sh.fx[0][h1.i] + X1);
+                s = lad(sh.la, s, sh.fx[1][h1.i] + Y1);
+                t0[h1.i] = s;
             }
-            if ((W.from - d - 1) % 10 == 0) {
-                double *t0 = terms + total_at * 2 * term_stride;
-                if (in1) {
-                    double s = f + h1.M;
-                    s = lad(sh.la, s, sh.fx[0][tid] + X1);
-                    s = lad(sh.la, s, sh.fx[1][tid] + Y1);
-                    t0[h1.i] = s;
+            if (k > 1 && h2.i < h2.n) {
+                // the slot of d+2 this thread held: its predecessors' forward values on d
+                const int4 below = sh.info[k & (kInfoRing - 1)];
+                auto fm = [&](int st, int32_t q) {
+                    const int32_t j = q - below.x;
+                    return j >= 0 && j < below.y ? sh.fm[st][j] : kNegInf;
+                };
+                double w = kNegInf;
+                for (int32_t j = 0, p = h2.pred.x; j < h2.pred.y; ++j, p += h2.pred.z) {
+                    w = lad(sh.la, w, fm(S_M, p) + (h2.e + tMC));
+                    w = lad(sh.la, w, fm(S_X, p) + (h2.e + tMX));
+                    w = lad(sh.la, w, fm(S_Y, p) + (h2.e + tMY));
                 }
-                if (k > 1 && h2.i < h2.n) {
-                    // the slot of d+2 this thread held: its predecessors' forward values on d
-                    double w = kNegInf;
-                    if constexpr (!kMulti) {
-                        const int p = h2.pred.x & (NT - 1);
-                        w = lad(sh.la, sh.fm[S_M][p] + (h2.e + tMC), sh.fm[S_X][p] + (h2.e + tMX));
-                        w = lad(sh.la, w, sh.fm[S_Y][p] + (h2.e + tMY));
-                    } else {
-                        for (int32_t j = 0, p = h2.pred.x; j < h2.pred.y; ++j, p += h2.pred.z) {
-                            w = lad(sh.la, w, sh.fm[S_M][p & (NT - 1)] + (h2.e + tMC));
-                            w = lad(sh.la, w, sh.fm[S_X][p & (NT - 1)] + (h2.e + tMX));
-                            w = lad(sh.la, w, sh.fm[S_Y][p & (NT - 1)] + (h2.e + tMY));
-                        }
-                    }
-                    t0[term_stride + h2.i] = w + h2.M;
-                }
-                ++total_at;
+                t0[term_stride + h2.i] = w + h2.M;
             }
+            ++total_at;
         }
         X1 = vX;
         Y1 = vY;
         h2 = h1;
-        h1 = Held64{o0.i, o0.n, o0.at, make_int4(nb.z, nb.w, o0.step, 0), e.x, kNegInf};
-        f1 = o0.f;
+        h1 = Held64{o0.i, o0.n, make_int4(nb.z, nb.w, o0.step, 0), o0.e.x, kNegInf};
         o0 = o1;
     }
+    bar64(NT + kHelpers64);                          // the last match values go out
+}
+
+template <int NT, bool kMulti>
+__device__ __forceinline__ void backward_copies64(const Region64 &R, const Window &W, Backward64Shared<NT, kMulti> &sh) {
+    const int lane = threadIdx.x & 31;
+    const int32_t steps = W.D - W.T;
+    InfoStream<-1> info;
+    info.open(sh.info, R.info, R.n, W.D);
+    auto issue = [&](int32_t k, const int4 &in) {
+        if (k < steps) {
+            const int32_t d = W.D - k;
+            const bool post = d <= W.from, total = post && (W.from - d) % 10 == 0;
+            const int b = k & (kRing64 - 1);
+            const double *e = R.E + 2 * ((int64_t) in.z + in.x), *f = R.F + 3 * ((int64_t) in.z + in.x);
+            const Path64 *path = R.path + in.x;
+#pragma unroll
+            for (int w = 0; w < NT / 32; ++w) {
+                const int i = lane + 32 * w;
+                if (i < in.y) {
+                    copy64_16(&sh.e[b][i], e + 2 * i);
+                    if constexpr (NT <= 256) copy64_8(&sh.gx[b][i], &path[i].gapx);
+                    if constexpr (kMulti) {
+                        copy64_8(&sh.nb[b][i].x, &path[i].succ);
+                        copy64_8(&sh.nb[b][i].z, &path[i].pred);
+                        copy64_4(&sh.step[b][i], &path[i].pred_step);
+                    }
+                    if (post) copy64_8(&sh.f[b][i], f + 3 * i);
+                    if (total) {
+                        copy64_8(&sh.fx[0][i], f + 3 * i + S_X);
+                        copy64_8(&sh.fx[1][i], f + 3 * i + S_Y);
+                    }
+                }
+            }
+            if (total) {
+                const int4 bl = info.at(k + 1);
+                const double *g = R.F + 3 * ((int64_t) bl.z + bl.x);
+                for (int i = lane; i < bl.y; i += 32)
+                    for (int st = 0; st < 3; ++st) copy64_8(&sh.fm[st][i], g + 3 * i + st);
+            }
+        }
+        copy64_commit();
+    };
+#pragma unroll
+    for (int k = 0; k < kBehind64; ++k) issue(k, info.at(k));
+    copy64_wait<kBehind64 - 2>();
+    int4 in = info.at(kBehind64);
+    bar64(NT + kHelpers64);
+    for (int32_t k = 0; k <= steps; ++k) {
+        bar64(NT + kHelpers64);
+        issue(k + kBehind64, in);
+        info.advance(k);
+        in = info.at(k + kBehind64 + 1);
+        copy64_wait<kBehind64 - 2>();                // every copy of d-2 and above has landed
+    }
+    bar64(NT + kHelpers64);
     copy64_wait<0>();
+}
+
+// at step k d+2's F.B of the match state, and (expectations) its values, go to their stores
+template <int NT, bool kMulti>
+__device__ __forceinline__ void backward_results64(const Region64 &R, const Window &W, Backward64Shared<NT, kMulti> &sh,
+                                                   int expect) {
+    const int lane = threadIdx.x & 31;
+    const int32_t steps = W.D - W.T;
+    bar64(NT + kHelpers64);
+    bar64(NT + kHelpers64);
+    bar64(NT + kHelpers64);                          // steps 0 and 1 (a match value is there two steps on)
+    int4 in = sh.info[0];
+    for (int32_t k = 0; k < steps; ++k) {            // the anti-diagonal that goes out
+        bar64(NT + kHelpers64);
+        if (W.D - k <= W.from) {
+            const int64_t z = (int64_t) in.z + in.x + lane;
+#pragma unroll
+            for (int w = 0; w < NT / 32; ++w) {
+                const int i = lane + 32 * w, at = (in.x + i) & (NT - 1);
+                if (i < in.y) {
+                    const double m = sh.vm[k & 1][at];
+                    R.S[z + 32 * w] = sh.f[k & (kRing64 - 1)][i] + m;
+                    if (expect) {
+                        double *b = R.B + 3 * (z + 32 * w);
+                        b[S_M] = m;
+                        b[S_X] = sh.vx[k & 3][at];
+                        b[S_Y] = sh.vy[k & 3][at];
+                    }
+                }
+            }
+        }
+        in = sh.info[(k + 1) & (kInfoRing - 1)];
+    }
+}
+
+template <int NT, bool kMulti, bool kSX>
+__global__ void __launch_bounds__(NT + kHelpers64) backward64(const Model64 *models, const Region64 *tasks,
+                                                              const Window64 *windows, double *terms, int64_t term_stride,
+                                                              int expect) {
+    extern __shared__ double2 smem64[];
+    using Sh = Backward64Shared<NT, kMulti>;
+    Sh &sh = *reinterpret_cast<Sh *>(smem64);
+    const Window64 wt = windows[blockIdx.x];
+    const Region64 R = tasks[wt.task];
+    const Window W = R.win[wt.win];
+    if (threadIdx.x < 16) log_add_table64(sh.la, threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x < NT)
+        backward_sweep64<NT, kMulti, kSX>(models[R.model].t, R, wt, W, sh, terms, term_stride, expect);
+    else if (threadIdx.x < NT + 32) backward_copies64<NT, kMulti>(R, W, sh);
+    else backward_results64<NT, kMulti>(R, W, sh, expect);
 }
 
 // ------------------------------------------------------------------------------------------------
