@@ -64,7 +64,7 @@ struct Region64 {
     double *loglik;
     int32_t *status;
     // resident kernels (sa_fp64_resident.cuh): per anti-diagonal {first path, paths, first slot - first
-    // path, window}; the paths; F.B of the match state per slot; the region's first window among the
+    // path, window}; the paths; the backward match value per slot; the region's first window among the
     // set's; the read's accumulators; the region's first column in the read
     const int4 *info;
     const struct Path64 *path;
@@ -719,7 +719,7 @@ namespace {
 // resident route: its store of every anti-diagonal, at most (the rings of the other route take a few
 // MB a region whatever its length), and the threads its sweeps may use
 constexpr size_t kResidentBytes = (size_t) 24 << 30;
-constexpr int kResidentThreads[] = {128, 256, 512};
+constexpr int kResidentThreads[] = {128, 256, 480};
 
 // host plan of one region: geometry (band, windows) and its paths
 struct PlainRegion {
@@ -1071,7 +1071,7 @@ size_t resident_layout(PlainSet *s, unsigned char *host, unsigned char *dev) {
     const size_t o_P = take((size_t) s->n_rows * sizeof(double));
     s->p_bytes = (size_t) s->n_rows * sizeof(double);
     const size_t o_rows = take((size_t) s->n_rows * sizeof(int32_t));
-    const size_t o_terms = take((size_t) s->n_totals * 2 * (size_t) s->term_stride * sizeof(double));
+    const size_t o_terms = take((size_t) s->n_totals * kTotalRows * (size_t) s->term_stride * sizeof(double));
     std::vector<size_t> o_E(nreg), o_S(nreg), o_B(nreg), o_F((size_t) s->n_run_tasks), o_sv((size_t) s->n_stitch);
     size_t t = 0;
     auto first_row = [](const PlainRegion &pr, size_t q) {   // of task q's store
@@ -1188,7 +1188,7 @@ size_t resident_layout(PlainSet *s, unsigned char *host, unsigned char *dev) {
                 windows[nw] = Window64{(int32_t) ntask, w, (int32_t) nt, 0};
                 task_of[nw] = (int32_t) ntask;
                 for (int32_t d = W.from; d > W.T; d -= 10)
-                    totals[nt++] = Total64{(int32_t) i, d, d < W.D ? 1 : 0, d == r.n ? 1 : 0};
+                    totals[nt++] = Total64{(int32_t) i, d, w, (int16_t) (d < W.D), (int16_t) (d == r.n)};
             }
         }
         for (size_t q = 0; q < pr.cuts.size(); ++q) {
@@ -1494,8 +1494,8 @@ bool sweeps64(PlainSet *s, const SetOut &O, cudaStream_t stream) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd) != cudaSuccess ||
         cudaFuncSetAttribute(b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd) != cudaSuccess)
         return false;
-    f<<<(unsigned) s->n_run_tasks, NT + kHelpers64, fwd, stream>>>(s->d_models, s->d_tasks, O);
-    b<<<(unsigned) s->n_windows, NT + kHelpers64, bwd, stream>>>(s->d_models, s->d_tasks, s->d_windows, s->d_terms, s->term_stride,
+    f<<<(unsigned) s->n_run_tasks, kSweepThreads64<NT>, fwd, stream>>>(s->d_models, s->d_tasks, O);
+    b<<<(unsigned) s->n_windows, kSweepThreads64<NT>, bwd, stream>>>(s->d_models, s->d_tasks, s->d_windows, s->d_terms, s->term_stride,
                                                    s->expect ? 1 : 0);
     return cudaGetLastError() == cudaSuccess;
 }
@@ -1512,10 +1512,11 @@ sa_status resident_sweeps(PlainSet *s, const SetOut &O, cudaStream_t stream) {
     if (s->multi) ok = s->nt == 128 ? sweeps64<128, true>(s, O, stream) : sweeps64<256, true>(s, O, stream);
     else if (s->nt == 128) ok = sweeps64<128, false>(s, O, stream);
     else if (s->nt == 256) ok = sweeps64<256, false>(s, O, stream);
-    else ok = sweeps64<512, false>(s, O, stream);
+    else ok = sweeps64<480, false>(s, O, stream);
     if (!ok) return SA_E_CUDA;
-    totals64<<<(unsigned) ((s->n_totals + 63) / 64), 64, 0, stream>>>(s->d_regions, s->d_totals, s->n_totals, s->d_terms,
-                                                                     s->term_stride, s->multi ? 1 : 0);
+    totals64<<<(unsigned) ((s->n_totals + kTotalWarps - 1) / kTotalWarps), 32 * kTotalWarps, 0, stream>>>(
+        s->d_models, s->d_regions, s->d_tasks, s->d_task_of, s->d_totals, s->n_totals, s->d_terms, s->term_stride,
+        s->multi ? 1 : 0);
     count_launch(4);
     return cudaGetLastError() == cudaSuccess ? SA_OK : SA_E_CUDA;
 }
@@ -1534,10 +1535,12 @@ sa_status resident_outputs(PlainSet *s, const ExpectOut *reads, const int32_t *f
     const unsigned nc = (unsigned) s->n_chunks, nr = (unsigned) s->regs.size();
     // regions that do not run have no counts
     if (cudaMemsetAsync(s->d_count_rows, 0, (size_t) s->n_rows * sizeof(int32_t), stream) != cudaSuccess) return SA_E_CUDA;
-    outputs64<kAssign, false><<<nc, 256, 0, stream>>>(s->d_regions, s->d_chunk_region, s->d_chunk_d0, s->d_row_base, O);
+    outputs64<kAssign, false><<<nc, 256, 0, stream>>>(s->d_regions, s->d_tasks, s->d_task_of, s->d_chunk_region, s->d_chunk_d0,
+                                                     s->d_row_base, O);
     scan64<<<nr, 1024, 0, stream>>>(s->d_regions, s->d_row_base, O);
     place64<<<1, 32, 0, stream>>>((int64_t) nr, s->d_region_total, s->d_region_count, s->d_count, first);
-    outputs64<kAssign, true><<<nc, 256, 0, stream>>>(s->d_regions, s->d_chunk_region, s->d_chunk_d0, s->d_row_base, O);
+    outputs64<kAssign, true><<<nc, 256, 0, stream>>>(s->d_regions, s->d_tasks, s->d_task_of, s->d_chunk_region, s->d_chunk_d0,
+                                                     s->d_row_base, O);
     count_launch(4);
     return cudaGetLastError() == cudaSuccess ? SA_OK : SA_E_CUDA;
 }

@@ -3,9 +3,9 @@
 //
 //   emit64      the emissions of every path slot
 //   forward64   a CTA per forward segment, a path per thread: stores every anti-diagonal's values
-//   backward64  a CTA per traceback window, a path per thread: stores F.B of the match state of every
-//               slot, and the terms of the total probabilities
-//   totals64    a thread per total probability (the reference's sequential folds)
+//   backward64  a CTA per traceback window, a path per thread: stores the match value of every slot, and
+//               what the total probabilities need
+//   totals64    a warp per total probability (the reference's sequential folds)
 //   posterior pairs: count64, scan64, place64, write64, in the reference's order; or, in
 //   expectations mode, transitions64, kmers64 and finish64 (and the HDP machine's assignments with
 //   the pairs' kernels)
@@ -23,9 +23,7 @@
 // route only if they span at most NT paths.
 #pragma once
 
-constexpr int kAhead64 = 6;            // anti-diagonals between a copy and its use (forward)
-constexpr int kBehind64 = 5;           // and backward, where a row is read once more after its use
-constexpr int kHelpers64 = 64;         // threads of the warps beside a sweep's: copies, results
+constexpr int kAhead64 = 6;            // anti-diagonals between a copy and its use
 constexpr int kRing64 = 8;             // rows of the copy rings
 constexpr int kInfoRing = 128;         // rows of band facts kept
 
@@ -47,8 +45,12 @@ struct Window64 {
 
 struct Total64 {
     int32_t region, d;                 // anti-diagonal
-    int32_t have_next, last;           // d < D; d ends the region
+    int32_t win;                       // its window in the region
+    int16_t have_next, last;           // d < D; d ends the region
 };
+// what the backward sweep leaves of a total's anti-diagonal d, by slot: match, gap-X and gap-Y values of
+// d, match values of d+1
+constexpr int kTotalRows = 4;
 
 __device__ __forceinline__ void copy64_4(void *dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src)
@@ -180,13 +182,13 @@ __device__ __forceinline__ double lad(const LogAdd64 &t, double x, double y) {
     return pick64(x, y, ((c[0] * d + c[16]) * d + c[32]) * d + c[48], d);
 }
 
-// four independent ones, stage by stage
-__device__ __forceinline__ void lad4(const LogAdd64 &t, const double (&x)[4], const double (&y)[4], double (&r)[4]) {
-    double d[4], p[4], b[4], c[4], e[4];
+// two independent ones, stage by stage
+__device__ __forceinline__ void lad2(const LogAdd64 &t, const double (&x)[2], const double (&y)[2], double (&r)[2]) {
+    double d[2], p[2], b[2], c[2], e[2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) d[j] = fabs(x[j] - y[j]);
+    for (int j = 0; j < 2; ++j) d[j] = fabs(x[j] - y[j]);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j) {
         const double *q = piece64(t, d[j]);
         p[j] = q[0];
         b[j] = q[16];
@@ -194,172 +196,214 @@ __device__ __forceinline__ void lad4(const LogAdd64 &t, const double (&x)[4], co
         e[j] = q[48];
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
+    for (int j = 0; j < 2; ++j) p[j] = p[j] * d[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] + b[j];
+    for (int j = 0; j < 2; ++j) p[j] = p[j] + b[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
+    for (int j = 0; j < 2; ++j) p[j] = p[j] * d[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] + c[j];
+    for (int j = 0; j < 2; ++j) p[j] = p[j] + c[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] * d[j];
+    for (int j = 0; j < 2; ++j) p[j] = p[j] * d[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = p[j] + e[j];
+    for (int j = 0; j < 2; ++j) p[j] = p[j] + e[j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) r[j] = pick64(x[j], y[j], p[j], d[j]);
+    for (int j = 0; j < 2; ++j) r[j] = pick64(x[j], y[j], p[j], d[j]);
+}
+
+// ------------------------------------------------------------------------------------------------
+// the sweeps' warps
+// ------------------------------------------------------------------------------------------------
+// A sweep is a chain of anti-diagonals and its warps issue in order, so what counts is how much one
+// warp does a step.  Four log_adds of a step are independent of one another; two groups of NT threads
+// take two each (gap-X and gap-Y of d; the match state but for its last term, and the last term of the
+// anti-diagonal next to it), and two more warps take what is not the recursion: the copies, and the
+// stores.  Operands lie by thread, those of slots outside the band as log 0, which makes a path that is
+// not there drop out without a test.  Cycles a step of the forward sweep: one group with its own copies
+// and stores 895, with bank conflicts gone 805, with the two helper warps 600 (290 of them without the
+// log_adds), in this form @@CYC@@.
+template <int NT>
+constexpr int kHelperWarps64 = NT <= 256 ? 2 : 1;   // of the copies, and as many of the stores
+template <int NT>
+constexpr int kSweepThreads64 = 2 * NT + 64 * kHelperWarps64<NT>;
+
+// Path q stays on thread q mod NT of a group: 128, 256, or (what a CTA of 1,024 threads holds twice, one-path
+// sets only) 480.
+template <int NT>
+constexpr bool kPow2 = (NT & (NT - 1)) == 0;
+
+// the slot that thread t holds on an anti-diagonal whose first path is lo (beyond it: at or past its end)
+template <int NT>
+__device__ __forceinline__ int32_t slot64(int32_t t, int32_t lo) {
+    if constexpr (kPow2<NT>) return (t - lo) & (NT - 1);
+    const int32_t i = t - lo % NT;
+    return i < 0 ? i + NT : i;
+}
+
+// the thread of path q
+template <int NT>
+__device__ __forceinline__ int32_t thread64(int32_t q) {
+    if constexpr (kPow2<NT>) return q & (NT - 1);
+    return q % NT;
 }
 
 // ------------------------------------------------------------------------------------------------
 // forward sweep of one segment
 // ------------------------------------------------------------------------------------------------
-// On anti-diagonal d a thread computes, side by side, the four log_adds whose operands are at hand:
-// gap-X of d (its neighbours on d-1), gap-Y of d (own column on d-1), all but the last term of the
-// match state of d+1 (neighbours on d-1), and the last term of d's.  So a step takes one log_add's
-// latency, a barrier and a shared-memory round trip, where the states one after another took four.
-// The sweep's warps issue in order, so two more warps take what is not the recursion: the copies, and
-// the stores of the values.
 template <int NT, bool kMulti>
 struct Forward64Shared {
     LogAdd64 la;
     int4 info[kInfoRing];
-    double2 e[kRing64][NT];            // by slot of the anti-diagonal
+    double2 e[kRing64][NT];            // by thread
     double gx[kRing64][NT];
     int4 pred[kMulti ? kRing64 : 1][kMulti ? NT : 1];   // pred, pred_n, pred_step
     double v[2][3][NT];                // states by thread, by parity of the anti-diagonal
 };
 
-// what a thread needs of an anti-diagonal beside the values, in registers before its step
-template <bool kMulti>
-struct ForwardOwn64 {
-    bool in;
-    double2 e;
-    double gx;
-    int4 pr;
-};
-
+// predecessors of a thread's path on the k-th anti-diagonal
 template <int NT, bool kMulti>
-__device__ __forceinline__ ForwardOwn64<kMulti> forward_own64(const Forward64Shared<NT, kMulti> &sh, int32_t k) {
-    const int4 in = sh.info[k & (kInfoRing - 1)];
-    const int b = k & (kRing64 - 1);
-    const int32_t i = (threadIdx.x - in.x) & (NT - 1);
-    ForwardOwn64<kMulti> o;
-    o.in = i < in.y;
-    o.e = sh.e[b][i];
-    o.gx = sh.gx[b][i];
-    if constexpr (kMulti) o.pr = o.in ? sh.pred[b][i] : make_int4(0, 0, 0, 0);
-    else o.pr = make_int4((threadIdx.x - 1) & (NT - 1), 1, 0, 0);
-    return o;
+__device__ __forceinline__ int4 preds64(const Forward64Shared<NT, kMulti> &sh, int32_t k, int tid) {
+    if constexpr (kMulti) return sh.pred[k & (kRing64 - 1)][tid];
+    return make_int4(tid ? tid - 1 : NT - 1, 1, 0, 0);
 }
 
+// gap-X (lower neighbours, d-1) and gap-Y (own path, d-1) of d
 template <int NT, bool kMulti, bool kSX>
-__device__ __forceinline__ void forward_sweep64(const double *mt, const Region64 &R, Forward64Shared<NT, kMulti> &sh) {
-    const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY], tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX],
-                 tOY = mt[T_OY], tEY = mt[T_EY];
+__device__ __forceinline__ void forward_gaps64(const double *mt, const Region64 &R, Forward64Shared<NT, kMulti> &sh) {
+    const double tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX], tOY = mt[T_OY], tEY = mt[T_EY];
     const int tid = threadIdx.x;
     const int32_t s = R.s0 <= 1 ? 1 : R.s0, steps = R.win[R.w1 - 1].D - s + 1;
-    // the values of s-2 (parity 0, as s) and s-1
-    double M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf;
-    for (int st = 0; st < 3; ++st) sh.v[0][st][tid] = kNegInf;
-    if (R.s0 <= 1) {
-        if (tid == 0) {   // startStateProb / raggedStartStateProb (stateMachine.c:1022-1032) on anti-diagonal 0
-            M1 = R.ragged_left ? kNegInf : 0.0;
-            X1 = Y1 = R.ragged_left ? 0.0 : kNegInf;
-        }
-    } else {   // a later segment: every slot of s-2 and s-1 starts at 0
-        const int4 i2 = R.info[s - 2], i1 = R.info[s - 1];
-        const double z = ((tid - i2.x) & (NT - 1)) < i2.y ? 0.0 : kNegInf;
-        for (int st = 0; st < 3; ++st) sh.v[0][st][tid] = z;
-        M1 = X1 = Y1 = ((tid - i1.x) & (NT - 1)) < i1.y ? 0.0 : kNegInf;
-    }
-    sh.v[1][S_M][tid] = M1;
-    sh.v[1][S_X][tid] = X1;
-    sh.v[1][S_Y][tid] = Y1;
-    bar64(NT + kHelpers64);            // the first rows are ready
-    ForwardOwn64<kMulti> o0 = forward_own64<NT, kMulti>(sh, 0), o1 = forward_own64<NT, kMulti>(sh, 1);
-    // match state: all terms but the last, and that
-    double most = kNegInf, last = kNegInf;
-    for (int32_t a = 0, p = o0.pr.x; a < o0.pr.y; ++a, p += o0.pr.z) {
-        const int w = p & (NT - 1);
-        if (a) most = lad(sh.la, most, last);
-        most = lad(sh.la, most, sh.v[0][S_M][w] + (o0.e.x + tMC));
-        most = lad(sh.la, most, sh.v[0][S_X][w] + (o0.e.x + tMX));
-        last = sh.v[0][S_Y][w] + (o0.e.x + tMY);
-    }
-    bar64(NT + kHelpers64);            // s-2's values are read
+    bar64(kSweepThreads64<NT>);      // s-1's values and the first rows are there
+    double Y1 = sh.v[1][S_Y][tid];
+    double eY = sh.e[0][tid].y, gx = sh.gx[0][tid];
+    int4 pr = preds64(sh, 0, tid);
 #pragma unroll 1
     for (int32_t k = 0; k < steps; ++k) {
-        const double eOX = o0.gx + tOX, eEX = o0.gx + tEX, eSX = o0.gx + tSX;
-        const double eMC = o1.e.x + tMC, eMX = o1.e.x + tMX, eMY = o1.e.x + tMY;
-        double x[4], y[4], r[4];
-        x[1] = M1 + (o0.e.y + tOY);
-        y[1] = Y1 + (o0.e.y + tEY);
-        x[2] = most;
-        y[2] = last;
-        bar64(NT + kHelpers64);        // d-1's values, d+2's operands
+        const double eOX = gx + tOX, eEX = gx + tEX, eSX = gx + tSX, eOY = eY + tOY;
+        double x[2], y[2], r[2];
+        y[1] = Y1 + (eY + tEY);
+        const int p = kMulti ? pr.x & (NT - 1) : pr.x;
+        bar64(kSweepThreads64<NT>);  // d-1's values, d+1's operands
         const double(&v)[3][NT] = sh.v[(k + 1) & 1];
-        const int p0 = o0.pr.x & (NT - 1), p1 = o1.pr.x & (NT - 1);
-        x[0] = v[S_M][p0] + eOX;
-        y[0] = v[S_X][p0] + eEX;
-        x[3] = v[S_M][p1] + eMC;
-        y[3] = v[S_X][p1] + eMX;
+        x[0] = v[S_M][p] + eOX;
+        y[0] = v[S_X][p] + eEX;
+        x[1] = v[S_M][tid] + eOY;
         double lY = 0.0;
-        if (kSX) lY = v[S_Y][p0] + eSX;
-        last = v[S_Y][p1] + eMY;
-        const ForwardOwn64<kMulti> o2 = forward_own64<NT, kMulti>(sh, k + 2);
-        if constexpr (kMulti) {
-            if (o0.pr.y == 0) x[0] = y[0] = lY = kNegInf;
-            if (o1.pr.y == 0) x[3] = y[3] = last = kNegInf;
-        }
-        lad4(sh.la, x, y, r);
+        if (kSX) lY = v[S_Y][p] + eSX;
+        eY = sh.e[(k + 1) & (kRing64 - 1)][tid].y;
+        gx = sh.gx[(k + 1) & (kRing64 - 1)][tid];
+        const int4 pr_next = preds64(sh, k + 1, tid);
+        if constexpr (kMulti)
+            if (pr.y == 0) x[0] = y[0] = lY = kNegInf;
+        lad2(sh.la, x, y, r);
         if (kSX) r[0] = lad(sh.la, r[0], lY);
-        most = r[3];
         if constexpr (kMulti) {
-            for (int32_t a = 1, p = o0.pr.x + o0.pr.z; a < o0.pr.y; ++a, p += o0.pr.z) {
-                const int w = p & (NT - 1);
+            for (int32_t a = 1, q = pr.x + pr.z; a < pr.y; ++a, q += pr.z) {
+                const int w = q & (NT - 1);
                 r[0] = lad(sh.la, r[0], v[S_M][w] + eOX);
                 r[0] = lad(sh.la, r[0], v[S_X][w] + eEX);
                 if (kSX) r[0] = lad(sh.la, r[0], v[S_Y][w] + eSX);
             }
-            for (int32_t a = 1, p = o1.pr.x + o1.pr.z; a < o1.pr.y; ++a, p += o1.pr.z) {
-                const int w = p & (NT - 1);
+        }
+        sh.v[k & 1][S_X][tid] = r[0];
+        sh.v[k & 1][S_Y][tid] = r[1];
+        Y1 = r[1];
+        pr = pr_next;
+    }
+    bar64(kSweepThreads64<NT>);      // the last anti-diagonal's values go out
+}
+
+// the match state (middle neighbours, two anti-diagonals back): of d+1 all terms but the last, of d that
+template <int NT, bool kMulti>
+__device__ __forceinline__ void forward_match64(const double *mt, const Region64 &R, Forward64Shared<NT, kMulti> &sh) {
+    const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY];
+    const int tid = threadIdx.x - NT;
+    const int32_t s = R.s0 <= 1 ? 1 : R.s0, steps = R.win[R.w1 - 1].D - s + 1;
+    // the values of s-1 (parity 1); s-2's are log 0, or 0 where a later segment starts
+    double z = kNegInf, m = kNegInf, g = kNegInf;
+    if (R.s0 <= 1) {
+        if (tid == 0) {   // startStateProb / raggedStartStateProb (stateMachine.c:1022-1032) on anti-diagonal 0
+            m = R.ragged_left ? kNegInf : 0.0;
+            g = R.ragged_left ? 0.0 : kNegInf;
+        }
+    } else {
+        const int4 i2 = R.info[s - 2], i1 = R.info[s - 1];
+        if (slot64<NT>(tid, i2.x) < i2.y) z = 0.0;
+        if (slot64<NT>(tid, i1.x) < i1.y) m = g = 0.0;
+    }
+    sh.v[0][S_M][tid] = z;             // s-2's, read before step 0 writes over them
+    sh.v[1][S_M][tid] = m;
+    sh.v[1][S_X][tid] = g;
+    sh.v[1][S_Y][tid] = g;
+    bar64(kSweepThreads64<NT>);
+    int4 pr = preds64(sh, 0, tid);
+    double e = sh.e[0][tid].x, most = kNegInf, last = kNegInf;
+    for (int32_t a = 0, q = pr.x; a < pr.y; ++a, q += pr.z) {
+        const double b = sh.v[0][S_M][kMulti ? q & (NT - 1) : q];   // every state's value there
+        if (a) most = lad(sh.la, most, last);
+        most = lad(sh.la, most, b + (e + tMC));
+        most = lad(sh.la, most, b + (e + tMX));
+        last = b + (e + tMY);
+    }
+    pr = preds64(sh, 1, tid);
+    e = sh.e[1][tid].x;
+#pragma unroll 1
+    for (int32_t k = 0; k < steps; ++k) {
+        const double eMC = e + tMC, eMX = e + tMX, eMY = e + tMY;
+        double x[2], y[2], r[2];
+        x[0] = most;
+        y[0] = last;
+        const int p = kMulti ? pr.x & (NT - 1) : pr.x;
+        bar64(kSweepThreads64<NT>);  // d-1's values, d+2's operands
+        const double(&v)[3][NT] = sh.v[(k + 1) & 1];
+        x[1] = v[S_M][p] + eMC;
+        y[1] = v[S_X][p] + eMX;
+        last = v[S_Y][p] + eMY;
+        e = sh.e[(k + 2) & (kRing64 - 1)][tid].x;
+        const int4 pr_next = preds64(sh, k + 2, tid);
+        if constexpr (kMulti)
+            if (pr.y == 0) x[1] = y[1] = last = kNegInf;
+        lad2(sh.la, x, y, r);
+        most = r[1];
+        if constexpr (kMulti) {
+            for (int32_t a = 1, q = pr.x + pr.z; a < pr.y; ++a, q += pr.z) {
+                const int w = q & (NT - 1);
                 most = lad(sh.la, most, last);
                 most = lad(sh.la, most, v[S_M][w] + eMC);
                 most = lad(sh.la, most, v[S_X][w] + eMX);
                 last = v[S_Y][w] + eMY;
             }
         }
-        X1 = o0.in ? r[0] : kNegInf;
-        Y1 = o0.in ? r[1] : kNegInf;
-        M1 = o0.in ? r[2] : kNegInf;
-        sh.v[k & 1][S_M][tid] = M1;
-        sh.v[k & 1][S_X][tid] = X1;
-        sh.v[k & 1][S_Y][tid] = Y1;
-        o0 = o1;
-        o1 = o2;
+        sh.v[k & 1][S_M][tid] = r[0];
+        pr = pr_next;
     }
-    bar64(NT + kHelpers64);            // the last anti-diagonal's values go out
+    bar64(kSweepThreads64<NT>);
 }
 
+// part: which of the warps of the copies
 template <int NT, bool kMulti>
-__device__ __forceinline__ void forward_copies64(const Region64 &R, Forward64Shared<NT, kMulti> &sh) {
+__device__ __forceinline__ void forward_copies64(const Region64 &R, Forward64Shared<NT, kMulti> &sh, InfoStream<1> &info,
+                                                 int part) {
     const int lane = threadIdx.x & 31;
     const int32_t s = R.s0 <= 1 ? 1 : R.s0, steps = R.win[R.w1 - 1].D - s + 1;
-    InfoStream<1> info;
-    info.open(sh.info, R.info, R.n, s);
     auto issue = [&](int32_t k, const int4 &in) {
         const int b = k & (kRing64 - 1);
         const double *e = R.E + 2 * ((int64_t) in.z + in.x);
         const Path64 *path = R.path + in.x;
 #pragma unroll
-        for (int w = 0; w < NT / 32; ++w) {
-            const int i = lane + 32 * w;
+        for (int w = 0; w < NT / 32; w += kHelperWarps64<NT>) {
+            const int t = lane + 32 * (w + part), i = slot64<NT>(t, in.x);
             if (i < in.y) {
-                copy64_16(&sh.e[b][i], e + 2 * i);
-                copy64_8(&sh.gx[b][i], &path[i].gapx);
+                copy64_16(&sh.e[b][t], e + 2 * i);
+                copy64_8(&sh.gx[b][t], &path[i].gapx);
                 if constexpr (kMulti) {
-                    copy64_8(&sh.pred[b][i].x, &path[i].pred);
-                    copy64_8(&sh.pred[b][i].z, &path[i].pred_step);
+                    copy64_8(&sh.pred[b][t].x, &path[i].pred);
+                    copy64_8(&sh.pred[b][t].z, &path[i].pred_step);
                 }
+            } else {
+                sh.e[b][t] = make_double2(kNegInf, kNegInf);
+                sh.gx[b][t] = kNegInf;
+                if constexpr (kMulti) sh.pred[b][t].y = 0;
             }
         }
         copy64_commit();
@@ -368,23 +412,24 @@ __device__ __forceinline__ void forward_copies64(const Region64 &R, Forward64Sha
     for (int k = 0; k < kAhead64; ++k) issue(k, info.at(k));
     copy64_wait<kAhead64 - 3>();
     int4 in = info.at(kAhead64);
-    bar64(NT + kHelpers64);
-    bar64(NT + kHelpers64);
+    bar64(kSweepThreads64<NT>);
     for (int32_t k = 0; k < steps; ++k) {
-        bar64(NT + kHelpers64);
+        bar64(kSweepThreads64<NT>);
         issue(k + kAhead64, in);
-        info.advance(k);
+        if (part == 0) info.advance(k);
         in = info.at(k + kAhead64 + 1);
         copy64_wait<kAhead64 - 3>();   // every copy of d+3 and before has landed
     }
-    bar64(NT + kHelpers64);
+    bar64(kSweepThreads64<NT>);
     copy64_wait<0>();
 }
 
-// at step k d-1's values go to the store and, where a stitch is, to its side
+// at step k d-1's values go to the store and, where a stitch is, to its side; part: which of the warps
 template <int NT, bool kMulti>
-__device__ __forceinline__ void forward_results64(const Region64 &R, const SetOut &O, Forward64Shared<NT, kMulti> &sh) {
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void forward_results64(const Region64 &R, const SetOut &O, Forward64Shared<NT, kMulti> &sh,
+                                                  int part) {
+    constexpr int NW = NT / 32 / kHelperWarps64<NT>;
+    const int lane = 32 * part + (threadIdx.x & 31), stride = 32 * kHelperWarps64<NT>;
     const int32_t s = R.s0 <= 1 ? 1 : R.s0, steps = R.win[R.w1 - 1].D - s + 1;
     if (R.s0 <= 1 && lane == 0) {
         double *c = R.F + 3 * (int64_t) R.info[0].z;
@@ -392,48 +437,58 @@ __device__ __forceinline__ void forward_results64(const Region64 &R, const SetOu
         c[S_X] = c[S_Y] = R.ragged_left ? 0.0 : kNegInf;
     }
     const int32_t b_in = R.st_in >= 0 ? O.stitch[R.st_in].b : -10, b_out = R.st_out >= 0 ? O.stitch[R.st_out].b : -10;
-    bar64(NT + kHelpers64);
-    bar64(NT + kHelpers64);
-    bar64(NT + kHelpers64);            // step 0
+    bar64(kSweepThreads64<NT>);
+    bar64(kSweepThreads64<NT>);        // step 0
     int4 in = sh.info[0];
     for (int32_t k = 1; k <= steps; ++k) {
         const int32_t r = s + k - 1;   // the anti-diagonal that goes out
         double *c = R.F + 3 * ((int64_t) in.z + in.x + lane);
-        int at[NT / 32];
-#pragma unroll
-        for (int w = 0; w < NT / 32; ++w) at[w] = (in.x + lane + 32 * w) & (NT - 1);
-        bar64(NT + kHelpers64);
+        bar64(kSweepThreads64<NT>);
         const double(&v)[3][NT] = sh.v[(k - 1) & 1];
+        const int4 in_next = sh.info[k & (kInfoRing - 1)];
 #pragma unroll
-        for (int w = 0; w < NT / 32; ++w) {
-            if (lane + 32 * w < in.y) {
-                c[96 * w + S_M] = v[S_M][at[w]];
-                c[96 * w + S_X] = v[S_X][at[w]];
-                c[96 * w + S_Y] = v[S_Y][at[w]];
+        for (int w0 = 0; w0 < NW; w0 += 4) {   // as many values in flight as registers allow
+            double o[3][4];
+#pragma unroll
+            for (int w = w0; w < w0 + 4 && w < NW; ++w) {
+                const int at = thread64<NT>(in.x + lane + stride * w);
+#pragma unroll
+                for (int st = 0; st < 3; ++st) o[st][w - w0] = v[st][at];
+            }
+#pragma unroll
+            for (int w = w0; w < w0 + 4 && w < NW; ++w) {
+                if (lane + stride * w < in.y) {
+#pragma unroll
+                    for (int st = 0; st < 3; ++st) c[3 * stride * w + st] = o[st][w - w0];
+                }
             }
         }
         if (r == b_in - 1 || r == b_in || r == b_out - 1 || r == b_out) {
             const bool side = r == b_in - 1 || r == b_in;
             const Stitch64 S = O.stitch[side ? R.st_in : R.st_out];
-            double *o = S.vals + 3 * (int64_t) (side ? r - (b_in - 1) : 2 + r - (b_out - 1)) * S.stride;
-            for (int i = lane; i < in.y; i += 32)
-                for (int st = 0; st < 3; ++st) o[3 * i + st] = v[st][(in.x + i) & (NT - 1)];
+            double *to = S.vals + 3 * (int64_t) (side ? r - (b_in - 1) : 2 + r - (b_out - 1)) * S.stride;
+            for (int i = lane; i < in.y; i += stride)
+                for (int st = 0; st < 3; ++st) to[3 * i + st] = v[st][thread64<NT>(in.x + i)];
         }
-        in = sh.info[k & (kInfoRing - 1)];
+        in = in_next;
     }
 }
 
 template <int NT, bool kMulti, bool kSX>
-__global__ void __launch_bounds__(NT + kHelpers64) forward64(const Model64 *models, const Region64 *tasks, SetOut O) {
+__global__ void __launch_bounds__(kSweepThreads64<NT>) forward64(const Model64 *models, const Region64 *tasks, SetOut O) {
     extern __shared__ double2 smem64[];
     using Sh = Forward64Shared<NT, kMulti>;
     Sh &sh = *reinterpret_cast<Sh *>(smem64);
     const Region64 R = tasks[blockIdx.x];
+    const int helper = ((int) threadIdx.x - 2 * NT) >> 5;
+    InfoStream<1> info{sh.info, nullptr, 0, 0, make_int4(0, 0, 0, 0)};
     if (threadIdx.x < 16) log_add_table64(sh.la, threadIdx.x);
+    if (helper == 0) info.open(sh.info, R.info, R.n, R.s0 <= 1 ? 1 : R.s0);
     __syncthreads();
-    if (threadIdx.x < NT) forward_sweep64<NT, kMulti, kSX>(models[R.model].t, R, sh);
-    else if (threadIdx.x < NT + 32) forward_copies64<NT, kMulti>(R, sh);
-    else forward_results64<NT, kMulti>(R, O, sh);
+    if (threadIdx.x < NT) forward_gaps64<NT, kMulti, kSX>(models[R.model].t, R, sh);
+    else if (threadIdx.x < 2 * NT) forward_match64<NT, kMulti>(models[R.model].t, R, sh);
+    else if (helper < kHelperWarps64<NT>) forward_copies64<NT, kMulti>(R, sh, info, helper);
+    else forward_results64<NT, kMulti>(R, O, sh, helper - kHelperWarps64<NT>);
     __syncthreads();
     if (R.st_in >= 0) stitch_arrive64(R, O, R.st_in);
     if (R.st_out >= 0) stitch_arrive64(R, O, R.st_out);
@@ -443,341 +498,358 @@ __global__ void __launch_bounds__(NT + kHelpers64) forward64(const Model64 *mode
 // backward sweep of one traceback window
 // ------------------------------------------------------------------------------------------------
 // A path's values go to its predecessors already summed with its emission and the transitions (the
-// pushed sums of backward_cell), so a predecessor only folds.  As forward, the log_adds of a step are
-// side by side: gap-X and gap-Y of d, the match state of d but for its last term, and the last term of
-// d+1's (which nothing needs before d-1).  What d+1's match value goes into (F.B, the terms of a total
-// probability's two folds: F.B on that anti-diagonal, and the matches from the one before it over it
-// into the one after, dotted with B there) is therefore written a step late or later.
+// pushed sums of backward_cell), so a predecessor only folds.  The last term of d+1's match state is
+// folded at step d, which nothing needs before d-1.  The values go out for the launches after this one:
+// the match values of the window's own anti-diagonals, all of an anti-diagonal with a total probability,
+// and the match values of the one above it.
 template <int NT, bool kMulti>
 struct Backward64Shared {
     LogAdd64 la;
     int4 info[kInfoRing];
-    double2 e[kRing64][NT];            // by slot of the anti-diagonal
-    double gx[NT > 256 ? 1 : kRing64][NT > 256 ? 1 : NT];   // (512 threads read it where it is: no room)
-    int4 nb[kMulti ? kRing64 : 1][kMulti ? NT : 1];        // succ, succ_n; pred, pred_n
-    int32_t step[kMulti ? kRing64 : 1][kMulti ? NT : 1];   // pred_step
-    double f[kRing64][NT];             // forward match value
-    double fx[2][NT];                  // forward gap values of a total's anti-diagonal
-    double fm[3][NT];                  // forward values of the anti-diagonal before it
-    double a[2][3][NT];                // sums for the match predecessors, by thread, by parity
-    double b[2][3][NT];                // sums for the gap-X predecessors, by thread, by parity
-    double vm[2][NT];                  // match values by thread, by parity of the anti-diagonal
-    double vx[4][NT], vy[4][NT];       // gap values (expectations)
+    double2 e[kRing64][NT];            // by thread
+    double gx[NT > 256 ? 1 : kRing64][NT > 256 ? 1 : NT];   // (480 threads read it where it is: no room)
+    int2 succ[kMulti ? kRing64 : 1][kMulti ? NT : 1];      // succ, succ_n
+    double a[2][3][NT];                // sums for the match predecessors, by parity
+    double b[2][3][NT];                // sums for the gap-X predecessors, by parity
+    double u[2][NT];                   // the gap-Y sum for the own path's match state, by parity
+    double vm[2][NT];                  // match values, by parity of the anti-diagonal
+    double vx[4][NT], vy[4][NT];       // gap values
 };
-
-static_assert(sizeof(Backward64Shared<512, false>) <= 227 * 1024 && sizeof(Backward64Shared<256, true>) <= 227 * 1024 &&
-                  sizeof(Forward64Shared<512, false>) <= 227 * 1024,
+static_assert(sizeof(Backward64Shared<480, false>) <= 227 * 1024 && sizeof(Backward64Shared<256, true>) <= 227 * 1024 &&
+                  sizeof(Forward64Shared<480, false>) <= 227 * 1024,
               "a CTA's shared memory");
 
-// the path a thread holds on an anti-diagonal
-struct Held64 {
-    int32_t i, n;                      // its slot, and the anti-diagonal's slots
-    int4 pred;                         // its predecessors: first, count, step
-    double e;                          // its match emission
-    double M;                          // its match value
-};
+// successors of a thread's path on the k-th anti-diagonal
+template <int NT, bool kMulti>
+__device__ __forceinline__ int2 succs64(const Backward64Shared<NT, kMulti> &sh, int32_t k, int tid) {
+    if constexpr (kMulti) return sh.succ[k & (kRing64 - 1)][tid];
+    return make_int2(tid < NT - 1 ? tid + 1 : 0, 1);
+}
 
+// gap-X and gap-Y of d
 template <int NT, bool kMulti, bool kSX>
-__device__ __forceinline__ void backward_sweep64(const double *mt, const Region64 &R, const Window64 &wt, const Window &W,
-                                                 Backward64Shared<NT, kMulti> &sh, double *terms, int64_t term_stride,
-                                                 int expect) {
-    const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY], tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX],
-                 tOY = mt[T_OY], tEY = mt[T_EY];
+__device__ __forceinline__ void backward_gaps64(const double *mt, const Region64 &R, const Window &W,
+                                                Backward64Shared<NT, kMulti> &sh) {
+    const double tOX = mt[T_OX], tEX = mt[T_EX], tSX = mt[T_SX], tOY = mt[T_OY], tEY = mt[T_EY];
     const int tid = threadIdx.x;
     const int32_t steps = W.D - W.T;
     // endStateProb / raggedEndStateProb (stateMachine.c:1034-1061) on the traceback anti-diagonal
     const bool ragged_end = W.at_end && R.ragged_right;
-    const double e0 = ragged_end ? (tOX + tOY) / 2.0 : tMC, e1 = ragged_end ? tEX : tMX, e2 = ragged_end ? tEY : tMY;
-    for (int k = 0; k < 2; ++k)
-        for (int st = 0; st < 3; ++st) sh.a[k][st][tid] = sh.b[k][st][tid] = kNegInf;
-    struct Own {
-        int32_t i, n;
-        double2 e;
-        double gx;
-        int4 nb;
-        int32_t step;
-    };
-    auto own = [&](int32_t k) -> Own {
-        const int4 in = sh.info[k & (kInfoRing - 1)];
-        const int b = k & (kRing64 - 1);
-        Own o;
-        o.i = (tid - in.x) & (NT - 1);
-        o.n = k < steps ? in.y : 0;
-        o.e = sh.e[b][o.i];
-        if constexpr (NT > 256) o.gx = o.i < o.n ? __ldg(&R.path[in.x + o.i].gapx) : 0.0;
-        else o.gx = sh.gx[b][o.i];
-        o.step = 0;
-        if constexpr (kMulti) {
-            o.nb = o.i < o.n ? sh.nb[b][o.i] : make_int4(0, 0, 0, 0);
-            o.step = sh.step[b][o.i];
+    const double e1 = ragged_end ? tEX : mt[T_MFGX], e2 = ragged_end ? tEY : mt[T_MFGY];
+    for (int st = 0; st < 3; ++st) sh.b[1][st][tid] = kNegInf;
+    sh.u[1][tid] = kNegInf;
+    auto skip = [&](int32_t k) -> double {
+        if constexpr (NT > 256) {
+            const int4 in = sh.info[k & (kInfoRing - 1)];
+            const int32_t i = slot64<NT>(tid, in.x);
+            return k < steps && i < in.y ? __ldg(&R.path[in.x + i].gapx) : kNegInf;
         } else {
-            o.nb = make_int4(in.x + o.i + 1, 1, in.x + o.i - 1, 1);
+            return sh.gx[k & (kRing64 - 1)][tid];
         }
-        return o;
     };
-    bar64(NT + kHelpers64);                          // the first rows are ready
-    Own o0 = own(0);
-    double u0 = kNegInf, u1 = kNegInf;               // own path's gap-Y sums of d+1
-    double most = kNegInf, last = kNegInf;           // its match state on d+1: all terms but one, and that
-    double X1 = kNegInf, Y1 = kNegInf;               // its gap values on d+1
-    Held64 h1{0, 0, make_int4(0, 0, 0, 0), 0.0, kNegInf}, h2 = h1;   // the paths held on d+1, d+2
-    int64_t total_at = wt.first_total;
-    int32_t until = W.D - W.from;                    // steps until the next total's anti-diagonal
+    bar64(kSweepThreads64<NT>);                    // the first rows are ready
+    double u1 = kNegInf;                             // own path's gap-Y sum of d+1 for gap-Y
+    double eY = sh.e[0][tid].y, gx = skip(0);
+    int2 nb = succs64(sh, 0, tid);
 #pragma unroll 1
-    for (int32_t k = 0; k <= steps; ++k) {           // k == steps: only what is a step late
-        const bool inb = o0.i < o0.n;
-        const int4 nb = o0.nb;
-        double x[4], y[4], r[4];
-        bar64(NT + kHelpers64);                      // d+1's sums for gap-X predecessors, d+2's for match predecessors
+    for (int32_t k = 0; k < steps; ++k) {
+        const double gOX = gx + tOX, gEX = gx + tEX, gSX = gx + tSX, eOY = eY + tOY, eEY = eY + tEY;
+        double x[2], y[2], r[2];
+        const int p = kMulti ? nb.x & (NT - 1) : nb.x;
+        y[1] = u1;
+        bar64(kSweepThreads64<NT>);                // d+1's sums for gap-X predecessors, d+2's for match predecessors
         const double(&a)[3][NT] = sh.a[k & 1];
         const double(&c)[3][NT] = sh.b[(k + 1) & 1];
-        const int p0 = nb.x & (NT - 1);
-        x[0] = a[1][p0];
-        y[0] = c[1][p0];
-        x[1] = a[2][p0];
-        y[1] = u1;
-        x[2] = a[0][p0];
-        y[2] = u0;
-        x[3] = most;
-        y[3] = last;
-        double l = c[0][p0], lY = 0.0;
-        if (kSX) lY = c[2][p0];
-        const Own o1 = own(k + 1);
+        x[0] = a[1][p];
+        y[0] = c[1][p];
+        x[1] = a[2][p];
+        double lY = 0.0;
+        if (kSX) lY = c[2][p];
+        eY = sh.e[(k + 1) & (kRing64 - 1)][tid].y;
+        gx = skip(k + 1);
+        const int2 nb_next = succs64(sh, k + 1, tid);
         if constexpr (kMulti) {
-            if (nb.y == 0) x[0] = y[0] = x[1] = x[2] = l = lY = kNegInf;
+            if (nb.y == 0) x[0] = y[0] = x[1] = lY = kNegInf;
             for (int32_t j = 1; j < nb.y; ++j) {
-                const int w = (nb.x + j) & (NT - 1);
-                x[0] = lad(sh.la, x[0], a[1][w]);
-                x[1] = lad(sh.la, x[1], a[2][w]);
-                x[2] = lad(sh.la, x[2], a[0][w]);
+                x[0] = lad(sh.la, x[0], a[1][(nb.x + j) & (NT - 1)]);
+                x[1] = lad(sh.la, x[1], a[2][(nb.x + j) & (NT - 1)]);
             }
         }
-        lad4(sh.la, x, y, r);
+        lad2(sh.la, x, y, r);
         if (kSX) r[1] = lad(sh.la, r[1], lY);
         if constexpr (kMulti) {
             for (int32_t j = 1; j < nb.y; ++j) {
-                const int w = (nb.x + j) & (NT - 1);
-                r[2] = lad(sh.la, r[2], l);
-                l = c[0][w];
-                r[0] = lad(sh.la, r[0], c[1][w]);
-                if (kSX) r[1] = lad(sh.la, r[1], c[2][w]);
+                r[0] = lad(sh.la, r[0], c[1][(nb.x + j) & (NT - 1)]);
+                if (kSX) r[1] = lad(sh.la, r[1], c[2][(nb.x + j) & (NT - 1)]);
             }
         }
-        const bool in1 = h1.i < h1.n;
-        h1.M = in1 ? r[3] : kNegInf;
         if (k == 0) {
-            r[2] = e0;
-            l = kNegInf;
             r[0] = e1;
             r[1] = e2;
         }
-        most = r[2];
-        last = l;
-        const double vX = inb ? r[0] : kNegInf, vY = inb ? r[1] : kNegInf;
-        // match sums of d+1 (a buffer's parity is its anti-diagonal's plus one), gap sums of d
-        sh.a[(k + 1) & 1][0][tid] = in1 ? h1.M + (h1.e + tMC) : kNegInf;
-        sh.a[(k + 1) & 1][1][tid] = in1 ? h1.M + (h1.e + tMX) : kNegInf;
-        sh.a[(k + 1) & 1][2][tid] = in1 ? h1.M + (h1.e + tMY) : kNegInf;
-        sh.b[k & 1][0][tid] = inb ? vX + (o0.gx + tOX) : kNegInf;
-        sh.b[k & 1][1][tid] = inb ? vX + (o0.gx + tEX) : kNegInf;
-        if (kSX) sh.b[k & 1][2][tid] = inb ? vX + (o0.gx + tSX) : kNegInf;
-        u0 = inb ? vY + (o0.e.y + tOY) : kNegInf;
-        u1 = inb ? vY + (o0.e.y + tEY) : kNegInf;
-        sh.vm[(k + 1) & 1][tid] = h1.M;              // of the anti-diagonal before, for the warp of the results
-        if (expect) {
-            sh.vx[k & 3][tid] = vX;
-            sh.vy[k & 3][tid] = vY;
-        }
-        if (k == until + 1) {
-            // d+1 is a total's: its terms
-            until += 10;
-            double *t0 = terms + total_at * 2 * term_stride;
-            if (in1) {
-                double s = sh.f[(k - 1) & (kRing64 - 1)][h1.i] + h1.M;
-                s = lad(sh.la, s, sh.fx[0][h1.i] + X1);
-                s = lad(sh.la, s, sh.fx[1][h1.i] + Y1);
-                t0[h1.i] = s;
-            }
-            if (k > 1 && h2.i < h2.n) {
-                // the slot of d+2 this thread held: its predecessors' forward values on d
-                const int4 below = sh.info[k & (kInfoRing - 1)];
-                auto fm = [&](int st, int32_t q) {
-                    const int32_t j = q - below.x;
-                    return j >= 0 && j < below.y ? sh.fm[st][j] : kNegInf;
-                };
-                double w = kNegInf;
-                for (int32_t j = 0, p = h2.pred.x; j < h2.pred.y; ++j, p += h2.pred.z) {
-                    w = lad(sh.la, w, fm(S_M, p) + (h2.e + tMC));
-                    w = lad(sh.la, w, fm(S_X, p) + (h2.e + tMX));
-                    w = lad(sh.la, w, fm(S_Y, p) + (h2.e + tMY));
-                }
-                t0[term_stride + h2.i] = w + h2.M;
-            }
-            ++total_at;
-        }
-        X1 = vX;
-        Y1 = vY;
-        h2 = h1;
-        h1 = Held64{o0.i, o0.n, make_int4(nb.z, nb.w, o0.step, 0), o0.e.x, kNegInf};
-        o0 = o1;
+        sh.b[k & 1][0][tid] = r[0] + gOX;
+        sh.b[k & 1][1][tid] = r[0] + gEX;
+        if (kSX) sh.b[k & 1][2][tid] = r[0] + gSX;
+        sh.u[k & 1][tid] = r[1] + eOY;
+        u1 = r[1] + eEY;
+        sh.vx[k & 3][tid] = r[0];
+        sh.vy[k & 3][tid] = r[1];
+        nb = nb_next;
     }
-    bar64(NT + kHelpers64);                          // the last match values go out
+    bar64(kSweepThreads64<NT>);
+    bar64(kSweepThreads64<NT>);
+}
+
+// the match state: of d all terms but the last, of d+1 that
+template <int NT, bool kMulti>
+__device__ __forceinline__ void backward_match64(const double *mt, const Region64 &R, const Window &W,
+                                                 Backward64Shared<NT, kMulti> &sh) {
+    const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY];
+    const int tid = threadIdx.x - NT;
+    const int32_t steps = W.D - W.T;
+    const bool ragged_end = W.at_end && R.ragged_right;
+    const double e0 = ragged_end ? (mt[T_OX] + mt[T_OY]) / 2.0 : tMC;
+    for (int k = 0; k < 2; ++k)
+        for (int st = 0; st < 3; ++st) sh.a[k][st][tid] = kNegInf;
+    bar64(kSweepThreads64<NT>);
+    double most = kNegInf, last = kNegInf;           // the match state on d+1: all terms but one, and that
+    double e1 = kNegInf, e = sh.e[0][tid].x;         // emissions of d+1 and d
+    int2 nb = succs64(sh, 0, tid);
+#pragma unroll 1
+    for (int32_t k = 0; k <= steps; ++k) {           // k == steps: only the last term of the last one
+        const double eMC = e1 + tMC, eMX = e1 + tMX, eMY = e1 + tMY;
+        double x[2], y[2], r[2];
+        x[0] = most;
+        y[0] = last;
+        const int p = kMulti ? nb.x & (NT - 1) : nb.x;
+        bar64(kSweepThreads64<NT>);
+        const double(&a)[3][NT] = sh.a[k & 1];
+        const double(&c)[3][NT] = sh.b[(k + 1) & 1];
+        x[1] = a[0][p];
+        y[1] = sh.u[(k + 1) & 1][tid];
+        double l = c[0][p];
+        const double e_next = sh.e[(k + 1) & (kRing64 - 1)][tid].x;
+        const int2 nb_next = succs64(sh, k + 1, tid);
+        if constexpr (kMulti) {
+            if (nb.y == 0) x[1] = l = kNegInf;
+            for (int32_t j = 1; j < nb.y; ++j) x[1] = lad(sh.la, x[1], a[0][(nb.x + j) & (NT - 1)]);
+        }
+        lad2(sh.la, x, y, r);
+        if constexpr (kMulti) {
+            for (int32_t j = 1; j < nb.y; ++j) {
+                r[1] = lad(sh.la, r[1], l);
+                l = c[0][(nb.x + j) & (NT - 1)];
+            }
+        }
+        most = k == 0 ? e0 : r[1];
+        last = k == 0 ? kNegInf : l;
+        // a buffer's parity is its anti-diagonal's plus one
+        sh.a[(k + 1) & 1][0][tid] = r[0] + eMC;
+        sh.a[(k + 1) & 1][1][tid] = r[0] + eMX;
+        sh.a[(k + 1) & 1][2][tid] = r[0] + eMY;
+        sh.vm[(k + 1) & 1][tid] = r[0];
+        e1 = e;
+        e = e_next;
+        nb = nb_next;
+    }
+    bar64(kSweepThreads64<NT>);                      // the last match values go out
 }
 
 template <int NT, bool kMulti>
-__device__ __forceinline__ void backward_copies64(const Region64 &R, const Window &W, Backward64Shared<NT, kMulti> &sh) {
+__device__ __forceinline__ void backward_copies64(const Region64 &R, const Window &W, Backward64Shared<NT, kMulti> &sh,
+                                                  InfoStream<-1> &info, int part) {
     const int lane = threadIdx.x & 31;
     const int32_t steps = W.D - W.T;
-    InfoStream<-1> info;
-    info.open(sh.info, R.info, R.n, W.D);
     auto issue = [&](int32_t k, const int4 &in) {
-        if (k < steps) {
-            const int32_t d = W.D - k;
-            const bool post = d <= W.from, total = post && (W.from - d) % 10 == 0;
-            const int b = k & (kRing64 - 1);
-            const double *e = R.E + 2 * ((int64_t) in.z + in.x), *f = R.F + 3 * ((int64_t) in.z + in.x);
-            const Path64 *path = R.path + in.x;
+        const int32_t n = k < steps ? in.y : 0;
+        const int b = k & (kRing64 - 1);
+        const double *e = R.E + 2 * ((int64_t) in.z + in.x);
+        const Path64 *path = R.path + in.x;
 #pragma unroll
-            for (int w = 0; w < NT / 32; ++w) {
-                const int i = lane + 32 * w;
-                if (i < in.y) {
-                    copy64_16(&sh.e[b][i], e + 2 * i);
-                    if constexpr (NT <= 256) copy64_8(&sh.gx[b][i], &path[i].gapx);
-                    if constexpr (kMulti) {
-                        copy64_8(&sh.nb[b][i].x, &path[i].succ);
-                        copy64_8(&sh.nb[b][i].z, &path[i].pred);
-                        copy64_4(&sh.step[b][i], &path[i].pred_step);
-                    }
-                    if (post) copy64_8(&sh.f[b][i], f + 3 * i);
-                    if (total) {
-                        copy64_8(&sh.fx[0][i], f + 3 * i + S_X);
-                        copy64_8(&sh.fx[1][i], f + 3 * i + S_Y);
-                    }
-                }
-            }
-            if (total) {
-                const int4 bl = info.at(k + 1);
-                const double *g = R.F + 3 * ((int64_t) bl.z + bl.x);
-                for (int i = lane; i < bl.y; i += 32)
-                    for (int st = 0; st < 3; ++st) copy64_8(&sh.fm[st][i], g + 3 * i + st);
+        for (int w = 0; w < NT / 32; w += kHelperWarps64<NT>) {
+            const int t = lane + 32 * (w + part), i = slot64<NT>(t, in.x);
+            if (i < n) {
+                copy64_16(&sh.e[b][t], e + 2 * i);
+                if constexpr (NT <= 256) copy64_8(&sh.gx[b][t], &path[i].gapx);
+                if constexpr (kMulti) copy64_8(&sh.succ[b][t], &path[i].succ);
+            } else {
+                sh.e[b][t] = make_double2(kNegInf, kNegInf);
+                if constexpr (NT <= 256) sh.gx[b][t] = kNegInf;
+                if constexpr (kMulti) sh.succ[b][t] = make_int2(0, 0);
             }
         }
         copy64_commit();
     };
 #pragma unroll
-    for (int k = 0; k < kBehind64; ++k) issue(k, info.at(k));
-    copy64_wait<kBehind64 - 2>();
-    int4 in = info.at(kBehind64);
-    bar64(NT + kHelpers64);
+    for (int k = 0; k < kAhead64; ++k) issue(k, info.at(k));
+    copy64_wait<kAhead64 - 2>();
+    int4 in = info.at(kAhead64);
+    bar64(kSweepThreads64<NT>);
     for (int32_t k = 0; k <= steps; ++k) {
-        bar64(NT + kHelpers64);
-        issue(k + kBehind64, in);
-        info.advance(k);
-        in = info.at(k + kBehind64 + 1);
-        copy64_wait<kBehind64 - 2>();                // every copy of d-2 and above has landed
+        bar64(kSweepThreads64<NT>);
+        issue(k + kAhead64, in);
+        if (part == 0) info.advance(k);
+        in = info.at(k + kAhead64 + 1);
+        copy64_wait<kAhead64 - 2>();                 // every copy of d-2 and above has landed
     }
-    bar64(NT + kHelpers64);
+    bar64(kSweepThreads64<NT>);
     copy64_wait<0>();
 }
 
-// at step k d+2's F.B of the match state, and (expectations) its values, go to their stores
+// at step k d+2's values go to their stores
 template <int NT, bool kMulti>
-__device__ __forceinline__ void backward_results64(const Region64 &R, const Window &W, Backward64Shared<NT, kMulti> &sh,
-                                                   int expect) {
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void backward_results64(const Region64 &R, const Window64 &wt, const Window &W,
+                                                   Backward64Shared<NT, kMulti> &sh, double *terms, int64_t term_stride,
+                                                   int expect, int part) {
+    constexpr int NW = NT / 32 / kHelperWarps64<NT>;
+    const int lane = 32 * part + (threadIdx.x & 31), stride = 32 * kHelperWarps64<NT>;
     const int32_t steps = W.D - W.T;
-    bar64(NT + kHelpers64);
-    bar64(NT + kHelpers64);
-    bar64(NT + kHelpers64);                          // steps 0 and 1 (a match value is there two steps on)
+    int32_t until = W.D - W.from;                    // the k of the next total's anti-diagonal
+    double *t = terms + (int64_t) wt.first_total * kTotalRows * term_stride + lane;
+    bar64(kSweepThreads64<NT>);
+    bar64(kSweepThreads64<NT>);
+    bar64(kSweepThreads64<NT>);                      // steps 0 and 1 (a match value is there two steps on)
     int4 in = sh.info[0];
     for (int32_t k = 0; k < steps; ++k) {            // the anti-diagonal that goes out
-        bar64(NT + kHelpers64);
-        if (W.D - k <= W.from) {
-            const int64_t z = (int64_t) in.z + in.x + lane;
+        const int64_t z = (int64_t) in.z + in.x + lane;
+        const bool post = W.D - k <= W.from, total = k == until, above = k == until - 1 && until < steps;
+        bar64(kSweepThreads64<NT>);
+        const int4 in_next = sh.info[(k + 1) & (kInfoRing - 1)];
+        if (post || above) {
 #pragma unroll
-            for (int w = 0; w < NT / 32; ++w) {
-                const int i = lane + 32 * w, at = (in.x + i) & (NT - 1);
-                if (i < in.y) {
-                    const double m = sh.vm[k & 1][at];
-                    R.S[z + 32 * w] = sh.f[k & (kRing64 - 1)][i] + m;
-                    if (expect) {
-                        double *b = R.B + 3 * (z + 32 * w);
-                        b[S_M] = m;
-                        b[S_X] = sh.vx[k & 3][at];
-                        b[S_Y] = sh.vy[k & 3][at];
-                    }
+            for (int w = 0; w < NW; ++w) {
+                if (lane + stride * w >= in.y) continue;
+                const int at = thread64<NT>(in.x + lane + stride * w);
+                const double m = sh.vm[k & 1][at];
+                if (post) R.S[z + stride * w] = m;
+                if (expect && post) {
+                    double *b = R.B + 3 * (z + stride * w);
+                    b[S_M] = m;
+                    b[S_X] = sh.vx[k & 3][at];
+                    b[S_Y] = sh.vy[k & 3][at];
                 }
+                if (total) {
+                    t[stride * w] = m;
+                    t[term_stride + stride * w] = sh.vx[k & 3][at];
+                    t[2 * term_stride + stride * w] = sh.vy[k & 3][at];
+                }
+                if (above) t[3 * term_stride + stride * w] = m;
             }
         }
-        in = sh.info[(k + 1) & (kInfoRing - 1)];
+        if (total) {
+            until += 10;
+            t += kTotalRows * term_stride;
+        }
+        in = in_next;
     }
 }
 
 template <int NT, bool kMulti, bool kSX>
-__global__ void __launch_bounds__(NT + kHelpers64) backward64(const Model64 *models, const Region64 *tasks,
-                                                              const Window64 *windows, double *terms, int64_t term_stride,
-                                                              int expect) {
+__global__ void __launch_bounds__(kSweepThreads64<NT>) backward64(const Model64 *models, const Region64 *tasks,
+                                                                 const Window64 *windows, double *terms,
+                                                                 int64_t term_stride, int expect) {
     extern __shared__ double2 smem64[];
     using Sh = Backward64Shared<NT, kMulti>;
     Sh &sh = *reinterpret_cast<Sh *>(smem64);
     const Window64 wt = windows[blockIdx.x];
     const Region64 R = tasks[wt.task];
     const Window W = R.win[wt.win];
+    const int helper = ((int) threadIdx.x - 2 * NT) >> 5;
+    InfoStream<-1> info{sh.info, nullptr, 0, 0, make_int4(0, 0, 0, 0)};
     if (threadIdx.x < 16) log_add_table64(sh.la, threadIdx.x);
+    if (helper == 0) info.open(sh.info, R.info, R.n, W.D);
     __syncthreads();
-    if (threadIdx.x < NT)
-        backward_sweep64<NT, kMulti, kSX>(models[R.model].t, R, wt, W, sh, terms, term_stride, expect);
-    else if (threadIdx.x < NT + 32) backward_copies64<NT, kMulti>(R, W, sh);
-    else backward_results64<NT, kMulti>(R, W, sh, expect);
+    if (threadIdx.x < NT) backward_gaps64<NT, kMulti, kSX>(models[R.model].t, R, W, sh);
+    else if (threadIdx.x < 2 * NT) backward_match64<NT, kMulti>(models[R.model].t, R, W, sh);
+    else if (helper < kHelperWarps64<NT>) backward_copies64<NT, kMulti>(R, W, sh, info, helper);
+    else backward_results64<NT, kMulti>(R, wt, W, sh, terms, term_stride, expect, helper - kHelperWarps64<NT>);
 }
 
 // ------------------------------------------------------------------------------------------------
-// total probabilities: a thread each
+// total probabilities: a warp each
 // ------------------------------------------------------------------------------------------------
-// diagonalCalculationTotalProbability (pairwiseAligner.c:1182-1200) over the terms: cells in ascending
-// order, a cell's paths folded first (hdCell_totalProbability); the two sums side by side.
-__global__ void __launch_bounds__(64) totals64(const Region64 *regions, const Total64 *totals, int64_t n, const double *terms,
-                                               int64_t term_stride, int multi) {
+// diagonalCalculationTotalProbability (pairwiseAligner.c:1182-1200): F.B on d in ascending cell order, a
+// cell's paths folded first (hdCell_totalProbability), then the matches from d-1 over d into d+1, dotted
+// with B(d+1).  The lanes make both folds' terms, 128 slots at a time, and two of them fold.
+constexpr int kTotalWarps = 2;
+constexpr int kTotalSlots = 128;
+
+__global__ void __launch_bounds__(32 * kTotalWarps) totals64(const Model64 *models, const Region64 *regions,
+                                                             const Region64 *tasks, const int32_t *task_of,
+                                                             const Total64 *totals, int64_t n, const double *terms,
+                                                             int64_t term_stride, int multi) {
     __shared__ LogAdd64 la;
+    __shared__ double term[kTotalWarps][2][kTotalSlots];
+    __shared__ int32_t cols[kTotalWarps][2][kTotalSlots];
     if (threadIdx.x < 16) log_add_table64(la, threadIdx.x);
     __syncthreads();
-    const int64_t at = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t at = blockIdx.x * (int64_t) kTotalWarps + warp;
     if (at >= n) return;
     const Total64 T = totals[at];
     const Region64 &R = regions[T.region];
-    const double *t0 = terms + at * 2 * term_stride, *t1 = t0 + term_stride;
-    const int4 in = R.info[T.d];
-    const int4 in1 = T.have_next ? R.info[T.d + 1] : make_int4(0, 0, 0, 0);
-    double total = kNegInf, through = kNegInf;
-    if (!multi) {
-        const int32_t most = max(in.y, in1.y);
-#pragma unroll 4
-        for (int32_t i = 0; i < most; ++i) {
-            const double a = i < in.y ? t0[i] : kNegInf, b = i < in1.y ? t1[i] : kNegInf;
-            total = lad(la, total, a);        // log_add(x, log 0) is x
-            through = lad(la, through, b);
-        }
-    } else {
-        auto fold = [&](const double *t, const int4 &f) {
-            double v = kNegInf, cell = kNegInf;
-            int32_t col = -1;
-            for (int32_t i = 0; i < f.y; ++i) {
-                const int32_t c = R.path[f.x + i].col;
-                if (c != col) {
-                    v = lad(la, v, cell);
-                    cell = kNegInf;
-                    col = c;
-                }
-                cell = lad(la, cell, t[i]);
+    const double *mt = models[R.model].t;
+    const double tMC = mt[T_MC], tMX = mt[T_MFGX], tMY = mt[T_MFGY];
+    const double *F = tasks[task_of[R.win_base + T.win]].F;   // the segment that swept the window
+    const double *t = terms + at * kTotalRows * term_stride;
+    const int4 in = R.info[T.d], in1 = T.have_next ? R.info[T.d + 1] : make_int4(0, 0, 0, 0), bl = R.info[T.d - 1];
+    double v = kNegInf, cell = kNegInf;        // lane 0: the fold on d; lane 1: through d
+    int32_t col = -1;
+    for (int32_t k0 = 0; k0 < max(in.y, in1.y); k0 += kTotalSlots) {
+#pragma unroll
+        for (int w = 0; w < kTotalSlots / 32; ++w) {
+            const int j = lane + 32 * w, i = k0 + j;
+            if (i < in.y) {
+                const double *f = F + 3 * ((int64_t) in.z + in.x + i);
+                double s = f[S_M] + t[i];
+                s = lad(la, s, f[S_X] + t[term_stride + i]);
+                s = lad(la, s, f[S_Y] + t[2 * term_stride + i]);
+                term[warp][0][j] = s;
+                if (multi) cols[warp][0][j] = R.path[in.x + i].col;
             }
-            return lad(la, v, cell);
-        };
-        total = fold(t0, in);
-        if (T.have_next) through = fold(t1, in1);
+            if (i < in1.y) {
+                const int32_t q = in1.x + i;
+                const double e = R.E[2 * ((int64_t) in1.z + q)];
+                double s = kNegInf;
+                const int32_t cnt = multi ? R.path[q].pred_n : 1, step = multi ? R.path[q].pred_step : 1;
+                for (int32_t c = 0, p = multi ? R.path[q].pred : q - 1; c < cnt; ++c, p += step) {
+                    const bool there = p >= bl.x && p < bl.x + bl.y;
+                    const double *f = F + 3 * ((int64_t) bl.z + (there ? p : bl.x));
+                    s = lad(la, s, (there ? f[S_M] : kNegInf) + (e + tMC));
+                    s = lad(la, s, (there ? f[S_X] : kNegInf) + (e + tMX));
+                    s = lad(la, s, (there ? f[S_Y] : kNegInf) + (e + tMY));
+                }
+                term[warp][1][j] = s + t[3 * term_stride + i];
+                if (multi) cols[warp][1][j] = R.path[q].col;
+            }
+        }
+        __syncwarp();
+        if (lane < 2) {
+            const int32_t m = min(kTotalSlots, (lane ? in1.y : in.y) - k0);
+            const double *s = term[warp][lane];
+            if (!multi) {
+#pragma unroll 4
+                for (int32_t j = 0; j < m; ++j) v = lad(la, v, s[j]);
+            } else {
+                for (int32_t j = 0; j < m; ++j) {
+                    if (cols[warp][lane][j] != col) {
+                        v = lad(la, v, cell);
+                        cell = kNegInf;
+                        col = cols[warp][lane][j];
+                    }
+                    cell = lad(la, cell, s[j]);
+                }
+            }
+        }
+        __syncwarp();
     }
-    if (T.have_next) total = lad(la, total, through);
-    R.P[T.d] = total;
-    if (T.last) *R.loglik = total;
+    if (multi) v = lad(la, v, cell);
+    const double through = __shfl_sync(0xffffffffu, v, 1);
+    if (lane == 0) {
+        if (T.have_next) v = lad(la, v, through);
+        R.P[T.d] = v;
+        if (T.last) *R.loglik = v;
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -796,8 +868,8 @@ struct Output64 {
 
 // the number of outputs of slot q on d, and (write) the outputs
 template <bool kAssign>
-__device__ __forceinline__ int slot_hits(const Region64 &R, const Output64 &O, int64_t at, double total, int32_t x,
-                                         int32_t y, double &p, unsigned &which) {
+__device__ __forceinline__ int slot_hits(const Region64 &R, const double *F, const Output64 &O, int64_t at, double total,
+                                         int32_t x, int32_t y, double &p, unsigned &which) {
     if (kAssign) {   // match transitions at or above the threshold, from match, gap-X, gap-Y
         which = 0;
         if (R.B[3 * at] >= 0.0)
@@ -806,13 +878,14 @@ __device__ __forceinline__ int slot_hits(const Region64 &R, const Output64 &O, i
         return __popc(which);
     }
     if (x <= 0 || y <= 0) return 0;
-    p = exp(R.S[at] - total);
+    p = exp((F[3 * at] + R.S[at]) - total);
     return p >= O.threshold ? 1 : 0;
 }
 
 template <bool kAssign, bool kWrite>
-__global__ void __launch_bounds__(256) outputs64(const Region64 *regions, const int32_t *chunk_region,
-                                                 const int32_t *chunk_d0, const int64_t *row_base, Output64 O) {
+__global__ void __launch_bounds__(256) outputs64(const Region64 *regions, const Region64 *tasks, const int32_t *task_of,
+                                                 const int32_t *chunk_region, const int32_t *chunk_d0,
+                                                 const int64_t *row_base, Output64 O) {
     const int32_t region = chunk_region[blockIdx.x];
     const Region64 &R = regions[region];
     if (kAssign && !O.reads[R.reader].hdp) return;
@@ -823,6 +896,7 @@ __global__ void __launch_bounds__(256) outputs64(const Region64 *regions, const 
         const int4 in = R.info[d];
         const Window W = R.win[in.w];
         const int32_t place = W.T + W.from - d;
+        const double *F = kAssign ? nullptr : tasks[task_of[R.win_base + in.w]].F;   // the segment that swept the window
         const double total = R.P[W.from - 10 * ((W.from - d) / 10)];
         int64_t base = kWrite ? O.region_total[region] + count[place] : 0;
         int32_t found = 0;
@@ -836,7 +910,7 @@ __global__ void __launch_bounds__(256) outputs64(const Region64 *regions, const 
             if (k < in.y) {
                 x = R.path[q].col;
                 y = d - x;
-                hits = slot_hits<kAssign>(R, O, at, total, x, y, p, which);
+                hits = slot_hits<kAssign>(R, F, O, at, total, x, y, p, which);
             }
             if (!__any_sync(0xffffffffu, hits > 0)) continue;
             int32_t inc = hits;
