@@ -7,25 +7,27 @@
 // address per operand (24 warp instructions per band cell, issue 19 to 30 % busy).
 //
 // How.  Column x lives on thread x mod NT, whichever way the band moves.  A cell's neighbours are then
-// on the same thread (the same column) or the one beside it (column x - 1 forward, x + 1 backward):
-// shuffles, and one shared float4 per warp's edge.  Threads outside the band hold -inf, which makes
-// every absent neighbour drop out of logAdd.  Three anti-diagonals' columns never share a thread: the
-// host takes this path for a batch only if any three consecutive anti-diagonals span at most
-// column_span(NT) columns.  A sweep is a chain of anti-diagonals and its warps issue in order, so
-// every instruction that is not the recursion lengthens the chain: three more warps take them, each
-// with less to do a step than the sweep, since they issue in order too (one warp for all of it made
-// the step 760 cycles; the sweep alone takes under 300).  One works out the renormalisation shifts,
-// one brings band facts and copies operands into shared memory kAhead anti-diagonals ahead, and one
-// takes the results out: forward, the values, bases and publication of windows; backward, the total
-// probabilities (sequential folds), posteriors and pairs, ten anti-diagonals at a time.
+// on the same thread (the same column) or the one beside it (column x - 1 forward, x + 1 backward): one
+// shared float4 each (shuffles and an edge per warp took ten instructions a step more).  Threads outside
+// the band hold -inf, which makes every absent neighbour drop out of logAdd.  Three anti-diagonals'
+// columns never share a thread: the host takes this path for a batch only if any three consecutive
+// anti-diagonals span at most column_span(NT) columns.  A sweep is a chain of anti-diagonals and its
+// warps issue in order, so every instruction that is not the recursion lengthens the chain: four more
+// warps take them, each with less to do a step than the sweep, since they issue in order too (one warp
+// for all of it made the step 760 cycles; the sweep alone takes under 300).  One works out the
+// renormalisation shifts, one brings band facts and copies operands into shared memory kAhead
+// anti-diagonals ahead, and two take the results out: forward, the values, bases and publication of
+// windows; backward, ten anti-diagonals at a time, one the total probabilities (sequential folds), the
+// other posteriors and pairs (one warp for both made a window's step 530 cycles longer than the sweep's
+// at 512 threads: 2,300 of them).
 //
 // The arithmetic is that of ForwardSweep and window_task, operation for operation, so the values are
 // theirs bit for bit.
 //
 // Measured on B200, the worker launch with cells by their place in the band / with four columns a lane,
-// a warp per window, and every thread its own copies / in this form: 8 reads of 8 to 12 kb (2.1e7 cells,
-// 71 segments) 3.52 / 2.35 / 1.27 ms, 30 reads of 8 to 30 kb (1.5e8 cells) 5.36 / 3.85 / 3.04 ms, 6 reads
-// of 3 to 8 kb at expansion 200 (512 threads) 6.79 / - / 3.88 ms.
+// a warp per window, and every thread its own copies / with three helper warps / in this form: 8 reads of
+// 8 to 12 kb (2.1e7 cells, 71 segments) 3.52 / 2.35 / 1.27 / 1.10 ms, 30 reads of 8 to 30 kb (1.5e8 cells)
+// 5.36 / 3.85 / 3.04 / 2.92 ms, 6 reads of 3 to 8 kb at expansion 200 (512 threads) 6.79 / - / 3.88 / 2.98 ms.
 #pragma once
 
 namespace sa {
@@ -115,8 +117,11 @@ __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync
 __device__ __forceinline__ void bar_arrive(int id, int n) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
-enum { kBarRow = 1, kBarFull = 2, kBarEmpty = 4 };   // kBarFull + b, kBarEmpty + b: block buffer b
-constexpr int kHelpers = 96;             // threads of the warps beside a sweep's: shifts, copies, results
+// kBarFull + b, kBarTotal + b, kBarEmpty + b: block buffer b
+enum { kBarRow = 1, kBarFull = 2, kBarTotal = 4, kBarEmpty = 6, kBarResults = 8 };
+// threads of the warps beside a sweep's: shifts, copies, and two of the results (forward: the cells;
+// backward: totals, and posteriors)
+constexpr int kHelpers = 128;
 
 // ------------------------------------------------------------------------------------------------
 // band facts of a sweep, 32 anti-diagonals at a time, by its service warp
@@ -201,9 +206,8 @@ struct ColumnForwardShared {
     float2 e[kRows][NT];                 // match and extra-event emissions, by cell
     InfoRing info;
     RowFacts row[4];
-    float4 edge[2][NT / 32];             // match, gap-X, gap-Y of a warp's last column, by parity
-    float part[2][NT / 32];              // the warps' largest values, by parity
-    float v[2][3][NT];                   // values by thread, by parity
+    float4 v[2][NT];                     // match, gap-X, gap-Y by thread, by parity
+    float part[2][NT / 32];              // the warps' largest values, by parity (more than 128 threads)
 };
 
 template <int NT>
@@ -213,13 +217,14 @@ struct ColumnWindowShared {
     RowFacts row[4];
     float f[kRows][NT];                  // forward match values, by cell
     float ops[5][NT];                    // a total's anti-diagonal d: gap-X, gap-Y of d; match, gap-X, gap-Y of d-1
-    float4 edge[2][NT / 32];             // match and its emission a row back, gap-X, skip emission of a warp's
-                                         // first column, by parity
-    float part[2][NT / 32];
+    float4 v[2][NT];                     // match and its emission a row back, gap-X, skip emission by thread,
+                                         // by parity
+    float part[2][NT / 32];              // the warps' largest values, by parity
     // for the posteriors' warp: by anti-diagonal of the sweep, its base and this window's; and two
     // blocks of kBlock anti-diagonals: F.B of the match state by thread, the two folds' terms, and the
     // shift and gamma of the total's anti-diagonal
     double fb[kPostRows], bb[kPostRows];
+    double total[2];                     // the blocks' total probabilities
     int2 post[kPostRows];                // first column, width
     float s[2][kBlock][NT];
     float chain[2][2][NT];
@@ -310,98 +315,8 @@ __device__ __forceinline__ void warp_stitch_arrive(const Args &A, int32_t si) {
     if (__shfl_sync(0xffffffffu, before, 0) == 1) warp_stitch_check(A, si);
 }
 
-// ------------------------------------------------------------------------------------------------
-// forward sweep of one segment
-// ------------------------------------------------------------------------------------------------
-// On anti-diagonal d a thread folds, side by side: gap-X of d (left column on d-1), gap-Y of d (own
-// column on d-1), the match state of d+1 but for its last term (left column on d-1), and the last
-// term of d's: one logAdd's latency, a barrier and a shared-memory read a step.
-template <int NT, bool kSX, bool kGX>
-__device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs) {
-    constexpr int NW = NT / 32;
-    const Args &A = *c.A;
-    const RegionDesc &R = c.R;
-    const float *t = c.t;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int32_t dbeg = S.d_begin, s = dbeg - S.warm + (dbeg == 0 ? 1 : 0), steps = S.d_end - s + 1;
-    // own column on d-1, and d's match state but for its last term, and that term
-    float M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf, most = kNegInf, last = kNegInf;
-    float mxw;                           // this warp's largest value on d-1
-    if (dbeg == 0) {
-        // anti-diagonal 0: startStateProb / raggedStartStateProb (stateMachine.c:1022-1032), column 0
-        const float s0 = R.ragged_left ? kNegInf : 0.0f, s1 = R.ragged_left ? 0.0f : kNegInf;
-        if (tid == 0) {
-            M1 = s0;
-            X1 = Y1 = s1;
-        }
-        mxw = warp == 0 ? fmaxf(s0, s1) : kNegInf;
-    } else {
-        // a later segment: every band cell of s-2 and s-1 starts at 0
-        const int2 r2 = raw_meta(A, R.diag_base, s - 2, R.n), r1 = raw_meta(A, R.diag_base, s - 1, R.n);
-        if (((tid - ((s - 1 + r1.x) >> 1)) & (NT - 1)) < (r1.y & kWidthMask)) M1 = X1 = Y1 = 0.0f;
-        const bool left = ((tid - 1 - ((s - 2 + r2.x) >> 1)) & (NT - 1)) < (r2.y & kWidthMask);
-        const float z = left ? 0.0f : kNegInf;
-        most = lac(z + t[T_MC], z + t[T_MFGX]);
-        last = z + t[T_MFGY];
-        mxw = 0.0f;
-    }
-    if (lane == 0) fs->part[1][warp] = mxw;
-    if (lane == 31) fs->edge[1][warp] = make_float4(M1, X1, Y1, 0.0f);
-    const float4 *edge = &fs->edge[0][(warp + NW - 1) & (NW - 1)];
-    bar_sync(kBarRow, NT + kHelpers);          // the first rows are ready
-    RowFacts row = fs->row[0];
-    bool inb = ((tid - row.xf) & (NT - 1)) < (row.w & kWidthMask);
-    float2 e = fs->e[0][(tid - row.xf) & (NT - 1)];
-    float gx = 0.0f;
-    if (kGX) gx = raw_gapx(c, row.xf + ((tid - row.xf) & (NT - 1)));
-#pragma unroll 2
-    for (int32_t k = 0; k < steps; ++k) {
-        float lM = __shfl_up_sync(0xffffffffu, M1, 1), lX = __shfl_up_sync(0xffffffffu, X1, 1),
-              lY = __shfl_up_sync(0xffffffffu, Y1, 1);
-        float x[4], y[4], r[4];
-        x[1] = M1 + t[T_OY];
-        y[1] = Y1 + t[T_EY];
-        x[2] = most;
-        y[2] = last;
-        bar_sync(kBarRow, NT + kHelpers);      // d-1's edges; d+1's facts and emissions
-        const float4 ed = edge[((k + 1) & 1) * NW];
-        const RowFacts next = fs->row[(k + 1) & 3];
-        if (lane == 0) {
-            lM = ed.x;
-            lX = ed.y;
-            lY = ed.z;
-        }
-        x[0] = lM + t[T_OX];
-        y[0] = lX + t[T_EX];
-        x[3] = lM + t[T_MC];
-        y[3] = lX + t[T_MFGX];
-        const int32_t i = (tid - next.xf) & (NT - 1);
-        const float2 e_next = fs->e[(k + 1) & (kRows - 1)][i];
-        lacs<4>(x, y, r);
-        if (kSX) r[0] = lac(r[0], lY + t[T_SX]);
-        const float vX = r[0] + ((kGX ? gx : c.gx) + row.sh1);
-        const float vY = r[1] + (e.y + row.sh1);
-        const float vM = r[2] + (e.x + row.sh2);
-        most = r[3];
-        last = lY + t[T_MFGY];
-        M1 = inb ? vM : kNegInf;
-        X1 = inb ? vX : kNegInf;
-        Y1 = inb ? vY : kNegInf;
-        if (lane == 31) fs->edge[k & 1][warp] = make_float4(M1, X1, Y1, 0.0f);
-        mxw = warp_max1(fmaxf(M1, fmaxf(X1, Y1)));
-        if (lane == 0) fs->part[k & 1][warp] = mxw;
-        fs->v[k & 1][0][tid] = M1;
-        fs->v[k & 1][1][tid] = X1;
-        fs->v[k & 1][2][tid] = Y1;
-        row = next;
-        inb = i < (next.w & kWidthMask);
-        e = e_next;
-        if (kGX) gx = raw_gapx(c, row.xf + i);
-    }
-    bar_sync(kBarRow, NT + kHelpers);          // the last anti-diagonal's values go out
-}
-
-// The largest of the warps' values (part: one row of them)
+// The largest of the warps' values (part: one row of them), and a warp's share of it.  A sweep of up to
+// 128 threads leaves both to the warp of the shifts; wider, that warp would read too long.
 template <int NW>
 __device__ __forceinline__ float part_max(const float *part) {
     float m[NW];
@@ -413,6 +328,87 @@ __device__ __forceinline__ float part_max(const float *part) {
         for (int w = 0; w < NW / 2; ++w)
             if (w < o) m[w] = fmaxf(m[w], m[w + o]);
     return m[0];
+}
+
+__device__ __forceinline__ void part_of(float *part, float m, float x, float y) {
+    const float mx = warp_max1(fmaxf(m, fmaxf(x, y)));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = mx;
+}
+
+// ------------------------------------------------------------------------------------------------
+// forward sweep of one segment
+// ------------------------------------------------------------------------------------------------
+// On anti-diagonal d a thread folds, side by side: gap-X of d (left column on d-1), gap-Y of d (own
+// column on d-1), the match state of d+1 but for its last term (left column on d-1), and the last
+// term of d's: one logAdd's latency, a barrier and a shared-memory read a step.
+template <int NT, bool kSX, bool kGX>
+__device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs) {
+    const Args &A = *c.A;
+    const RegionDesc &R = c.R;
+    const float *t = c.t;
+    const int tid = threadIdx.x;
+    const int32_t dbeg = S.d_begin, s = dbeg - S.warm + (dbeg == 0 ? 1 : 0), steps = S.d_end - s + 1;
+    // own column on d-1, and d's match state but for its last term, and that term
+    float M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf, most = kNegInf, last = kNegInf;
+    if (dbeg == 0) {
+        // anti-diagonal 0: startStateProb / raggedStartStateProb (stateMachine.c:1022-1032), column 0
+        const float s0 = R.ragged_left ? kNegInf : 0.0f, s1 = R.ragged_left ? 0.0f : kNegInf;
+        if (tid == 0) {
+            M1 = s0;
+            X1 = Y1 = s1;
+        }
+    } else {
+        // a later segment: every band cell of s-2 and s-1 starts at 0
+        const int2 r2 = raw_meta(A, R.diag_base, s - 2, R.n), r1 = raw_meta(A, R.diag_base, s - 1, R.n);
+        if (((tid - ((s - 1 + r1.x) >> 1)) & (NT - 1)) < (r1.y & kWidthMask)) M1 = X1 = Y1 = 0.0f;
+        const bool left = ((tid - 1 - ((s - 2 + r2.x) >> 1)) & (NT - 1)) < (r2.y & kWidthMask);
+        const float z = left ? 0.0f : kNegInf;
+        most = lac(z + t[T_MC], z + t[T_MFGX]);
+        last = z + t[T_MFGY];
+    }
+    fs->v[1][tid] = make_float4(M1, X1, Y1, 0.0f);
+    if (NT > 128) part_of(fs->part[1], M1, X1, Y1);
+    const float4 *left = &fs->v[0][(tid + NT - 1) & (NT - 1)];   // the column before
+    bar_sync(kBarRow, NT + kHelpers);          // the first rows are ready
+    RowFacts row = fs->row[0];
+    bool inb = ((tid - row.xf) & (NT - 1)) < (row.w & kWidthMask);
+    float2 e = fs->e[0][(tid - row.xf) & (NT - 1)];
+    float gx = 0.0f;
+    if (kGX) gx = raw_gapx(c, row.xf + ((tid - row.xf) & (NT - 1)));
+#pragma unroll 2
+    for (int32_t k = 0; k < steps; ++k) {
+        float x[4], y[4], r[4];
+        x[1] = M1 + t[T_OY];
+        y[1] = Y1 + t[T_EY];
+        x[2] = most;
+        y[2] = last;
+        bar_sync(kBarRow, NT + kHelpers);      // d-1's values; d+1's facts and emissions
+        const float4 l = left[((k + 1) & 1) * NT];
+        const RowFacts next = fs->row[(k + 1) & 3];
+        x[0] = l.x + t[T_OX];
+        y[0] = l.y + t[T_EX];
+        x[3] = l.x + t[T_MC];
+        y[3] = l.y + t[T_MFGX];
+        const int32_t i = (tid - next.xf) & (NT - 1);
+        const float2 e_next = fs->e[(k + 1) & (kRows - 1)][i];
+        lacs<4>(x, y, r);
+        if (kSX) r[0] = lac(r[0], l.z + t[T_SX]);
+        const float vX = r[0] + ((kGX ? gx : c.gx) + row.sh1);
+        const float vY = r[1] + (e.y + row.sh1);
+        const float vM = r[2] + (e.x + row.sh2);
+        most = r[3];
+        last = l.z + t[T_MFGY];
+        M1 = inb ? vM : kNegInf;
+        X1 = inb ? vX : kNegInf;
+        Y1 = inb ? vY : kNegInf;
+        fs->v[k & 1][tid] = make_float4(M1, X1, Y1, 0.0f);
+        if (NT > 128) part_of(fs->part[k & 1], M1, X1, Y1);
+        row = next;
+        inb = i < (next.w & kWidthMask);
+        e = e_next;
+        if (kGX) gx = raw_gapx(c, row.xf + i);
+    }
+    bar_sync(kBarRow, NT + kHelpers);          // the last anti-diagonal's values go out
 }
 
 // The forward sweep's shifts: at step k (anti-diagonal d) those of d+2, from the maximum of d-1.
@@ -427,7 +423,19 @@ __device__ __forceinline__ void column_forward_shifts(const Segment &S, ColumnFo
 #pragma unroll 2
     for (int32_t k = 0; k < steps; ++k) {
         bar_sync(kBarRow, NT + kHelpers);
-        const float mx = part_max<NT / 32>(fs->part[(k + 1) & 1]);
+        float mx;
+        if constexpr (NT > 128) {
+            mx = part_max<NT / 32>(fs->part[(k + 1) & 1]);
+        } else {
+            const float4 *v = &fs->v[(k + 1) & 1][lane];
+            float most[NT / 32];
+#pragma unroll
+            for (int w = 0; w < NT / 32; ++w) {
+                const float4 u = v[32 * w];
+                most[w] = fmaxf(u.x, fmaxf(u.y, u.z));
+            }
+            mx = warp_max1(part_max<NT / 32>(most));
+        }
         const float d2 = ((mx > kNegInf ? mx : 0.0f) - d1) - d0;
         if (lane == 0) *reinterpret_cast<float2 *>(&fs->row[(k + 2) & 3].sh1) = make_float2(-d2, -d1 - d2);
         d0 = d1;
@@ -481,18 +489,19 @@ __device__ __forceinline__ void column_forward_copies(const Ctx &c, const Segmen
 }
 
 // The forward sweep's results: at step k d-1's values, base and shift go out, a window that closes there
-// is published, and a stitch there gets its side.
+// is published, and a stitch there gets its side.  Two warps, `part` 0 and 1, share the cells.
 template <int NT>
-__device__ __forceinline__ void column_forward_results(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs) {
-    constexpr int NW = NT / 32;
+__device__ __forceinline__ void column_forward_results(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs,
+                                                       int part) {
+    constexpr int NW = NT / 64;          // cells a lane has, 64 apart
     const Args &A = *c.A;
     const RegionDesc &R = c.R;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, cell = lane + 32 * part;
     const int64_t db = R.diag_base;
     const int32_t dbeg = S.d_begin, dend = S.d_end;
     const int32_t s = dbeg - S.warm + (dbeg == 0 ? 1 : 0), steps = dend - s + 1;
     float *Freg = A.F + 3 * R.cell_base;
-    if (dbeg == 0 && lane == 0) {
+    if (dbeg == 0 && cell == 0) {
         const float s0 = R.ragged_left ? kNegInf : 0.0f, s1 = R.ragged_left ? 0.0f : kNegInf;
         Freg[ST_M] = s0;
         Freg[ST_X] = s1;
@@ -512,25 +521,25 @@ __device__ __forceinline__ void column_forward_results(const Ctx &c, const Segme
         const int32_t r = s + k - 1;     // the anti-diagonal that goes out
         const int32_t W = in.y & kWidthMask;
         const bool own = r > dbeg, gaps = (in.y & kFlagStoreGaps) != 0;
-        float *Fd = Freg + 3 * (int64_t) in.z + lane;
+        float *Fd = Freg + 3 * (int64_t) in.z + cell;
         int at[NW];
 #pragma unroll
-        for (int w = 0; w < NW; ++w) at[w] = (in.x + lane + 32 * w) & (NT - 1);
+        for (int w = 0; w < NW; ++w) at[w] = (in.x + cell + 64 * w) & (NT - 1);
         bar_sync(kBarRow, NT + kHelpers);
-        const float(*v)[NT] = fs->v[(k - 1) & 1];
+        const float4 *v = fs->v[(k - 1) & 1];
         if (own) {
             float o[NW];
 #pragma unroll
-            for (int w = 0; w < NW; ++w) o[w] = v[0][at[w]];
+            for (int w = 0; w < NW; ++w) o[w] = v[at[w]].x;
 #pragma unroll
             for (int w = 0; w < NW; ++w)
-                if (lane + 32 * w < W) Fd[32 * w] = o[w];
+                if (cell + 64 * w < W) Fd[64 * w] = o[w];
             if (gaps) {
 #pragma unroll
                 for (int w = 0; w < NW; ++w) {
-                    if (lane + 32 * w < W) {
-                        Fd[W + 32 * w] = v[1][at[w]];
-                        Fd[2 * W + 32 * w] = v[2][at[w]];
+                    if (cell + 64 * w < W) {
+                        Fd[W + 64 * w] = v[at[w]].y;
+                        Fd[2 * W + 64 * w] = v[at[w]].z;
                     }
                 }
             }
@@ -545,14 +554,14 @@ __device__ __forceinline__ void column_forward_results(const Ctx &c, const Segme
             qshift = delta;
         }
         if (q == 31 || window_end || r == dend) {
-            if (lane <= q && r - q + lane > dbeg) {
+            if (part == 0 && lane <= q && r - q + lane > dbeg) {
                 A.base[db + (r - q) + lane] = qbase;
                 A.fshift[db + (r - q) + lane] = qshift;
             }
             if (window_end) {
                 __threadfence();         // this anti-diagonal and all before it, device-wide
-                __syncwarp();
-                if (lane == 0) {
+                bar_sync(kBarResults, 64);
+                if (cell == 0) {
                     const unsigned p = atomicAdd(&A.ctl->pub, 1u);
                     if ((int64_t) p < A.n_windows) atomicExch(A.ready + p, (int32_t) (R.win_base + wi));
                 }
@@ -564,9 +573,13 @@ __device__ __forceinline__ void column_forward_results(const Ctx &c, const Segme
             const int32_t si = in_side ? S.stitch_in : S.stitch_out, b = in_side ? dbeg : dend;
             const StitchDesc sd = A.stitch[si];
             float *o = A.stitch_vals + sd.voff + (in_side ? 0 : 3 * (sd.w0 + sd.w1)) + (r == b ? 3 * sd.w0 : 0);
-            for (int i = lane; i < W; i += 32)
-                for (int st = 0; st < 3; ++st) o[st * W + i] = v[st][(in.x + i) & (NT - 1)];
-            if (r == b && lane == 0) {
+            for (int i = cell; i < W; i += 64) {
+                const float4 u = v[(in.x + i) & (NT - 1)];
+                o[i] = u.x;
+                o[W + i] = u.y;
+                o[2 * W + i] = u.z;
+            }
+            if (r == b && cell == 0) {
                 // as ForwardSweep: back from the base past b
                 const double past = base + (double) delta_next, base_b = past - (double) delta_next;
                 double *bs = in_side ? A.stitch_res[si].sbase : A.stitch_res[si].tbase;
@@ -579,9 +592,9 @@ __device__ __forceinline__ void column_forward_results(const Ctx &c, const Segme
     }
     if (S.stitch_in >= 0 || S.stitch_out >= 0) {
         __threadfence();                 // the stitch's values, before the counts below
-        __syncwarp();
-        if (S.stitch_in >= 0) warp_stitch_arrive(A, S.stitch_in);
-        if (S.stitch_out >= 0) warp_stitch_arrive(A, S.stitch_out);
+        bar_sync(kBarResults, 64);
+        if (S.stitch_in >= 0 && part == 0) warp_stitch_arrive(A, S.stitch_in);
+        if (S.stitch_out >= 0 && part == 1) warp_stitch_arrive(A, S.stitch_out);
     }
 }
 
@@ -669,7 +682,6 @@ __device__ __forceinline__ float2 column_folds(float *chain, int na, int nb) {
 // ------------------------------------------------------------------------------------------------
 template <int NT, bool kSX, bool kGX>
 __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &Wn, ColumnWindowShared<NT> *ws) {
-    constexpr int NW = NT / 32;
     const RegionDesc &R = c.R;
     const float *t = c.t;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -679,12 +691,12 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
     const float e0 = ragged_end ? (t[T_OX] + t[T_OY]) / 2.0f : t[T_MC];
     const float e1 = ragged_end ? t[T_EX] : t[T_MFGX];
     const float e2 = ragged_end ? t[T_EY] : t[T_MFGY];
-    if (lane == 0) ws->edge[1][warp] = make_float4(kNegInf, 0.0f, kNegInf, 0.0f);
-    const float4 *edge = &ws->edge[0][(warp + 1) & (NW - 1)];
-    // own column: values and emissions of d+1, match value and emission of d+2
-    float M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf, M2 = kNegInf;
+    ws->v[1][tid] = make_float4(kNegInf, 0.0f, kNegInf, 0.0f);
+    const float4 *right = &ws->v[0][(tid + 1) & (NT - 1)];   // the column after
+    // own column: values and emissions of d+1
+    float M1 = kNegInf, Y1 = kNegInf;
     float2 e1r = make_float2(0.0f, 0.0f);
-    float eM2 = 0.0f, gx = 0.0f, gx1 = 0.0f;
+    float gx = 0.0f;
     int32_t i1 = 0, W1 = 0, xf1 = 0;     // its cell, the width and the first column of d+1
     int32_t left = rows;                 // posterior anti-diagonals to come
     int32_t block = 0, in_block = 0;
@@ -697,21 +709,13 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
     for (int32_t k = 0; k < steps; ++k) {
         const int32_t W = row.y & kWidthMask;
         const bool inb = i < W;
-        float nM = __shfl_down_sync(0xffffffffu, M2, 1), nE = __shfl_down_sync(0xffffffffu, eM2, 1),
-              nX = __shfl_down_sync(0xffffffffu, X1, 1), nG = kGX ? __shfl_down_sync(0xffffffffu, gx1, 1) : c.gx;
-        bar_sync(kBarRow, NT + 64);      // d+1's edges, d's shifts; d-1's facts and operands
-        const float4 ed = edge[((k + 1) & 1) * NW];
+        bar_sync(kBarRow, NT + 64);      // d+1's values, d's shifts; d-1's facts and operands
+        const float4 n = right[((k + 1) & 1) * NT];
         const float2 sh = *reinterpret_cast<const float2 *>(&ws->row[k & 3].sh1);
         const int2 next = *reinterpret_cast<const int2 *>(&ws->row[(k + 1) & 3].xf);
-        if (lane == 31) {
-            nM = ed.x;
-            nE = ed.y;
-            nX = ed.z;
-            if (kGX) nG = ed.w;
-        }
-        const float me = nM + (nE + sh.y);
+        const float me = n.x + (n.y + sh.y);
         const float ue = Y1 + (e1r.y + sh.x);
-        const float le = nX + (nG + sh.x);
+        const float le = n.z + ((kGX ? n.w : c.gx) + sh.x);
         float x[3], y[3], r[3];
         x[0] = me + t[T_MC];
         y[0] = ue + t[T_OY];
@@ -731,7 +735,7 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
             r[2] = e2;
         }
         const float vM = inb ? r[0] : kNegInf, vX = inb ? r[1] : kNegInf, vY = inb ? r[2] : kNegInf;
-        if (lane == 0) ws->edge[k & 1][warp] = make_float4(M1, e1r.x, vX, gx);
+        ws->v[k & 1][tid] = make_float4(M1, e1r.x, vX, gx);
         const float mx = warp_max1(fmaxf(vM, fmaxf(vX, vY)));
         if (lane == 0) ws->part[k & 1][warp] = mx;
         if ((row.y & kRowPost) != 0) {
@@ -770,13 +774,9 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
                 in_block = 0;
             }
         }
-        M2 = M1;
-        eM2 = e1r.x;
         M1 = vM;
-        X1 = vX;
         Y1 = vY;
         e1r = e;
-        gx1 = gx;
         i1 = i;
         W1 = W;
         xf1 = row.x;
@@ -897,8 +897,29 @@ __device__ __forceinline__ void column_window_copies(const Ctx &c, const Window 
     copy_wait<0>();
 }
 
-// The window's total probabilities, posteriors and pairs (one warp): a block's total first, then its
-// anti-diagonals in the reference's order, descending, cells ascending.
+// The window's total probabilities (one warp), a block's at a time.
+template <int NT>
+__device__ __forceinline__ void column_window_totals(const Window &Wn, ColumnWindowShared<NT> *ws) {
+    const int lane = threadIdx.x & 31;
+    const int32_t rows = Wn.from - Wn.T, blocks = (rows + kBlock - 1) / kBlock;
+    for (int32_t q = 0; q < blocks; ++q) {
+        const int b = q & 1;
+        bar_sync(kBarFull + b, NT + 32);
+        const int2 widths = ws->widths[b];
+        const float2 ff = column_folds<NT / 32>(&ws->chain[b][0][0], widths.x, widths.y);
+        const float2 th = ws->through[b];
+        // the through-part is relative to base_F(d-1) + base_B(d+1)
+        const float ptil = lac(ff.x, ff.y - th.x - th.y);
+        const int32_t k0 = Wn.D - Wn.from + q * kBlock;   // the total's anti-diagonal
+        if (lane == 0) ws->total[b] = (double) ptil + ws->fb[k0 & (kPostRows - 1)] + ws->bb[k0 & (kPostRows - 1)];
+        __syncwarp();
+        bar_arrive(kBarTotal + b, 64);
+    }
+}
+
+// The window's posteriors and pairs (one warp): a block's anti-diagonals in the reference's order,
+// descending, cells ascending.  Most of an anti-diagonal's cells are far below the threshold, so only
+// the groups of 32 that hold one above it are looked at closely.
 template <int NT>
 __device__ __forceinline__ void column_window_post(const Ctx &c, const Window &Wn, const WindowTask &wt, int64_t gw,
                                                    ColumnWindowShared<NT> *ws) {
@@ -908,19 +929,15 @@ __device__ __forceinline__ void column_window_post(const Ctx &c, const Window &W
     const int lane = threadIdx.x & 31;
     const int32_t rows = Wn.from - Wn.T, blocks = (rows + kBlock - 1) / kBlock;
     // a cell can only reach the threshold if its logarithm does
-    const float log_threshold = A.threshold > 0.0f ? logf(A.threshold) - 1e-3f : kNegInf;
-    double pref = 0.0, ll = 0.0;
+    const bool every = !(A.threshold > 0.0f);
+    const float log_threshold = every ? kNegInf : logf(A.threshold) - 1e-3f;
+    double ll = 0.0;
     int64_t n_out = 0;
     for (int32_t q = 0; q < blocks; ++q) {
         const int b = q & 1;
-        bar_sync(kBarFull + b, NT + 32);
-        const int2 widths = ws->widths[b];
-        const float2 ff = column_folds<NT / 32>(&ws->chain[b][0][0], widths.x, widths.y);
-        const float2 th = ws->through[b];
-        // the through-part is relative to base_F(d-1) + base_B(d+1)
-        const float ptil = lac(ff.x, ff.y - th.x - th.y);
+        bar_sync(kBarTotal + b, 64);
+        const double pref = ws->total[b];
         const int32_t top = Wn.from - q * kBlock, k0 = Wn.D - top;   // the total's anti-diagonal
-        pref = (double) ptil + ws->fb[k0 & (kPostRows - 1)] + ws->bb[k0 & (kPostRows - 1)];
         if (top == R.n) ll = pref;
         const int m = min(kBlock, rows - q * kBlock);
         // lane j: what the block's j-th anti-diagonal needs
@@ -931,20 +948,18 @@ __device__ __forceinline__ void column_window_post(const Ctx &c, const Window &W
             const float kd = __shfl_sync(0xffffffffu, kd_lane, j);
             const int32_t xf = __shfl_sync(0xffffffffu, row_lane.x, j), W = __shfl_sync(0xffffffffu, row_lane.y, j);
             const int32_t d = top - j;
-            float v[NW], most = kNegInf;
+            const float *s = ws->s[b][j];
+            unsigned mine = 0;
 #pragma unroll
             for (int w = 0; w < NW; ++w) {
                 const int i = lane + 32 * w;
-                v[w] = ws->s[b][j][(xf + i) & (NT - 1)] + kd;
-                if (i >= W) v[w] = kNegInf;
-                most = fmaxf(most, v[w]);
+                const float v = s[(xf + i) & (NT - 1)] + kd;
+                if (i < W && (v > log_threshold || every)) mine |= 1u << w;
             }
-            if (!__any_sync(0xffffffffu, most > log_threshold || A.threshold <= 0.0f)) continue;
-#pragma unroll
-            for (int w = 0; w < NW; ++w) {
-                const int i = lane + 32 * w;
+            for (unsigned groups = __reduce_or_sync(0xffffffffu, mine); groups; groups &= groups - 1) {
+                const int i = lane + 32 * (__ffs(groups) - 1);
                 const int32_t x = xf + i, y = d - x;
-                const float p = __expf(v[w]);
+                const float p = __expf(s[x & (NT - 1)] + kd);
                 const bool hit = i < W && x > 0 && y > 0 && p >= A.threshold;
                 const unsigned bal = __ballot_sync(0xffffffffu, hit);
                 if (hit) {
@@ -983,7 +998,7 @@ __device__ __forceinline__ void column_forward(const Ctx &c, const Segment &sg, 
     if (threadIdx.x < NT) column_forward_sweep<NT, kSX, kGX>(c, sg, fs);
     else if (threadIdx.x < NT + 32) column_forward_shifts<NT>(sg, fs);
     else if (threadIdx.x < NT + 64) column_forward_copies<NT>(c, sg, fs);
-    else column_forward_results<NT>(c, sg, fs);
+    else column_forward_results<NT>(c, sg, fs, (threadIdx.x - NT - 64) >> 5);
 }
 
 template <int NT, bool kSX, bool kGX>
@@ -993,6 +1008,7 @@ __device__ __forceinline__ void column_window(const Ctx &c, ColumnWindowShared<N
     if (threadIdx.x < NT) column_window_sweep<NT, kSX, kGX>(c, Wn, ws);
     else if (threadIdx.x < NT + 32) column_window_shifts<NT>(c, Wn, ws);
     else if (threadIdx.x < NT + 64) column_window_copies<NT>(c, Wn, wt, ws);
+    else if (threadIdx.x < NT + 96) column_window_totals<NT>(Wn, ws);
     else column_window_post<NT>(c, Wn, wt, id, ws);
 }
 
@@ -1050,7 +1066,7 @@ __global__ void __launch_bounds__(NT + kHelpers, MINB) column_worker(const __gri
             else column_window<NT, false, true>(c, &cs->w, id);
         }
         // the posteriors' warp wrote the window's pairs and counts
-        if (tid >= NT + 64) read_unit_done<32>(A, c.R.read, tid & 31, nullptr);
+        if (tid >= NT + 96) read_unit_done<32>(A, c.R.read, tid & 31, nullptr);
         __syncthreads();
     }
 }

@@ -15,7 +15,8 @@
 // anti-diagonal and sweep: latency, not arithmetic (issue 0.1 a cycle on its SM, FP64 pipe 3 %).
 // Here the paths of the reference are numbered along it and path q stays on thread q mod NT, so its own
 // column's previous value is in a register and its neighbours' are one shared-memory read away; the
-// operands come by asynchronous copy kAhead64 anti-diagonals ahead; and a step's log_adds are independent.  Windows run side by side, and logarithms, exponentials, totals and outputs are off the
+// operands come by asynchronous copy kAhead64 anti-diagonals ahead; and a step's log_adds are
+// independent.  Windows run side by side, and logarithms, exponentials, totals and outputs are off the
 // sweeps' chain.  Measured on B200: see the dispatch rule in plain_create.
 //
 // A slot not in the band holds log 0 for that anti-diagonal, so an absent neighbour drops out of
@@ -217,11 +218,12 @@ __device__ __forceinline__ void lad2(const LogAdd64 &t, const double (&x)[2], co
 // A sweep is a chain of anti-diagonals and its warps issue in order, so what counts is how much one
 // warp does a step.  Four log_adds of a step are independent of one another; two groups of NT threads
 // take two each (gap-X and gap-Y of d; the match state but for its last term, and the last term of the
-// anti-diagonal next to it), and two more warps take what is not the recursion: the copies, and the
-// stores.  Operands lie by thread, those of slots outside the band as log 0, which makes a path that is
-// not there drop out without a test.  Cycles a step of the forward sweep: one group with its own copies
-// and stores 895, with bank conflicts gone 805, with the two helper warps 600 (290 of them without the
-// log_adds), in this form @@CYC@@.
+// anti-diagonal next to it), and more warps take what is not the recursion: the copies, and the stores,
+// two of each while a CTA has room.  Operands lie by thread, those of slots outside the band as log 0,
+// which makes a path that is not there drop out without a test.  Cycles a step of the forward sweep: one
+// group with its own copies and stores 895, with bank conflicts gone 805, with helper warps 600, with two
+// groups 465 (250 of them without the log_adds).  Backward, where the terms of the totals were the match
+// group's too and one warp copied: 853, with two warps and the totals' terms in a launch of their own 520.
 template <int NT>
 constexpr int kHelperWarps64 = NT <= 256 ? 2 : 1;   // of the copies, and as many of the stores
 template <int NT>
