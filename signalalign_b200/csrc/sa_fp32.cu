@@ -139,6 +139,7 @@ struct sa_batch {
     int64_t n_segs = 0, n_stitch = 0, stitch_floats = 0;
     int64_t cells = 0, out_total = 0;
     int32_t max_width = 0;
+    bool any_hdp = false, any_gaussian = false;   // machines with HDP emissions, and others
     int32_t max_span = 0;         // columns that three consecutive anti-diagonals span at most
     float threshold = 0.01f;
     // inputs, staged on the host with the device layout (one copy uploads them all)
@@ -889,14 +890,20 @@ sa_status sa_batch_upload(sa_batch *b, void *stream) {
             m.gapx_value = uni ? (float) sm->gapx[0] : 0.0f;
         }
         for (int j = 0; j < 9; ++j) m.t[j] = (float) sm->t[j];
-        if (sm->emission == SA_EMIT_HDP) {
+        if (sm->emission != SA_EMIT_HDP) {
+            b->any_gaussian = true;
+        } else {
+            b->any_hdp = true;
             const HdpTables &h = sm->hdp;
             m.hdp64.match = sm->dev.match;
-            m.hdp64.grid = sm->dev.hdp_grid;
             m.hdp64.density = sm->dev.hdp_density;
             m.hdp64.slope = sm->dev.hdp_slope;
             m.hdp64.kmer_row = sm->dev.hdp_kmer_row;
             m.hdp64.grid_length = h.grid_length;
+            m.hdp64.start = h.grid_start;
+            m.hdp64.stop = h.grid_stop;
+            m.hdp64.step = (h.grid_stop - h.grid_start) / (double) (h.grid_length - 1);
+            m.hdp64.dx = h.grid[1] - h.grid[0];
         }
     }
     sa_status st = SA_OK;
@@ -949,9 +956,10 @@ sa_status sa_batch_run(sa_batch *b, void *stream) {
             for (cudaEvent_t &e : b->ev) cudaEventCreate(&e);
         const bool timing = b->owns_device && b->ev[3];
         if (timing) cudaEventRecord(b->ev[0], s);
-        emission_kernel<<<(unsigned) std::max<int64_t>(1, std::min<int64_t>((int64_t) sms * cfg.emission_ctas_per_sm,
-                                                                            (a.n_chunks + kEmitWarps - 1) / kEmitWarps)),
-                          32 * kEmitWarps, 0, s>>>(a);
+        const auto grid = (unsigned) std::max<int64_t>(1, std::min<int64_t>((int64_t) sms * cfg.emission_ctas_per_sm,
+                                                                            (a.n_chunks + kEmitWarps - 1) / kEmitWarps));
+        if (b->any_gaussian) emission_kernel<<<grid, 32 * kEmitWarps, 0, s>>>(a);
+        if (b->any_hdp) emission_hdp_kernel<<<grid, 32 * kEmitWarps, 0, s>>>(a);
         if (timing) cudaEventRecord(b->ev[1], s);
         launch_worker(b, a, cfg, sms, s);
         if (timing) cudaEventRecord(b->ev[2], s);
@@ -962,7 +970,7 @@ sa_status sa_batch_run(sa_batch *b, void *stream) {
             cudaEventRecord(b->ev[3], s);
             b->timed = true;
         }
-        count_launch(b->d_done ? 2 : 3);
+        count_launch((b->any_gaussian ? 1 : 0) + (b->any_hdp ? 1 : 0) + (b->d_done ? 1 : 2));
         if (cudaGetLastError() != cudaSuccess) st = SA_E_CUDA;
     }
     if (!st && b->plain) st = plain_run(b->plain, s);

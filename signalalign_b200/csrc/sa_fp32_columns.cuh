@@ -685,7 +685,7 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
     const RegionDesc &R = c.R;
     const float *t = c.t;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int32_t D = Wn.D, steps = Wn.D - Wn.T, rows = Wn.from - Wn.T;
+    const int32_t steps = Wn.D - Wn.T, rows = Wn.from - Wn.T;
     // end-state values on D (stateMachine.c:1034-1061)
     const bool ragged_end = Wn.at_end && R.ragged_right;
     const float e0 = ragged_end ? (t[T_OX] + t[T_OY]) / 2.0f : t[T_MC];

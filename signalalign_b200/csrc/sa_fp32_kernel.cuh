@@ -68,11 +68,12 @@ enum { T_MC = 0, T_MFGX, T_MFGY, T_OX, T_OY, T_EX, T_EY, T_SX, T_SY };
 // below the FP32 range in the tails, and the spline's terms cancel there)
 struct Hdp64 {
     const double *match;      // n_kmers x 5 (level mean in column 0)
-    const double *grid;       // grid_length knots
     const double *density;    // rows x grid_length
     const double *slope;      // rows x grid_length
     const int64_t *kmer_row;  // n_kmers
     int64_t grid_length;
+    // knot i is start + i step (linspace, hdp_math_utils.c:497-509), the last one stop; dx: the first two's distance
+    double start, stop, step, dx;
 };
 
 struct ModelDesc {
@@ -432,48 +433,158 @@ constexpr int kEmitCols = 4;   // column slots per lane of the column-stationary
 struct EmitStage {
     float4 kca[kEmitSpan], kcb[kEmitSpan];
     float4 ev[kEmitSpan];
-    double mean[kEmitSpan];     // FP64 event means (HDP)
-    int32_t kid[kEmitSpan];
 };
 
 // getHdpKmerDensity (stateMachine.c:468-495): log((1/var) * max(0, spline(descaled mean))) with the
-// spline of grid_spline_interp (hdp_math_utils.c:471-495), in FP64 as the reference computes it
-__device__ __forceinline__ float emit_hdp64(const Hdp64 &h, int32_t kid, double mean, const ReadScale64 &rs) {
+// spline of grid_spline_interp (hdp_math_utils.c:471-495), in FP64 as the reference computes it.  In
+// three stages, so that several cells' table reads can be under way together: the descaled mean and
+// its knot, the reads, the value.
+struct HdpRow {
+    const double *y, *sl;       // densities and slopes of the k-mer's row (null: it has none)
+    double mu;                  // its level mean
+};
+struct HdpCell {
+    double u, xl, yl, yr, sl, sr;
+    int64_t il;
+};
+
+__device__ __forceinline__ HdpRow hdp_row(const Hdp64 &h, int32_t kid) {
     const int64_t row = h.kmer_row[kid];
-    if (row < 0) return kNegInf;
-    const double mu = h.match[(int64_t) kid * 5];
+    if (row < 0) return HdpRow{nullptr, nullptr, 0.0};
+    return HdpRow{h.density + row * h.grid_length, h.slope + row * h.grid_length, h.match[(int64_t) kid * 5]};
+}
+
+__device__ __forceinline__ void hdp_knot(HdpCell &cell, double mean, double mu, const ReadScale64 &rs, const Hdp64 &h) {
     const double u = (mean + rs.var * mu - rs.scale * mu - rs.shift) / rs.var;
-    const double *x = h.grid, *y = h.density + row * h.grid_length, *sl = h.slope + row * h.grid_length;
-    const int64_t len = h.grid_length;
+    const int64_t il = (int64_t) ((u - h.start) / h.dx), last = h.grid_length - 2;
+    cell.u = u;
+    cell.il = il > last ? last : (il < 0 ? 0 : il);
+    cell.xl = __dadd_rn(h.start, __dmul_rn((double) cell.il, h.step));
+}
+
+__device__ __forceinline__ void hdp_read(HdpCell &cell, const HdpRow &r) {
+    cell.yl = __ldg(r.y + cell.il);
+    cell.yr = __ldg(r.y + cell.il + 1);
+    cell.sl = __ldg(r.sl + cell.il);
+    cell.sr = __ldg(r.sl + cell.il + 1);
+}
+
+__device__ __forceinline__ float hdp_value(const HdpCell &cell, const ReadScale64 &rs, const Hdp64 &h) {
+    const double u = cell.u, x0 = h.start, xe = h.stop, dx = h.dx;
     double d;
-    if (u <= x[0]) {
-        d = y[0] - sl[0] * (x[0] - u);
-    } else if (u >= x[len - 1]) {
-        d = y[len - 1] + sl[len - 1] * (u - x[len - 1]);
+    if (u <= x0) {
+        d = cell.yl - cell.sl * (x0 - u);
+    } else if (u >= xe) {
+        d = cell.yr + cell.sr * (u - xe);
     } else {
-        const double dx = x[1] - x[0];
-        int64_t il = (int64_t) ((u - x[0]) / dx);
-        il = il > len - 2 ? len - 2 : (il < 0 ? 0 : il);
-        const double dy = y[il + 1] - y[il];
-        const double a = sl[il] * dx - dy, b = dy - sl[il + 1] * dx;
-        const double tl = (u - x[il]) / dx, tr = 1.0 - tl;
-        d = tr * y[il] + tl * y[il + 1] + tl * tr * (a * tr + b * tl);
+        const double dy = cell.yr - cell.yl;
+        const double a = cell.sl * dx - dy, b = dy - cell.sr * dx;
+        const double tl = (u - cell.xl) / dx, tr = 1.0 - tl;
+        d = tr * cell.yl + tl * cell.yr + tl * tr * (a * tr + b * tl);
     }
     return d > 0.0 ? (float) log((1.0 / rs.var) * d) : kNegInf;
 }
 
-__device__ __forceinline__ void emit_cell(const Ctx &c, const KmerConst32 &k, int32_t kid, const float4 &v,
-                                          double mean64, bool ok, float &em, float &ey) {
-    em = ey = kNegInf;
-    if (!ok) return;
-    if (c.hdp) {
-        em = ey = emit_hdp64(c.M->hdp64, kid, mean64, c.A->read_scale64[c.R.read]);
-    } else {
-        const Event32 e{v.x, v.y, v.z, v.w};
-        emit_gauss(k, e, c.rs, em, ey);
+// a chunk's anti-diagonals: lane k has the k-th one's band facts and first cell, and the chunk's ranges of
+// columns and rows
+struct ChunkRows {
+    int2 mt;
+    int32_t w, off;
+    int32_t xlo, xhi, ylo, yhi;
+};
+
+__device__ __forceinline__ ChunkRows chunk_rows(const Args &A, const Ctx &c, const Chunk &C) {
+    const int lane = threadIdx.x & 31;
+    ChunkRows r;
+    r.mt = lane < C.nd ? __ldg(A.meta + c.R.diag_base + C.d0 + lane) : make_int2(0, 0);
+    r.w = r.mt.y & kWidthMask;
+    int32_t off = r.w;   // inclusive prefix of the widths, then exclusive
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t t = __shfl_up_sync(0xffffffffu, off, o);
+        if (lane >= o) off += t;
+    }
+    r.off = off - r.w;
+    const int32_t dk = C.d0 + lane, Lk = r.mt.x, Rk = r.mt.x + 2 * (r.w - 1);
+    const bool in = lane < C.nd;
+    r.xlo = __reduce_min_sync(0xffffffffu, in ? (dk + Lk) >> 1 : INT32_MAX);
+    r.xhi = __reduce_max_sync(0xffffffffu, in ? (dk + Rk) >> 1 : INT32_MIN);
+    r.ylo = __reduce_min_sync(0xffffffffu, in ? (dk - Rk) >> 1 : INT32_MAX);
+    r.yhi = __reduce_max_sync(0xffffffffu, in ? (dk - Lk) >> 1 : INT32_MIN);
+    return r;
+}
+
+// The emissions of HDP machines' regions, column-stationary: a warp takes a chunk 64 columns at a time, a
+// lane keeps the rows and means of two in registers and has the table reads of both under way together.
+// What bounds it are those reads, at random places of a k-mer's 32 KB, and the latency of the FP64
+// divisions and logarithms around them, so it has few registers and little shared memory, for many warps
+// on an SM.  12 reads of 5 to 15 kb (3.1e7 cells): a cell after another, each behind its k-mer's row and
+// mean and the grid (four dependent reads, 20 warps an SM) 1.20 ms; four columns a lane (12 warps) 0.79 ms;
+// this way 0.67 ms.
+constexpr int kHdpCols = 2;
+__global__ void __launch_bounds__(32 * kEmitWarps, 5) emission_hdp_kernel(const __grid_constant__ Args A) {
+    __shared__ double means[kEmitWarps][kEmitSpan];
+    const int lane = threadIdx.x & 31;
+    double *mean = means[threadIdx.x >> 5];
+    const int64_t warps = (int64_t) gridDim.x * (blockDim.x >> 5);
+    for (int64_t ch = blockIdx.x * (int64_t) (blockDim.x >> 5) + (threadIdx.x >> 5); ch < A.n_chunks; ch += warps) {
+        const Chunk C = A.chunks[ch];
+        Ctx c;
+        ctx_init(c, A, C.region);
+        if (!c.hdp) continue;
+        const ChunkRows r = chunk_rows(A, c, C);
+        const Hdp64 h = c.M->hdp64;
+        const ReadScale64 rs = A.read_scale64[c.R.read];
+        const bool staged = r.yhi - r.ylo < kEmitSpan;   // else their means are read where they are
+        const auto *event = A.events_raw + c.R.event_base;
+        for (int q = lane; staged && q <= r.yhi - r.ylo; q += 32)
+            mean[q] = __ldg(event + clampi(r.ylo + q - 1, 0, max(c.R.lY - 1, 0))).x;
+        __syncwarp();
+        for (int32_t x0 = r.xlo + lane; x0 - lane <= r.xhi; x0 += 32 * kHdpCols) {
+            HdpRow row[kHdpCols];
+#pragma unroll
+            for (int q = 0; q < kHdpCols; ++q) {
+                const int32_t x = x0 + 32 * q;
+                row[q] = HdpRow{nullptr, nullptr, 0.0};
+                if (x <= r.xhi && x >= 1 && x <= c.R.lX) row[q] = hdp_row(h, __ldg(A.kmer + c.R.kmer_base + x - 1));
+            }
+            for (int k = 0; k < C.nd; ++k) {
+                const int32_t d = C.d0 + k;
+                const int32_t L = __shfl_sync(0xffffffffu, r.mt.x, k);
+                const int32_t W = __shfl_sync(0xffffffffu, r.w, k);
+                float2 *Ed = A.E + (C.cell + __shfl_sync(0xffffffffu, r.off, k));
+                const int32_t i0 = x0 - ((d + L) >> 1);   // the first column's cell
+                HdpCell cell[kHdpCols];
+                bool live[kHdpCols];
+#pragma unroll
+                for (int q = 0; q < kHdpCols; ++q) {
+                    const int32_t i = i0 + 32 * q, y = d - x0 - 32 * q;
+                    live[q] = i >= 0 && i < W && row[q].y && y >= 1 && y <= c.R.lY;
+                    if (live[q]) {
+                        hdp_knot(cell[q], staged ? mean[y - r.ylo] : __ldg(event + (y - 1)).x, row[q].mu, rs, h);
+                        hdp_read(cell[q], row[q]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < kHdpCols; ++q) {
+                    const int32_t i = i0 + 32 * q;
+                    if (i < 0 || i >= W) continue;
+                    const float e = live[q] ? hdp_value(cell[q], rs, h) : kNegInf;
+                    Ed[i] = make_float2(e, e);
+                }
+            }
+        }
+        __syncwarp();   // the means are rewritten by the warp's next chunk
     }
 }
 
+__device__ __forceinline__ void emit_cell(const Ctx &c, const KmerConst32 &k, const float4 &v, bool ok, float &em,
+                                          float &ey) {
+    em = ey = kNegInf;
+    if (ok) emit_gauss(k, Event32{v.x, v.y, v.z, v.w}, c.rs, em, ey);
+}
+
+// those of the other machines' regions
 __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_constant__ Args A) {
     __shared__ EmitStage stage[kEmitWarps];
     const int lane = threadIdx.x & 31;
@@ -483,27 +594,10 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
         const Chunk C = A.chunks[ch];
         Ctx c;
         ctx_init(c, A, C.region);
-        const int2 mt = lane < C.nd ? __ldg(A.meta + c.R.diag_base + C.d0 + lane) : make_int2(0, 0);
-        const int32_t w = mt.y & kWidthMask;
-        int32_t off = w;   // inclusive prefix of the widths, then exclusive
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t t = __shfl_up_sync(0xffffffffu, off, o);
-            if (lane >= o) off += t;
-        }
-        off -= w;
-        // column and row ranges of the chunk's cells, over all its anti-diagonals
-        int32_t xlo, xhi, ylo, yhi;
-        {
-            const int32_t dk = C.d0 + lane, Lk = mt.x, Rk = mt.x + 2 * (w - 1);
-            const bool in = lane < C.nd;
-            xlo = __reduce_min_sync(0xffffffffu, in ? (dk + Lk) >> 1 : INT32_MAX);
-            xhi = __reduce_max_sync(0xffffffffu, in ? (dk + Rk) >> 1 : INT32_MIN);
-            ylo = __reduce_min_sync(0xffffffffu, in ? (dk - Rk) >> 1 : INT32_MAX);
-            yhi = __reduce_max_sync(0xffffffffu, in ? (dk - Lk) >> 1 : INT32_MIN);
-        }
+        if (c.hdp) continue;
+        const auto [mt, w, off, xlo, xhi, ylo, yhi] = chunk_rows(A, c, C);
         const bool staged = xhi - xlo < kEmitSpan && yhi - ylo < kEmitSpan;
-        const bool by_column = staged && !c.hdp && xhi - xlo < 32 * kEmitCols;
+        const bool by_column = staged && xhi - xlo < 32 * kEmitCols;
         if (by_column) {
             // Gaussian emissions, column-stationary: lane l owns columns xlo + l + 32 q and keeps their
             // k-mer constants in registers for the whole chunk, so a cell reads only its event from
@@ -556,18 +650,16 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
                 const float4 ka = __ldg(kp), kb = __ldg(kp + 1);
                 st.kca[q] = ka;
                 st.kcb[q] = kb;
-                st.kid[q] = kid;
             }
             for (int q = lane; q <= yhi - ylo; q += 32) {
                 const int32_t y = ylo + q;
                 const int32_t yc = clampi(y - 1, 0, max(c.R.lY - 1, 0));
                 st.ev[q] = __ldg(reinterpret_cast<const float4 *>(A.events + c.R.event_base + yc));
-                if (c.hdp) st.mean[q] = __ldg(A.events_raw + c.R.event_base + yc).x;
             }
             __syncwarp();
         }
-        // every other chunk (HDP emissions, or a chunk spanning more than 128 columns or the stage's
-        // rows): a lane per cell of each anti-diagonal
+        // every other chunk (spanning more than 128 columns or the stage's rows): a lane per cell of each
+        // anti-diagonal
         for (int k = 0; k < (by_column ? 0 : C.nd); ++k) {
             const int32_t d = C.d0 + k;
             const int32_t L = __shfl_sync(0xffffffffu, mt.x, k);
@@ -580,8 +672,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
                 if (staged) {
                     const float4 ka = st.kca[x - xlo], kb = st.kcb[x - xlo];
                     const KmerConst32 kk{ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
-                    emit_cell(c, kk, st.kid[x - xlo], st.ev[y - ylo], c.hdp ? st.mean[y - ylo] : 0.0, ok,
-                              em, ey);
+                    emit_cell(c, kk, st.ev[y - ylo], ok, em, ey);
                 } else {
                     const int32_t kid = ok ? __ldg(A.kmer + c.R.kmer_base + x - 1) : 0;
                     const float4 *kp = reinterpret_cast<const float4 *>(c.M->kc + kid);
@@ -589,7 +680,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps) emission_kernel(const __grid_
                     const KmerConst32 kk{ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
                     const int32_t yc = clampi(y - 1, 0, max(c.R.lY - 1, 0));
                     const float4 v = __ldg(reinterpret_cast<const float4 *>(A.events + c.R.event_base + yc));
-                    emit_cell(c, kk, kid, v, c.hdp ? __ldg(A.events_raw + c.R.event_base + yc).x : 0.0, ok, em, ey);
+                    emit_cell(c, kk, v, ok, em, ey);
                 }
                 Ed[i] = make_float2(em, ey);
             }
