@@ -1,7 +1,13 @@
 """HDP emissions a group of 64 columns at a time: bands within a group, past it and past the staged means,
 grids of an odd and an even number of knots, k-mers without a row, a machine's own scaling, and a batch
-that mixes HDP and Gaussian machines; against the FP64 oracle, within what the batched form's other tests
-allow its FP32 arithmetic (posteriors 1e-4)."""
+that mixes HDP and Gaussian machines; against the FP64 oracle.
+
+Tolerance: the FP32 arithmetic's 1e-4, and one jump of the reference's logAdd.  At its cut-off its value
+drops by the cubic's excess over the argument, h = 4.5e-4, and FP32 arithmetic (differences good to about
+1e-5) can find itself on the other side of the cut-off than FP64 in a cell of a pair's path; that moves the
+cell's logarithm by h and the posterior by at most h.  The pairs themselves (those that differ by more than
+the tolerance from the threshold on either side) have to be the same.  These inputs give 1.2e-4 and less
+than 1.4e-4, bit for bit the same with the emissions computed a cell at a time."""
 import numpy as np
 import pytest
 
@@ -11,7 +17,9 @@ from signalalign_b200 import synth
 import workloads as W
 
 pytestmark = pytest.mark.gpu
-FP32_TOL = 1e-4
+# the cubic's last piece at the cut-off of 7.5, less 7.5
+CUTOFF_JUMP = ((-0.000458661602210 * 7.5 + 0.009695946122598) * 7.5 + 0.930734667215156) * 7.5 + 0.168037164329057 - 7.5
+FP32_TOL = 1e-4 + CUTOFF_JUMP
 
 
 @pytest.fixture(scope="module")
