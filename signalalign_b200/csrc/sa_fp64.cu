@@ -780,6 +780,7 @@ struct PlainSet {
     size_t p_bytes = 0;
     // resident route
     bool resident = false, expect = false, multi = false, finite_sx = false;
+    bool segments = false;       // as asked for, whichever route
     int nt = 128;
     int64_t n_windows = 0, n_totals = 0, n_chunks = 0, n_rows = 0, n_run_tasks = 0;
     int64_t term_stride = 1;
@@ -1385,6 +1386,13 @@ void plan_route(PlainSet *s, const sa_read *reads, size_t max_bytes) {
     s->resident = true;
 }
 
+// The set by rings after all, and whole regions where there are no pairs
+void plan_rings(PlainSet *s) {
+    s->resident = false;
+    plan_segments(s, s->segments && !s->expect);
+    plain_layout(s, nullptr, nullptr);
+}
+
 // Plans a set of reads for the plain form.  Reads that fail planning keep their status and get no
 // regions.  `max_bytes` bounds the device block (SA_E_CAPACITY above it).
 sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p, size_t max_bytes, PlainSet **out,
@@ -1455,14 +1463,12 @@ sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p
     s->cap = cap;
     s->expect = expect;
     if (!rings) plan_route(s, reads, max_bytes);
-    segments = segments || (expect && s->resident);
-    plan_segments(s, segments);
+    s->segments = segments;
+    plan_segments(s, segments || (expect && s->resident));
     plain_layout(s, nullptr, nullptr);
     if (s->resident && s->dev_bytes > std::min(kResidentBytes, max_bytes)) {
-        // more than the store may hold: the rings, and whole regions where there are no pairs
-        s->resident = false;
-        plan_segments(s, segments && !expect);
-        plain_layout(s, nullptr, nullptr);
+        // more than the store may hold
+        plan_rings(s);
     }
     if (s->dev_bytes > max_bytes) {
         delete s;
@@ -1475,6 +1481,11 @@ sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p
 // Device block, staged inputs and their upload (async on `stream`); models must be resident.
 sa_status plain_upload(PlainSet *s, cudaStream_t stream) {
     sa_status st = mem_get(MemKind::Device, s->device, s->dev_bytes, s->dev);
+    if (st == SA_E_NOMEM && s->resident && !s->expect) {
+        // no room for the store: the rings take a few MB a region
+        plan_rings(s);
+        st = mem_get(MemKind::Device, s->device, s->dev_bytes, s->dev);
+    }
     if (!st) st = mem_get(MemKind::Pinned, s->device, s->in_bytes, s->host_in);
     if (!st) st = mem_get(MemKind::Pinned, s->device, s->res_bytes, s->host_res);
     if (st) return st;
@@ -2141,7 +2152,9 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
     }
     mem_put(blk);
     cudaSetDevice(prev_dev);
+    const bool no_room = st == SA_E_NOMEM && s->resident;   // for the store: the rings take a few MB a region
     plain_destroy(s);
+    if (no_room) return expectations_batch(reads, n, p, ex, read_status, true);
     for (int64_t i : again)
         if (!st) st = expectations_batch(reads + i, 1, p, ex + i, read_status + i, true);
     return st;

@@ -92,3 +92,49 @@ def test_expectations(api, expansion, repeat):
     np.testing.assert_allclose(got["posteriors"], want["posteriors"], rtol=1e-9)
     np.testing.assert_allclose(got["event_expectations"], want["event_expectations"], rtol=1e-9, atol=1e-9)
     assert np.array_equal(got["observed"], want["observed"])
+
+
+_NO_ROOM = """
+import numpy as np, torch
+from signalalign_b200 import api, synth
+import workloads as W
+from oracle import oracle as orc
+cfg = synth.config1(seed=321, n_reads=1, span=(20000, 20000))
+rd, m = cfg["reads"][0], W.gaussian_model(cfg)
+sm = W.gpu_model(api, m, orc.EMIT_DESCALED, rd)
+p = api.pairwiseAlignmentBandingParameters_construct(diagonal_expansion=50)
+def call(bases, events):
+    before = api.kernel_launch_count()
+    anchors = rd["anchors"][(rd["anchors"][:, 0] < bases - 9) & (rd["anchors"][:, 1] < events - 3)]
+    got = api.getAlignedPairsUsingAnchors(sm, rd["reference"][:bases], rd["events"][:events], anchors, p)
+    return got, api.kernel_launch_count() - before
+def expect():
+    return api.getExpectationsUsingAnchors(sm, rd["reference"], rd["events"], rd["anchors"], p)
+api.set_segment_policy(-1, 1024)           # one ring a read
+call(400, 600)                             # the machine's tables
+free = torch.cuda.mem_get_info()[0]
+held = torch.empty(free - (100 << 20), dtype=torch.uint8, device="cuda")
+(rings, few), e_rings = call(20000, len(rd["events"])), expect()
+del held
+torch.cuda.empty_cache()
+(resident, more), e_resident = call(20000, len(rd["events"])), expect()
+assert few < more, (few, more)
+assert len(rings) == len(resident) > 10000
+for f in ("x", "y", "kmer"):
+    assert np.array_equal(rings[f], resident[f]), f
+assert np.abs(rings["score"] - resident["score"]).max() <= 100     # posteriors 1e-5
+np.testing.assert_allclose(e_rings["transitions"], e_resident["transitions"], rtol=1e-6)
+print("ok", few, more)
+"""
+
+
+def test_no_room_for_the_store(api):
+    """A device without room for the resident store (256 MB for this read) runs the rings, in a process
+    of its own: blocks that other calls left for reuse would be room."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "tests")]))
+    got = subprocess.run([sys.executable, "-c", _NO_ROOM], env=env, capture_output=True, text=True, timeout=600)
+    assert got.returncode == 0 and got.stdout.startswith("ok"), got.stdout + got.stderr
