@@ -1319,8 +1319,7 @@ void plan_resident(const sa_state_machine *sm, PlainRegion &pr) {
     }
 }
 
-// Forward segments (alignment runs, and expectations on the resident route): long regions cut at
-// window starts like the batched form's, the automatic cap from twice the set's anti-diagonals per
+// Forward segments (alignment runs): long regions cut at window starts like the batched form's, the automatic cap from twice the set's anti-diagonals per
 // CTA slot (four plain CTAs per SM)
 void plan_segments(PlainSet *s, bool segments) {
     int32_t policy = -1, warm0 = 1024;
@@ -1386,10 +1385,10 @@ void plan_route(PlainSet *s, const sa_read *reads, size_t max_bytes) {
     s->resident = true;
 }
 
-// The set by rings after all, and whole regions where there are no pairs
+// The set by rings after all
 void plan_rings(PlainSet *s) {
     s->resident = false;
-    plan_segments(s, s->segments && !s->expect);
+    plan_segments(s, s->segments);
     plain_layout(s, nullptr, nullptr);
 }
 
@@ -1464,7 +1463,7 @@ sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p
     s->expect = expect;
     if (!rings) plan_route(s, reads, max_bytes);
     s->segments = segments;
-    plan_segments(s, segments || (expect && s->resident));
+    plan_segments(s, segments);
     plain_layout(s, nullptr, nullptr);
     if (s->resident && s->dev_bytes > std::min(kResidentBytes, max_bytes)) {
         // more than the store may hold
@@ -1890,7 +1889,7 @@ extern "C" sa_status sa_getAlignedPairsUsingAnchors(const sa_state_machine *sm_c
 struct ExpectPlan {
     std::vector<Kmer64> kmers;
     std::vector<Column64> cols;
-    std::vector<int64_t> read_chunk, read_task;   // per running read its first chunk and task, and the ends
+    std::vector<int64_t> read_chunk;   // per running read its first chunk, and the end
     std::vector<int32_t> first;                   // per region the first region of its read
     bool hdp = false;
 };
@@ -1898,17 +1897,13 @@ struct ExpectPlan {
 static void plan_expectations(const PlainSet *s, const sa_read *reads, const std::vector<int64_t> &run, ExpectPlan &E) {
     E.first.resize(s->regs.size());
     for (size_t r = 0; r < s->regs.size(); ++r) E.first[r] = (int32_t) s->read_first[s->regs[r].read];
-    int64_t chunks = 0, tasks = 0;
+    int64_t chunks = 0;
     std::vector<int32_t> at, dlo, dhi;
     for (size_t j = 0; j < run.size(); ++j) {
         const int64_t i = run[j];
         E.read_chunk.push_back(chunks);
-        E.read_task.push_back(tasks);
         const int64_t r0 = s->read_first[i], r1 = r0 + s->read_count[i];
-        for (int64_t r = r0; r < r1; ++r) {
-            chunks += (s->regs[r].rg.lX + s->regs[r].rg.lY + 32) / 32;
-            tasks += 1 + (int64_t) s->regs[r].cuts.size();
-        }
+        for (int64_t r = r0; r < r1; ++r) chunks += (s->regs[r].rg.lX + s->regs[r].rg.lY + 32) / 32;
         if (reads[i].sm->emission == SA_EMIT_HDP) {
             E.hdp = true;
             continue;
@@ -1938,7 +1933,6 @@ static void plan_expectations(const PlainSet *s, const sa_read *reads, const std
         }
     }
     E.read_chunk.push_back(chunks);
-    E.read_task.push_back(tasks);
 }
 
 // Expectations of many reads: on the resident route every read's sweeps side by side and its
@@ -2026,12 +2020,10 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
     const size_t o_kmers = total; total += up(sizeof(Kmer64) * E.kmers.size());
     const size_t o_cols = total; total += up(sizeof(Column64) * E.cols.size());
     const size_t o_rchunk = total; total += up(sizeof(int64_t) * E.read_chunk.size());
-    const size_t o_rtask = total; total += up(sizeof(int64_t) * E.read_task.size());
     const size_t o_first = total; total += up(sizeof(int32_t) * E.first.size());
     const size_t staged = total;
     const size_t o_partial = total; total += s->resident ? up(sizeof(double) * 9 * (size_t) s->n_chunks) : 0;
     std::vector<unsigned char> host(staged, 0);
-    std::vector<int64_t> again;
     MemBlock blk;
     st = plain_upload(s, nullptr);
     if (!st) st = mem_get(MemKind::Device, s->device, total, blk);
@@ -2070,7 +2062,6 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
         put(o_kmers, E.kmers.data(), sizeof(Kmer64) * E.kmers.size());
         put(o_cols, E.cols.data(), sizeof(Column64) * E.cols.size());
         put(o_rchunk, E.read_chunk.data(), sizeof(int64_t) * E.read_chunk.size());
-        put(o_rtask, E.read_task.data(), sizeof(int64_t) * E.read_task.size());
         put(o_first, E.first.data(), sizeof(int32_t) * E.first.size());
         SetOut O;
         std::memset(&O, 0, sizeof(O));
@@ -2081,10 +2072,6 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
             st = SA_E_CUDA;
         const auto *X = reinterpret_cast<const ExpectOut *>(d + o_xs);
         if (!st && s->resident) {
-            O.stitch = s->d_stitch;
-            O.stres = s->d_stres;
-            O.fail = s->d_fail;
-            O.stitch_tol = s->stitch_tol;
             auto *partial = reinterpret_cast<double *>(d + o_partial);
             st = resident_sweeps(s, O, nullptr);
             if (!st) {
@@ -2094,9 +2081,7 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
                     kmers64<<<(unsigned) ((E.kmers.size() + 3) / 4), 128>>>(
                         s->d_models, s->d_regions, reinterpret_cast<const Kmer64 *>(d + o_kmers), (int64_t) E.kmers.size(),
                         reinterpret_cast<const Column64 *>(d + o_cols), X);
-                finish64<<<(unsigned) run.size(), 256>>>(X, reinterpret_cast<const int64_t *>(d + o_rchunk), partial,
-                                                        s->d_tasks, reinterpret_cast<const int64_t *>(d + o_rtask),
-                                                        s->d_stres);
+                finish64<<<(unsigned) run.size(), 256>>>(X, reinterpret_cast<const int64_t *>(d + o_rchunk), partial);
                 count_launch(E.kmers.empty() ? 2 : 3);
                 if (cudaGetLastError() != cudaSuccess) st = SA_E_CUDA;
             }
@@ -2115,18 +2100,10 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
         if (!st && cudaMemcpy(host.data(), d, o_xs, cudaMemcpyDeviceToHost) != cudaSuccess) st = SA_E_CUDA;
         if (!st) {
             const auto *res = static_cast<const unsigned char *>(s->host_res.ptr);
-            const auto *fail = reinterpret_cast<const int32_t *>(res + s->res_fail);
             const auto *counts = reinterpret_cast<const int64_t *>(res + s->res_region_count);
             for (size_t j = 0; j < run.size(); ++j) {
                 const int64_t i = run[j];
                 const Off &o = off[j];
-                bool agreed = true;   // a read with a disagreeing stitch: again, whole, from its accumulators
-                for (int64_t r = s->read_first[i]; s->resident && r < s->read_first[i] + s->read_count[i]; ++r)
-                    agreed = agreed && !fail[r];
-                if (!agreed) {
-                    again.push_back(i);
-                    continue;
-                }
                 const auto *acc = reinterpret_cast<const double *>(host.data() + o.acc);
                 ex[i].likelihood = acc[0];
                 for (int k = 0; k < 9; ++k) ex[i].transitions[k] = acc[k + 1];
@@ -2154,10 +2131,7 @@ static sa_status expectations_batch(const sa_read *reads, int64_t n, const sa_pa
     cudaSetDevice(prev_dev);
     const bool no_room = st == SA_E_NOMEM && s->resident;   // for the store: the rings take a few MB a region
     plain_destroy(s);
-    if (no_room) return expectations_batch(reads, n, p, ex, read_status, true);
-    for (int64_t i : again)
-        if (!st) st = expectations_batch(reads + i, 1, p, ex + i, read_status + i, true);
-    return st;
+    return no_room ? expectations_batch(reads, n, p, ex, read_status, true) : st;
 }
 
 extern "C" sa_status sa_getExpectationsUsingAnchors(const sa_state_machine *sm_c, const char *reference,

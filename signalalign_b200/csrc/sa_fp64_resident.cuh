@@ -17,7 +17,7 @@
 // column's previous value is in a register and its neighbours' are one shared-memory read away; the
 // operands come by asynchronous copy kAhead64 anti-diagonals ahead; and a step's log_adds are
 // independent.  Windows run side by side, and logarithms, exponentials, totals and outputs are off the
-// sweeps' chain.  Measured on B200: see the dispatch rule in plain_create.
+// sweeps' chain.  Measured on B200: see the rule in plan_route.
 //
 // A slot not in the band holds log 0 for that anti-diagonal, so an absent neighbour drops out of
 // log_add.  No two paths of three consecutive anti-diagonals share a thread: the host takes this
@@ -1204,10 +1204,8 @@ __global__ void __launch_bounds__(128) kmers64(const Model64 *models, const Regi
     }
 }
 
-// A read's likelihood and transition expectations from its blocks' sums, a CTA per read.  Anti-diagonals
-// a later segment swept have their totals in its frame: the stitches' constants bring them back.
-__global__ void __launch_bounds__(256) finish64(const ExpectOut *XS, const int64_t *read_chunk, const double *partial,
-                                                const Region64 *tasks, const int64_t *read_task, const Stitch64Res *stres) {
+// A read's likelihood and transition expectations from its blocks' sums, a CTA per read.
+__global__ void __launch_bounds__(256) finish64(const ExpectOut *XS, const int64_t *read_chunk, const double *partial) {
     __shared__ double sums[8][9];
     const ExpectOut &X = XS[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1227,12 +1225,6 @@ __global__ void __launch_bounds__(256) finish64(const ExpectOut *XS, const int64
     for (int j = 0; j < 9; ++j) {
         acc[j] = 0.0;
         for (int w = 0; w < 8; ++w) acc[j] += sums[w][j];
-    }
-    double delta = 0.0;
-    for (int64_t t = read_task[blockIdx.x]; t < read_task[blockIdx.x + 1]; ++t) {
-        const Region64 &R = tasks[t];
-        delta = R.st_in >= 0 ? delta + stres[R.st_in].delta : 0.0;
-        if (R.st_in >= 0) acc[8] += delta * (double) (R.win[R.w1 - 1].from - R.win[R.w0].T);
     }
     X.acc[0] += acc[8];
     constexpr int to[8] = {S_M * 3 + S_X, S_X * 3 + S_X, S_Y * 3 + S_X, S_M * 3 + S_M,

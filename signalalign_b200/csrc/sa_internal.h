@@ -202,8 +202,7 @@ bool batch_run_events(const sa_batch *b, cudaEvent_t *start, cudaEvent_t *end);
 // for reads whose references have degenerate ('X') positions.
 struct PlainSet;
 // segments: cut long regions into forward segments (alignment runs; not the expectations mode)
-// expect: for getExpectations (no pairs; forward segments only on the resident route); rings: not the
-// resident route
+// expect: for getExpectations (no pairs); rings: not the resident route
 sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p, size_t max_bytes, PlainSet **out,
                        bool segments = false, bool expect = false, bool rings = false);
 // scale of the set's stitch tolerance (negative: every stitch disagrees and its region re-runs whole)
