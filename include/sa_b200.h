@@ -277,7 +277,7 @@ sa_status sa_batch_set_wait_limit(sa_batch *b, int64_t cycles);
  * posteriors do not depend on the constant, and the log-likelihood adds it back.  A read whose
  * check disagrees is re-run unsegmented at download, so results never depend on it.
  * segment_diags: < 0 keeps every region whole; > 0 caps a segment's sweep (warm-up included);
- * 0 (default) picks twice the batch's forward anti-diagonals per worker CTA, at least 4096 (a large
+ * 0 (default) picks twice the batch's forward anti-diagonals per worker CTA, at least 2800 (a large
  * batch, bound by its total work, then keeps nearly every region whole; a small one splits).
  * warmup_diags: default 1024, at least 64.  Applies to batches created afterwards. */
 sa_status sa_setSegmentPolicy(int32_t segment_diags, int32_t warmup_diags);

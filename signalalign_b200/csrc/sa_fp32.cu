@@ -334,10 +334,15 @@ int planning_threads() {
 // chain and its total work (forward and traceback-window work per anti-diagonal together cost about
 // twice a worker CTA's forward step, measured on B200), so only chains longer than the total work
 // are cut: a large batch keeps nearly every region whole (no warm-up overhead), a small one (a
-// serving micro-batch) splits its long reads for latency.
+// serving micro-batch) splits its long reads for latency.  kSegMin: shorter pieces shorten the longest
+// chain and add warm-up work, 1,050 anti-diagonals a piece at expansion 50.  Run and download on B200 at
+// 4,096 / 2,900 / 2,600 / 2,300: one 10 kb read 1.23 / 0.94 / 0.93 / 0.93 ms, 20 reads of 8 to 12 kb 3.51 /
+// 3.28 / 3.22 / 3.18, 8 of them 1.86 / 1.83 / 1.81 / 1.97, 12 HDP reads of 5 to 15 kb 3.12 / 2.96 / 2.98 /
+// 2.99, 8 reads at expansion 20 1.76 / 1.66 / 1.67 / 1.69, 10 reads with sites (FP64) 3.90 / 3.44 / 3.30 /
+// 3.34.  At expansion 200 the warm-up alone is 4,010, and plan_cuts lets no piece own less than that.
 std::atomic<int32_t> g_seg_target{0};
 std::atomic<int32_t> g_seg_warm{1024};
-constexpr int64_t kSegMin = 4096;
+constexpr int64_t kSegMin = 2800;
 
 // Warm-up of a region's later segments: the start's influence dies out over a few band widths
 // (measured on the oracle's FP64 sweep: within 4.2 widths at diagonal expansion 50, 5.9 at 200), so
