@@ -343,6 +343,9 @@ int planning_threads() {
 std::atomic<int32_t> g_seg_target{0};
 std::atomic<int32_t> g_seg_warm{1024};
 constexpr int64_t kSegMin = 2800;
+// The no-allocation entry's: more pieces have more stitches, and what fits its scratch has to fit still.  Its
+// short reads gain nothing (five of 300 to 1,500 bp 1.29 ms either way).
+constexpr int64_t kSegMinNoAlloc = 4096;
 
 // Warm-up of a region's later segments: the start's influence dies out over a few band widths
 // (measured on the oracle's FP64 sweep: within 4.2 widths at diagonal expansion 50, 5.9 at 200), so
@@ -507,7 +510,7 @@ sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, 
             }
             if (sms <= 0) sms = 148;
             const int64_t slots = (int64_t) sms * std::max(1, launch_for(std::max(device, 0), wc).ctas_per_sm);
-            target = std::max<int64_t>(kSegMin, 2 * fwd_diags / slots);
+            target = std::max<int64_t>(pinned ? kSegMin : kSegMinNoAlloc, 2 * fwd_diags / slots);
         }
         for (int64_t r = 0; r < n_reads; ++r) {
             ReadPlan &rp = plan[r];
@@ -759,7 +762,9 @@ Args batch_args(const sa_batch *b) {
 
 // The persistent worker over a.n_segs forward segments and a.n_windows windows: column-resident CTAs of
 // 128, 256 or 512 columns where the bands fit them, the CTA form for other bands and for launch
-// configurations that ask for it.
+// configurations that ask for it.  Narrower CTAs leave room for more of them; a band takes the first it
+// fits.  The CTA form / columns on B200: 256 reads at expansion 50 (128 threads) 18.8 / 13.1 ms, 6 reads of 3
+// to 8 kb at expansion 200 (512 threads) 6.8 / 3.0.
 void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
     auto launch = [&](auto kern, int threads, size_t smem) {
         int per_sm = 0;

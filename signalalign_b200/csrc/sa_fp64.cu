@@ -1358,9 +1358,10 @@ void plan_segments(PlainSet *s, bool segments) {
 // The resident route for sets whose bands fit its threads (the paths of three consecutive
 // anti-diagonals, and a path's neighbours beyond them, on threads of their own) and, in plain_create,
 // whose store fits kResidentBytes.  Both sides measured on B200, whole call, rings
-// then resident: one 1 kb read 14.0 and 2.1 ms, one 3 kb read with sites 29.4 and 3.8, ten reads of
-// 1 to 10 kb with sites 48 and 5.6, the expectations of six reads of 1 to 5 kb 222 and 6.0.
-// The rings stay for wider bands, for larger sets, and for regions re-run whole.
+// then resident: one 1 kb read 14.6 and 1.08 ms, one 3 kb read with sites 29.8 and 2.05, ten reads of
+// 1 to 10 kb with sites 47 and 3.4, the expectations of six reads of 1 to 5 kb 221 and 6.4.
+// The rings stay for wider bands, for larger sets, where the device has no room for the store, and for
+// regions re-run whole.
 void plan_route(PlainSet *s, const sa_read *reads, size_t max_bytes) {
     int32_t span = 0, paths = 1;
     int64_t slots = 0;

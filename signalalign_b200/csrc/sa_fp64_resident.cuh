@@ -6,7 +6,7 @@
 //   backward64  a CTA per traceback window, a path per thread: stores the match value of every slot, and
 //               what the total probabilities need
 //   totals64    a warp per total probability (the reference's sequential folds)
-//   posterior pairs: count64, scan64, place64, write64, in the reference's order; or, in
+//   posterior pairs: outputs64 (counts), scan64, place64, outputs64, in the reference's order; or, in
 //   expectations mode, transitions64, kmers64 and finish64 (and the HDP machine's assignments with
 //   the pairs' kernels)
 //
