@@ -433,7 +433,7 @@ def run_saturate(args):
             "reads_per_sec": len(reads) / (t / 1e3), "read_errors": bad,
             "kernels_ms": {"emission_kernel": statistics.mean(k[0] for k in kern), "worker_kernel": wk,
                            "gather_pairs": statistics.mean(k[2] for k in kern)},
-            "roofline": {"kernel": "worker_kernel", "bound": "fp32", "achieved": achieved, "peak": peak,
+            "roofline": {"kernel": "column_worker", "bound": "fp32", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak}}
     print(json.dumps(line), flush=True)
 
@@ -813,9 +813,9 @@ def main():
                                 "kernels)",
                         "sequential": {"value": e2e_seq_value, "ms_per_step": float(te.item()),
                                        "mode": "one synchronous sa_align_batch call per step"}},
-                "plain_fp64": {"value": plain_value, "unit": UNIT, "sample": "%d reads, one launch per read" % len(sample),
+                "plain_fp64": {"value": plain_value, "unit": UNIT, "sample": "%d reads, one call per read" % len(sample),
                                "batched_over_plain": value / world / plain_value},
-                "roofline": {"kernel": "worker_kernel", "bound": "fp32", "achieved": achieved, "peak": peak,
+                "roofline": {"kernel": "column_worker", "bound": "fp32", "achieved": achieved, "peak": peak,
                              "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic,
                              "kernel_ms": wk_ms,
                              "note": "%.0f FP32 FLOP per band cell (transitions of both sweeps + posterior; "
