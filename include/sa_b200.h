@@ -238,7 +238,8 @@ sa_status sa_batch_kernel_ms(const sa_batch *b, double *emission_ms, double *wor
 typedef struct {
     int32_t ctas_per_sm;           /* worker CTAs per SM (at most the kernel's occupancy; default 2) */
     int32_t grid_per_region;       /* worker grid at most this many CTAs per region (default 3) */
-    int32_t warp_windows;          /* class 1: a traceback window per warp (1, default) or per CTA (0) */
+    int32_t warp_windows;          /* columns resident on threads where the band fits (1, default), or
+                                    * cells by their place in the band (0) */
     int32_t emission_ctas_per_sm;  /* emission kernel grid, CTAs per SM (default 16) */
 } sa_launch_config;
 

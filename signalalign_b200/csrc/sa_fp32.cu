@@ -92,8 +92,9 @@ std::mutex g_launch_mutex;
 std::map<std::pair<std::string, int>, sa_launch_config> g_launch;   // (device name, width class)
 
 // the choices measured on B200: two worker CTAs per SM, at most three CTAs per region (a forward CTA
-// and about two CTAs of window warps, so small batches on other streams run beside it), a window
-// per warp for bands up to 128 cells, 16 emission CTAs per SM
+// and two for windows: more contend with the forward sweeps for issue slots, 8 served reads at 2 / 4 / 8 a
+// region 1.88 / 2.20 / 2.55 ms, 6 reads at expansion 200 at 1 / 2 / 3 / 4 5.5 / 3.8 / 3.6 / 3.6), columns
+// resident on threads, 16 emission CTAs per SM
 sa_launch_config default_launch() { return sa_launch_config{2, 3, 1, 16}; }
 
 bool valid_launch(const sa_launch_config &c) {

@@ -3,8 +3,8 @@
 //   1. emission_kernel: the match and extra-event emissions of every band cell, written to the
 //      emission store.  Fully parallel (a warp per run of 32 anti-diagonals); it takes the
 //      Gaussian / HDP density work off the sequential sweeps.
-//   2. column_worker (sa_fp32_columns.cuh; bands up to about 124 columns) or worker_kernel (wider
-//      bands): persistent CTAs of 128 threads pull tasks from one device counter.  The first
+//   2. column_worker (sa_fp32_columns.cuh; bands up to 510 columns) or worker_kernel (wider
+//      bands): persistent CTAs pull tasks from one device counter.  The first
 //      claims are forward segments (longest first); every later claim is a slot of a ready queue of
 //      traceback windows.  A forward segment sweeps a run of a region's anti-diagonals (the whole
 //      region, or a piece of a long one; see Segment) anti-diagonal by anti-diagonal (cells spread
@@ -1568,8 +1568,8 @@ __device__ void read_unit_done(const Args &A, int32_t r, int tid, Shared *sh) {
 
 // CPT: cells per thread (128 threads per region).  The first claims are forward sweeps, one per CTA;
 // once none is left, windows are claimed, one per CTA.  MINB: CTAs per SM the registers are budgeted
-// for.  Serves the batches column_worker cannot take, and launch configurations without a window per
-// warp.
+// for.  Serves the batches column_worker cannot take, and launch configurations that ask for the
+// CTA form.
 template <int CPT, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) worker_kernel(const __grid_constant__ Args A) {
     extern __shared__ float4 smem_raw[];
