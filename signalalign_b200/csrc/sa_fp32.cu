@@ -340,10 +340,14 @@ int planning_threads() {
 // 4,096 / 2,900 / 2,600 / 2,300: one 10 kb read 1.23 / 0.94 / 0.93 / 0.93 ms, 20 reads of 8 to 12 kb 3.51 /
 // 3.28 / 3.22 / 3.18, 8 of them 1.86 / 1.83 / 1.81 / 1.97, 12 HDP reads of 5 to 15 kb 3.12 / 2.96 / 2.98 /
 // 2.99, 8 reads at expansion 20 1.76 / 1.66 / 1.67 / 1.69, 10 reads with sites (FP64) 3.90 / 3.44 / 3.30 /
-// 3.34.  At expansion 200 the warm-up alone is 4,010, and plan_cuts lets no piece own less than that.
+// 3.34.
+// A region whose warm-up leaves a floor of 2,800 no room (bands of 274 cells and more) has the floor of wide
+// bands: without one it would not be cut at all.  Whole / cut at 4,096: 4 reads of 2 to 10 kb at expansion 300
+// 7.85 / 4.18 ms, 4 reads of 5 to 19 kb with sites there (FP64) 1,214 / 232.
 std::atomic<int32_t> g_seg_target{0};
 std::atomic<int32_t> g_seg_warm{1024};
 constexpr int64_t kSegMin = 2800;
+constexpr int64_t kSegMinWide = 4096;
 // The no-allocation entry's: more pieces have more stitches, and what fits its scratch has to fit still.  Its
 // short reads gain nothing (five of 300 to 1,500 bp 1.29 ms either way).
 constexpr int64_t kSegMinNoAlloc = 4096;
@@ -353,6 +357,9 @@ constexpr int64_t kSegMinNoAlloc = 4096;
 // ten widths of the region's widest anti-diagonal, and at least the policy's warm-up.
 int32_t region_warm(const Region &rg, int32_t warm) { return std::max<int32_t>(warm, 10 * rg.max_width); }
 
+// a cap has to leave this much after the warm-up
+constexpr int64_t kSegSlack = 64;
+
 // Window indices (>= 1) whose T starts a new segment of region rg: k pieces of about equal sweep
 // time (L + warm each; the first piece owns L + warm anti-diagonals and needs no warm-up, and L is
 // at least warm), each cut at the first window start at or after its ideal place, none leaving less
@@ -360,7 +367,7 @@ int32_t region_warm(const Region &rg, int32_t warm) { return std::max<int32_t>(w
 void plan_cuts(const Region &rg, int64_t target, int32_t warm, std::vector<int32_t> &cuts) {
     cuts.clear();
     const int64_t n = rg.lX + rg.lY;
-    if (target <= (int64_t) warm + 64 || n <= target) return;
+    if (target <= (int64_t) warm + kSegSlack || n <= target) return;
     // pieces: sweeps of at most `target`, and none owning fewer anti-diagonals than its warm-up
     const int64_t k = std::min((n - warm + (target - warm) - 1) / (target - warm), (n - warm) / warm);
     if (k < 2) return;
@@ -373,6 +380,11 @@ void plan_cuts(const Region &rg, int64_t target, int32_t warm, std::vector<int32
         cuts.push_back((int32_t) j);
         ++j;
     }
+}
+
+// the automatic cap of one region, from the batch's
+int64_t region_cap(int64_t target, int32_t warm) {
+    return target <= (int64_t) warm + kSegSlack ? std::max(target, kSegMinWide) : target;
 }
 
 // one read's plan before packing
@@ -518,7 +530,8 @@ sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, 
             rp.cuts.assign(rp.regs.size(), {});
             for (size_t gi = 0; gi < rp.regs.size(); ++gi) {
                 const Region &rg = rp.regs[gi];
-                if (policy >= 0) plan_cuts(rg, target, region_warm(rg, warm), rp.cuts[gi]);
+                const int32_t wr = region_warm(rg, warm);
+                if (policy >= 0) plan_cuts(rg, policy == 0 ? region_cap(target, wr) : target, wr, rp.cuts[gi]);
                 rp.segs += 1 + (int64_t) rp.cuts[gi].size();
                 rp.stitches += (int64_t) rp.cuts[gi].size();
                 for (int32_t j : rp.cuts[gi]) {
@@ -1345,6 +1358,7 @@ void segment_policy(int32_t &target, int32_t &warm) {
     warm = g_seg_warm.load();
 }
 int64_t segment_min() { return kSegMin; }
+int64_t segment_cap(int64_t target, int32_t warm) { return region_cap(target, warm); }
 int32_t segment_warm(const Region &rg, int32_t warm) { return region_warm(rg, warm); }
 void segment_cuts(const Region &rg, int64_t target, int32_t warm, std::vector<int32_t> &cuts) {
     plan_cuts(rg, target, warm, cuts);

@@ -1345,7 +1345,7 @@ void plan_segments(PlainSet *s, bool segments) {
         pr.warm = 0;
         if (segments && policy >= 0) {
             const int32_t wr = segment_warm(pr.rg, warm0);
-            segment_cuts(pr.rg, target, wr, pr.cuts);
+            segment_cuts(pr.rg, policy == 0 ? segment_cap(target, wr) : target, wr, pr.cuts);
             pr.warm = wr;
         }
         s->task_first[i] = s->n_tasks;

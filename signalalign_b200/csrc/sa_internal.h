@@ -156,9 +156,11 @@ sa_status mem_get(MemKind kind, int device, size_t bytes, MemBlock &out);
 void mem_put(MemBlock &b);
 
 // forward-segment planning shared by both forms (sa_fp32.cu): the policy (cap, -1 off, 0 automatic;
-// warm-up), the automatic cap's floor, a region's warm-up and its cuts (window indices)
+// warm-up), the automatic cap's floor, one region's automatic cap from the batch's, a region's warm-up
+// and its cuts (window indices)
 void segment_policy(int32_t &target, int32_t &warm);
 int64_t segment_min();
+int64_t segment_cap(int64_t target, int32_t warm);
 int32_t segment_warm(const Region &rg, int32_t warm);
 void segment_cuts(const Region &rg, int64_t target, int32_t warm, std::vector<int32_t> &cuts);
 
