@@ -982,7 +982,8 @@ sa_status sa_batch_run(sa_batch *b, void *stream) {
         if (timing) cudaEventRecord(b->ev[0], s);
         const auto grid = (unsigned) std::max<int64_t>(1, std::min<int64_t>((int64_t) sms * cfg.emission_ctas_per_sm,
                                                                             (a.n_chunks + kEmitWarps - 1) / kEmitWarps));
-        if (b->any_gaussian) emission_kernel<<<grid, 32 * kEmitWarps, 0, s>>>(a);
+        const size_t room = b->max_width > kEmitWide ? kEmitRoom : 0;
+        if (b->any_gaussian) emission_kernel<<<grid, 32 * kEmitWarps, room, s>>>(a);
         if (b->any_hdp) emission_hdp_kernel<<<grid, 32 * kEmitWarps, 0, s>>>(a);
         if (timing) cudaEventRecord(b->ev[1], s);
         launch_worker(b, a, cfg, sms, s);

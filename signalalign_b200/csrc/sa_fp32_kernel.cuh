@@ -427,6 +427,13 @@ __device__ __forceinline__ void ring_init(float *base, int wmax) {
 constexpr int kEmitWarps = 4;
 constexpr int kEmitSpan = 192;
 constexpr int kEmitCols = 4;   // column slots per lane of the column-stationary Gaussian path
+// Chunks past the stage read constants and events through L1, which has what the CTAs' shared memory
+// leaves.  Six CTAs an SM leave it next to nothing, five a quarter of an SM's: batches with bands wider
+// than kEmitWide (their chunks drift by about half their anti-diagonals) launch with kEmitRoom bytes a CTA
+// they do not use, which makes it five.  64 reads of 2 to 10 kb, without / with: width 168 0.46 / 0.47 ms,
+// 188 1.07 / 0.95, 208 1.65 / 1.36, 254 2.71 / 1.86, 358 3.94 / 2.71, 508 5.75 / 3.83; width 108 0.22 / 0.24.
+constexpr int kEmitWide = kEmitSpan - kChunkDiags / 2;
+constexpr size_t kEmitRoom = 2048;
 // The k-mer constants are staged as two float4 halves in separate arrays: lanes reading consecutive
 // columns then load 16-byte strides, which shared memory serves without bank conflicts (32-byte
 // records would put two lanes on every bank group).
