@@ -777,8 +777,10 @@ Args batch_args(const sa_batch *b) {
 // The persistent worker over a.n_segs forward segments and a.n_windows windows: column-resident CTAs of
 // 128, 256 or 512 columns where the bands fit them, the CTA form for other bands and for launch
 // configurations that ask for it.  Narrower CTAs leave room for more of them; a band takes the first it
-// fits.  The CTA form / columns on B200: 256 reads at expansion 50 (128 threads) 18.8 / 13.1 ms, 6 reads of 3
-// to 8 kb at expansion 200 (512 threads) 6.8 / 3.0.
+// fits, its last two columns with the sweeps compiled for that.  The CTA form / columns on B200: 256 reads
+// at expansion 50 (128 threads) 18.8 / 13.1 ms, 6 reads of 3 to 8 kb at expansion 200 (512 threads) 6.8 / 3.0.
+// The next wider CTA / full columns: 256 reads of 2 to 10 kb with a span of 128 12.1 / 7.5 ms, of 256 28.6 /
+// 12.8, 128 reads with a span of 512 (the CTA form) 23.6 / 16.6.
 void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
     auto launch = [&](auto kern, int threads, size_t smem) {
         int per_sm = 0;
@@ -789,10 +791,13 @@ void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg
                                                                     (int64_t) cfg.grid_per_region * a.n_segs));
         kern<<<(unsigned) grid, (unsigned) threads, smem, s>>>(a);
     };
-    if (cfg.warp_windows && b->max_span <= column_span(512)) {
-        if (b->max_span <= column_span(128)) launch(column_worker<128, 3>, 128 + kHelpers, sizeof(ColumnShared<128>));
-        else if (b->max_span <= column_span(256)) launch(column_worker<256, 2>, 256 + kHelpers, sizeof(ColumnShared<256>));
-        else launch(column_worker<512, 1>, 512 + kHelpers, sizeof(ColumnShared<512>));
+    auto columns = [&](auto plain, auto full, int nt, size_t smem) {
+        launch(b->max_span <= column_span(nt) ? plain : full, nt + kHelpers, smem);
+    };
+    if (cfg.warp_windows && b->max_span <= 512) {
+        if (b->max_span <= 128) columns(column_worker<128, 3, false>, column_worker<128, 3, true>, 128, sizeof(ColumnShared<128>));
+        else if (b->max_span <= 256) columns(column_worker<256, 2, false>, column_worker<256, 2, true>, 256, sizeof(ColumnShared<256>));
+        else columns(column_worker<512, 1, false>, column_worker<512, 1, true>, 512, sizeof(ColumnShared<512>));
         return;
     }
     const int cls = a.wmax / kThreads;

@@ -11,7 +11,8 @@
 // shared float4 each (shuffles and an edge per warp took ten instructions a step more).  Threads outside
 // the band hold -inf, which makes every absent neighbour drop out of logAdd.  Three anti-diagonals'
 // columns never share a thread: the host takes this path for a batch only if any three consecutive
-// anti-diagonals span at most column_span(NT) columns.  A sweep is a chain of anti-diagonals and its
+// anti-diagonals span at most NT columns.  Past column_span(NT) the thread beside the band's edge may hold
+// its other end: sweeps compiled for that (kFull) leave that neighbour out by its column.  A sweep is a chain of anti-diagonals and its
 // warps issue in order, so every instruction that is not the recursion lengthens the chain: four more
 // warps take them, each with less to do a step than the sweep, since they issue in order too (one warp
 // for all of it made the step 760 cycles; the sweep alone takes under 300).  One works out the
@@ -33,7 +34,7 @@
 namespace sa {
 namespace fp32 {
 
-// NT threads hold bands up to column_span(NT) columns (a neighbour's column included)
+// NT threads hold bands up to column_span(NT) columns (a neighbour's column included), and with kFull NT
 __host__ __device__ constexpr int column_span(int nt) { return nt - 2; }
 
 constexpr int kAhead = 6;                // anti-diagonals between a copy and its use
@@ -341,7 +342,7 @@ __device__ __forceinline__ void part_of(float *part, float m, float x, float y) 
 // On anti-diagonal d a thread folds, side by side: gap-X of d (left column on d-1), gap-Y of d (own
 // column on d-1), the match state of d+1 but for its last term (left column on d-1), and the last
 // term of d's: one logAdd's latency, a barrier and a shared-memory read a step.
-template <int NT, bool kSX, bool kGX>
+template <int NT, bool kSX, bool kGX, bool kFull>
 __device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment &S, ColumnForwardShared<NT> *fs) {
     const Args &A = *c.A;
     const RegionDesc &R = c.R;
@@ -350,6 +351,7 @@ __device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment
     const int32_t dbeg = S.d_begin, s = dbeg - S.warm + (dbeg == 0 ? 1 : 0), steps = S.d_end - s + 1;
     // own column on d-1, and d's match state but for its last term, and that term
     float M1 = kNegInf, X1 = kNegInf, Y1 = kNegInf, most = kNegInf, last = kNegInf;
+    int32_t xf1 = 0;                     // first column of d-1
     if (dbeg == 0) {
         // anti-diagonal 0: startStateProb / raggedStartStateProb (stateMachine.c:1022-1032), column 0
         const float s0 = R.ragged_left ? kNegInf : 0.0f, s1 = R.ragged_left ? 0.0f : kNegInf;
@@ -361,7 +363,12 @@ __device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment
         // a later segment: every band cell of s-2 and s-1 starts at 0
         const int2 r2 = raw_meta(A, R.diag_base, s - 2, R.n), r1 = raw_meta(A, R.diag_base, s - 1, R.n);
         if (((tid - ((s - 1 + r1.x) >> 1)) & (NT - 1)) < (r1.y & kWidthMask)) M1 = X1 = Y1 = 0.0f;
-        const bool left = ((tid - 1 - ((s - 2 + r2.x) >> 1)) & (NT - 1)) < (r2.y & kWidthMask);
+        bool left = ((tid - 1 - ((s - 2 + r2.x) >> 1)) & (NT - 1)) < (r2.y & kWidthMask);
+        if (kFull) {
+            const int32_t xf = (s + raw_meta(A, R.diag_base, s, R.n).x) >> 1;
+            left = left && xf + ((tid - xf) & (NT - 1)) > ((s - 2 + r2.x) >> 1);
+            xf1 = (s - 1 + r1.x) >> 1;
+        }
         const float z = left ? 0.0f : kNegInf;
         most = lac(z + t[T_MC], z + t[T_MFGX]);
         last = z + t[T_MFGY];
@@ -372,6 +379,7 @@ __device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment
     bar_sync(kBarRow, NT + kHelpers);          // the first rows are ready
     RowFacts row = fs->row[0];
     bool inb = ((tid - row.xf) & (NT - 1)) < (row.w & kWidthMask);
+    int32_t x0 = row.xf + ((tid - row.xf) & (NT - 1));   // own column on d
     float2 e = fs->e[0][(tid - row.xf) & (NT - 1)];
     float gx = 0.0f;
     if (kGX) gx = raw_gapx(c, row.xf + ((tid - row.xf) & (NT - 1)));
@@ -383,13 +391,18 @@ __device__ __forceinline__ void column_forward_sweep(const Ctx &c, const Segment
         x[2] = most;
         y[2] = last;
         bar_sync(kBarRow, NT + kHelpers);      // d-1's values; d+1's facts and emissions
-        const float4 l = left[((k + 1) & 1) * NT];
+        float4 l = left[((k + 1) & 1) * NT];
         const RowFacts next = fs->row[(k + 1) & 3];
+        const int32_t i = (tid - next.xf) & (NT - 1);
+        if (kFull) {   // no column before d-1's first (a thread in the band on d and on d+1 has one column)
+            if ((inb ? x0 : next.xf + i) <= xf1) l.x = l.y = l.z = kNegInf;
+            xf1 = row.xf;
+            x0 = next.xf + i;
+        }
         x[0] = l.x + t[T_OX];
         y[0] = l.y + t[T_EX];
         x[3] = l.x + t[T_MC];
         y[3] = l.y + t[T_MFGX];
-        const int32_t i = (tid - next.xf) & (NT - 1);
         const float2 e_next = fs->e[(k + 1) & (kRows - 1)][i];
         lacs<4>(x, y, r);
         if (kSX) r[0] = lac(r[0], l.z + t[T_SX]);
@@ -680,7 +693,7 @@ __device__ __forceinline__ float2 column_folds(float *chain, int na, int nb) {
 // ------------------------------------------------------------------------------------------------
 // backward sweep of one traceback window
 // ------------------------------------------------------------------------------------------------
-template <int NT, bool kSX, bool kGX>
+template <int NT, bool kSX, bool kGX, bool kFull>
 __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &Wn, ColumnWindowShared<NT> *ws) {
     const RegionDesc &R = c.R;
     const float *t = c.t;
@@ -698,6 +711,7 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
     float2 e1r = make_float2(0.0f, 0.0f);
     float gx = 0.0f;
     int32_t i1 = 0, W1 = 0, xf1 = 0;     // its cell, the width and the first column of d+1
+    int32_t hi1 = -1, hi2 = -1;          // last columns of d+1 and d+2
     int32_t left = rows;                 // posterior anti-diagonals to come
     int32_t block = 0, in_block = 0;
     bar_sync(kBarRow, NT + 64);          // the first rows are ready
@@ -710,7 +724,8 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
         const int32_t W = row.y & kWidthMask;
         const bool inb = i < W;
         bar_sync(kBarRow, NT + 64);      // d+1's values, d's shifts; d-1's facts and operands
-        const float4 n = right[((k + 1) & 1) * NT];
+        float4 n = right[((k + 1) & 1) * NT];
+        if (kFull && row.x + i >= max(hi1, hi2)) n.x = n.z = kNegInf;   // no column after their last
         const float2 sh = *reinterpret_cast<const float2 *>(&ws->row[k & 3].sh1);
         const int2 next = *reinterpret_cast<const int2 *>(&ws->row[(k + 1) & 3].xf);
         const float me = n.x + (n.y + sh.y);
@@ -780,6 +795,10 @@ __device__ __forceinline__ void column_window_sweep(const Ctx &c, const Window &
         i1 = i;
         W1 = W;
         xf1 = row.x;
+        if (kFull) {
+            hi2 = hi1;
+            hi1 = row.x + W - 1;
+        }
         row = next;
         i = i_next;
         e = e_next;
@@ -993,26 +1012,26 @@ __device__ __forceinline__ void column_window_post(const Ctx &c, const Window &W
 // ------------------------------------------------------------------------------------------------
 // NT / 32 warps sweep, beside the three others.  The first claims are forward segments (longest
 // first); once none is left, windows.
-template <int NT, bool kSX, bool kGX>
+template <int NT, bool kSX, bool kGX, bool kFull>
 __device__ __forceinline__ void column_forward(const Ctx &c, const Segment &sg, ColumnForwardShared<NT> *fs) {
-    if (threadIdx.x < NT) column_forward_sweep<NT, kSX, kGX>(c, sg, fs);
+    if (threadIdx.x < NT) column_forward_sweep<NT, kSX, kGX, kFull>(c, sg, fs);
     else if (threadIdx.x < NT + 32) column_forward_shifts<NT>(sg, fs);
     else if (threadIdx.x < NT + 64) column_forward_copies<NT>(c, sg, fs);
     else column_forward_results<NT>(c, sg, fs, (threadIdx.x - NT - 64) >> 5);
 }
 
-template <int NT, bool kSX, bool kGX>
+template <int NT, bool kSX, bool kGX, bool kFull>
 __device__ __forceinline__ void column_window(const Ctx &c, ColumnWindowShared<NT> *ws, int64_t id) {
     const Window Wn = c.A->windows[id];
     const WindowTask wt = c.A->wtask[id];
-    if (threadIdx.x < NT) column_window_sweep<NT, kSX, kGX>(c, Wn, ws);
+    if (threadIdx.x < NT) column_window_sweep<NT, kSX, kGX, kFull>(c, Wn, ws);
     else if (threadIdx.x < NT + 32) column_window_shifts<NT>(c, Wn, ws);
     else if (threadIdx.x < NT + 64) column_window_copies<NT>(c, Wn, wt, ws);
     else if (threadIdx.x < NT + 96) column_window_totals<NT>(Wn, ws);
     else column_window_post<NT>(c, Wn, wt, id, ws);
 }
 
-template <int NT, int MINB>
+template <int NT, int MINB, bool kFull>
 __global__ void __launch_bounds__(NT + kHelpers, MINB) column_worker(const __grid_constant__ Args A) {
     ColumnShared<NT> *cs = reinterpret_cast<ColumnShared<NT> *>(column_smem);
     const int tid = threadIdx.x;
@@ -1038,11 +1057,11 @@ __global__ void __launch_bounds__(NT + kHelpers, MINB) column_worker(const __gri
         ctx_init(c, A, sg.region);
         const bool sx = c.t[T_SX] > kNegInf;
         if (c.gx_uniform) {
-            if (sx) column_forward<NT, true, false>(c, sg, &cs->f);
-            else column_forward<NT, false, false>(c, sg, &cs->f);
+            if (sx) column_forward<NT, true, false, kFull>(c, sg, &cs->f);
+            else column_forward<NT, false, false, kFull>(c, sg, &cs->f);
         } else {
-            if (sx) column_forward<NT, true, true>(c, sg, &cs->f);
-            else column_forward<NT, false, true>(c, sg, &cs->f);
+            if (sx) column_forward<NT, true, true, kFull>(c, sg, &cs->f);
+            else column_forward<NT, false, true, kFull>(c, sg, &cs->f);
         }
         __syncthreads();
     }
@@ -1059,11 +1078,11 @@ __global__ void __launch_bounds__(NT + kHelpers, MINB) column_worker(const __gri
         ctx_init(c, A, A.wtask[id].region);
         const bool sx = c.t[T_SX] > kNegInf;
         if (c.gx_uniform) {
-            if (sx) column_window<NT, true, false>(c, &cs->w, id);
-            else column_window<NT, false, false>(c, &cs->w, id);
+            if (sx) column_window<NT, true, false, kFull>(c, &cs->w, id);
+            else column_window<NT, false, false, kFull>(c, &cs->w, id);
         } else {
-            if (sx) column_window<NT, true, true>(c, &cs->w, id);
-            else column_window<NT, false, true>(c, &cs->w, id);
+            if (sx) column_window<NT, true, true, kFull>(c, &cs->w, id);
+            else column_window<NT, false, true, kFull>(c, &cs->w, id);
         }
         // the posteriors' warp wrote the window's pairs and counts
         if (tid >= NT + 96) read_unit_done<32>(A, c.R.read, tid & 31, nullptr);

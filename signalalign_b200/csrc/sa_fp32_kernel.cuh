@@ -3,8 +3,9 @@
 //   1. emission_kernel: the match and extra-event emissions of every band cell, written to the
 //      emission store.  Fully parallel (a warp per run of 32 anti-diagonals); it takes the
 //      Gaussian / HDP density work off the sequential sweeps.
-//   2. column_worker (sa_fp32_columns.cuh; bands up to 510 columns) or worker_kernel (wider
-//      bands): persistent CTAs pull tasks from one device counter.  The first
+//   2. column_worker (sa_fp32_columns.cuh; any three consecutive anti-diagonals within 512 columns) or
+//      worker_kernel (past that, and where the launch configuration asks for it): persistent CTAs pull
+//      tasks from one device counter.  The first
 //      claims are forward segments (longest first); every later claim is a slot of a ready queue of
 //      traceback windows.  A forward segment sweeps a run of a region's anti-diagonals (the whole
 //      region, or a piece of a long one; see Segment) anti-diagonal by anti-diagonal (cells spread

@@ -2,7 +2,8 @@
 first to the last of any three consecutive anti-diagonals; the reads here are chosen by it (anchors
 every 50 positions, one of several seeds, an expansion), and the span is checked.
 
-FP32: the emissions of bands wider than 176 cells are launched with room for L1.  Every case, in a batch with a narrow read and cut
+FP32: 128, 256 or 512 threads hold spans of up to their number; of the last two, whose band's ends lie on
+neighbouring threads, with sweeps of their own.  Every case, in a batch with a narrow read and cut
 into forward segments, against the FP64 oracle (posteriors 1e-4, log-likelihood 1e-3 relative, the FP32
 form's bounds) and against the CTA form, whose values the column-resident form has bit for bit."""
 import numpy as np
@@ -56,7 +57,8 @@ def _width_class(rd, expansion, k=6):
     return 1 if w <= 128 else (2 if w <= 256 else 4)
 
 
-@pytest.mark.parametrize("span", [175, 176, 177, 178, 300, 400])
+@pytest.mark.parametrize("span", [125, 126, 127, 128, 129, 175, 176, 177, 178, 253, 254, 255, 256, 257, 300, 400,
+                                  509, 510, 511, 512])
 def test_fp32(api, span):
     cfg, rd, expansion = read_of_span(span, 3400 if span < 260 else 6400)
     m = W.gaussian_model(cfg)
@@ -89,3 +91,34 @@ def test_fp32(api, span):
         assert abs(columns.log_likelihood(i) - total) <= 1e-3 * abs(total)
         assert np.array_equal(columns.pairs(i), cta.pairs(i))
         assert columns.log_likelihood(i) == cta.log_likelihood(i)
+
+
+@pytest.mark.parametrize("span", [127, 128, 256])
+@pytest.mark.parametrize("finite_sx,skips", [(True, False), (False, True), (True, True)])
+def test_fp32_machines(api, span, finite_sx, skips):
+    """a finite SWITCH_TO_X and skip emissions that differ between k-mers, ends not ragged"""
+    cfg, rd, expansion = read_of_span(span, 1300)
+    m = dict(W.gaussian_model(cfg))
+    m["t"] = np.array(m["t"], dtype=np.float64)
+    if finite_sx:
+        m["t"][7] = m["t"][8] = -3.0
+    if skips:
+        m["gapx"] = np.log(np.random.Generator(np.random.PCG64(5)).uniform(0.02, 0.3, m["n_kmers"]))
+    inp = _input(api, W.gpu_model(api, m, orc.EMIT_DESCALED), rd)
+    inp.ragged_left = inp.ragged_right = False
+    p = api.pairwiseAlignmentBandingParameters_construct(diagonal_expansion=expansion)
+    want = orc.aligned_pairs(W.oracle_model(m, orc.EMIT_DESCALED, rd), rd["reference"], rd["events"], rd["anchors"],
+                             orc.params(threshold=p.threshold, expansion=expansion), False, False)
+    cls = _width_class(rd, expansion)
+    saved = api.get_launch_config(0, cls)
+    try:
+        api.set_launch_config(0, cls, dict(saved, warp_windows=1))
+        columns = api.align_batch([inp], p)
+        api.set_launch_config(0, cls, dict(saved, warp_windows=0))
+        cta = api.align_batch([inp], p)
+    finally:
+        api.set_launch_config(0, cls, saved)
+    assert columns.status(0) == 0 and len(want) > 100
+    assert W.max_posterior_error(want, columns.pairs(0), p.threshold) <= 1e-4
+    assert np.array_equal(columns.pairs(0), cta.pairs(0))
+    assert columns.log_likelihood(0) == cta.log_likelihood(0)
