@@ -280,7 +280,8 @@ sa_status sa_batch_set_wait_limit(sa_batch *b, int64_t cycles);
  * segment_diags: < 0 keeps every region whole; > 0 caps a segment's sweep (warm-up included);
  * 0 (default) picks twice the batch's forward anti-diagonals per worker CTA, at least 2800 (a large
  * batch, bound by its total work, then keeps nearly every region whole; a small one splits; 4096 in
- * sa_align_batch_noalloc, and for regions whose warm-up leaves the cap less than 64).
+ * sa_align_batch_noalloc, and for regions whose warm-up leaves the cap less than 64; the FP64 form
+ * sweeps regions of up to 4096 anti-diagonals whole).
  * warmup_diags: default 1024, at least 64.  Applies to batches created afterwards. */
 sa_status sa_setSegmentPolicy(int32_t segment_diags, int32_t warmup_diags);
 sa_status sa_getSegmentPolicy(int32_t *segment_diags, int32_t *warmup_diags);
