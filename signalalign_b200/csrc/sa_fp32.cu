@@ -721,6 +721,12 @@ sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, 
     return SA_OK;
 }
 
+// width class of the batch's launch configuration: 1, 2 or 4 times kThreads cells
+int batch_width_class(const sa_batch *b) {
+    const int cpt = std::max(1, (b->max_width + kThreads - 1) / kThreads);
+    return cpt <= 1 ? 1 : (cpt <= 2 ? 2 : 4);
+}
+
 // kernel arguments of a batch's run (launch-dependent fields set by the caller)
 Args batch_args(const sa_batch *b) {
     Args a;
@@ -768,8 +774,7 @@ Args batch_args(const sa_batch *b) {
     a.read_wdone = b->d_read_wdone;
     a.done_host = b->d_done;
     a.done_seq = b->run_seq;
-    const int cpt = std::max(1, (b->max_width + kThreads - 1) / kThreads);
-    a.wmax = (cpt <= 1 ? 1 : (cpt <= 2 ? 2 : 4)) * kThreads;
+    a.wmax = batch_width_class(b) * kThreads;
     a.spin_limit = b->wait_limit;
     return a;
 }
@@ -781,30 +786,41 @@ Args batch_args(const sa_batch *b) {
 // at expansion 50 (128 threads) 18.8 / 13.1 ms, 6 reads of 3 to 8 kb at expansion 200 (512 threads) 6.8 / 3.0.
 // The next wider CTA / full columns: 256 reads of 2 to 10 kb with a span of 128 12.1 / 7.5 ms, of 256 28.6 /
 // 12.8, 128 reads with a span of 512 (the CTA form) 23.6 / 16.6.
-void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
-    auto launch = [&](auto kern, int threads, size_t smem) {
-        int per_sm = 0;
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-        per_sm = std::max(1, std::min(per_sm, cfg.ctas_per_sm));
-        const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t) sms * per_sm,
-                                                                    (int64_t) cfg.grid_per_region * a.n_segs));
-        kern<<<(unsigned) grid, (unsigned) threads, smem, s>>>(a);
+struct Worker {
+    void (*kernel)(const Args);
+    int threads;
+    size_t smem;
+};
+
+// columns: as the launch configuration asks
+Worker pick_worker(const sa_batch *b, bool columns) {
+    auto of = [&](auto plain, auto full, int nt, size_t smem) {
+        return Worker{b->max_span <= column_span(nt) ? plain : full, nt + kHelpers, smem};
     };
-    auto columns = [&](auto plain, auto full, int nt, size_t smem) {
-        launch(b->max_span <= column_span(nt) ? plain : full, nt + kHelpers, smem);
-    };
-    if (cfg.warp_windows && b->max_span <= 512) {
-        if (b->max_span <= 128) columns(column_worker<128, 3, false>, column_worker<128, 3, true>, 128, sizeof(ColumnShared<128>));
-        else if (b->max_span <= 256) columns(column_worker<256, 2, false>, column_worker<256, 2, true>, 256, sizeof(ColumnShared<256>));
-        else columns(column_worker<512, 1, false>, column_worker<512, 1, true>, 512, sizeof(ColumnShared<512>));
-        return;
+    if (columns && b->max_span <= 512) {
+        if (b->max_span <= 128) return of(column_worker<128, 3, false>, column_worker<128, 3, true>, 128, sizeof(ColumnShared<128>));
+        if (b->max_span <= 256) return of(column_worker<256, 2, false>, column_worker<256, 2, true>, 256, sizeof(ColumnShared<256>));
+        return of(column_worker<512, 1, false>, column_worker<512, 1, true>, 512, sizeof(ColumnShared<512>));
     }
-    const int cls = a.wmax / kThreads;
-    const size_t smem = sizeof(Shared) + sizeof(float) * (size_t) worker_area_floats(cls);
-    if (cls == 1) launch(worker_kernel<1, 2>, kThreads, smem);
-    else if (cls == 2) launch(worker_kernel<2, 1>, kThreads, smem);
-    else launch(worker_kernel<4, 1>, kThreads, smem);
+    const int cls = batch_width_class(b);
+    return Worker{cls == 1 ? worker_kernel<1, 2> : (cls == 2 ? worker_kernel<2, 1> : worker_kernel<4, 1>), kThreads,
+                  sizeof(Shared) + sizeof(float) * (size_t) worker_area_floats(cls)};
+}
+
+// CTAs of it that an SM holds
+int worker_occupancy(const Worker &w) {
+    int per_sm = 0;
+    if (w.smem > 48 * 1024) cudaFuncSetAttribute(w.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) w.smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, w.kernel, w.threads, w.smem);
+    return std::max(1, per_sm);
+}
+
+void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
+    const Worker w = pick_worker(b, cfg.warp_windows != 0);
+    const int per_sm = std::min(worker_occupancy(w), cfg.ctas_per_sm);
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t) sms * per_sm,
+                                                                (int64_t) cfg.grid_per_region * a.n_segs));
+    w.kernel<<<(unsigned) grid, (unsigned) w.threads, w.smem, s>>>(a);
 }
 
 // Reads whose stitch disagreed run again with every region as one segment (after the batch's
@@ -973,10 +989,8 @@ sa_status sa_batch_run(sa_batch *b, void *stream) {
         st = SA_E_CUDA;
     if (!st && nr > 0) {
         Args a = batch_args(b);
-        const int cpt = std::max(1, (b->max_width + kThreads - 1) / kThreads);
-        const int cpt_pow2 = cpt <= 1 ? 1 : (cpt <= 2 ? 2 : 4);
-        b->width_class = cpt_pow2;
-        const sa_launch_config cfg = b->has_cfg ? b->cfg : launch_for(b->device, cpt_pow2);
+        b->width_class = batch_width_class(b);
+        const sa_launch_config cfg = b->has_cfg ? b->cfg : launch_for(b->device, b->width_class);
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
         sms = std::max(1, sms);
@@ -1291,16 +1305,19 @@ sa_status sa_loadLaunchConfigs(const char *path) {
 sa_status sa_tuneLaunchConfig(sa_batch *b, void *stream, int32_t repeats, sa_launch_config *best, double *best_ms,
                               int32_t *n_tried) {
     if (!b || !best || !best_ms || !n_tried || repeats < 1 || !b->owns_device) return SA_E_ARG;
-    const int cpt = std::max(1, (b->max_width + kThreads - 1) / kThreads);
-    const int wc = cpt <= 1 ? 1 : (cpt <= 2 ? 2 : 4);
+    const int wc = batch_width_class(b);
+    // both forms of the worker, each at up to as many CTAs per SM as it can have
     std::vector<sa_launch_config> cand;
-    for (int cps : {1, 2, 3})
-        for (int gpr : {2, 3, 4, 6})
-            for (int ww : {1, 0})
-                for (int ecs : {8, 16, 32}) {
-                    if (wc != 1 && (ww == 0 || cps >= 2)) continue;   // wider bands: CTA windows, one CTA per SM
-                    cand.push_back(sa_launch_config{cps, gpr, ww, ecs});
-                }
+    for (int ww : {1, 0}) {
+        int prev = 0;
+        cudaGetDevice(&prev);
+        if (cudaSetDevice(b->device) != cudaSuccess) return SA_E_CUDA;
+        const int most = std::min(3, worker_occupancy(pick_worker(b, ww != 0)));
+        cudaSetDevice(prev);
+        for (int cps = 1; cps <= most; ++cps)
+            for (int gpr : {2, 3, 4, 6})
+                for (int ecs : {8, 16, 32}) cand.push_back(sa_launch_config{cps, gpr, ww, ecs});
+    }
     double best_t = 1e300;
     sa_launch_config best_c = default_launch();
     int tried = 0;
