@@ -1487,14 +1487,24 @@ sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p
 
 // Device block, staged inputs and their upload (async on `stream`); models must be resident.
 sa_status plain_upload(PlainSet *s, cudaStream_t stream) {
-    sa_status st = mem_get(MemKind::Device, s->device, s->dev_bytes, s->dev);
+    sa_status st = SA_OK;
+    // a batch uploaded again has its blocks
+    auto have = [&](MemBlock &b, size_t bytes, auto &&get) {
+        if (st || b.bytes >= bytes) return;
+        mem_put(b);
+        st = get(bytes, b);
+    };
+    auto device = [&](size_t bytes, MemBlock &b) { return mem_get(MemKind::Device, s->device, bytes, b); };
+    auto pinned = [&](size_t bytes, MemBlock &b) { return mem_get(MemKind::Pinned, s->device, bytes, b); };
+    have(s->dev, s->dev_bytes, device);
     if (st == SA_E_NOMEM && s->resident && !s->expect) {
         // no room for the store: the rings take a few MB a region
         plan_rings(s);
-        st = mem_get(MemKind::Device, s->device, s->dev_bytes, s->dev);
+        st = SA_OK;
+        have(s->dev, s->dev_bytes, device);
     }
-    if (!st) st = mem_get(MemKind::Pinned, s->device, s->in_bytes, s->host_in);
-    if (!st) st = mem_get(MemKind::Pinned, s->device, s->res_bytes, s->host_res);
+    have(s->host_in, s->in_bytes, pinned);
+    have(s->host_res, s->res_bytes, pinned);
     if (st) return st;
     plain_layout(s, static_cast<unsigned char *>(s->host_in.ptr), static_cast<unsigned char *>(s->dev.ptr));
     if (cudaMemcpyAsync(s->dev.ptr, s->host_in.ptr, s->in_bytes, cudaMemcpyHostToDevice, stream) != cudaSuccess)
