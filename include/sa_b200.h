@@ -157,7 +157,12 @@ sa_status sa_getSplitPoints(const int64_t *anchors, int64_t n_anchors, int64_t l
                             int64_t split_matrix_bigger_than_this, int32_t ragged_left, int32_t ragged_right,
                             int64_t *regions, int64_t max_regions, int64_t *n_regions);
 
-/* ---- plain FP64 form: one read per launch ---- */
+/* ---- plain FP64 form ----
+ * Device memory (this call, the expectations calls and a batch's reads with 'X' positions): about 52 bytes a
+ * path slot of the band (77 in the expectations calls; 0.25 GiB for a 20 kb read at expansion 50) while that
+ * is at most 24 GiB a call and, past 4 GiB, at most half of what is free on the device; else, and where an
+ * allocation fails, a few MB a forward segment and slower sweeps with the same results.  The library keeps
+ * blocks for later calls, at most 16 GiB of these. */
 
 /* getAlignedPairsUsingAnchors(sM, sX, sY, anchorPairs, p, diagonalCalculationPosteriorMatchProbs,
  * raggedLeft, raggedRight) (pairwiseAligner.c:1871-1899), which splits at large anchor gaps

@@ -717,7 +717,7 @@ sa_status compute_kmer_logs(sa_state_machine *sm) {
 namespace {
 
 // resident route: its store of every anti-diagonal, at most (the rings of the other route take a few
-// MB a region whatever its length), and the threads its sweeps may use
+// MB a segment whatever its length; see also mem_get_store), and the threads its sweeps may use
 constexpr size_t kResidentBytes = (size_t) 24 << 30;
 constexpr int kResidentThreads[] = {128, 256, 480};
 // regions up to this many anti-diagonals are swept whole
@@ -1494,7 +1494,9 @@ sa_status plain_upload(PlainSet *s, cudaStream_t stream) {
         mem_put(b);
         st = get(bytes, b);
     };
-    auto device = [&](size_t bytes, MemBlock &b) { return mem_get(MemKind::Device, s->device, bytes, b); };
+    auto device = [&](size_t bytes, MemBlock &b) {
+        return s->resident ? mem_get_store(s->device, bytes, b) : mem_get(MemKind::Device, s->device, bytes, b);
+    };
     auto pinned = [&](size_t bytes, MemBlock &b) { return mem_get(MemKind::Pinned, s->device, bytes, b); };
     have(s->dev, s->dev_bytes, device);
     if (st == SA_E_NOMEM && s->resident && !s->expect) {

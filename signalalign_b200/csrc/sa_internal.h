@@ -151,8 +151,11 @@ struct MemBlock {
     size_t bytes = 0;
     int device = -1;
     MemKind kind = MemKind::Heap;
+    bool store = false;
 };
 sa_status mem_get(MemKind kind, int device, size_t bytes, MemBlock &out);
+// a device block for a store whose size goes with the input: see sa_memory.cpp
+sa_status mem_get_store(int device, size_t bytes, MemBlock &out);
 void mem_put(MemBlock &b);
 
 // forward-segment planning shared by both forms (sa_fp32.cu): the policy (cap, -1 off, 0 automatic;
