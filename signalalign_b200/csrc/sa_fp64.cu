@@ -793,7 +793,6 @@ struct PlainSet {
     int32_t *d_count_rows = nullptr;
     double *d_terms = nullptr;
     size_t res_region_count = 0;
-    std::vector<int64_t> read_chunk;   // expectations: first chunk of each running read, and the end
     MemBlock host_pairs;
     // results: a read's pairs lie in host_pairs (resident route) or in its own vector
     std::vector<std::vector<sa_aligned_pair>> pairs;
@@ -1245,20 +1244,20 @@ void plan_region(const PathTable &pt, int32_t asz, int64_t kpow, PlainRegion &pr
         pr.psuf[q] = pr.pid[q] < 0 ? -1 : (int32_t) (pr.pid[q] % kpow);
     }
     pr.stride = 1;
-    for (int32_t d = 0; d <= n; ++d) {
-        const int64_t x0 = (d + rg.xmy_l[d]) / 2, x1 = (d + rg.xmy_r[d]) / 2;
-        pr.stride = std::max<int32_t>(pr.stride, pr.pfirst[x1 + 1] - pr.pfirst[x0]);
-    }
     pr.max_paths = 1;
     for (int64_t x = 0; x <= rg.lX; ++x) pr.max_paths = std::max(pr.max_paths, pr.pfirst[x + 1] - pr.pfirst[x]);
     // paths of any three consecutive anti-diagonals, first to last
-    int32_t lo3[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, hi3[3] = {-1, -1, -1};
+    int32_t lo1 = INT32_MAX, lo2 = INT32_MAX, hi1 = -1, hi2 = -1;   // of d-1 and d-2
     pr.slots = 0;
     for (int32_t d = 0; d <= n; ++d) {
-        lo3[d % 3] = pr.pfirst[(d + rg.xmy_l[d]) / 2];
-        hi3[d % 3] = pr.pfirst[(d + rg.xmy_r[d]) / 2 + 1] - 1;
-        pr.slots += hi3[d % 3] - lo3[d % 3] + 1;
-        pr.span = std::max(pr.span, std::max({hi3[0], hi3[1], hi3[2]}) - std::min({lo3[0], lo3[1], lo3[2]}) + 1);
+        const int32_t lo = pr.pfirst[(d + rg.xmy_l[d]) / 2], hi = pr.pfirst[(d + rg.xmy_r[d]) / 2 + 1] - 1;
+        pr.slots += hi - lo + 1;
+        pr.stride = std::max(pr.stride, hi - lo + 1);
+        pr.span = std::max(pr.span, std::max(hi, std::max(hi1, hi2)) - std::min(lo, std::min(lo1, lo2)) + 1);
+        lo2 = lo1;
+        lo1 = lo;
+        hi2 = hi1;
+        hi1 = hi;
     }
     int32_t span = 0;
     for (const Window &w : rg.windows) span = std::max(span, w.D - w.T + 1);
@@ -1383,7 +1382,8 @@ void plan_route(PlainSet *s, const sa_read *reads, size_t max_bytes) {
     for (int nt : kResidentThreads)
         if (!s->nt && span <= nt) s->nt = nt;
     if (!s->nt || (s->multi && s->nt > 256)) return;
-    if ((size_t) slots * 48 > std::min(kResidentBytes, max_bytes)) return;   // not worth planning in full
+    // not worth planning in full
+    if ((size_t) slots * (s->expect ? 72 : 48) > std::min(kResidentBytes, max_bytes)) return;
     s->finite_sx = false;
     for (PlainRegion &pr : s->regs) {
         plan_resident(reads[pr.read].sm, pr);
@@ -1458,10 +1458,7 @@ sa_status plain_create(const sa_read *reads, int64_t n_reads, const sa_params &p
             }
             const int64_t n = pr.rg.lX + pr.rg.lY;
             cap += 4 * (n + 1) * std::min<int64_t>(pr.max_paths, 4) + 256;
-            for (int32_t d = 0; d <= n; ++d) {
-                const int64_t x0 = (d + pr.xl[d]) / 2, x1 = (d + pr.xr[d]) / 2;
-                s->cells += pr.pfirst[x1 + 1] - pr.pfirst[x0];
-            }
+            s->cells += pr.slots;
             s->regs.push_back(std::move(pr));
         }
         s->read_count[r] = (int64_t) s->regs.size() - s->read_first[r];
