@@ -337,10 +337,10 @@ int planning_threads() {
 // are cut: a large batch keeps nearly every region whole (no warm-up overhead), a small one (a
 // serving micro-batch) splits its long reads for latency.  kSegMin: shorter pieces shorten the longest
 // chain and add warm-up work, 1,050 anti-diagonals a piece at expansion 50.  Run and download on B200 at
-// 4,096 / 2,900 / 2,600 / 2,300: one 10 kb read 1.23 / 0.94 / 0.93 / 0.93 ms, 20 reads of 8 to 12 kb 3.51 /
-// 3.28 / 3.22 / 3.18, 8 of them 1.86 / 1.83 / 1.81 / 1.97, 12 HDP reads of 5 to 15 kb 3.12 / 2.96 / 2.98 /
-// 2.99, 8 reads at expansion 20 1.76 / 1.66 / 1.67 / 1.69, 10 reads with sites (FP64) 3.90 / 3.44 / 3.30 /
-// 3.34.
+// caps of 4,096 / 2,900 / 2,800 / 2,600 / 2,300: one 10 kb read 1.15 / 0.86 / 0.86 / 0.86 / 0.85 ms, 20 reads of
+// 8 to 12 kb 2.15 / 1.90 / 1.81 / 1.80 / 1.80, 8 of them 1.35 / 1.28 / 1.28 / 1.27 / 1.45, 12 HDP reads of 5 to
+// 15 kb 2.33 / 2.18 / 2.19 / 2.24 / 2.20, 8 reads at expansion 20 1.10 / 0.89 / 0.89 / 0.87 / 0.87 and at 100
+// 2.23 / 1.99 / 1.99 / 1.99 / 1.99, 10 reads with sites (FP64) 2.61 / 2.57 / 2.47 / 2.38 / 2.33.
 // A region whose warm-up leaves a floor of 2,800 no room (bands of 274 cells and more) has the floor of wide
 // bands: without one it would not be cut at all.  Whole / cut at 4,096: 4 reads of 2 to 10 kb at expansion 300
 // 7.85 / 4.18 ms, 4 reads of 5 to 19 kb with sites there (FP64) 1,214 / 232.
@@ -426,8 +426,10 @@ int32_t column_extent(const Region &rg) {
 // over reads), then the packed inputs, written straight into a host staging block (pinned when
 // `pinned`): per region its descriptor, per-anti-diagonal meta and emission chunks, per window its
 // task and output segment, per read its k-mer ids, skip emissions and events; and the LPT order.
+// seg_min: the floor of the automatic segment cap.
 // Returns SA_E_CAPACITY for a band wider than the kernel's widest ring.
-sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, bool pinned, sa_batch *b) {
+sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, bool pinned, int64_t seg_min,
+                     sa_batch *b) {
     b->n_reads = n_reads;
     b->host_pinned = pinned;
     b->threshold = (float) p->threshold;
@@ -526,7 +528,7 @@ sa_status plan_batch(const sa_read *reads, int64_t n_reads, const sa_params *p, 
             }
             if (sms <= 0) sms = 148;
             const int64_t slots = (int64_t) sms * std::max(1, launch_for(std::max(device, 0), wc).ctas_per_sm);
-            target = std::max<int64_t>(pinned ? kSegMin : kSegMinNoAlloc, 2 * fwd_diags / slots);
+            target = std::max<int64_t>(seg_min, 2 * fwd_diags / slots);
         }
         for (int64_t r = 0; r < n_reads; ++r) {
             ReadPlan &rp = plan[r];
@@ -888,7 +890,7 @@ sa_status sa_batch_create(const sa_read *reads, int64_t n_reads, const sa_params
     if (st) return st;
     auto *b = new (std::nothrow) sa_batch();
     if (!b) return SA_E_NOMEM;
-    st = plan_batch(reads, n_reads, p, true, b);
+    st = plan_batch(reads, n_reads, p, true, kSegMin, b);
     if (!st) {
         int prev = 0;
         cudaGetDevice(&prev);
@@ -1368,7 +1370,7 @@ sa_status batch_plan_host(const sa_read *reads, int64_t n_reads, const sa_params
     if (st) return st;
     auto *b = new (std::nothrow) sa_batch();
     if (!b) return SA_E_NOMEM;
-    st = plan_batch(reads, n_reads, p, false, b);
+    st = plan_batch(reads, n_reads, p, false, kSegMinNoAlloc, b);
     if (st) {
         delete b;
         return st;

@@ -614,10 +614,9 @@ __device__ __forceinline__ void column_forward_results(const Ctx &c, const Segme
 // ------------------------------------------------------------------------------------------------
 // the two ordered folds of a refresh
 // ------------------------------------------------------------------------------------------------
-// ordered_fold2 on chain[0..na) and chain[128..128 + nb), with the same result: half the warp folds
-// each, and of the values after the first largest one only those within the 7.5 cut-off of it are
-// folded (the running result is at least the largest value by then, so logAdd returns it unchanged
-// for any other).
+// ordered_fold on chain[0..na) and on chain[32 NC..32 NC + nb), side by side: half the warp folds each, and
+// of the values after the first largest one only those within the 7.5 cut-off of it are folded (the
+// running result is at least the largest value by then, so logAdd returns it unchanged for any other).
 template <int NC>
 __device__ __forceinline__ float2 column_folds(float *chain, int na, int nb) {
     const int lane = threadIdx.x & 31;
@@ -1010,7 +1009,7 @@ __device__ __forceinline__ void column_window_post(const Ctx &c, const Window &W
 // ------------------------------------------------------------------------------------------------
 // the persistent worker of column-resident batches
 // ------------------------------------------------------------------------------------------------
-// NT / 32 warps sweep, beside the three others.  The first claims are forward segments (longest
+// NT / 32 warps sweep, beside four helper warps.  The first claims are forward segments (longest
 // first); once none is left, windows.
 template <int NT, bool kSX, bool kGX, bool kFull>
 __device__ __forceinline__ void column_forward(const Ctx &c, const Segment &sg, ColumnForwardShared<NT> *fs) {

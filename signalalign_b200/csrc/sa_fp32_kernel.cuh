@@ -1576,8 +1576,8 @@ __device__ void read_unit_done(const Args &A, int32_t r, int tid, Shared *sh) {
 
 // CPT: cells per thread (128 threads per region).  The first claims are forward sweeps, one per CTA;
 // once none is left, windows are claimed, one per CTA.  MINB: CTAs per SM the registers are budgeted
-// for.  Serves the batches column_worker cannot take, and launch configurations that ask for the
-// CTA form.
+// for.  Serves batches of which three consecutive anti-diagonals span more than 512 columns (a band of 512
+// cells that moves on all three), and launch configurations that ask for the CTA form.
 template <int CPT, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) worker_kernel(const __grid_constant__ Args A) {
     extern __shared__ float4 smem_raw[];

@@ -4,8 +4,9 @@
 
 Builds the benchmark workload (seeded synthetic reads, reference spans ~U(2 kb, 20 kb), 6-mer ACGT
 Gaussian table, diagonal expansion 50), uploads it once, and times every candidate configuration
-on it through sa_tuneLaunchConfig: worker CTAs per SM (1, 2 or 3), the worker grid's CTAs per region, columns resident on threads or the CTA form, and
-the emission kernel's grid.  The fastest is written to
+on it through sa_tuneLaunchConfig: columns resident on threads or the CTA form, worker CTAs per SM
+(as many as the kernel can have, 3 at most), the worker grid's CTAs per region, and the emission
+kernel's grid.  The fastest is written to
 launch_configs.tsv beside the library (one row per device name and band-width class; rows of other
 devices and classes are kept), which the library reads when it loads.
 """
