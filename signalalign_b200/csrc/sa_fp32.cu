@@ -812,6 +812,15 @@ Worker pick_worker(const sa_batch *b, bool columns) {
                   sizeof(Shared) + sizeof(float) * (size_t) worker_area_floats(cls)};
 }
 
+// A column-resident CTA takes about two microseconds to begin a window, which windows of a few posterior
+// anti-diagonals each do not repay: with 512 threads, one CTA an SM, a batch that fills the GPU with them runs
+// the CTA form.  64 reads of 2 to 10 kb at expansion 200, columns / the CTA form: traced back every 12
+// anti-diagonals, six of them new, 27.7 / 22.8 ms, every 20 (14 new) 18.3 / 17.7, every 30 (24) 14.7 / 16.0;
+// 8 reads every 12 6.5 / 8.7; at expansion 50 (128 threads) every 12 7.9 / 9.4.
+bool short_windows(const sa_batch *b, int sms) {
+    return b->max_span > 256 && b->n_diags < 16 * b->n_windows && b->n_diags > 2000 * (int64_t) sms;
+}
+
 // CTAs of it that an SM holds
 int worker_occupancy(const Worker &w) {
     int per_sm = 0;
@@ -821,7 +830,7 @@ int worker_occupancy(const Worker &w) {
 }
 
 void launch_worker(const sa_batch *b, const Args &a, const sa_launch_config &cfg, int sms, cudaStream_t s) {
-    const Worker w = pick_worker(b, cfg.warp_windows != 0);
+    const Worker w = pick_worker(b, cfg.warp_windows != 0 && !short_windows(b, sms));
     const int per_sm = std::min(worker_occupancy(w), cfg.ctas_per_sm);
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t) sms * per_sm,
                                                                 (int64_t) cfg.grid_per_region * a.n_segs));
