@@ -4,7 +4,7 @@
 //      emission store.  Fully parallel (a warp per run of 32 anti-diagonals); it takes the
 //      Gaussian / HDP density work off the sequential sweeps.
 //   2. column_worker (sa_fp32_columns.cuh; any three consecutive anti-diagonals within 512 columns) or
-//      worker_kernel (past that, and where the launch configuration asks for it): persistent CTAs pull
+//      worker_kernel (past that, for very short windows, and where asked for): persistent CTAs pull
 //      tasks from one device counter.  The first
 //      claims are forward segments (longest first); every later claim is a slot of a ready queue of
 //      traceback windows.  A forward segment sweeps a run of a region's anti-diagonals (the whole
@@ -1577,7 +1577,8 @@ __device__ void read_unit_done(const Args &A, int32_t r, int tid, Shared *sh) {
 // CPT: cells per thread (128 threads per region).  The first claims are forward sweeps, one per CTA;
 // once none is left, windows are claimed, one per CTA.  MINB: CTAs per SM the registers are budgeted
 // for.  Serves batches of which three consecutive anti-diagonals span more than 512 columns (a band of 512
-// cells that moves on all three), and launch configurations that ask for the CTA form.
+// cells that moves on all three), full batches of wide bands with very short windows, and launch
+// configurations that ask for the CTA form.
 template <int CPT, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) worker_kernel(const __grid_constant__ Args A) {
     extern __shared__ float4 smem_raw[];
